@@ -2,6 +2,8 @@
 // argument checking, dispatch to the kernels, thread-local error messages.
 #include <cuda.h>
 
+#include <algorithm>
+#include <cmath>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -80,6 +82,83 @@ int check_plane(const pz_plane& p, const char* what, int idx, bool pairs) {
     return fail(PZ_EINVAL, "%s[%d]: this output is written in pixel pairs; base and pitch must be 2-element aligned",
                 what, idx);
   return PZ_OK;
+}
+
+// The tensor-core operands B [2*nns][KP] of an NNEDI3 model, chunk-major:
+// chunk c of NC neurons (NC = 32, or nns when below) is NC softmax-branch rows
+// followed by NC Elliott-branch rows.  Row = [weights (T taps), sum of the
+// weights, the bias in pieces, 0...]; against A rows [x_hat, mean*invstd, 1, 1,
+// 1, 0...] the MMA yields the whole pre-activation <x,w>*invstd + b.  Softmax
+// rows are scaled by log2(e) so the epilogue takes exp2 directly.  Stored as
+// no-swizzle K-major core matrices (8 rows x 8 halves; K-neighbours 64 halves
+// apart, 8-row groups 8*KP apart).
+//   wts_h  FP16 values (the fast form)
+//   wts_s  two FP16 pieces of each value, [hi][lo]: hi = fp16(v), lo =
+//          fp16(v - hi), v scaled by the power of two that brings the largest
+//          magnitude to 2^13..2^14.  Every value down to 2^-16 of the largest
+//          then keeps 22 bits or more, and a smaller one an absolute error of
+//          2^-39 of the largest.  Not made (the CUDA cores run the model)
+//          when a value is not finite or the power lies outside 2^-8..2^30,
+//          where the blend's products could leave FP32's range.
+int upload_operands(pz_model* m, const std::vector<float>& w, const std::vector<float>& bias) {
+  const int n = m->nns, T = m->win_w * m->win_h, NC = pz::nnedi3_tc_chunk(n);
+  const int KP = (T + 4 + 15) / 16 * 16;  // taps, mean term, three bias pieces, padded to a K step
+  const double kLog2e = 1.4426950408889634;
+  std::vector<double> v((size_t)2 * n * (T + 2));  // [row][weights, sum, bias], row as stored
+  double top = 0.0;
+  bool finite = true;
+  for (int r = 0; r < 2 * n; r++) {
+    const int k = r / (2 * NC) * NC + r % NC, br = r % (2 * NC) / NC;
+    const double scale = br == 0 ? kLog2e : 1.0;
+    double* row = &v[(size_t)r * (T + 2)];
+    double sum = 0.0;
+    for (int t = 0; t < T; t++) {
+      const double x = w[((size_t)k * 2 + br) * T + t];
+      sum += x;
+      row[t] = x * scale;
+    }
+    row[T] = sum * scale;
+    row[T + 1] = bias[2 * k + br] * scale;
+    for (int t = 0; t < T + 2; t++) {
+      finite = finite && std::isfinite(row[t]);
+      top = std::max(top, std::fabs(row[t]));
+    }
+  }
+  const size_t piece = (size_t)2 * n * KP;
+  const int exp2 = top > 0.0 && finite ? 13 - std::ilogb(top) : 0;
+  const bool split = finite && exp2 >= -8 && exp2 <= 30;
+  const __half zero = __float2half_rn(0.0f);
+  std::vector<__half> h(piece, zero), s(2 * piece, zero);
+  auto at = [&](int r, int t) { return (size_t)(r >> 3) * 8 * KP + (t >> 3) * 64 + (r & 7) * 8 + (t & 7); };
+  auto half_of = [](double x) { return __float2half_rn((float)x); };
+  auto val = [](__half x) { return (double)__half2float(x); };
+  for (int r = 0; r < 2 * n; r++) {
+    const double* row = &v[(size_t)r * (T + 2)];
+    for (int t = 0; t <= T; t++) {
+      h[at(r, t)] = half_of(row[t]);
+      if (split) {
+        const double x = std::ldexp(row[t], exp2);
+        const __half hi = half_of(x);
+        s[at(r, t)] = hi;
+        s[piece + at(r, t)] = half_of(x - val(hi));
+      }
+    }
+    double b = row[T + 1], x = split ? std::ldexp(b, exp2) : 0.0;
+    for (int t = T + 1; t <= T + 3; t++) {  // two pieces (fast form), three (split)
+      if (t < T + 3) {
+        h[at(r, t)] = half_of(b);
+        b -= val(h[at(r, t)]);
+      }
+      s[at(r, t)] = half_of(x);
+      x -= val(s[at(r, t)]);
+    }
+  }
+  int rc = upload(&m->d_wts_h, h.data(), piece * 2);
+  if (!rc && split) {
+    m->split_one = (float)std::ldexp(1.0, exp2);
+    rc = upload(&m->d_wts_s, s.data(), 2 * piece * 2);
+  }
+  return rc;
 }
 
 }  // namespace
@@ -181,8 +260,6 @@ int pz_model_create(const pz_model_desc* d, pz_model** out) {
     m->win_h = d->win_h;
     const int T = d->win_w * d->win_h, n = d->nns;
     std::vector<float> w((size_t)n * 2 * T), cs((size_t)n * 2), bias((size_t)n * 2);
-    const int KP = (T + 3 + 15) / 16 * 16;  // taps + (mean term, bias hi, bias lo), padded to a K step
-    std::vector<__half> wh((size_t)n * 2 * KP, __float2half_rn(0.0f));
     for (int k = 0; k < n; k++) {
       double sa = 0, sb = 0;
       for (int t = 0; t < T; t++) {
@@ -197,38 +274,9 @@ int pz_model_create(const pz_model_desc* d, pz_model** out) {
       bias[2 * k] = d->bias_a[k];
       bias[2 * k + 1] = d->bias_b[k];
     }
-    // tensor-core operand B [2*nns][KP] FP16, chunk-major: chunk c of NC
-    // neurons (NC = 32, or nns when below) is NC softmax-branch rows followed by
-    // NC Elliott-branch rows.  Row = [weights (T taps), sum of the weights,
-    // bias hi, bias lo, 0...]; against A rows [x_hat, mean*invstd, 1, 1, 0...]
-    // the MMA yields the whole pre-activation <x,w>*invstd + b.  Softmax rows
-    // are scaled by log2(e) so the epilogue takes exp2 directly.  Stored as
-    // no-swizzle K-major core matrices (8 rows x 8 halves; K-neighbours 64
-    // halves apart, 8-row groups 8*KP apart).
-    const int NC = pz::nnedi3_tc_chunk(n);
-    const double kLog2e = 1.4426950408889634;
-    for (int r = 0; r < 2 * n; r++) {
-      const int chunk = r / (2 * NC), within = r % (2 * NC);
-      const int k = chunk * NC + within % NC, br = within / NC;
-      const double scale = br == 0 ? kLog2e : 1.0;
-      auto put = [&](int t, double v) {
-        wh[(size_t)(r >> 3) * 8 * KP + (t >> 3) * 64 + (r & 7) * 8 + (t & 7)] = __float2half_rn((float)v);
-      };
-      double sum = 0.0;
-      for (int t = 0; t < T; t++) {
-        const double v = w[((size_t)k * 2 + br) * T + t];
-        sum += v;
-        put(t, v * scale);
-      }
-      const double b = (br == 0 ? d->bias_a[k] : d->bias_b[k]) * scale;
-      const float bhi = __half2float(__float2half_rn((float)b));
-      put(T, sum * scale);
-      put(T + 1, bhi);
-      put(T + 2, b - bhi);
-    }
     if ((rc = upload(&m->d_wts, w.data(), w.size() * 4)) || (rc = upload(&m->d_cs, cs.data(), cs.size() * 4)) ||
         (rc = upload(&m->d_bias, bias.data(), bias.size() * 4)) ||
-        (rc = upload(&m->d_wts_h, wh.data(), wh.size() * 2))) {
+        (pz::nnedi3_tc_supported(n, d->win_h) && (rc = upload_operands(m, w, bias)))) {
       pz_model_destroy(m);
       return rc;
     }
@@ -354,6 +402,7 @@ void pz_model_destroy(pz_model* m) {
   cudaFree(m->d_cs);
   cudaFree(m->d_bias);
   cudaFree(m->d_wts_h);
+  cudaFree(m->d_wts_s);
   delete m;
 }
 
@@ -443,15 +492,8 @@ int pz_run(const pz_model* m, const pz_plane* in, int n_in, pz_plane* out, int n
 
   if (m->family == PZ_NNEDI3) {
     const int ax = nn_axes(o);
-    const bool fast = o && o->precision == PZ_PREC_FAST && pz::nnedi3_tc_supported(m->nns, m->win_h);
-    pz::NnArgs a{};
-    a.nns = m->nns;
-    a.win_h = m->win_h;
-    a.wts = m->d_wts;
-    a.cs = m->d_cs;
-    a.bias = m->d_bias;
-    a.wts_h = m->d_wts_h;
-    a.err = err;
+    const int precision = o ? o->precision : PZ_PREC_FP32;
+    pz::NnArgs a = pz::nn_args(m, err);
     void* tmp = nullptr;
     bool own_tmp = false;
     if (ax == 3) {
@@ -472,7 +514,7 @@ int pz_run(const pz_model* m, const pz_plane* in, int n_in, pz_plane* out, int n
       a.out_pitch = dpitch;
       a.W = sw;
       a.H = sh;
-      return fast ? pz::launch_nnedi3_tc(a, xpass, dt, s) : pz::launch_nnedi3_simt(a, xpass, dt, s);
+      return pz::launch_nnedi3(a, precision, xpass, dt, s);
     };
     rc = 0;
     if (ax == 3) {

@@ -47,6 +47,9 @@ struct NnArgs {
   const float* cs;          // [nns][2]: column sums of A and B
   const float* bias;        // [nns][2]
   const __half* wts_h;      // FP16 packed weights for the tensor-core kernel
+  const __half* wts_s;      // the same as two FP16 pieces (hi, lo), scaled, or null
+  float split_one;          // the power of two that wts_s is scaled by
+  float split_unit;         // its inverse
   int* err;                 // device error word
 };
 
@@ -56,6 +59,7 @@ int launch_lattice(const RavuArgs& a, int radius, int chmode, int dtype, cudaStr
 int launch_zoom(const RavuArgs& a, int radius, int chmode, bool ar, int dtype, cudaStream_t s);
 int launch_nnedi3_simt(const NnArgs& a, bool xpass, int dtype, cudaStream_t s);
 int launch_nnedi3_tc(const NnArgs& a, bool xpass, int dtype, cudaStream_t s);
+int launch_nnedi3_split(const NnArgs& a, bool xpass, int dtype, cudaStream_t s);
 bool nnedi3_tc_supported(int nns, int win_h);
 // Neurons per group of the tensor-core weight operand: the host stores B
 // chunk-major, NC softmax rows then NC Elliott rows per group.

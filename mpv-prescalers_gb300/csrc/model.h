@@ -22,6 +22,8 @@ struct pz_model {
   float* d_cs = nullptr;    // [nns][2]
   float* d_bias = nullptr;  // [nns][2]
   __half* d_wts_h = nullptr;
+  __half* d_wts_s = nullptr;  // split operand of the plain FP32 form (null: CUDA cores)
+  float split_one = 1.0f;     // the power of two it is scaled by
   int device = 0;
 };
 
@@ -74,6 +76,38 @@ inline void select_lut(const pz_model* m, int precision, RavuArgs* a) {
 inline int default_tile_rows(const pz_model* m) {
   if (m->family == PZ_RAVU_LITE && (m->radius == 2 || (m->radius == 4 && m->ar != 0.0f))) return 8;
   return 4;
+}
+
+// The neurons of an NNEDI3 model, as the doubling passes take them.
+inline NnArgs nn_args(const pz_model* m, int* err) {
+  NnArgs a{};
+  a.nns = m->nns;
+  a.win_h = m->win_h;
+  a.wts = m->d_wts;
+  a.cs = m->d_cs;
+  a.bias = m->d_bias;
+  a.wts_h = m->d_wts_h;
+  a.wts_s = m->d_wts_s;
+  a.split_one = m->split_one;
+  a.split_unit = 1.0f / m->split_one;
+  a.err = err;
+  return a;
+}
+
+// One doubling pass in the form `precision` asks for.  The fast form runs
+// its neurons on the tensor cores in FP16; every other form keeps FP32 values
+// and runs them there as two FP16 pieces each.  1080p to 2160p, FP32 planes,
+// split against CUDA cores: nns128 8x6 523 against 4919 us, nns16 8x4 189
+// against 491 us; 160x90 nns32 8x4 the same (both are the two launches).  The
+// error against 64 bits is 0.5-0.65x the CUDA cores' for every nns and window
+// (nns128 8x6 at 640x360: 8.6e-8 against 1.46e-7 relative).  Models of other
+// shapes, or with weights that the pieces cannot hold, stay on the CUDA cores.
+inline int launch_nnedi3(const NnArgs& a, int precision, bool xpass, int dtype, cudaStream_t s) {
+  if (nnedi3_tc_supported(a.nns, a.win_h)) {
+    if (precision == PZ_PREC_FAST) return launch_nnedi3_tc(a, xpass, dtype, s);
+    if (a.wts_s) return launch_nnedi3_split(a, xpass, dtype, s);
+  }
+  return launch_nnedi3_simt(a, xpass, dtype, s);
 }
 
 // Scratch of a ravu lattice chain: the int11 plane, FP32 [channels][H][W].

@@ -1,4 +1,6 @@
-// NNEDI3 doubling pass, plain FP32 on the CUDA cores.
+// NNEDI3 doubling pass, plain FP32 on the CUDA cores: neuron counts that the
+// tensor-core kernel is not built for, and weights that its two FP16 pieces
+// cannot hold (see launch_nnedi3, model.h).
 //
 // Reference: nnedi3-nns16-win8x4.hook:15-104 (double_y: 8x4 window,
 // normalisation, nns neuron pairs, softmax-weighted Elliott blend) and its

@@ -101,15 +101,8 @@ extern "C" int pz_nnedi3_run_static(const pz_model* m, const pz_plane* in, pz_pl
   if ((rc = resolve_static(&addr))) return rc;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
 
-  const bool fast = o && o->precision == PZ_PREC_FAST && pz::nnedi3_tc_supported(m->nns, m->win_h);
-  pz::NnArgs a{};
-  a.nns = m->nns;
-  a.win_h = m->win_h;
-  a.wts = m->d_wts;
-  a.cs = m->d_cs;
-  a.bias = m->d_bias;
-  a.wts_h = m->d_wts_h;
-  a.err = addr.err;
+  const int precision = o ? o->precision : PZ_PREC_FP32;
+  pz::NnArgs a = pz::nn_args(m, addr.err);
   auto pass = [&](bool xpass, const void* src, int sw, int sh, int spitch, void* dst, int dpitch) {
     a.in = src;
     a.in_pitch = spitch;
@@ -117,7 +110,7 @@ extern "C" int pz_nnedi3_run_static(const pz_model* m, const pz_plane* in, pz_pl
     a.out_pitch = dpitch;
     a.W = sw;
     a.H = sh;
-    return fast ? pz::launch_nnedi3_tc(a, xpass, dt, s) : pz::launch_nnedi3_simt(a, xpass, dt, s);
+    return pz::launch_nnedi3(a, precision, xpass, dt, s);
   };
   if (ax == 3) {
     rc = pass(false, in->data, W, H, in->pitch, addr.scratch, W);

@@ -4,28 +4,45 @@
 // window, nns neuron pairs, exp-weighted Elliott blend); pass geometry as in
 // the CUDA-core kernel (nnedi3_simt.cu).
 //
-// Per CTA tile of 128 interpolated pixels (4 warps x 32 consecutive pixels):
-//   1. the window tile is staged in shared memory; each thread normalises its
-//      pixel's window, x_hat = (x - mean) * invstd, and writes it as one FP16
-//      row of the A operand [128 x T] (K-major, no-swizzle core matrices:
-//      8 rows x 16 bytes, LBO = 128 B between K-neighbours, SBO = T*16 B
-//      between 8-row groups);
-//   2. one thread issues T/16 tcgen05.mma.kind::f16 instructions (M = 128,
-//      N = 2*nns, or two N = 256 halves for nns256) against the resident
-//      weight operand B [2*nns x T] (rows 0..nns-1: softmax branch, nns..:
-//      Elliott branch), accumulating FP32 in tensor memory, and commits to an
-//      mbarrier;
-//   3. after the (time-bounded) mbarrier wait, warp w reads TMEM lanes
-//      32w..32w+31 -- one lane per pixel -- with tcgen05.ld.32x32b.x32 and
-//      runs the epilogue in FP32: s1 = D + mean*invstd*sum(A_k) + a_k,
-//      e = exp(s1), s2 likewise, wsum += e, vsum += e * s2 / (1 + |s2|).
-// The mean term restores <x, A_k> * invstd exactly (x_hat is centred).
-// The CTA is persistent: weights and TMEM are set up once per CTA.
+// One persistent CTA per SM: NG groups of 4 warps and one MMA-issuing warp
+// per group.  The groups share the weight operand B in shared memory (one
+// bulk copy per CTA); each works on its own M-tiles of 128 interpolated
+// pixels (4 rows x 32 columns, one thread and one TMEM lane per pixel):
+//   1. the window tile is staged in shared memory (its loads are in flight
+//      while the previous tile's neurons run); each thread normalises its
+//      pixel's window, x_hat = (x - mean) * invstd, into one row of A
+//      [128 x KP] FP16 (K-major, no-swizzle core matrices: 8 rows x 16 bytes,
+//      LBO = 128 B between K-neighbours, SBO = KP*16 B between 8-row groups),
+//      followed by mean*invstd and ones, which multiply B's columns of weight
+//      sums and biases;
+//   2. the group's issuing thread runs tcgen05.mma.kind::f16 (M = 128, N = 64,
+//      K = 16) for 32-neuron chunks into two alternating TMEM accumulators and
+//      commits each to an mbarrier;
+//   3. each warp reads its 32 TMEM lanes with tcgen05.ld.32x32b and runs the
+//      blend in FP32: e = exp2(s1) (softmax rows of B are in log2 units),
+//      wsum += e, vsum += e * s2 / (1 + |s2|).
+// Every hand-off is an mbarrier between the warps that need it (A written,
+// chunk accumulated, chunk read); the one barrier among a group's warps is
+// the window tile's, once per tile.  A is free once the last chunk's MMAs are
+// done, so the next tile is normalised before the last chunk is blended: its
+// first MMAs run under that blend.
+//
+// SPLIT (the plain FP32 form): every operand value is two FP16 pieces, hi +
+// lo, which together hold 22-24 bits, and a chunk is three products, A_lo B_hi
+// + A_hi B_lo + A_hi B_hi in FP32, the small ones first.  A power of two (the
+// model's) scales B so that its pieces stay clear of FP16's subnormals.
+//
+// Bound by issue in the blend (about 14 instructions a neuron pair, three of
+// them MUFU) and in the normalisation (about 8 a tap).  1080p to 2160p, nns128
+// 8x6: 384 us fast (438 us as four CTAs an SM, each with its own copy of B and
+// a CTA barrier per chunk), 523 us split (4919 us on the CUDA cores); nns256 8x6
+// at 720p 283 us fast (443 us: two CTAs an SM had room).
 //
 // Every mbarrier wait is bounded (kWaitNs of %globaltimer).  A wait that runs
-// out ends the CTA's loop; before the tensor memory is freed, the issuing
-// thread commits once more and waits (bounded again) until every MMA it has
-// issued has completed, so no MMA can still write the freed columns; the
+// out sets the CTA's abort flag: from then on nobody waits, nothing is stored,
+// and the loops run out through the same barriers; before the tensor memory
+// is freed, each issuing thread commits once more and waits (bounded) until
+// its MMAs have completed, so no MMA can still write the freed columns; the
 // failure is reported as kErrWaitTimeout in the device error word.
 #include "async.cuh"
 #include "kernels.h"
@@ -33,7 +50,7 @@
 namespace pz {
 namespace {
 
-constexpr int kThreads = 128;  // 4 warps, one TMEM lane quarter each
+constexpr int kGroup = 128;  // threads per group: 4 warps, one TMEM lane quarter each
 
 // tcgen05 shared-memory matrix descriptor, no swizzle, K-major.
 __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
@@ -63,31 +80,27 @@ __device__ __forceinline__ void mma_commit(uint32_t mbar) {
                : "memory");
 }
 
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
-  uint32_t r[32];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
-        "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
-        "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(taddr));
-#pragma unroll
-  for (int i = 0; i < 32; i++) v[i] = __uint_as_float(r[i]);
-}
-
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[32]) {
-  uint32_t r[16];
+// 16 columns of this warp's lanes; the values are valid after tmem_wait16.
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
       "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]), "=f"(v[8]),
+        "=f"(v[9]), "=f"(v[10]), "=f"(v[11]), "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15])
       : "r"(taddr));
-#pragma unroll
-  for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
+}
+
+// Wait for this thread's TMEM loads; the operands tie the loaded registers to
+// the wait, so that no use of them can be scheduled before it.
+__device__ __forceinline__ void tmem_wait16(float (&a)[16], float (&b)[16]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+f"(a[0]), "+f"(a[1]), "+f"(a[2]), "+f"(a[3]), "+f"(a[4]), "+f"(a[5]), "+f"(a[6]), "+f"(a[7]),
+                 "+f"(a[8]), "+f"(a[9]), "+f"(a[10]), "+f"(a[11]), "+f"(a[12]), "+f"(a[13]), "+f"(a[14]), "+f"(a[15]),
+                 "+f"(b[0]), "+f"(b[1]), "+f"(b[2]), "+f"(b[3])
+               :
+               : "memory");
+  asm volatile("" : "+f"(b[4]), "+f"(b[5]), "+f"(b[6]), "+f"(b[7]), "+f"(b[8]), "+f"(b[9]), "+f"(b[10]), "+f"(b[11]),
+                    "+f"(b[12]), "+f"(b[13]), "+f"(b[14]), "+f"(b[15]));
 }
 
 __device__ __forceinline__ float exp2f_approx(float x) {
@@ -96,281 +109,369 @@ __device__ __forceinline__ float exp2f_approx(float x) {
   return r;
 }
 
-__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ float rcp_approx(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
+__device__ __forceinline__ void mbar_arrive(uint32_t mbar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(mbar) : "memory");
+}
+
+// Barrier among the 128 threads of group g (named barriers 1..4; 0 is the CTA's).
+__device__ __forceinline__ void group_sync(int g) {
+  asm volatile("bar.sync %0, %1;" ::"r"(g + 1), "n"(kGroup) : "memory");
+}
+
+// Shape of one instantiation.
+template <int WH, int NNS, bool XP, bool SPLIT>
+struct TcShape {
+  static constexpr int NT = 8 * WH;                   // window taps
+  static constexpr int KP = (NT + 4 + 15) / 16 * 16;  // K: taps, mean term, bias pieces, zero pad
+  static constexpr int NC = NNS < 32 ? NNS : 32;      // neurons per chunk
+  static constexpr int NCH = NNS / NC;                // chunks per tile
+  static constexpr int CCOL = 2 * NC;                 // TMEM columns per chunk buffer
+  static constexpr int NP = SPLIT ? 2 : 1;            // FP16 pieces per operand value
+  static constexpr int DY0 = -(WH / 2 - 1);
+  static constexpr int OX0 = XP ? DY0 : -3, OX1 = XP ? WH / 2 : 4;
+  static constexpr int OY0 = XP ? -3 : DY0, OY1 = XP ? 4 : WH / 2;
+  static constexpr int TW = 32 + OX1 - OX0, TH = 4 + OY1 - OY0;
+  static constexpr uint32_t BPIECE = 2 * NNS * KP * 2;  // bytes of one piece of B / of a group's A
+  static constexpr uint32_t APIECE = 128 * KP * 2;
+  static constexpr uint32_t GROUP_BYTES = NP * APIECE + (TW * TH * 4 + 127) / 128 * 128;
+  static constexpr uint32_t kSmemMax = 227 * 1024 - 1024;  // less the static shared memory
+  // groups per CTA: four fill the SM's tensor memory (128 columns each, two
+  // 32-neuron buffers); fewer where the split operands leave less room
+  static constexpr int fit = (int)((kSmemMax - NP * BPIECE) / GROUP_BYTES);
+  static constexpr int NG = fit < 4 ? fit : 4;
+  static constexpr int THREADS = NG * (kGroup + 32);
+  static constexpr uint32_t TCOLS = NG * 2 * CCOL <= 64 ? 64 : (NG * 2 * CCOL <= 128 ? 128 : (NG * 2 * CCOL <= 256 ? 256 : 512));
+  static constexpr uint32_t SMEM = NP * BPIECE + NG * GROUP_BYTES;
+  static_assert(NNS % NC == 0 && NC % 16 == 0, "neuron count must be a multiple of 16");
+  static_assert(NG >= 1 && NG * 2 * CCOL <= 512, "operands must fit shared and tensor memory");
+};
+
 // Neurons are processed in chunks of NC (32, or 16 for nns16): chunk k's
-// accumulator holds NC softmax-branch and NC Elliott-branch columns, and two
-// chunk buffers alternate in tensor memory (4*NC columns per CTA), so up to
-// four CTAs share an SM's 512 columns.  The MMA of chunk k+2 is issued as
-// soon as every warp has read chunk k, and runs under chunk k's epilogue.
+// accumulator holds NC softmax-branch and NC Elliott-branch columns; the MMA
+// of chunk k+2 is issued as soon as every warp of the group has read chunk k.
 // Operand B is stored chunk-major: rows [2*NC*k, 2*NC*k + NC) are the
 // softmax weights of neurons k*NC.., the next NC rows their Elliott weights.
-template <int WH, int NNS, bool XP, typename T>
-__global__ void __launch_bounds__(kThreads) nn_tc_kernel(const __grid_constant__ NnArgs p) {
-  constexpr int NT = 8 * WH;                 // window taps
-  constexpr int KP = (NT + 3 + 15) / 16 * 16;  // K: taps, mean term, bias hi/lo, zero pad
-  constexpr int NC = NNS < 32 ? NNS : 32;    // neurons per chunk
-  constexpr int NCH = NNS / NC;              // chunks per tile
-  constexpr int CCOL = 2 * NC;               // TMEM columns per chunk buffer
-  constexpr int TCOLS = 2 * CCOL;            // two buffers
-  constexpr int DY0 = -(WH / 2 - 1);
-  constexpr int OX0 = XP ? DY0 : -3, OX1 = XP ? WH / 2 : 4;
-  constexpr int OY0 = XP ? -3 : DY0, OY1 = XP ? 4 : WH / 2;
-  constexpr int TW = 32 + OX1 - OX0, TH = 4 + OY1 - OY0;
-  constexpr uint32_t SBO = KP * 16;          // bytes between 8-row groups (A and B)
-  constexpr uint32_t LBO = 128;              // bytes between K-adjacent core matrices
-  static_assert(NNS % NC == 0 && NC % 16 == 0, "neuron count must be a multiple of 16");
+template <int WH, int NNS, bool XP, typename T, bool SPLIT>
+__global__ void __launch_bounds__(TcShape<WH, NNS, XP, SPLIT>::THREADS, 1) nn_tc_kernel(const __grid_constant__ NnArgs p) {
+  using S = TcShape<WH, NNS, XP, SPLIT>;
+  constexpr int NT = S::NT, KP = S::KP, NC = S::NC, NCH = S::NCH, CCOL = S::CCOL, NG = S::NG;
+  constexpr int TW = S::TW, TH = S::TH;
+  constexpr uint32_t SBO = KP * 16;  // bytes between 8-row groups (A and B)
+  constexpr uint32_t LBO = 128;      // bytes between K-adjacent core matrices
 
   extern __shared__ __align__(1024) unsigned char smem[];
-  unsigned char* sB = smem;                                    // [2*NNS x KP] f16
-  unsigned char* sA = sB + 2 * NNS * KP * 2;                   // [128 x KP] f16
-  float* tile = reinterpret_cast<float*>(sA + 128 * KP * 2);   // [TH][TW]
-  __shared__ __align__(8) unsigned long long mbar[3];  // two chunk buffers, drain
+  unsigned char* sB = smem;  // [NP][2*NNS x KP] f16, then per group [NP][128 x KP] f16 and the window tile
+  struct GroupBars {
+    unsigned long long afull, full[2], empty[2], drain;
+  };
+  __shared__ __align__(8) GroupBars bars[NG];
+  __shared__ __align__(8) unsigned long long bbar;
   __shared__ uint32_t tmem_base;
   __shared__ int abort_flag;
+  volatile int* const aborted = &abort_flag;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  {  // one-time setup: the weight operand
-    const uint4* src = reinterpret_cast<const uint4*>(p.wts_h);
-    uint4* dst = reinterpret_cast<uint4*>(sB);
-    for (int i = tid; i < 2 * NNS * KP * 2 / 16; i += kThreads) dst[i] = __ldg(src + i);
+  if (tid == 0) {
+    for (int g = 0; g < NG; g++) {
+      mbar_init(smem_u32(&bars[g].afull), 4);  // one arrival per warp of the group
+      for (int b = 0; b < 2; b++) {
+        mbar_init(smem_u32(&bars[g].full[b]), 1);   // tcgen05.commit
+        mbar_init(smem_u32(&bars[g].empty[b]), 4);  // one arrival per warp
+      }
+      mbar_init(smem_u32(&bars[g].drain), 1);
+    }
+    mbar_init(smem_u32(&bbar), 1);
+    abort_flag = 0;
+    fence_async_smem();
+    // the weight operand, one bulk copy (read by the MMAs only)
+    mbar_arrive_expect_tx(smem_u32(&bbar), S::NP * S::BPIECE);
+    asm volatile(
+        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(sB)),
+        "l"(reinterpret_cast<uint64_t>(SPLIT ? p.wts_s : p.wts_h)), "r"(S::NP * S::BPIECE), "r"(smem_u32(&bbar))
+        : "memory");
   }
   if (warp == 0) {
+    __syncwarp();
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base)),
-                 "r"(TCOLS));
+                 "r"(S::TCOLS));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
-  if (tid == 0) {
-    mbar_init(smem_u32(&mbar[0]), 1);
-    mbar_init(smem_u32(&mbar[1]), 1);
-    mbar_init(smem_u32(&mbar[2]), 1);
-    abort_flag = 0;
-  }
-  fence_async_smem();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = tmem_base;
-  const uint32_t mb0 = smem_u32(&mbar[0]), mb1 = smem_u32(&mbar[1]);
-  const uint32_t a_addr = smem_u32(sA), b_addr = smem_u32(sB);
-  constexpr uint32_t IDESC = instr_desc(128, CCOL);
-  // D[buf] (+)= A x B[chunk]^T over the whole K; completion on mbar[buf]
-  auto issue_chunk = [&](int chunk, int buf) {
-#pragma unroll
-    for (int ks = 0; ks < KP / 16; ks++) {
-      const uint64_t ad = smem_desc(a_addr + ks * 2 * LBO, LBO, SBO);
-      const uint64_t bd = smem_desc(b_addr + (uint32_t)chunk * (CCOL / 8) * SBO + ks * 2 * LBO, LBO, SBO);
-      mma_f16(tmem + buf * CCOL, ad, bd, IDESC, ks > 0 ? 1u : 0u);
-    }
-    mma_commit(buf ? mb1 : mb0);
-  };
-
-  const T* in = static_cast<const T*>(p.in);
-  T* out = static_cast<T*>(p.out);
   const int tiles_x = (p.W + 31) / 32, tiles_y = (p.H + 3) / 4;
   const int ntiles = tiles_x * tiles_y;
-  uint32_t phase = 0;  // bit b: parity of mbar[b]'s next phase
+  const int stride = NG * gridDim.x;  // tiles go over the SMs first, then over each SM's groups
 
-  // the window tile of the next tile is loaded into registers while the
-  // current tile's neurons run (at most PF values per thread)
-  constexpr int PF = (TW * TH + kThreads - 1) / kThreads;
-  float pre[PF];
-  auto prefetch = [&](int tid_) {
-    if (tid_ >= ntiles) return;
-    const int px0 = (tid_ % tiles_x) * 32, py0 = (tid_ / tiles_x) * 4;
-#pragma unroll
-    for (int r = 0; r < PF; r++) {
-      const int i = tid + r * kThreads;
-      if (i < TW * TH) {
-        const int ty = i / TW, tx = i % TW;
-        const int gx = clampi(px0 + OX0 + tx, 0, p.W - 1), gy = clampi(py0 + OY0 + ty, 0, p.H - 1);
-        pre[r] = ldp(in + (size_t)gy * p.in_pitch + gx);
-      }
+  // true once the phase has completed; false when the CTA has given up
+  auto wait = [&](const unsigned long long* bar, uint32_t parity) {
+    const uint32_t mb = smem_u32(bar);
+    if (mbar_try(mb, parity)) return true;
+    const unsigned long long t0 = globaltimer();
+    while (!*aborted) {
+      if (mbar_try(mb, parity)) return true;
+      if (globaltimer() - t0 > kWaitNs) *aborted = 1;
     }
+    return false;
   };
-  prefetch(blockIdx.x);
-  for (int tile_id = blockIdx.x; tile_id < ntiles; tile_id += gridDim.x) {
-    const int x0 = (tile_id % tiles_x) * 32, y0 = (tile_id / tiles_x) * 4;
+
+  if (warp >= 4 * NG) {
+    // ---- the MMA-issuing warp of group g (one thread)
+    const int g = warp - 4 * NG;
+    if (lane == 0) {
+      GroupBars& B = bars[g];
+      constexpr uint32_t IDESC = instr_desc(128, CCOL);
+      const uint32_t a_addr = smem_u32(sB + S::NP * S::BPIECE + g * S::GROUP_BYTES), b_addr = smem_u32(sB);
+      const uint32_t dcol = tmem + g * 2 * CCOL;
+      bool ok = wait(&bbar, 0u);
+      int c = 0, it = 0;  // chunks and tiles issued so far
+      for (int t = g * gridDim.x + blockIdx.x; ok && t < ntiles; t += stride, it++) {
+        if (!(ok = wait(&B.afull, it & 1))) break;
+        for (int k = 0; k < NCH; k++, c++) {
+          const int b = c & 1, u = c >> 1;
+          if (u > 0 && !(ok = wait(&B.empty[b], (u - 1) & 1))) break;
+          tc_fence_after();
+          // D[b] = A x B[chunk]^T over the whole K; completion on full[b]
+          uint32_t acc = 0;
 #pragma unroll
-    for (int r = 0; r < PF; r++) {
-      const int i = tid + r * kThreads;
-      if (i < TW * TH) tile[i] = pre[r];
+          for (int pr = 0; pr < (SPLIT ? 3 : 1); pr++) {
+            const uint32_t ap = a_addr + (SPLIT && pr == 0 ? S::APIECE : 0);
+            const uint32_t bp = b_addr + (SPLIT && pr == 1 ? S::BPIECE : 0) + (uint32_t)k * (CCOL / 8) * SBO;
+#pragma unroll
+            for (int ks = 0; ks < KP / 16; ks++) {
+              mma_f16(dcol + b * CCOL, smem_desc(ap + ks * 2 * LBO, LBO, SBO), smem_desc(bp + ks * 2 * LBO, LBO, SBO),
+                      IDESC, acc);
+              acc = 1;
+            }
+          }
+          mma_commit(smem_u32(&B.full[b]));
+        }
+      }
+      // no MMA may still write tensor memory when it is freed, nor B still land
+      mma_commit(smem_u32(&B.drain));
+      if (!mbar_wait_bounded(smem_u32(&B.drain), 0u)) *aborted = 1;
+      if (g == 0 && !mbar_wait_bounded(smem_u32(&bbar), 0u)) *aborted = 1;
     }
-    __syncthreads();
-    // ---- normalise this thread's window into its A row (pixel m = tid)
-    // The sums run as 8 independent partial sums (one per window column):
-    // the window's loads and adds form no serial chain of NT steps.
-    const int m = tid, px = lane, py = warp;
-    float xv[NT];
+    __syncwarp();
+  } else {
+    // ---- a group's warps: windows into A, accumulators into pixels
+    const int g = warp >> 2, m = tid & (kGroup - 1), py = warp & 3;
+    GroupBars& B = bars[g];
+    unsigned char* sA = sB + S::NP * S::BPIECE + g * S::GROUP_BYTES;
+    float* tile = reinterpret_cast<float*>(sA + S::NP * S::APIECE);
+    const T* in = static_cast<const T*>(p.in);
+    T* out = static_cast<T*>(p.out);
+
+    // the window tile of a later tile, loaded into registers ahead of use
+    constexpr int PF = (TW * TH + kGroup - 1) / kGroup;
+    float pre[PF];
+    auto prefetch = [&](int t) {
+      if (t >= ntiles) return;
+      const int px0 = (t % tiles_x) * 32, py0 = (t / tiles_x) * 4;
 #pragma unroll
-    for (int t = 0; t < NT; t++) {
-      const int dx = t % 8 - 3, dy = t / 8 + DY0;
-      const int ox = XP ? dy : dx, oy = XP ? dx : dy;
-      xv[t] = tile[(py + oy - OY0) * TW + px + ox - OX0];
-    }
-    float ps[8];
+      for (int r = 0; r < PF; r++) {
+        const int i = m + r * kGroup;
+        if (i < TW * TH) {
+          const int ty = i / TW, tx = i % TW;
+          const int gx = clampi(px0 + S::OX0 + tx, 0, p.W - 1), gy = clampi(py0 + S::OY0 + ty, 0, p.H - 1);
+          pre[r] = ldp(in + (size_t)gy * p.in_pitch + gx);
+        }
+      }
+    };
+    // a tile's pixel: window mean and standard deviation, the pixel copied through
+    struct Pixel {
+      float mean, stdv, orig;
+    };
+    // stage the prefetched window tile and write this thread's row of A.  All
+    // warps of the group have read the tile before (their arrivals on afull
+    // precede the MMAs whose completion brought this warp here).
+    auto normalise = [&]() {
 #pragma unroll
-    for (int c = 0; c < 8; c++) ps[c] = xv[c];
+      for (int r = 0; r < PF; r++) {
+        const int i = m + r * kGroup;
+        if (i < TW * TH) tile[i] = pre[r];
+      }
+      group_sync(g);
+      // 8 independent partial sums (one per window column): no serial chain of
+      // NT steps
+      Pixel px;
+      float xv[NT];
 #pragma unroll
-    for (int t = 8; t < NT; t++) ps[t % 8] += xv[t];
-    const float mean = (((ps[0] + ps[1]) + (ps[2] + ps[3])) + ((ps[4] + ps[5]) + (ps[6] + ps[7]))) * (1.0f / NT);
+      for (int t = 0; t < NT; t++) {
+        const int dx = t % 8 - 3, dy = t / 8 + S::DY0;
+        const int ox = XP ? dy : dx, oy = XP ? dx : dy;
+        xv[t] = tile[(py + oy - S::OY0) * TW + lane + ox - S::OX0];
+      }
+      px.orig = tile[(py - S::OY0) * TW + lane - S::OX0];
+      float ps[8];
 #pragma unroll
-    for (int c = 0; c < 8; c++) {
-      const float d = xv[c] - mean;
-      ps[c] = d * d;
-    }
+      for (int c = 0; c < 8; c++) ps[c] = xv[c];
 #pragma unroll
-    for (int t = 8; t < NT; t++) {
-      const float d = xv[t] - mean;
-      ps[t % 8] = fmaf(d, d, ps[t % 8]);
-    }
-    const float var = (((ps[0] + ps[1]) + (ps[2] + ps[3])) + ((ps[4] + ps[5]) + (ps[6] + ps[7]))) * (1.0f / NT);
-    const float invstd = var >= kFltEps ? rsqrtf(var) : 0.0f;
-    const float stdv = var * invstd;
-    const float orig = tile[(py - OY0) * TW + px - OX0];
-    {  // A row: [x_hat (NT), mean * invstd, 1, 1, 0...], x_hat = x * invstd - mean * invstd
+      for (int t = 8; t < NT; t++) ps[t % 8] += xv[t];
+      px.mean = (((ps[0] + ps[1]) + (ps[2] + ps[3])) + ((ps[4] + ps[5]) + (ps[6] + ps[7]))) * (1.0f / NT);
+#pragma unroll
+      for (int t = 0; t < NT; t++) xv[t] -= px.mean;
+#pragma unroll
+      for (int c = 0; c < 8; c++) ps[c] = xv[c] * xv[c];
+#pragma unroll
+      for (int t = 8; t < NT; t++) ps[t % 8] = fmaf(xv[t], xv[t], ps[t % 8]);
+      const float var = (((ps[0] + ps[1]) + (ps[2] + ps[3])) + ((ps[4] + ps[5]) + (ps[6] + ps[7]))) * (1.0f / NT);
+      const float invstd = var >= kFltEps ? (SPLIT ? 1.0f / sqrtf(var) : rsqrtf(var)) : 0.0f;
+      px.stdv = var * invstd;
+      // A row: [x_hat (NT), mean * invstd, 1, 1, 1, 0...].  A mean term beyond
+      // FP16's range is cut: the output is then clamped whatever the neurons
+      // say (|mean| > 22 against a deviation below mean / 60000)
+      const float mterm = fminf(fmaxf(px.mean * invstd, -60000.0f), 60000.0f);
       unsigned char* row = sA + (m >> 3) * SBO + (m & 7) * 16;
-      const float mterm = mean * invstd;
 #pragma unroll
       for (int kc = 0; kc < KP / 8; kc++) {
-        __half2 h[4];
+        __half2 h[4], l[4];
 #pragma unroll
         for (int j = 0; j < 4; j++) {
-          const int t = 8 * kc + 2 * j;
-          const float v0 = t < NT ? fmaf(xv[t], invstd, -mterm) : (t == NT ? mterm : (t <= NT + 2 ? 1.0f : 0.0f));
-          const float v1 = t + 1 < NT ? fmaf(xv[t + 1], invstd, -mterm)
-                                      : (t + 1 == NT ? mterm : (t + 1 <= NT + 2 ? 1.0f : 0.0f));
-          h[j] = __floats2half2_rn(v0, v1);
+          float v[2];
+#pragma unroll
+          for (int q = 0; q < 2; q++) {
+            const int t = 8 * kc + 2 * j + q;
+            v[q] = t < NT ? xv[t < NT ? t : 0] * invstd : (t == NT ? mterm : (t <= NT + 3 ? 1.0f : 0.0f));
+          }
+          h[j] = __floats2half2_rn(v[0], v[1]);
+          if (SPLIT) {
+            const float2 f = __half22float2(h[j]);
+            l[j] = __floats2half2_rn(v[0] - f.x, v[1] - f.y);
+          }
         }
         *reinterpret_cast<uint4*>(row + kc * LBO) = *reinterpret_cast<uint4*>(h);
+        if (SPLIT) *reinterpret_cast<uint4*>(row + S::APIECE + kc * LBO) = *reinterpret_cast<uint4*>(l);
       }
-    }
-    fence_async_smem();
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    if (tid == 0) {
-      issue_chunk(0, 0);
-      if (NCH > 1) issue_chunk(1, 1);
-    }
-    prefetch(tile_id + gridDim.x);  // in flight during the epilogue
-    // ---- epilogue: lane m of TMEM holds pixel m's pre-activations
-    // (softmax branch already in log2 units, Elliott branch as is)
-    float wsum = 0.0f, vsum = 0.0f;
-    const uint32_t lane_addr = tmem + ((uint32_t)(warp * 32) << 16);
-#pragma unroll 1
-    for (int k = 0; k < NCH; k++) {
-      const int b = k & 1;
-      if (!mbar_wait_bounded(b ? mb1 : mb0, (phase >> b) & 1u)) atomicExch(&abort_flag, 1);
-      phase ^= 1u << b;
-      tc_fence_after();
-      float s1[32], s2[32];
-      if (NC == 32) {
-        tmem_ld32(lane_addr + b * CCOL, s1);
-        tmem_ld32(lane_addr + b * CCOL + NC, s2);
-      } else {
-        tmem_ld16(lane_addr + b * CCOL, s1);
-        tmem_ld16(lane_addr + b * CCOL + NC, s2);
-      }
-      tmem_wait_ld();
+      fence_async_smem();
       tc_fence_before();
-      __syncthreads();  // every warp has read buffer b
-      if (abort_flag) break;
-      if (tid == 0 && k + 2 < NCH) {
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&B.afull));
+      return px;
+    };
+
+    int t = g * gridDim.x + blockIdx.x;
+    Pixel cur{}, nxt{};
+    if (t < ntiles) {
+      prefetch(t);
+      cur = normalise();
+      prefetch(t + stride);
+    }
+    const uint32_t lane_addr = tmem + g * 2 * CCOL + ((uint32_t)(py * 32) << 16);
+    const float one = SPLIT ? p.split_one : 1.0f, unit = SPLIT ? p.split_unit : 1.0f;
+    int c = 0;
+    for (; t < ntiles; t += stride) {
+      float2 wsum = make_float2(0.0f, 0.0f);
+      float vsum = 0.0f;
+#pragma unroll 1
+      for (int k = 0; k < NCH; k++, c++) {
+        const int b = c & 1;
+        (void)wait(&B.full[b], (c >> 1) & 1);
         tc_fence_after();
-        issue_chunk(k + 2, b);
-      }
+        if (k == NCH - 1 && t + stride < ntiles) {
+          nxt = normalise();
+          prefetch(t + 2 * stride);
+        }
+        // the accumulators in steps of 16 neurons: both branches' columns
+        // (the next step's loads are in flight during this step's arithmetic)
+        float s1[2][16], s2[2][16];
+        const uint32_t col = lane_addr + b * CCOL;
+        tmem_ld16(col, s1[0]);
+        tmem_ld16(col + NC, s2[0]);
 #pragma unroll
-      for (int j = 0; j < NC; j += 2) {
-        const float b0 = s2[j], b1 = s2[j + 1];
-        const float e0 = exp2f_approx(s1[j]), e1 = exp2f_approx(s1[j + 1]);
-        // b/(1+|b|) for two neurons from one reciprocal of the product
-        const float d0 = 1.0f + fabsf(b0), d1 = 1.0f + fabsf(b1);
-        const float r = __fdividef(1.0f, d0 * d1);
-        wsum += e0 + e1;
-        vsum += (e0 * b0 * d1 + e1 * b1 * d0) * r;
+        for (int q = 0; q < NC / 16; q++) {
+          tmem_wait16(s1[q & 1], s2[q & 1]);
+          if (q + 1 < NC / 16) {
+            tmem_ld16(col + 16 * (q + 1), s1[(q + 1) & 1]);
+            tmem_ld16(col + NC + 16 * (q + 1), s2[(q + 1) & 1]);
+          } else {  // this warp has read buffer b
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&B.empty[b]));
+          }
+          const float(&a)[16] = s1[q & 1];
+          const float(&d)[16] = s2[q & 1];
+#pragma unroll
+          for (int j = 0; j < 16; j += 2) {
+            float2 l = make_float2(a[j], a[j + 1]);
+            if (SPLIT) l = __fmul2_rn(l, make_float2(unit, unit));
+            const float2 e = make_float2(exp2f_approx(l.x), exp2f_approx(l.y));
+            // s / (1 + |s|) for two neurons from one reciprocal of the product
+            const float d0 = one + fabsf(d[j]), d1 = one + fabsf(d[j + 1]);
+            const float2 n = __fmul2_rn(e, make_float2(d[j], d[j + 1]));
+            wsum = __fadd2_rn(wsum, e);
+            vsum = fmaf(fmaf(n.x, d1, n.y * d0), rcp_approx(d0 * d1), vsum);
+          }
+        }
       }
-    }
-    if (abort_flag) break;
-    const int gx = x0 + px, gy = y0 + py;
-    if (gx < p.W && gy < p.H) {
-      const float v = clampf(mean + 5.0f * vsum / wsum * stdv, 0.0f, 1.0f);
-      if (XP) {
-        stp2(out + (size_t)gy * p.out_pitch + 2 * gx, orig, v);
-      } else {
-        stp(out + (size_t)(2 * gy) * p.out_pitch + gx, orig);
-        stp(out + (size_t)(2 * gy + 1) * p.out_pitch + gx, v);
+      const int gx = (t % tiles_x) * 32 + lane, gy = (t / tiles_x) * 4 + py;
+      if (gx < p.W && gy < p.H && !*aborted) {
+        const float v = clampf(cur.mean + 5.0f * vsum / (wsum.x + wsum.y) * cur.stdv, 0.0f, 1.0f);
+        if (XP) {
+          stp2(out + (size_t)gy * p.out_pitch + 2 * gx, cur.orig, v);
+        } else {
+          stp(out + (size_t)(2 * gy) * p.out_pitch + gx, cur.orig);
+          stp(out + (size_t)(2 * gy + 1) * p.out_pitch + gx, v);
+        }
       }
+      cur = nxt;
     }
-    __syncthreads();  // A tile and tile free for the next tile
   }
-  if (tid == 0) {  // no MMA may still write tensor memory when it is freed
-    mma_commit(smem_u32(&mbar[2]));
-    if (!mbar_wait_bounded(smem_u32(&mbar[2]), 0u)) abort_flag = 1;
-  }
-  __syncthreads();
-  if (abort_flag && tid == 0) atomicCAS(p.err, 0, kErrWaitTimeout);
   tc_fence_before();
   __syncthreads();
+  if (*aborted && tid == 0) atomicCAS(p.err, 0, kErrWaitTimeout);
   if (warp == 0) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TCOLS));
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(S::TCOLS));
   }
 }
 
-template <int WH, int NNS, bool XP, typename T>
+template <int WH, int NNS, bool XP, typename T, bool SPLIT>
 int launch_one(const NnArgs& a, cudaStream_t s) {
-  constexpr int NT = 8 * WH;
-  constexpr int DY0 = -(WH / 2 - 1);
-  constexpr int TW = 32 + (XP ? WH / 2 - DY0 : 7), TH = 4 + (XP ? 7 : WH / 2 - DY0);
-  // CTAs per SM are capped by tensor memory (512 columns per SM, 4*NC per
-  // CTA): the shared-memory request is raised so that no more CTAs than fit
-  // in TMEM can be resident, so tcgen05.alloc never waits on a neighbour.
-  constexpr int NC = NNS < 32 ? NNS : 32;
-  constexpr int per_sm = 512 / (4 * NC) > 4 ? 4 : 512 / (4 * NC);
-  int dev = 0, sms = 0, sm_smem = 0, blk_smem = 0;
+  using S = TcShape<WH, NNS, XP, SPLIT>;
+  int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64) return -95;
-  cudaDeviceGetAttribute(&sm_smem, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
-  cudaDeviceGetAttribute(&blk_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-  constexpr int KP = (NT + 3 + 15) / 16 * 16;
-  const size_t need = (size_t)2 * NNS * KP * 2 + 128 * KP * 2 + TW * TH * 4;
-  const size_t cap = (size_t)sm_smem / (per_sm + 1) + 1024;
-  const size_t smem = need > cap ? need : cap;
-  if (smem > (size_t)blk_smem) return -95;
-  auto kern = nn_tc_kernel<WH, NNS, XP, T>;
+  auto kern = nn_tc_kernel<WH, NNS, XP, T, SPLIT>;
   static bool configured[64] = {};  // per instantiation and device
   if (!configured[dev]) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM) != cudaSuccess)
       return -5;
     configured[dev] = true;
   }
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int ntiles = ((a.W + 31) / 32) * ((a.H + 3) / 4);
-  const int grid = ntiles < sms * per_sm ? ntiles : sms * per_sm;
-  kern<<<grid, kThreads, smem, s>>>(a);
+  kern<<<ntiles < sms ? ntiles : sms, S::THREADS, S::SMEM, s>>>(a);
   return 0;
 }
 
-template <int WH, bool XP, typename T>
+template <int WH, bool XP, typename T, bool SPLIT>
 int dispatch_nns(const NnArgs& a, cudaStream_t s) {
   switch (a.nns) {
-    case 16: return launch_one<WH, 16, XP, T>(a, s);
-    case 32: return launch_one<WH, 32, XP, T>(a, s);
-    case 64: return launch_one<WH, 64, XP, T>(a, s);
-    case 128: return launch_one<WH, 128, XP, T>(a, s);
-    case 256: return launch_one<WH, 256, XP, T>(a, s);
+    case 16: return launch_one<WH, 16, XP, T, SPLIT>(a, s);
+    case 32: return launch_one<WH, 32, XP, T, SPLIT>(a, s);
+    case 64: return launch_one<WH, 64, XP, T, SPLIT>(a, s);
+    case 128: return launch_one<WH, 128, XP, T, SPLIT>(a, s);
+    case 256: return launch_one<WH, 256, XP, T, SPLIT>(a, s);
   }
   return -95;
 }
 
-template <typename T>
+template <typename T, bool SPLIT>
 int launch_t(const NnArgs& a, bool xp, cudaStream_t s) {
-  if (a.win_h == 4) return xp ? dispatch_nns<4, true, T>(a, s) : dispatch_nns<4, false, T>(a, s);
-  if (a.win_h == 6) return xp ? dispatch_nns<6, true, T>(a, s) : dispatch_nns<6, false, T>(a, s);
+  if (a.win_h == 4) return xp ? dispatch_nns<4, true, T, SPLIT>(a, s) : dispatch_nns<4, false, T, SPLIT>(a, s);
+  if (a.win_h == 6) return xp ? dispatch_nns<6, true, T, SPLIT>(a, s) : dispatch_nns<6, false, T, SPLIT>(a, s);
   return -95;
 }
 
@@ -384,7 +485,12 @@ int nnedi3_tc_chunk(int nns) { return nns < 32 ? nns : 32; }
 
 int launch_nnedi3_tc(const NnArgs& a, bool xpass, int dtype, cudaStream_t s) {
   if (!a.wts_h || !a.err) return -22;
-  return dtype == 0 ? launch_t<float>(a, xpass, s) : launch_t<__half>(a, xpass, s);
+  return dtype == 0 ? launch_t<float, false>(a, xpass, s) : launch_t<__half, false>(a, xpass, s);
+}
+
+int launch_nnedi3_split(const NnArgs& a, bool xpass, int dtype, cudaStream_t s) {
+  if (!a.wts_s || !a.err) return -22;
+  return dtype == 0 ? launch_t<float, true>(a, xpass, s) : launch_t<__half, true>(a, xpass, s);
 }
 
 }  // namespace pz

@@ -245,6 +245,24 @@ def test_nnedi3_fp32(name, axes):
     _check_nnedi3_fp32(hm, x, axes)
 
 
+@pytest.mark.parametrize("name,H,W", [("nnedi3-nns32-win8x6", 1, 1), ("nnedi3-nns128-win8x4", 4, 32),
+                                      ("nnedi3-nns64-win8x6", 5, 33), ("nnedi3-nns16-win8x4", 260, 641),
+                                      ("nnedi3-nns256-win8x6", 133, 330)])
+def test_nnedi3_tensor_core_tiles(name, H, W):
+    """Tile edges of the tensor-core passes (tiles of 32 x 4 pixels): less
+    than a tile, exactly one, one more row and column; and frames of several
+    tiles per group of every CTA (four groups on 152 SMs; two where the split
+    operands of nns256 8x6 leave no room for more), whose accumulators and
+    barriers are used over and over.  Plain FP32 against the oracle's 1e-5,
+    the fast form against its 2e-3."""
+    hm = _model(name)
+    x = synth.luma_plane(H, W, 77)
+    _check_nnedi3_fp32(hm, x, "yx")
+    y = hm.upscale(torch.from_numpy(x).cuda(), precision="fast").cpu().numpy().astype(np.float64)
+    ref, _ = oracle.nnedi3_upscale(hm.model, x)
+    assert np.abs(y - ref[0]).max() <= 2e-3
+
+
 def test_nnedi3_fp32_on_the_variance_gate():
     """Windows with variance near FLT_EPS: a plane of 0.5 with +-d
     perturbations on a few pixels so that var ~ eps; the bound per gate
