@@ -32,11 +32,13 @@
 // + A_hi B_lo + A_hi B_hi in FP32, the small ones first.  A power of two (the
 // model's) scales B so that its pieces stay clear of FP16's subnormals.
 //
-// Bound by issue in the blend (about 14 instructions a neuron pair, three of
-// them MUFU) and in the normalisation (about 8 a tap).  1080p to 2160p, nns128
-// 8x6: 384 us fast (438 us as four CTAs an SM, each with its own copy of B and
-// a CTA barrier per chunk), 523 us split (4919 us on the CUDA cores); nns256 8x6
-// at 720p 283 us fast (443 us: two CTAs an SM had room).
+// Bound by issue and latency in the blend (12 packed or scalar instructions
+// and 6 MUFU for four neurons) at four warps a scheduler (60 % issue, 37 % MUFU,
+// 23 % tensor pipe; 96 registers and 512 TMEM columns allow no fifth group).
+// 1080p to 2160p, nns128 8x6: 365 us fast (384 us with scalar sums over neuron
+// pairs; 438 us as four CTAs an SM, each with its own copy of B and a CTA barrier
+// per chunk), 485 us split (523 us; 4919 us on the CUDA cores); nns256 8x6 at
+// 720p 279 us fast (443 us: two CTAs an SM had room).
 //
 // Every mbarrier wait is bounded (kWaitNs of %globaltimer).  A wait that runs
 // out sets the CTA's abort flag: from then on nobody waits, nothing is stored,
@@ -303,30 +305,36 @@ __global__ void __launch_bounds__(TcShape<WH, NNS, XP, SPLIT>::THREADS, 1) nn_tc
         if (i < TW * TH) tile[i] = pre[r];
       }
       group_sync(g);
-      // 8 independent partial sums (one per window column): no serial chain of
-      // NT steps
+      // taps in FP32x2 pairs; 8 independent partial sums (one per window
+      // column): no serial chain of NT steps
       Pixel px;
-      float xv[NT];
+      float2 xv[NT / 2];
 #pragma unroll
       for (int t = 0; t < NT; t++) {
         const int dx = t % 8 - 3, dy = t / 8 + S::DY0;
         const int ox = XP ? dy : dx, oy = XP ? dx : dy;
-        xv[t] = tile[(py + oy - S::OY0) * TW + lane + ox - S::OX0];
+        const float v = tile[(py + oy - S::OY0) * TW + lane + ox - S::OX0];
+        if (t % 2 == 0) xv[t / 2].x = v;
+        else xv[t / 2].y = v;
       }
       px.orig = tile[(py - S::OY0) * TW + lane - S::OX0];
-      float ps[8];
+      float2 ps[4];
 #pragma unroll
-      for (int c = 0; c < 8; c++) ps[c] = xv[c];
+      for (int c = 0; c < 4; c++) ps[c] = xv[c];
 #pragma unroll
-      for (int t = 8; t < NT; t++) ps[t % 8] += xv[t];
-      px.mean = (((ps[0] + ps[1]) + (ps[2] + ps[3])) + ((ps[4] + ps[5]) + (ps[6] + ps[7]))) * (1.0f / NT);
+      for (int t = 4; t < NT / 2; t++) ps[t % 4] = __fadd2_rn(ps[t % 4], xv[t]);
+      auto total = [&]() {
+        const float2 q = __fadd2_rn(__fadd2_rn(ps[0], ps[1]), __fadd2_rn(ps[2], ps[3]));
+        return q.x + q.y;
+      };
+      px.mean = total() * (1.0f / NT);
 #pragma unroll
-      for (int t = 0; t < NT; t++) xv[t] -= px.mean;
+      for (int t = 0; t < NT / 2; t++) xv[t] = __fadd2_rn(xv[t], make_float2(-px.mean, -px.mean));
 #pragma unroll
-      for (int c = 0; c < 8; c++) ps[c] = xv[c] * xv[c];
+      for (int c = 0; c < 4; c++) ps[c] = __fmul2_rn(xv[c], xv[c]);
 #pragma unroll
-      for (int t = 8; t < NT; t++) ps[t % 8] = fmaf(xv[t], xv[t], ps[t % 8]);
-      const float var = (((ps[0] + ps[1]) + (ps[2] + ps[3])) + ((ps[4] + ps[5]) + (ps[6] + ps[7]))) * (1.0f / NT);
+      for (int t = 4; t < NT / 2; t++) ps[t % 4] = __ffma2_rn(xv[t], xv[t], ps[t % 4]);
+      const float var = total() * (1.0f / NT);
       const float invstd = var >= kFltEps ? (SPLIT ? 1.0f / sqrtf(var) : rsqrtf(var)) : 0.0f;
       px.stdv = var * invstd;
       // A row: [x_hat (NT), mean * invstd, 1, 1, 1, 0...].  A mean term beyond
@@ -339,16 +347,14 @@ __global__ void __launch_bounds__(TcShape<WH, NNS, XP, SPLIT>::THREADS, 1) nn_tc
         __half2 h[4], l[4];
 #pragma unroll
         for (int j = 0; j < 4; j++) {
-          float v[2];
-#pragma unroll
-          for (int q = 0; q < 2; q++) {
-            const int t = 8 * kc + 2 * j + q;
-            v[q] = t < NT ? xv[t < NT ? t : 0] * invstd : (t == NT ? mterm : (t <= NT + 3 ? 1.0f : 0.0f));
-          }
-          h[j] = __floats2half2_rn(v[0], v[1]);
+          const int t = 8 * kc + 2 * j;
+          const float2 v = t < NT ? __fmul2_rn(xv[t < NT ? t / 2 : 0], make_float2(invstd, invstd))
+                                  : (t == NT ? make_float2(mterm, 1.0f)
+                                             : (t == NT + 2 ? make_float2(1.0f, 1.0f) : make_float2(0.0f, 0.0f)));
+          h[j] = __floats2half2_rn(v.x, v.y);
           if (SPLIT) {
             const float2 f = __half22float2(h[j]);
-            l[j] = __floats2half2_rn(v[0] - f.x, v[1] - f.y);
+            l[j] = __floats2half2_rn(v.x - f.x, v.y - f.y);
           }
         }
         *reinterpret_cast<uint4*>(row + kc * LBO) = *reinterpret_cast<uint4*>(h);
@@ -372,8 +378,15 @@ __global__ void __launch_bounds__(TcShape<WH, NNS, XP, SPLIT>::THREADS, 1) nn_tc
     const float one = SPLIT ? p.split_one : 1.0f, unit = SPLIT ? p.split_unit : 1.0f;
     int c = 0;
     for (; t < ntiles; t += stride) {
-      float2 wsum = make_float2(0.0f, 0.0f);
-      float vsum = 0.0f;
+      float2 wsum = make_float2(0.0f, 0.0f), vsum = wsum;
+      // the accumulators in steps of 16 neurons, both branches' columns; a
+      // step's loads are in flight during the arithmetic of the step before
+      float s1[2][16], s2[2][16];
+      constexpr int STEPS = NC / 16;
+      auto load = [&](int b, int q) {
+        tmem_ld16(lane_addr + b * CCOL + 16 * q, s1[q]);
+        tmem_ld16(lane_addr + b * CCOL + NC + 16 * q, s2[q]);
+      };
 #pragma unroll 1
       for (int k = 0; k < NCH; k++, c++) {
         const int b = c & 1;
@@ -383,41 +396,41 @@ __global__ void __launch_bounds__(TcShape<WH, NNS, XP, SPLIT>::THREADS, 1) nn_tc
           nxt = normalise();
           prefetch(t + 2 * stride);
         }
-        // the accumulators in steps of 16 neurons: both branches' columns
-        // (the next step's loads are in flight during this step's arithmetic)
-        float s1[2][16], s2[2][16];
-        const uint32_t col = lane_addr + b * CCOL;
-        tmem_ld16(col, s1[0]);
-        tmem_ld16(col + NC, s2[0]);
+        load(b, 0);
 #pragma unroll
-        for (int q = 0; q < NC / 16; q++) {
-          tmem_wait16(s1[q & 1], s2[q & 1]);
-          if (q + 1 < NC / 16) {
-            tmem_ld16(col + 16 * (q + 1), s1[(q + 1) & 1]);
-            tmem_ld16(col + NC + 16 * (q + 1), s2[(q + 1) & 1]);
+        for (int q = 0; q < STEPS; q++) {
+          tmem_wait16(s1[q], s2[q]);
+          if (q + 1 < STEPS) {
+            load(b, q + 1);
           } else {  // this warp has read buffer b
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(&B.empty[b]));
           }
-          const float(&a)[16] = s1[q & 1];
-          const float(&d)[16] = s2[q & 1];
+          // sum of e s / (1 + |s|): neurons j and j+2 (and j+1, j+3) share one
+          // reciprocal, of the product of their denominators
 #pragma unroll
-          for (int j = 0; j < 16; j += 2) {
-            float2 l = make_float2(a[j], a[j + 1]);
-            if (SPLIT) l = __fmul2_rn(l, make_float2(unit, unit));
-            const float2 e = make_float2(exp2f_approx(l.x), exp2f_approx(l.y));
-            // s / (1 + |s|) for two neurons from one reciprocal of the product
-            const float d0 = one + fabsf(d[j]), d1 = one + fabsf(d[j + 1]);
-            const float2 n = __fmul2_rn(e, make_float2(d[j], d[j + 1]));
-            wsum = __fadd2_rn(wsum, e);
-            vsum = fmaf(fmaf(n.x, d1, n.y * d0), rcp_approx(d0 * d1), vsum);
+          for (int j = 0; j < 16; j += 4) {
+            float2 n[2], d[2];
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+              const int i = j + 2 * h;
+              float2 l = make_float2(s1[q][i], s1[q][i + 1]);
+              if (SPLIT) l = __fmul2_rn(l, make_float2(unit, unit));
+              const float2 e = make_float2(exp2f_approx(l.x), exp2f_approx(l.y));
+              d[h] = make_float2(one + fabsf(s2[q][i]), one + fabsf(s2[q][i + 1]));
+              n[h] = __fmul2_rn(e, make_float2(s2[q][i], s2[q][i + 1]));
+              wsum = __fadd2_rn(wsum, e);
+            }
+            const float2 dd = __fmul2_rn(d[0], d[1]);
+            const float2 nn = __ffma2_rn(n[0], d[1], __fmul2_rn(n[1], d[0]));
+            vsum = __ffma2_rn(nn, make_float2(rcp_approx(dd.x), rcp_approx(dd.y)), vsum);
           }
         }
       }
       const int gx = (t % tiles_x) * 32 + lane, gy = (t / tiles_x) * 4 + py;
       if (gx < p.W && gy < p.H && !*aborted) {
-        const float v = clampf(cur.mean + 5.0f * vsum / (wsum.x + wsum.y) * cur.stdv, 0.0f, 1.0f);
+        const float v = clampf(cur.mean + 5.0f * (vsum.x + vsum.y) / (wsum.x + wsum.y) * cur.stdv, 0.0f, 1.0f);
         if (XP) {
           stp2(out + (size_t)gy * p.out_pitch + 2 * gx, cur.orig, v);
         } else {
