@@ -324,7 +324,7 @@ int pz_model_create(const pz_model_desc* d, pz_model** out) {
   kp.log2_mode = d->strength_log2;
   if (kp.log2_mode) {
     kp.log2_scale = d->strength_scale;
-    kp.log2_max = (float)d->strength_max;
+    kp.log2_max = d->strength_max;
     kp.n_strength = d->strength_max + 1;
   } else {
     if (d->n_strength_thr != 2 && d->n_strength_thr != 3) {

@@ -24,7 +24,7 @@ struct KeyParams {
   int n_thr;
   int log2_mode;     // ravu: strength = clamp(floor(log2(l*scale+eps)), 0, max)
   float log2_scale;
-  float log2_max;
+  int log2_max;
   float coh0, coh1;  // coherence thresholds
   int n_strength;    // strength levels
   int rows;          // LUT keys (24 * n_strength * 3)
@@ -129,40 +129,94 @@ __device__ __forceinline__ void structure_tensor(const Get& get, const KeyParams
   }
 }
 
+// The structure tensors of E windows of one lattice that a thread evaluates
+// together: window e covers grid (X, Y) in [Off::x(e), +N) x [Off::y(e), +N),
+// and `get(X, Y)` returns the key input at lattice point (X, Y).  The points run
+// in lattice order, so that a derivative that several windows share (the same
+// stencil at the same point) is formed once; each window's own sums see their
+// terms in the order and rounding of structure_tensor<PACKED>.
+template <int N, bool FOUR, bool PACKED, int E, class Off, class Get>
+__device__ __forceinline__ void structure_tensors(const Get& get, const KeyParams& kp, float (&a)[E], float (&b)[E],
+                                                  float (&d)[E]) {
+  constexpr int P0 = N <= 4 ? 0 : 1;
+  constexpr int P1 = N <= 4 ? N : N - 1;
+  int x0 = Off::x(0), x1 = x0, y0 = Off::y(0), y1 = y0;
+#pragma unroll
+  for (int e = 1; e < E; e++) {
+    x0 = Off::x(e) < x0 ? Off::x(e) : x0;
+    x1 = Off::x(e) > x1 ? Off::x(e) : x1;
+    y0 = Off::y(e) < y0 ? Off::y(e) : y0;
+    y1 = Off::y(e) > y1 ? Off::y(e) : y1;
+  }
+  float2 ad[E];
+#pragma unroll
+  for (int e = 0; e < E; e++) {
+    ad[e] = make_float2(0.0f, 0.0f);
+    a[e] = b[e] = d[e] = 0.0f;
+  }
+#pragma unroll
+  for (int X = x0 + P0; X < x1 + P1; X++) {
+#pragma unroll
+    for (int Y = y0 + P0; Y < y1 + P1; Y++) {
+#pragma unroll
+      for (int e = 0; e < E; e++) {
+        const int px = X - Off::x(e), py = Y - Off::y(e);
+        if (px < P0 || px >= P1 || py < P0 || py >= P1) continue;
+        const int i = (px - P0) * (P1 - P0) + py - P0;
+        const bool fold = PACKED && stencil_kind(N, FOUR, px) == stencil_kind(N, FOUR, py);
+        auto sx = [&](int q) { return get(q + Off::x(e), Y); };
+        auto sy = [&](int q) { return get(X, q + Off::y(e)); };
+        const float gx = fold ? deriv_unscaled<N, FOUR>(sx, px) : deriv<N, FOUR>(sx, px);
+        const float gy = fold ? deriv_unscaled<N, FOUR>(sy, py) : deriv<N, FOUR>(sy, py);
+        const float w = fold ? kp.gwf[i] : kp.gw[i];
+        if constexpr (PACKED) {
+          const float gxw = __fmul_rn(gx, w), gyw = __fmul_rn(gy, w);
+          ad[e] = __ffma2_rn(make_float2(gx, gy), make_float2(gxw, gyw), ad[e]);
+          b[e] = fmaf(gxw, gy, b[e]);
+        } else {
+          a[e] += gx * gx * w;
+          b[e] += gx * gy * w;
+          d[e] += gy * gy * w;
+        }
+      }
+    }
+  }
+  if constexpr (PACKED) {
+#pragma unroll
+    for (int e = 0; e < E; e++) {
+      a[e] = ad[e].x;
+      d[e] = ad[e].y;
+    }
+  }
+}
+
 __device__ __forceinline__ float sqrt_approx(float x) {
   float r;
-  asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));  // NaN for x < 0, as in GLSL
+  // NaN for x < 0, as in GLSL.  Subnormal arguments count as zero: they mean
+  // eigenvalues below 2^-102, where every gate of ravu_key is closed anyway
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
   return r;
 }
 
 // floor(24 * theta / pi) with theta = mod(atan(y, x) + pi, pi) in [0, pi),
-// without the arctangent: the direction is folded into [0, pi/4] (a turn by
-// -pi/2, then a mirror about the diagonal) and the sector boundaries
-// k*pi/24 below it are counted by comparing y with tan(k*pi/24) * x.  Only
-// directions within FP32 rounding of a boundary can land in the neighbouring
-// sector (the oracle's boundary keys); a NaN component gives sector 0.
-__device__ __forceinline__ float angle_sector(float x, float y) {
-  if (y < 0.0f || (y == 0.0f && x < 0.0f)) {  // theta + pi: same direction mod pi
-    x = -x;
-    y = -y;
-  }
-  float base = 0.0f;
-  if (x < 0.0f) {  // theta in (pi/2, pi): turn by -pi/2
-    const float t = x;
-    x = y;
-    y = -t;
-    base = 12.0f;
-  }
-  const bool mirror = y > x;  // above pi/4: theta'' = pi/2 - theta'
-  if (mirror) {
-    const float t = x;
-    x = y;
-    y = t;
-  }
-  const float s = (float)((int)(y >= 0.131652498f * x) + (int)(y >= 0.267949192f * x) +
-                          (int)(y >= 0.414213562f * x) + (int)(y >= 0.577350269f * x) +
-                          (int)(y >= 0.767326988f * x) + (int)(y >= x));
-  return base + (mirror ? 11.0f - s : s);
+// without the arctangent: the direction is folded into [0, pi/4] (opposite
+// signs: theta above pi/2, turned back by pi/2; then a mirror about the
+// diagonal) and the sector boundaries k*pi/24 at or below it are counted in
+// three comparisons of y with tan(k*pi/24) * x (k = 4; then 2 or 6; then 1, 3 or
+// 5).  Only directions within FP32 rounding of a boundary can land in the
+// neighbouring sector (the oracle's boundary keys); NaN components fail every
+// comparison: sector 0, or 12 for x < 0.
+__device__ __forceinline__ int angle_sector(float x, float y) {
+  const bool turn = ((x < 0.0f) != (y < 0.0f)) && y != 0.0f;
+  const float u = fabsf(turn ? y : x), v = fabsf(turn ? x : y);
+  const bool mirror = v > u;
+  const float c = mirror ? v : u, s = mirror ? u : v;
+  const bool p = s >= 0.577350269f * c;
+  const bool q = s >= (p ? 1.0f : 0.267949192f) * c;
+  const bool r = s >= (p ? 0.767326988f : (q ? 0.414213562f : 0.131652498f)) * c;
+  int k = (p ? 4 : 0) + (q ? (p ? 1 : 2) : 0) + (r ? 1 : 0);
+  if (mirror) k = 11 - k;
+  return turn ? k + 12 : k;
 }
 
 // Eigen analysis + quantisation -> raw key (not clamped to the LUT).
@@ -182,21 +236,21 @@ __device__ __forceinline__ int ravu_key(float a, float b, float d, const KeyPara
   float delta = sqrt_approx(fmaxf(T * T * 0.25f - D, 0.0f));
   float L1 = T * 0.5f + delta, L2 = T * 0.5f - delta;
   float sqrtL1 = sqrt_approx(L1), sqrtL2 = sqrt_approx(L2);
-  const float angle = fabsf(b) < kFltEps ? 0.0f : angle_sector(b, L1 - a);
+  const int angle = fabsf(b) < kFltEps ? 0 : angle_sector(b, L1 - a);
   float lambda = sqrtL1;
-  float strength;
+  int strength;
   if (kp.log2_mode) {
     const float v = lambda * kp.log2_scale + kFltEps;
-    strength = clampf((float)((__float_as_int(v) >> 23) - 127), 0.0f, kp.log2_max);
+    strength = clampi((__float_as_int(v) >> 23) - 127, 0, kp.log2_max);
   } else if (kp.n_thr == 3) {
-    strength = lambda >= kp.thr[1] ? (lambda >= kp.thr[2] ? 3.0f : 2.0f) : (lambda >= kp.thr[0] ? 1.0f : 0.0f);
+    strength = lambda >= kp.thr[1] ? (lambda >= kp.thr[2] ? 3 : 2) : (lambda >= kp.thr[0] ? 1 : 0);
   } else {
-    strength = lambda >= kp.thr[1] ? 2.0f : (lambda >= kp.thr[0] ? 1.0f : 0.0f);
+    strength = lambda >= kp.thr[1] ? 2 : (lambda >= kp.thr[0] ? 1 : 0);
   }
   const float ssum = sqrtL1 + sqrtL2, sdif = sqrtL1 - sqrtL2;
-  float coherence = 0.0f;
-  if (!(ssum < kFltEps)) coherence = sdif >= kp.coh1 * ssum ? 2.0f : (sdif >= kp.coh0 * ssum ? 1.0f : 0.0f);
-  return (int)((angle * (float)kp.n_strength + strength) * 3.0f + coherence);
+  int coherence = 0;
+  if (!(ssum < kFltEps)) coherence = sdif >= kp.coh1 * ssum ? 2 : (sdif >= kp.coh0 * ssum ? 1 : 0);
+  return (angle * kp.n_strength + strength) * 3 + coherence;
 }
 
 // Anti-ringing powers of one value as FP32x2 pairs: (h^32, l^32) and

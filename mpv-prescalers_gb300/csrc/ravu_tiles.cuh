@@ -1,4 +1,4 @@
-// RAVU tile programs: one CTA of 32 x TR threads computes one tile of outputs.
+// RAVU tile programs: one CTA computes one tile of 32 x TR pixels.
 //
 // Each program is a struct with the shared-memory bytes it needs and a
 // device `run(p, x0, y0, smem)` that stages the tile (plus its radius halo)
@@ -16,7 +16,7 @@
 // Input tiles are 32 x TR input pixels (zoom: output pixels), TR = 4, 8 or 16
 // rows (a template argument of every program; 8 is the reference's own
 // workgroup height, compute/ravu-lite-r3.hook:22); thread t handles column
-// t % 32 of row t / 32.  Out-of-range reads replicate the edge texel (the mpv
+// t % 32 of row t / 32 (int11: of the P rows from P * (t / 32)).  Out-of-range reads replicate the edge texel (the mpv
 // texture border mode).
 #pragma once
 #include <cstddef>
@@ -33,24 +33,108 @@ constexpr int kTileW = 32, kBatchTileRows = 8;
 
 __host__ __device__ constexpr int cabs(int v) { return v < 0 ? -v : v; }
 
-// Stage all planes of a frame; RGB also gets a Rec.709 luma tile (the key
-// input); luma and yuv take their key input from plane 0.
-// NT threads share the work.
-template <int CM, int TW, int TH, int NT, typename T>
-__device__ __forceinline__ void stage_planes(float* tile, float* ltile, const RavuArgs& p, int x0, int y0) {
-  constexpr int C = CM == kLuma ? 1 : 3;
-  for (int i = threadIdx.x; i < TW * TH; i += NT) {
-    const int ty = i / TW, tx = i % TW;
-    const int gx = clampi(x0 + tx, 0, p.W - 1), gy = clampi(y0 + ty, 0, p.H - 1);
-    float v[3] = {0.f, 0.f, 0.f};
+// The window tiles of the frame-tile programs: 40 columns starting 4 left of
+// the tile's own 32, which hold every window up to radius 4 and keep groups of
+// 4 columns aligned in the plane (x0 - 4 is a multiple of 4) and in shared
+// memory.  Staging moves such quads: one 8- or 16-byte load and one 16-byte
+// shared store for 4 texels, where one texel at a time took as many address
+// and clamp instructions for each (ravu-r3 at 8-row
+// tiles 93.7 to 86.5 us, ravu-lite-ar-r3 64.4 to 56.3 us at 1080p).
+// Quads across the frame's left or right edge, and planes whose base or pitch
+// is not a multiple of a quad, go texel by texel with clamped columns.
+constexpr int kLead = 4, kTilePitch = kTileW + 8;
+
+template <typename T>
+struct Quad;
+template <>
+struct Quad<float> {
+  float4 v;
+  __device__ __forceinline__ void load(const float* p) { v = __ldg(reinterpret_cast<const float4*>(p)); }
+  __device__ __forceinline__ void load_shared(const float* p) { v = *reinterpret_cast<const float4*>(p); }
+  __device__ __forceinline__ void load1(const float* p, int a, int b, int c, int d) {
+    v = make_float4(__ldg(p + a), __ldg(p + b), __ldg(p + c), __ldg(p + d));
+  }
+  __device__ __forceinline__ float4 get() const { return v; }
+};
+template <>
+struct Quad<__half> {
+  uint2 v;
+  __device__ __forceinline__ void load(const __half* p) { v = __ldg(reinterpret_cast<const uint2*>(p)); }
+  __device__ __forceinline__ void load_shared(const __half* p) { v = *reinterpret_cast<const uint2*>(p); }
+  __device__ __forceinline__ void load1(const __half* p, int a, int b, int c, int d) {
+    const unsigned short* q = reinterpret_cast<const unsigned short*>(p);
+    v.x = __ldg(q + a) | (uint32_t)__ldg(q + b) << 16;
+    v.y = __ldg(q + c) | (uint32_t)__ldg(q + d) << 16;
+  }
+  __device__ __forceinline__ float4 get() const {
+    const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&v.x));
+    const float2 b = __half22float2(*reinterpret_cast<const __half2*>(&v.y));
+    return make_float4(a.x, a.y, b.x, b.y);
+  }
+};
+
+// One plane's window tile, rows y0 .. y0+TH-1 and columns x0-4 .. x0+35, in two
+// steps, so that the loads of all planes are in flight before the first store.
+template <int TH, int NT, typename T>
+struct QuadStage {
+  static constexpr int kQuads = kTilePitch / 4 * TH, IT = (kQuads + NT - 1) / NT;
+  Quad<T> q[IT];
+  __device__ __forceinline__ void load(const T* in, int pitch, int W, int H, int x0, int y0) {
+    const bool aligned = ((reinterpret_cast<uintptr_t>(in) | (uintptr_t)pitch * sizeof(T)) % (4 * sizeof(T))) == 0;
+#pragma unroll
+    for (int k = 0; k < IT; k++) {
+      const int i = threadIdx.x + k * NT;
+      if (kQuads % NT == 0 || i < kQuads) {
+        const int gx = x0 - kLead + i % (kTilePitch / 4) * 4, gy = clampi(y0 + i / (kTilePitch / 4), 0, H - 1);
+        const T* row = in + (size_t)gy * pitch;
+        if (aligned && gx >= 0 && gx + 3 < W) q[k].load(row + gx);
+        else q[k].load1(row, clampi(gx, 0, W - 1), clampi(gx + 1, 0, W - 1), clampi(gx + 2, 0, W - 1), clampi(gx + 3, 0, W - 1));
+      }
+    }
+  }
+  // the same from a box in shared memory whose rows hold bw texels
+  __device__ __forceinline__ void load_box(const T* box, int bw) {
+    each([&](int k, int i) { q[k].load_shared(box + i / (kTilePitch / 4) * bw + i % (kTilePitch / 4) * 4); });
+  }
+  template <class F>
+  __device__ __forceinline__ void each(const F& f) const {  // f(k, quad number)
+#pragma unroll
+    for (int k = 0; k < IT; k++)
+      if (kQuads % NT == 0 || (int)threadIdx.x + k * NT < kQuads) f(k, threadIdx.x + k * NT);
+  }
+};
+
+// The window tiles of C planes (`tile`, plane after plane; CM == kRgb: the
+// Rec.709 luma, the key input, as one more).
+template <int CM, int TH, int NT, typename T>
+struct TileStage {
+  static constexpr int C = CM == kLuma ? 1 : 3;
+  QuadStage<TH, NT, T> s[C];
+  template <class In>
+  __device__ __forceinline__ void load(const In& in, int W, int H, int x0, int y0) {  // in(c, &pitch): plane c
 #pragma unroll
     for (int c = 0; c < C; c++) {
-      v[c] = ldp(static_cast<const T*>(p.in[c]) + (size_t)gy * p.in_pitch[c] + gx);
-      tile[c * TW * TH + i] = v[c];
+      int pitch;
+      const T* base = in(c, pitch);
+      s[c].load(base, pitch, W, H, x0, y0);
     }
-    if (CM == kRgb) ltile[i] = rgb_luma(v[0], v[1], v[2]);
   }
-}
+  __device__ __forceinline__ void store(float* tile) const {
+    float4* t4 = reinterpret_cast<float4*>(tile);
+    s[0].each([&](int k, int i) {
+      float4 v[C];
+#pragma unroll
+      for (int c = 0; c < C; c++) {
+        v[c] = s[c].q[k].get();
+        t4[c * (kTilePitch / 4 * TH) + i] = v[c];
+      }
+      if constexpr (CM == kRgb)
+        t4[C * (kTilePitch / 4 * TH) + i] =
+            make_float4(rgb_luma(v[0].x, v[1].x, v[2].x), rgb_luma(v[0].y, v[1].y, v[2].y),
+                        rgb_luma(v[0].z, v[1].z, v[2].z), rgb_luma(v[0].w, v[1].w, v[2].w));
+    });
+  }
+};
 
 // ---------------------------------------------------------- TMA staging ---
 // Interior tiles (window fully inside the plane) can be staged by TMA: one
@@ -83,30 +167,41 @@ __host__ __device__ constexpr uint32_t tma_plane_bytes() {
 __device__ __forceinline__ float lds_f(const float* p) { return *p; }
 __device__ __forceinline__ float lds_f(const __half* p) { return __half2float(*p); }
 
-// Stage a w x h window whose first texel is column `off` of a bw x bh TMA
-// box at (bx, by) (bx a multiple of 8): thread 0 issues one box per plane
-// into the landing area (plane stride pb bytes), the CTA waits for it, and
-// the window is converted to the float tile (row pitch dp, plane stride
-// dps; RGB also the luma tile).  Returns 1, or -1 when the copy did not
-// complete within the wait bound (error word set, the tile abandoned and TMA
-// off for the rest of the CTA).  The outcome of the wait is made uniform across the
-// CTA, so every thread takes the same path through the tile's barriers.
-template <int CM, int NT, typename T>
-__device__ __forceinline__ int tma_stage_box(const RavuArgs& p, TmaCtx* t, int bx, int by, int bw, int bh,
-                                             uint32_t pb, int off, int w, int h, int dp, int dps, float* tile,
-                                             float* ltile) {
+// A bw x bh box per plane at (bx, by) (bx a multiple of 8) into the landing
+// area (plane stride pb bytes), issued by thread 0.
+template <int CM, typename T>
+__device__ __forceinline__ void tma_issue_box(TmaCtx* t, int bx, int by, int bw, int bh, uint32_t pb) {
   constexpr int C = CM == kLuma ? 1 : 3;
   if (threadIdx.x == 0) {
     mbar_arrive_expect_tx(t->mbar, (uint32_t)C * bw * bh * sizeof(T));
 #pragma unroll
     for (int c = 0; c < C; c++) tma_load_2d(t->raw + c * pb, &t->map[c], bx, by, t->mbar);
   }
+}
+// Wait for the boxes.  False when the copy did not complete within the wait
+// bound (error word set, the tile abandoned and TMA off for the rest of the
+// CTA).  The outcome is made uniform across the CTA, so every thread takes the
+// same path through the tile's barriers.
+__device__ __forceinline__ bool tma_wait_box(const RavuArgs& p, TmaCtx* t) {
   if (!__syncthreads_and(mbar_wait_bounded(t->mbar, t->phase))) {
     if (threadIdx.x == 0 && p.err) atomicCAS(p.err, 0, kErrWaitTimeout);
     t->dead = 1;
-    return -1;
+    return false;
   }
   t->phase ^= 1u;
+  return true;
+}
+
+// Stage a w x h window whose first texel is column `off` of such a box: the
+// window is converted to the float tile (row pitch dp, plane stride dps; RGB
+// also the luma tile).  Returns 1, or -1 when the wait ran out.
+template <int CM, int NT, typename T>
+__device__ __forceinline__ int tma_stage_box(const RavuArgs& p, TmaCtx* t, int bx, int by, int bw, int bh,
+                                             uint32_t pb, int off, int w, int h, int dp, int dps, float* tile,
+                                             float* ltile) {
+  constexpr int C = CM == kLuma ? 1 : 3;
+  tma_issue_box<CM, T>(t, bx, by, bw, bh, pb);
+  if (!tma_wait_box(p, t)) return -1;
   for (int i = threadIdx.x; i < w * h; i += NT) {
     const int ty = i / w, tx = i % w;
     float v[3] = {0.f, 0.f, 0.f};
@@ -120,16 +215,6 @@ __device__ __forceinline__ int tma_stage_box(const RavuArgs& p, TmaCtx* t, int b
   return 1;
 }
 
-// The TW x TH frame tile at (x0, y0) by TMA: 1 staged; 0 not an interior
-// tile, or no maps (use clamped loads); -1 the wait timed out.
-template <int CM, int TW, int TH, int NT, typename T>
-__device__ int stage_planes_tma(const RavuArgs& p, TmaCtx* t, int x0, int y0, float* tile, float* ltile) {
-  if (!t || !t->map || t->dead || x0 < 0 || y0 < 0 || x0 + TW > p.W || y0 + TH > p.H) return 0;
-  const int bx = x0 & ~7;
-  return tma_stage_box<CM, NT, T>(p, t, bx, y0, tma_box_w<TW>(), TH, tma_plane_bytes<TW, TH, T>(), x0 - bx, TW, TH,
-                                  TW, TW * TH, tile, ltile);
-}
-
 // A CTA whose TMA wait timed out may still have that copy in flight into its
 // landing area: before the CTA exits, thread 0 waits (bounded again) for the
 // outstanding phase, so the copy never lands in shared memory that another
@@ -139,16 +224,40 @@ __device__ __forceinline__ void tma_drain(const TmaCtx* t) {
   if (t && t->dead && threadIdx.x == 0) (void)mbar_wait_bounded(t->mbar, t->phase);
 }
 
-// Stage the frame tile by TMA when possible, else by clamped loads.
-// Returns false only when a TMA wait timed out (the tile is abandoned).
-template <int CM, int TW, int TH, int NT, typename T>
+// Stage the window tile of the frame whose own columns start at x0 (rows y0 ..
+// y0+TH-1): interior tiles from a TMA box per plane where the launch has maps,
+// the others by quads; `also` (its load, then its store) is more staging whose
+// loads overlap with the tile's.  Returns false only when a TMA wait timed out
+// (the tile is abandoned).
+struct NoStage {
+  __device__ __forceinline__ void load() {}
+  __device__ __forceinline__ void store() {}
+};
+template <int CM, int TH, int NT, typename T, class Also = NoStage>
 __device__ __forceinline__ bool stage_frame(const RavuArgs& p, TmaCtx* t, int x0, int y0, float* tile,
-                                            float* ltile) {
-  const int r = stage_planes_tma<CM, TW, TH, NT, T>(p, t, x0, y0, tile, ltile);
-  if (r == 0) stage_planes<CM, TW, TH, NT, T>(tile, ltile, p, x0, y0);
-  return r >= 0;
+                                            Also&& also = NoStage()) {
+  TileStage<CM, TH, NT, T> st;
+  constexpr int C = CM == kLuma ? 1 : 3, BW = tma_box_w<kTilePitch>();
+  const int wx = x0 - kLead;
+  if (t && t->map && !t->dead && wx >= 0 && y0 >= 0 && wx + kTilePitch <= p.W && y0 + TH <= p.H) {
+    constexpr uint32_t pb = tma_plane_bytes<kTilePitch, TH, T>();
+    const int bx = wx & ~7;
+    tma_issue_box<CM, T>(t, bx, y0, BW, TH, pb);
+    also.load();
+    if (!tma_wait_box(p, t)) return false;
+    // x0 is a multiple of 32, so the window starts 4 columns into the box: a
+    // quad's place in shared memory
+#pragma unroll
+    for (int c = 0; c < C; c++)
+      st.s[c].load_box(reinterpret_cast<const T*>(t->raw + c * pb) + (wx - bx), BW);
+  } else {
+    st.load([&](int c, int& pitch) { pitch = p.in_pitch[c]; return static_cast<const T*>(p.in[c]); }, p.W, p.H, x0, y0);
+    also.load();
+  }
+  st.store(tile);
+  also.store();
+  return true;
 }
-
 
 // One LUT texel: FP32 (float4) or, in the fast form, FP16 (4 halves in a
 // uint2, half the L1 traffic of the per-pixel row gathers).
@@ -195,12 +304,12 @@ struct LiteTile {
   static constexpr int N = 2 * R - 1, S = N * N, HALO = R - 1;
   static constexpr int kRows = TR, kThreads = kTileW * TR;
   static constexpr bool kOutputTiles = false;
-  static constexpr int TW = kTileW + N - 1, TH = TR + N - 1;
+  static constexpr int TW = kTilePitch, TH = TR + N - 1;
   // the value tile; the anti-ringing powers are formed per tap in registers
   // (ar_pow2): a shared table of each texel's four powers, formed once per
   // texel, measured 2-13 % slower (an extra barrier, 8 KB more shared memory
   // per CTA and a 16-byte shared load per tap)
-  static constexpr size_t smem_bytes = (size_t)((TW * TH + 3) & ~3) * 4;
+  static constexpr size_t smem_bytes = (size_t)TW * TH * 4;
 
   static constexpr int kPlanes = 1;
   // ravu-lite-ar-r4 at <= 48 registers (5 CTAs of 8 rows per SM) measured
@@ -213,12 +322,13 @@ struct LiteTile {
 
   __device__ static void run(const RavuArgs& p, int x0, int y0, float* smem, TmaCtx* tma = nullptr) {
     float* tile = smem;
-    if (!stage_frame<kLuma, TW, TH, kThreads, T>(p, tma, x0 - HALO, y0 - HALO, tile, nullptr)) return;
+    if (!stage_frame<kLuma, TH, kThreads, T>(p, tma, x0, y0 - HALO, tile)) return;
     __syncthreads();
     const int tx = threadIdx.x % kTileW, ty = threadIdx.x / kTileW;
     const int gx = x0 + tx, gy = y0 + ty;
     if (gx >= p.W || gy >= p.H) return;
-    auto get = [&](int kx, int ky) { return tile[(ty + ky) * TW + tx + kx]; };
+    const float* base = tile + ty * TW + tx + kLead - HALO;
+    auto get = [&](int kx, int ky) { return base[ky * TW + kx]; };
     float a, b, d;
     structure_tensor<N, false, kPackedTensor>(get, p.kp, a, b, d);
     const int key = ravu_key(a, b, d, p.kp);
@@ -312,7 +422,7 @@ struct ThreeXTile {
   static constexpr int N = 2 * R - 1, S = N * N, HALO = R - 1;
   static constexpr int kRows = TR, kThreads = kTileW * TR;
   static constexpr bool kOutputTiles = false;
-  static constexpr int TW = kTileW + N - 1, TH = TR + N - 1;
+  static constexpr int TW = kTilePitch, TH = TR + N - 1;
   static constexpr int C = CM == kLuma ? 1 : 3;
   static constexpr size_t smem_bytes = (size_t)(C + (CM == kRgb ? 1 : 0)) * TW * TH * 4;
   static constexpr int kPlanes = C;
@@ -321,16 +431,14 @@ struct ThreeXTile {
 
   __device__ static void run(const RavuArgs& p, int x0, int y0, float* smem, TmaCtx* tma = nullptr) {
     float* tile = smem;
-    float* ltile = smem + C * TW * TH;
-    if (!stage_frame<CM, TW, TH, kThreads, T>(p, tma, x0 - HALO, y0 - HALO, tile, ltile)) return;
+    if (!stage_frame<CM, TH, kThreads, T>(p, tma, x0, y0 - HALO, tile)) return;
     __syncthreads();
     const int tx = threadIdx.x % kTileW, ty = threadIdx.x / kTileW;
     const int gx = x0 + tx, gy = y0 + ty;
     if (gx >= p.W || gy >= p.H) return;
-    auto val = [&](int c, int t) { return tile[c * TW * TH + (ty + t % N) * TW + tx + t / N]; };
-    auto lum = [&](int kx, int ky) {
-      return CM == kRgb ? ltile[(ty + ky) * TW + tx + kx] : tile[(ty + ky) * TW + tx + kx];
-    };
+    const float* base = tile + ty * TW + tx + kLead - HALO;
+    auto val = [&](int c, int t) { return base[c * TW * TH + t % N * TW + t / N]; };
+    auto lum = [&](int kx, int ky) { return base[(CM == kRgb ? C * TW * TH : 0) + ky * TW + kx]; };
     float a, b, d;
     structure_tensor<N, false>(lum, p.kp, a, b, d);
     const int key = ravu_key(a, b, d, p.kp);
@@ -402,176 +510,204 @@ struct ThreeXTile {
   }
 };
 
-// The ravu keyed filter of one key evaluation: res[c] = sum over the S/2
-// mirrored tap pairs of (x_i + x_{S-1-i}) * w_i (ravu-r3.hook:126-146), the
-// weights w_i packed 4 to a texel.  Two tap pairs per FP32x2 FADD/FFMA.
-template <int S, int C, class Val>
-__device__ __forceinline__ void ravu_filter(const float4* L, const Val& val, float (&res)[C]) {
-  float2 acc[C];
-#pragma unroll
-  for (int c = 0; c < C; c++) acc[c] = make_float2(0.0f, 0.0f);
-#pragma unroll
-  for (int q = 0; q < (S / 2 + 3) / 4; q++) {
-    const float4 w4 = __ldg(L + q);
-#pragma unroll
-    for (int h = 0; h < 2; h++) {
-      const int i0 = 4 * q + 2 * h, i1 = i0 + 1;
-      const float2 w2 = h == 0 ? make_float2(w4.x, w4.y) : make_float2(w4.z, w4.w);
-      if (i1 < S / 2) {
-#pragma unroll
-        for (int c = 0; c < C; c++) {
-          const float2 s2 = __fadd2_rn(make_float2(val(c, i0), val(c, i1)),
-                                       make_float2(val(c, S - 1 - i0), val(c, S - 1 - i1)));
-          acc[c] = __ffma2_rn(s2, w2, acc[c]);
-        }
-      } else if (i0 < S / 2) {
-#pragma unroll
-        for (int c = 0; c < C; c++) acc[c].x = fmaf(val(c, i0) + val(c, S - 1 - i0), w2.x, acc[c].x);
-      }
-    }
-  }
-#pragma unroll
-  for (int c = 0; c < C; c++) res[c] = acc[c].x + acc[c].y;
-}
-
 // ------------------------------------------------------ ravu lattice -----
-// int11: the keyed filter over the input window (ravu-r3.hook:15-146).  Each
-// thread stores its pixel's int11 value into the compact FP32 int11 plane
-// (p.i11, [C][H][W]): one coalesced 4-byte store per channel.  The lattice
-// program below writes every output pixel.
+// Windows of a thread's P pixels, one below the other.
+struct OffDown {
+  __host__ __device__ static constexpr int x(int) { return 0; }
+  __host__ __device__ static constexpr int y(int e) { return e; }
+};
+
+// int11: the keyed filter over the input window (ravu-r3.hook:15-146):
+// res[c] = sum over the S/2 mirrored tap pairs of (x_i + x_{S-1-i}) * w_i, the
+// weights w_i packed 4 to a texel, even and odd i in the lanes of an FP32x2 sum.
+// A thread computes P pixels of one column, whose windows overlap in all but
+// one row each: loads, derivatives and staging are shared (33 shared loads and
+// stores a pixel at r3, from 73).  Each thread stores its int11 values into the
+// compact FP32 int11 plane (p.i11, [C][H][W]): one coalesced 4-byte store per
+// pixel and channel.  The lattice program below writes every output pixel.
+// Bound by issue (70 %) and by L1 (74 %), half of it the gathers of LUT rows.
+// 1080p, r3 luma: 26 us (34.4 us with one pixel a thread and texel staging).
 template <int R, int CM, typename T, int TR = 8>
 struct Int11Tile {
   static constexpr int N = 2 * R, S = N * N, HALO = R - 1;
-  static constexpr int kRows = TR, kThreads = kTileW * TR;
-  static constexpr bool kOutputTiles = false;
-  static constexpr int TW = kTileW + N - 1, TH = TR + N - 1;
   static constexpr int C = CM == kLuma ? 1 : 3;
+  static constexpr int P = 4;
+  static constexpr int kRows = TR, kThreads = kTileW * TR / P;
+  static constexpr bool kOutputTiles = false;
+  static constexpr int TW = kTilePitch, TH = TR + N - 1;
   static constexpr size_t smem_bytes = (size_t)(C + (CM == kRgb ? 1 : 0)) * TW * TH * 4;
   static constexpr int kPlanes = C;
-  // register caps measured best on GB300: r3 40 registers (6 CTAs of 8 rows
-  // per SM; 32 registers spill the packed structure tensor), r4 48, r2 the
-  // compiler's own allocation
-  static constexpr int kMaxRegs = R == 3 ? 40 : (R == 4 ? 48 : 0);
+  // r3 luma at 56 registers (of 66) is 1 % faster; the others lose by any cap
+  static constexpr int kMaxRegs = R == 3 && CM == kLuma ? 56 : 0;
   using Elem = T;
 
   __device__ static void run(const RavuArgs& p, int x0, int y0, float* smem, TmaCtx* tma = nullptr) {
     float* tile = smem;
-    float* ltile = smem + C * TW * TH;
-    if (!stage_frame<CM, TW, TH, kThreads, T>(p, tma, x0 - HALO, y0 - HALO, tile, ltile)) return;
+    if (!stage_frame<CM, TH, kThreads, T>(p, tma, x0, y0 - HALO, tile)) return;
     __syncthreads();
-    const int tx = threadIdx.x % kTileW, ty = threadIdx.x / kTileW;
+    const int tx = threadIdx.x % kTileW, ty = threadIdx.x / kTileW * P;
     const int gx = x0 + tx, gy = y0 + ty;
     if (gx >= p.W || gy >= p.H) return;
-    auto val = [&](int c, int i) { return tile[c * TW * TH + (ty + i % N) * TW + tx + i / N]; };
-    auto lum = [&](int kx, int ky) {
-      return CM == kRgb ? ltile[(ty + ky) * TW + tx + kx] : tile[(ty + ky) * TW + tx + kx];
-    };
-    float a, b, d;
-    structure_tensor<N, true>(lum, p.kp, a, b, d);
-    const int key = ravu_key(a, b, d, p.kp);
-    if (p.keys) p.keys[(size_t)gy * p.W + gx] = key;
-    const float4* L = p.lut + (size_t)min(max(key, 0), p.lut_rows - 1) * p.lut_cols;
-    float res[C];
-    ravu_filter<S, C>(L, val, res);
+    const float* base = tile + ty * TW + tx + kLead - HALO;
+    const float* lbase = base + (CM == kRgb ? C * TW * TH : 0);
+    float a[P], b[P], d[P];
+    structure_tensors<N, true, true, P, OffDown>([&](int X, int Y) { return lbase[Y * TW + X]; }, p.kp, a, b, d);
+    const float4* L[P];
+#pragma unroll
+    for (int e = 0; e < P; e++) {
+      const int key = ravu_key(a[e], b[e], d[e], p.kp);
+      if (p.keys && gy + e < p.H) p.keys[(size_t)(gy + e) * p.W + gx] = key;
+      L[e] = p.lut + (size_t)min(max(key, 0), p.lut_rows - 1) * p.lut_cols;
+    }
+    if (C > 1 || R == 4) asm volatile("" ::: "memory");  // no window value stays in a register from here
+    float2 acc[P][C];
+    float4 w4[P];
+#pragma unroll
+    for (int e = 0; e < P; e++)
+#pragma unroll
+      for (int c = 0; c < C; c++) acc[e][c] = make_float2(0.0f, 0.0f);
+#pragma unroll
+    for (int i = 0; i < S / 2; i += 2) {
+      const int X = i / N, Y = i % N;
+#pragma unroll
+      for (int e = 0; e < P; e++) {
+        if (i % 4 == 0) w4[e] = __ldg(L[e] + i / 4);
+        const float2 w2 = i % 4 == 0 ? make_float2(w4[e].x, w4[e].y) : make_float2(w4[e].z, w4[e].w);
+#pragma unroll
+        for (int c = 0; c < C; c++) {
+          auto v = [&](int x, int y) { return base[c * TW * TH + (y + e) * TW + x]; };
+          const float2 s2 = make_float2(v(X, Y) + v(N - 1 - X, N - 1 - Y), v(X, Y + 1) + v(N - 1 - X, N - 2 - Y));
+          acc[e][c] = __ffma2_rn(s2, w2, acc[e][c]);
+        }
+      }
+    }
     const size_t plane = (size_t)p.W * p.H;
 #pragma unroll
-    for (int c = 0; c < C; c++) {
-      float v = clampf(res[c], 0.f, 1.f);
-      if (p.i11_half) v = __half2float(__float2half_rn(v));
-      p.i11[c * plane + (size_t)gy * p.W + gx] = v;
+    for (int e = 0; e < P; e++) {
+      if (gy + e >= p.H) break;
+#pragma unroll
+      for (int c = 0; c < C; c++) {
+        float v = clampf(acc[e][c].x + acc[e][c].y, 0.f, 1.f);
+        if (p.i11_half) v = __half2float(__float2half_rn(v));
+        p.i11[c * plane + (size_t)(gy + e) * p.W + gx] = v;
+      }
     }
   }
 };
 
-// Where lattice sample k (grid (k/N, k%N)) of an int10 (L=0) or int01 (L=1)
-// pass reads: 0 = input, 1 = int11, at offsets (dx, dy).  The window is the
-// 45-degree lattice: s = kx+ky-(N-1), d = ky-kx (ravu-r3.hook:155-189 int10,
-// :289-323 int01).
+// The two lattice passes read windows turned by 45 degrees (s = kx+ky-(N-1),
+// d = ky-kx; ravu-r3.hook:155-189 int10, :289-323 int01) of the lattice that
+// interleaves input and int11 pixels.  int01's window is int10's one step back
+// along kx, so both are windows of one lattice (X, Y): int10 at X = kx, int01
+// at X = kx - 1.
+struct OffLattice {
+  __host__ __device__ static constexpr int x(int e) { return -e; }
+  __host__ __device__ static constexpr int y(int) { return 0; }
+};
+// Where lattice point (X, Y) lies: 0 = input, 1 = int11, at offset (dx, dy).
 template <int N>
-__host__ __device__ constexpr int lat_src(int k, int L) {
-  return (((k / N + k % N - (N - 1)) % 2 != 0) == (L == 0)) ? 0 : 1;
+__host__ __device__ constexpr int lat_src(int X, int Y) {
+  return (X + Y - (N - 1)) % 2 != 0 ? 0 : 1;
 }
 template <int N>
-__host__ __device__ constexpr int lat_dx(int k, int L) {
-  // int10: input (s+1)/2, int11 s/2; int01: input s/2, int11 (s-1)/2
-  return L == 0 ? (lat_src<N>(k, L) == 0 ? (k / N + k % N - (N - 1) + 1) / 2 : (k / N + k % N - (N - 1)) / 2)
-                : (lat_src<N>(k, L) == 0 ? (k / N + k % N - (N - 1)) / 2 : (k / N + k % N - (N - 1) - 1) / 2);
+__host__ __device__ constexpr int lat_dx(int X, int Y) {
+  return lat_src<N>(X, Y) == 0 ? (X + Y - (N - 1) + 1) / 2 : (X + Y - (N - 1)) / 2;
 }
 template <int N>
-__host__ __device__ constexpr int lat_dy(int k, int L) {
-  // int10: input d/2, int11 (d-1)/2; int01: input (d+1)/2, int11 d/2
-  return L == 0 ? (lat_src<N>(k, L) == 0 ? (k % N - k / N) / 2 : (k % N - k / N - 1) / 2)
-                : (lat_src<N>(k, L) == 0 ? (k % N - k / N + 1) / 2 : (k % N - k / N) / 2);
+__host__ __device__ constexpr int lat_dy(int X, int Y) {
+  return lat_src<N>(X, Y) == 0 ? (Y - X) / 2 : (Y - X - 1) / 2;
 }
 
 // int10 + int01: both lattice filters per input pixel (ravu-r3.hook:148-437).
 // The input tile and the int11 tile (from the FP32 int11 plane, clamped to
 // its edge: the clamp-to-edge of the int11 texture) are staged; each thread
-// then holds all four samples of its output 2x2 block -- input (0,0), int10
-// (1,0), int01 (0,1), int11 (1,1) -- and writes them as two pixel-pair rows.
+// evaluates both windows of a pixel, which share all but one column each of
+// the lattice: every lattice value is loaded once per use (key, filter) and
+// channel for the two, and a tap is one lane of an FP32x2 product with its
+// weight (no sums of mirrored taps first: the two windows mirror differently).
+// Bound by issue (69 %) and by L1 (76 %).  1080p, both passes together: ravu-r3
+// 79.0 us (100.9 us with each window by itself and texel staging), ravu-r4 209
+// (266), ravu-r4-yuv 279 (330).  It then holds all four samples of its output 2x2 block
+// -- input (0,0), int10 (1,0), int01 (0,1), int11 (1,1) -- and writes them as two
+// pixel-pair rows.
 template <int R, int CM, typename T, int TR = 8>
 struct LatticeTile {
   static constexpr int N = 2 * R, S = N * N;
   static constexpr int kRows = TR, kThreads = kTileW * TR;
   static constexpr bool kOutputTiles = false;
-  static constexpr int TW = kTileW + N - 1, TH = TR + N - 1;
+  static constexpr int TW = kTilePitch, TH = TR + N - 1;
   static constexpr int C = CM == kLuma ? 1 : 3;
   static constexpr int PL = C + (CM == kRgb ? 1 : 0);  // planes per tile set
   static constexpr size_t smem_bytes = (size_t)2 * PL * TW * TH * 4;
   static constexpr int kPlanes = C;
-  // register caps measured best on GB300: r3 48 registers (5 CTAs of 8 rows
-  // per SM), r4 80 (3), r2 the compiler's own allocation
-  static constexpr int kMaxRegs = R == 3 ? 48 : (R == 4 ? 80 : 0);
+  // luma at r2 / r3 is 2-4 % faster under these caps (of 44 / 60 registers);
+  // r4 and three channels lose by any (r3-yuv at 40: 162 against 126 us)
+  static constexpr int kMaxRegs = CM == kLuma && R <= 3 ? (R == 2 ? 40 : 48) : 0;
   using Elem = T;
 
   __device__ static void run(const RavuArgs& p, int x0, int y0, float* smem, TmaCtx* tma = nullptr) {
-    float* tin = smem;                      // input, offsets -(R-1) .. R
-    float* lin = tin + C * TW * TH;
-    float* t11 = smem + PL * TW * TH;       // int11, offsets -R .. R-1
-    float* l11 = t11 + C * TW * TH;
-    if (!stage_frame<CM, TW, TH, kThreads, T>(p, tma, x0 - (R - 1), y0 - (R - 1), tin, lin)) return;
+    float* tin = smem;                      // input, rows y0-(R-1) ..
+    float* t11 = smem + PL * TW * TH;       // int11, rows y0-R ..
     const size_t plane = (size_t)p.W * p.H;
-    for (int i = threadIdx.x; i < TW * TH; i += kThreads) {
-      const int ty = i / TW, tx = i % TW;
-      const int cx = clampi(x0 - R + tx, 0, p.W - 1), cy = clampi(y0 - R + ty, 0, p.H - 1);
-      float v[3] = {0.f, 0.f, 0.f};
-#pragma unroll
-      for (int c = 0; c < C; c++) {
-        v[c] = __ldg(p.i11 + c * plane + (size_t)cy * p.W + cx);
-        t11[c * TW * TH + i] = v[c];
+    struct {
+      TileStage<CM, TH, kThreads, float> st;
+      const RavuArgs& p;
+      float* t11;
+      int x0, y0;
+      __device__ __forceinline__ void load() {
+        st.load([&](int c, int& pitch) { pitch = p.W; return p.i11 + (size_t)c * p.W * p.H; }, p.W, p.H, x0, y0);
       }
-      if (CM == kRgb) l11[i] = rgb_luma(v[0], v[1], v[2]);
-    }
+      __device__ __forceinline__ void store() { st.store(t11); }
+    } i11{{}, p, t11, x0, y0 - R};
+    if (!stage_frame<CM, TH, kThreads, T>(p, tma, x0, y0 - (R - 1), tin, i11)) return;
     __syncthreads();
     const int tx = threadIdx.x % kTileW, ty = threadIdx.x / kTileW;
     const int gx = x0 + tx, gy = y0 + ty;
     if (gx >= p.W || gy >= p.H) return;
-    float res[2][C];
+    const float* bin = tin + (ty + R - 1) * TW + tx + kLead;
+    const float* b11 = t11 + (ty + R) * TW + tx + kLead;
+    auto val = [&](int c, int X, int Y) {
+      return (lat_src<N>(X, Y) == 0 ? bin : b11)[c * TW * TH + lat_dy<N>(X, Y) * TW + lat_dx<N>(X, Y)];
+    };
+    float a[2], b[2], d[2];
+    structure_tensors<N, true, true, 2, OffLattice>(
+        [&](int X, int Y) { return val(CM == kRgb ? C : 0, X, Y); }, p.kp, a, b, d);  // rgb: the luma tile is plane C
+    float4 w[2][(S / 2 + 3) / 4];
 #pragma unroll
-    for (int L = 0; L < 2; L++) {
-      auto idx = [&](int k) {
-        return lat_src<N>(k, L) == 0 ? (ty + lat_dy<N>(k, L) + R - 1) * TW + tx + lat_dx<N>(k, L) + R - 1
-                                     : (ty + lat_dy<N>(k, L) + R) * TW + tx + lat_dx<N>(k, L) + R;
-      };
-      auto val = [&](int c, int k) { return (lat_src<N>(k, L) == 0 ? tin : t11)[c * TW * TH + idx(k)]; };
-      auto lum = [&](int kx, int ky) {
-        const int k = kx * N + ky;
-        if (CM != kRgb) return val(0, k);
-        return (lat_src<N>(k, L) == 0 ? lin : l11)[idx(k)];
-      };
-      float a, b, d;
-      structure_tensor<N, true>(lum, p.kp, a, b, d);
-      const int key = ravu_key(a, b, d, p.kp);
-      if (p.keys) p.keys[(size_t)(1 + L) * p.W * p.H + (size_t)gy * p.W + gx] = key;
-      const float4* Lr = p.lut + (size_t)min(max(key, 0), p.lut_rows - 1) * p.lut_cols;
-      ravu_filter<S, C>(Lr, val, res[L]);
+    for (int e = 0; e < 2; e++) {
+      const int key = ravu_key(a[e], b[e], d[e], p.kp);
+      if (p.keys) p.keys[(size_t)(1 + e) * plane + (size_t)gy * p.W + gx] = key;
+      const float4* L = p.lut + (size_t)min(max(key, 0), p.lut_rows - 1) * p.lut_cols;
+#pragma unroll
+      for (int q = 0; q < (S / 2 + 3) / 4; q++) w[e][q] = __ldg(L + q);
     }
+    if (C > 1 || R == 4) asm volatile("" ::: "memory");  // no window value stays in a register from here
+    // weights i, i+1 (i even) of window e as a pair
+    auto wpair = [&](int e, int i) {
+      const float4& q = w[e][i / 4];
+      return i % 4 == 0 ? make_float2(q.x, q.y) : make_float2(q.z, q.w);
+    };
 #pragma unroll
     for (int c = 0; c < C; c++) {
+      float2 acc[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+#pragma unroll
+      for (int X = -1; X < N; X++) {
+#pragma unroll
+        for (int Y = 0; Y < N; Y += 2) {
+          const float v0 = val(c, X, Y), v1 = val(c, X, Y + 1);
+#pragma unroll
+          for (int e = 0; e < 2; e++) {
+            const int i = (X + e) * N + Y;  // taps i, i+1 of window e; the upper half mirrors the lower
+            if (i < 0 || i >= S) continue;
+            if (i < S / 2) acc[e] = __ffma2_rn(make_float2(v0, v1), wpair(e, i), acc[e]);
+            else acc[e] = __ffma2_rn(make_float2(v1, v0), wpair(e, S - 2 - i), acc[e]);
+          }
+        }
+      }
       T* o = static_cast<T*>(p.out[c]) + (size_t)(2 * gy) * p.out_pitch[c] + 2 * gx;
       // row 2i: input, int10; row 2i+1: int01, int11 (ravu-r3.hook:424-437)
-      stp2(o, tin[c * TW * TH + (ty + R - 1) * TW + tx + R - 1], clampf(res[0][c], 0.f, 1.f));
-      stp2(o + p.out_pitch[c], clampf(res[1][c], 0.f, 1.f), t11[c * TW * TH + (ty + R) * TW + tx + R]);
+      stp2(o, bin[c * TW * TH], clampf(acc[0].x + acc[0].y, 0.f, 1.f));
+      stp2(o + p.out_pitch[c], clampf(acc[1].x + acc[1].y, 0.f, 1.f), b11[c * TW * TH]);
     }
   }
 };

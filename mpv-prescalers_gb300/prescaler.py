@@ -99,9 +99,9 @@ class HookModel:
     @property
     def default_staging(self) -> str:
         """Halo staging used when none is asked for: TMA boxes for ravu-lite
-        (measured faster on GB300: ravu-lite-ar-r3 59 vs 64 us per 1080p
-        frame), clamped loads for the other programs (lattice, 3x and zoom
-        measured equal or 3-8 % faster with them)."""
+        (within 2 % of plain loads on GB300 at r2 and the anti-ringing r3 / r4:
+        ravu-lite-ar-r3 56 us per 1080p frame either way), plain loads for the
+        other programs (ravu-r3 79 against 83 us; 3x and zoom within 3 %)."""
         return "tma" if self.family == "lite" else "ldg"
 
     @property
@@ -290,9 +290,9 @@ class HookModel:
         (clamped loads) or "tma" (TMA boxes for interior tiles), default
         ``default_staging``; the pixels are identical, only the speed
         differs (see ``batch.autotune_staging``).
-        ``tile_rows``: RAVU tile height, 4, 8 or 16 rows of 32 pixels (one
-        thread per pixel; default: the library's measured choice for the
-        model's program, 4 rows but for ravu-lite r2 and ravu-lite-ar r4);
+        ``tile_rows``: RAVU tile height, 4, 8 or 16 rows of 32 pixels
+        (default: the library's measured choice for the model's program, 4
+        rows but for ravu-lite r2, ravu-lite-ar r4 and ravu-r2);
         again only the speed differs (see ``batch.autotune_tiles``).
         Returns the upscaled planes in the input's form (and the raw LUT
         keys as int32 when ``return_keys``).
