@@ -16,6 +16,7 @@
 #include "async.cuh"
 #include "kernels.h"
 #include "model.h"
+#include "ravu_tiles.cuh"
 
 namespace {
 
@@ -361,28 +362,45 @@ int pz_model_create(const pz_model_desc* d, pz_model** out) {
   }
   m->lut_rows = d->lut_rows;
   m->lut_cols = d->lut_cols;
+  // ravu-zoom's tables are held by LUT point (zoom_texel_at, ravu_tiles.cuh),
+  // the others as in the file; FP16 texels in rows padded to an even count, so
+  // that texel pairs are 16-byte loads
+  const bool zoom = d->family == PZ_RAVU_ZOOM;
+  const int nb = need_cols / 9;
+  m->lut_h_pitch = zoom ? 9 * ((nb + 1) & ~1) : (d->lut_cols + 1) & ~1;
   const size_t nval = (size_t)d->lut_rows * d->lut_cols * 4, bytes = nval * 4;
-  auto rounded = [&](const float* src) {  // every value rounded to FP16 (round to nearest even)
-    std::vector<float> r(nval);
-    for (size_t i = 0; i < nval; i++) r[i] = __half2float(__float2half_rn(src[i]));
+  auto laid_out = [&](const float* src, bool half, std::vector<float>* r) {
+    for (int y = 0; y < d->lut_rows; y++)
+      for (int c = 0; c < d->lut_cols; c++) {
+        size_t at;
+        if (zoom) {
+          const uint32_t x = c % 9, t = c / 9;
+          at = d->radius == 2 ? (half ? pz::zoom_texel_at<2, true>(y, x, t) : pz::zoom_texel_at<2, false>(y, x, t))
+                              : (half ? pz::zoom_texel_at<3, true>(y, x, t) : pz::zoom_texel_at<3, false>(y, x, t));
+        } else {
+          at = (size_t)y * (half ? m->lut_h_pitch : d->lut_cols) + c;
+        }
+        std::memcpy(&(*r)[at * 4], &src[((size_t)y * d->lut_cols + c) * 4], 16);
+      }
+  };
+  auto rounded = [](std::vector<float> r) {  // every value rounded to FP16 (round to nearest even)
+    for (float& v : r) v = __half2float(__float2half_rn(v));
     return r;
   };
-  // FP16 texels of the fast form, each row padded to an even texel count so
-  // that texel pairs are 16-byte loads
-  m->lut_h_pitch = (d->lut_cols + 1) & ~1;
-  std::vector<__half> luth((size_t)d->lut_rows * m->lut_h_pitch * 4, __float2half_rn(0.0f));
-  for (int r = 0; r < d->lut_rows; r++)
-    for (int c = 0; c < d->lut_cols * 4; c++)
-      luth[(size_t)r * m->lut_h_pitch * 4 + c] = __float2half_rn(d->lut[(size_t)r * d->lut_cols * 4 + c]);
-  const std::vector<float> lut16 = rounded(d->lut);
-  if ((rc = upload(&m->d_lut, d->lut, bytes)) || (rc = upload(&m->d_lut16, lut16.data(), bytes)) ||
+  std::vector<float> lut(nval), luthf((size_t)d->lut_rows * m->lut_h_pitch * 4, 0.0f);
+  laid_out(d->lut, false, &lut);
+  laid_out(d->lut, true, &luthf);
+  std::vector<__half> luth(luthf.size());
+  for (size_t i = 0; i < luthf.size(); i++) luth[i] = __float2half_rn(luthf[i]);
+  if ((rc = upload(&m->d_lut, lut.data(), bytes)) || (rc = upload(&m->d_lut16, rounded(lut).data(), bytes)) ||
       (rc = upload(&m->d_lut_h, luth.data(), luth.size() * 2))) {
     pz_model_destroy(m);
     return rc;
   }
   if (d->lut_ar) {
-    const std::vector<float> ar16 = rounded(d->lut_ar);
-    if ((rc = upload(&m->d_lut_ar, d->lut_ar, bytes)) || (rc = upload(&m->d_lut_ar16, ar16.data(), bytes))) {
+    std::vector<float> ar(nval);
+    laid_out(d->lut_ar, false, &ar);
+    if ((rc = upload(&m->d_lut_ar, ar.data(), bytes)) || (rc = upload(&m->d_lut_ar16, rounded(ar).data(), bytes))) {
       pz_model_destroy(m);
       return rc;
     }

@@ -253,19 +253,21 @@ __device__ __forceinline__ int ravu_key(float a, float b, float d, const KeyPara
   return (angle * kp.n_strength + strength) * 3 + coherence;
 }
 
-// Anti-ringing powers of one value as FP32x2 pairs: (h^32, l^32) and
-// (h^33, l^33) with h = 0.1 + v, l = 1.1 - v, pow(x, 32) by five squarings
-// (ravu-lite-ar-r3.hook:91-98); each lane rounds as a scalar FMUL would.
-__device__ __forceinline__ void ar_pow2(float v, float2& p32, float2& p33) {
-  const float2 hl = __ffma2_rn(make_float2(v, v), make_float2(1.0f, -1.0f), make_float2(0.1f, 1.1f));
-  float2 q = hl;
+// Anti-ringing powers of one value as an FP32x2 pair: (0.1 + v)^32 and
+// (1.1 - v)^32 by five squarings (ravu-lite-ar-r3.hook:91-98); each lane rounds
+// as a scalar FMUL would.
+__device__ __forceinline__ float2 ar_pow32(float v) {
+  float2 q = __ffma2_rn(make_float2(v, v), make_float2(1.0f, -1.0f), make_float2(0.1f, 1.1f));
 #pragma unroll
   for (int i = 0; i < 5; i++) q = __fmul2_rn(q, q);
-  p32 = q;
-  p33 = __fmul2_rn(q, hl);
+  return q;
 }
 
-// lo = 1.1 - lo2/lo; hi = hi2/hi - 0.1; mix(res, clamp(res, lo, hi), s).
+// The clamp of one output: mix(res, clamp(res, lo, hi), s).  The shaders bound
+// res by lo = 1.1 - sum g l^33 / sum g l^32 and hi = sum g h^33 / sum g h^32 -
+// 0.1 with h = 0.1 + v, l = 1.1 - v; both are means of v itself, weighted by
+// g l^32 and g h^32, and are taken as such: sums = (sum g h^32, sum g l^32),
+// means = (sum g h^32 v, sum g l^32 v).
 // The quotients are approximate (__fdividef, about 2 ulp, the precision a
 // shader's division has): they only move the clamp bounds, by < 3e-7.  Both
 // operands are scaled by 2^24 first, so that a subnormal denominator
@@ -274,10 +276,9 @@ __device__ __forceinline__ void ar_pow2(float v, float2& p32, float2& p33) {
 __device__ __forceinline__ float ar_quot(float n, float d) {
   return __fdividef(n * 16777216.0f, d * 16777216.0f);
 }
-__device__ __forceinline__ float ar_finish(float res, float lo, float hi, float lo2, float hi2, float s) {
-  float lob = 1.1f - ar_quot(lo2, lo);
-  float hib = ar_quot(hi2, hi) - 0.1f;
-  float c = fminf(fmaxf(res, lob), hib);
+__device__ __forceinline__ float ar_finish(float res, float2 sums, float2 means, float s) {
+  const float hib = ar_quot(means.x, sums.x), lob = ar_quot(means.y, sums.y);
+  const float c = fminf(fmaxf(res, lob), hib);
   return res * (1.0f - s) + c * s;
 }
 

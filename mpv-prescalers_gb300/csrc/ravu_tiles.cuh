@@ -19,12 +19,16 @@
 // t % 32 of row t / 32 (int11: of the P rows from P * (t / 32)).  Out-of-range reads replicate the edge texel (the mpv
 // texture border mode).
 #pragma once
+#include <atomic>
 #include <cstddef>
 #include <cstring>
 
 #include "async.cuh"
 #include "kernels.h"
 
+#ifndef PZ_ZOOM_REGS
+#define PZ_ZOOM_REGS 0
+#endif
 namespace pz {
 
 // Tile width in pixels (one warp per tile row); persistent batches run tiles
@@ -73,6 +77,18 @@ struct Quad<__half> {
   }
 };
 
+// May a plane be read in quads (at columns that are multiples of 4)?
+template <typename T>
+__device__ __forceinline__ bool quads_aligned(const T* in, int pitch) {
+  return ((reinterpret_cast<uintptr_t>(in) | (uintptr_t)pitch * sizeof(T)) % (4 * sizeof(T))) == 0;
+}
+// Columns gx .. gx+3 of a row (gx a multiple of 4), replicated past its ends.
+template <typename T>
+__device__ __forceinline__ void load_quad(Quad<T>& q, const T* row, int gx, int W, bool aligned) {
+  if (aligned && gx >= 0 && gx + 3 < W) q.load(row + gx);
+  else q.load1(row, clampi(gx, 0, W - 1), clampi(gx + 1, 0, W - 1), clampi(gx + 2, 0, W - 1), clampi(gx + 3, 0, W - 1));
+}
+
 // One plane's window tile, rows y0 .. y0+TH-1 and columns x0-4 .. x0+35, in two
 // steps, so that the loads of all planes are in flight before the first store.
 template <int TH, int NT, typename T>
@@ -80,16 +96,13 @@ struct QuadStage {
   static constexpr int kQuads = kTilePitch / 4 * TH, IT = (kQuads + NT - 1) / NT;
   Quad<T> q[IT];
   __device__ __forceinline__ void load(const T* in, int pitch, int W, int H, int x0, int y0) {
-    const bool aligned = ((reinterpret_cast<uintptr_t>(in) | (uintptr_t)pitch * sizeof(T)) % (4 * sizeof(T))) == 0;
+    const bool aligned = quads_aligned(in, pitch);
 #pragma unroll
     for (int k = 0; k < IT; k++) {
       const int i = threadIdx.x + k * NT;
-      if (kQuads % NT == 0 || i < kQuads) {
-        const int gx = x0 - kLead + i % (kTilePitch / 4) * 4, gy = clampi(y0 + i / (kTilePitch / 4), 0, H - 1);
-        const T* row = in + (size_t)gy * pitch;
-        if (aligned && gx >= 0 && gx + 3 < W) q[k].load(row + gx);
-        else q[k].load1(row, clampi(gx, 0, W - 1), clampi(gx + 1, 0, W - 1), clampi(gx + 2, 0, W - 1), clampi(gx + 3, 0, W - 1));
-      }
+      if (kQuads % NT == 0 || i < kQuads)
+        load_quad(q[k], in + (size_t)clampi(y0 + i / (kTilePitch / 4), 0, H - 1) * pitch,
+                  x0 - kLead + i % (kTilePitch / 4) * 4, W, aligned);
     }
   }
   // the same from a box in shared memory whose rows hold bw texels
@@ -119,7 +132,10 @@ struct TileStage {
       s[c].load(base, pitch, W, H, x0, y0);
     }
   }
-  __device__ __forceinline__ void store(float* tile) const {
+  // POW: beside the values of a luma tile, `pow` gets every texel's
+  // anti-ringing powers
+  template <bool POW = false>
+  __device__ __forceinline__ void store(float* tile, float4* pow = nullptr) const {
     float4* t4 = reinterpret_cast<float4*>(tile);
     s[0].each([&](int k, int i) {
       float4 v[C];
@@ -132,6 +148,11 @@ struct TileStage {
         t4[C * (kTilePitch / 4 * TH) + i] =
             make_float4(rgb_luma(v[0].x, v[1].x, v[2].x), rgb_luma(v[0].y, v[1].y, v[2].y),
                         rgb_luma(v[0].z, v[1].z, v[2].z), rgb_luma(v[0].w, v[1].w, v[2].w));
+      if constexpr (POW) {
+        const float2 a = ar_pow32(v[0].x), b = ar_pow32(v[0].y), c = ar_pow32(v[0].z), d = ar_pow32(v[0].w);
+        pow[2 * i] = make_float4(a.x, a.y, b.x, b.y);
+        pow[2 * i + 1] = make_float4(c.x, c.y, d.x, d.y);
+      }
     });
   }
 };
@@ -192,29 +213,6 @@ __device__ __forceinline__ bool tma_wait_box(const RavuArgs& p, TmaCtx* t) {
   return true;
 }
 
-// Stage a w x h window whose first texel is column `off` of such a box: the
-// window is converted to the float tile (row pitch dp, plane stride dps; RGB
-// also the luma tile).  Returns 1, or -1 when the wait ran out.
-template <int CM, int NT, typename T>
-__device__ __forceinline__ int tma_stage_box(const RavuArgs& p, TmaCtx* t, int bx, int by, int bw, int bh,
-                                             uint32_t pb, int off, int w, int h, int dp, int dps, float* tile,
-                                             float* ltile) {
-  constexpr int C = CM == kLuma ? 1 : 3;
-  tma_issue_box<CM, T>(t, bx, by, bw, bh, pb);
-  if (!tma_wait_box(p, t)) return -1;
-  for (int i = threadIdx.x; i < w * h; i += NT) {
-    const int ty = i / w, tx = i % w;
-    float v[3] = {0.f, 0.f, 0.f};
-#pragma unroll
-    for (int c = 0; c < C; c++) {
-      v[c] = lds_f(reinterpret_cast<const T*>(t->raw + c * pb) + ty * bw + tx + off);
-      tile[c * dps + ty * dp + tx] = v[c];
-    }
-    if (CM == kRgb) ltile[ty * dp + tx] = rgb_luma(v[0], v[1], v[2]);
-  }
-  return 1;
-}
-
 // A CTA whose TMA wait timed out may still have that copy in flight into its
 // landing area: before the CTA exits, thread 0 waits (bounded again) for the
 // outstanding phase, so the copy never lands in shared memory that another
@@ -233,9 +231,9 @@ struct NoStage {
   __device__ __forceinline__ void load() {}
   __device__ __forceinline__ void store() {}
 };
-template <int CM, int TH, int NT, typename T, class Also = NoStage>
+template <int CM, int TH, int NT, typename T, bool POW = false, class Also = NoStage>
 __device__ __forceinline__ bool stage_frame(const RavuArgs& p, TmaCtx* t, int x0, int y0, float* tile,
-                                            Also&& also = NoStage()) {
+                                            Also&& also = NoStage(), float4* pow = nullptr) {
   TileStage<CM, TH, NT, T> st;
   constexpr int C = CM == kLuma ? 1 : 3, BW = tma_box_w<kTilePitch>();
   const int wx = x0 - kLead;
@@ -254,23 +252,9 @@ __device__ __forceinline__ bool stage_frame(const RavuArgs& p, TmaCtx* t, int x0
     st.load([&](int c, int& pitch) { pitch = p.in_pitch[c]; return static_cast<const T*>(p.in[c]); }, p.W, p.H, x0, y0);
     also.load();
   }
-  st.store(tile);
+  st.template store<POW>(tile, pow);
   also.store();
   return true;
-}
-
-// One LUT texel: FP32 (float4) or, in the fast form, FP16 (4 halves in a
-// uint2, half the L1 traffic of the per-pixel row gathers).
-template <bool H16>
-__device__ __forceinline__ float4 lut_texel(const float4* f, const uint2* h, size_t i) {
-  if constexpr (H16) {
-    const uint2 q = __ldg(h + i);
-    const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&q.x));
-    const float2 b = __half22float2(*reinterpret_cast<const __half2*>(&q.y));
-    return make_float4(a.x, a.y, b.x, b.y);
-  } else {
-    return __ldg(f + i);
-  }
 }
 
 // Two adjacent FP32 texels i, i+1 (i even, row pitch even) as one 32-byte load.
@@ -305,11 +289,10 @@ struct LiteTile {
   static constexpr int kRows = TR, kThreads = kTileW * TR;
   static constexpr bool kOutputTiles = false;
   static constexpr int TW = kTilePitch, TH = TR + N - 1;
-  // the value tile; the anti-ringing powers are formed per tap in registers
-  // (ar_pow2): a shared table of each texel's four powers, formed once per
-  // texel, measured 2-13 % slower (an extra barrier, 8 KB more shared memory
-  // per CTA and a 16-byte shared load per tap)
-  static constexpr size_t smem_bytes = (size_t)TW * TH * 4;
+  // the value tile and (AR) each texel's two 32nd powers, formed while staging
+  // and read as 8 bytes a tap: TABLE_NUMS
+  static constexpr bool kTable = AR && (H16 || R == 2);
+  static constexpr size_t smem_bytes = (size_t)TW * TH * (kTable ? 12 : 4);
 
   static constexpr int kPlanes = 1;
   // ravu-lite-ar-r4 at <= 48 registers (5 CTAs of 8 rows per SM) measured
@@ -322,12 +305,15 @@ struct LiteTile {
 
   __device__ static void run(const RavuArgs& p, int x0, int y0, float* smem, TmaCtx* tma = nullptr) {
     float* tile = smem;
-    if (!stage_frame<kLuma, TH, kThreads, T>(p, tma, x0, y0 - HALO, tile)) return;
+    float* pow = tile + TW * TH;
+    if (!stage_frame<kLuma, TH, kThreads, T, kTable>(p, tma, x0, y0 - HALO, tile, NoStage(), reinterpret_cast<float4*>(pow)))
+      return;
     __syncthreads();
     const int tx = threadIdx.x % kTileW, ty = threadIdx.x / kTileW;
     const int gx = x0 + tx, gy = y0 + ty;
     if (gx >= p.W || gy >= p.H) return;
     const float* base = tile + ty * TW + tx + kLead - HALO;
+    const float2* pbase = reinterpret_cast<const float2*>(pow) + ty * TW + tx + kLead - HALO;
     auto get = [&](int kx, int ky) { return base[ky * TW + kx]; };
     float a, b, d;
     structure_tensor<N, false, kPackedTensor>(get, p.kp, a, b, d);
@@ -337,13 +323,23 @@ struct LiteTile {
     float4 w_next;  // H16: the odd texel of the pair loaded at the even one
     static_assert(S / 2 % 2 == 0, "texel pairs start at even columns");
     // FP32x2 sums: P = sum va*w, Q = sum vb*w, res = P + Q.wzyx; the
-    // anti-ringing sums of output k as (hi, lo) and (hi2, lo2) pairs
+    // anti-ringing sums of output k (ar_finish): G = sums, M = means
     float2 P01 = make_float2(0.f, 0.f), P23 = P01, Q01 = P01, Q23 = P01;
-    float2 HL[4], HL3[4];
+    float2 G[4], M[4];
 #pragma unroll
-    for (int k = 0; k < 4; k++) HL[k] = HL3[k] = P01;
+    for (int k = 0; k < 4; k++) G[k] = M[k] = P01;
+    // one AR tap: value v at window tap t, its weights g[k] (mirrored: g[3-k])
+    auto ar_tap = [&](float v, int t, const float (&g)[4], bool mirrored) {
+      const float2 h = kTable ? pbase[t % N * TW + t / N] : ar_pow32(v), hv = __fmul2_rn(h, make_float2(v, v));
 #pragma unroll
-    for (int c = 0; c < S / 2; c++) {
+      for (int k = 0; k < 4; k++) {
+        const float gk = g[mirrored ? 3 - k : k];
+        G[k] = __ffma2_rn(h, make_float2(gk, gk), G[k]);
+        M[k] = __ffma2_rn(hv, make_float2(gk, gk), M[k]);
+      }
+    };
+#pragma unroll
+    for (int c = 0; c <= S / 2; c++) {
       float4 w;
       if constexpr (H16) {
         if (c % 2 == 0) lut_pair_h16(p.lut_h, row + c, w, w_next);
@@ -356,54 +352,22 @@ struct LiteTile {
       const float2 a2 = make_float2(va, va), b2 = make_float2(vb, vb);
       P01 = __ffma2_rn(a2, w01, P01);
       P23 = __ffma2_rn(a2, w23, P23);
-      Q01 = __ffma2_rn(b2, w01, Q01);
-      Q23 = __ffma2_rn(b2, w23, Q23);
+      if (c < S / 2) {  // the centre tap is its own mirror
+        Q01 = __ffma2_rn(b2, w01, Q01);
+        Q23 = __ffma2_rn(b2, w23, Q23);
+      }
       if (AR && lite_ar_col<R>(c)) {
         const float g[4] = {fmaxf(w.x, 0.f), fmaxf(w.y, 0.f), fmaxf(w.z, 0.f), fmaxf(w.w, 0.f)};
-        float2 ha, ha3, hb, hb3;
-        ar_pow2(va, ha, ha3);
-        ar_pow2(vb, hb, hb3);
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-          const float2 gk = make_float2(g[k], g[k]), gr = make_float2(g[3 - k], g[3 - k]);
-          HL[k] = __ffma2_rn(ha, gk, HL[k]);
-          HL[k] = __ffma2_rn(hb, gr, HL[k]);
-          HL3[k] = __ffma2_rn(ha3, gk, HL3[k]);
-          HL3[k] = __ffma2_rn(hb3, gr, HL3[k]);
-        }
-      }
-    }
-    {
-      constexpr int c = S / 2;  // even: the centre texel and the row's padding
-      float4 w;
-      if constexpr (H16) lut_pair_h16(p.lut_h, row + c, w, w_next);
-      else w = __ldg(p.lut + row + c);
-      const float v = get(c / N, c % N);
-      const float2 v2 = make_float2(v, v);
-      P01 = __ffma2_rn(v2, make_float2(w.x, w.y), P01);
-      P23 = __ffma2_rn(v2, make_float2(w.z, w.w), P23);
-      if (AR) {
-        const float g[4] = {fmaxf(w.x, 0.f), fmaxf(w.y, 0.f), fmaxf(w.z, 0.f), fmaxf(w.w, 0.f)};
-        float2 hc, hc3;
-        ar_pow2(v, hc, hc3);
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-          const float2 gk = make_float2(g[k], g[k]);
-          HL[k] = __ffma2_rn(hc, gk, HL[k]);
-          HL3[k] = __ffma2_rn(hc3, gk, HL3[k]);
-        }
+        ar_tap(va, c, g, false);
+        if (c < S / 2) ar_tap(vb, S - 1 - c, g, true);
       }
     }
     float4 res = make_float4(P01.x + Q23.y, P01.y + Q23.x, P23.x + Q01.y, P23.y + Q01.x);
-    const float4 hi = make_float4(HL[0].x, HL[1].x, HL[2].x, HL[3].x);
-    const float4 lo = make_float4(HL[0].y, HL[1].y, HL[2].y, HL[3].y);
-    const float4 hi2 = make_float4(HL3[0].x, HL3[1].x, HL3[2].x, HL3[3].x);
-    const float4 lo2 = make_float4(HL3[0].y, HL3[1].y, HL3[2].y, HL3[3].y);
     if (AR) {  // no [0,1] clamp after anti-ringing (compute/ravu-lite-ar-r3.hook:166)
-      res.x = ar_finish(res.x, lo.x, hi.x, lo2.x, hi2.x, p.ar);
-      res.y = ar_finish(res.y, lo.y, hi.y, lo2.y, hi2.y, p.ar);
-      res.z = ar_finish(res.z, lo.z, hi.z, lo2.z, hi2.z, p.ar);
-      res.w = ar_finish(res.w, lo.w, hi.w, lo2.w, hi2.w, p.ar);
+      res.x = ar_finish(res.x, G[0], M[0], p.ar);
+      res.y = ar_finish(res.y, G[1], M[1], p.ar);
+      res.z = ar_finish(res.z, G[2], M[2], p.ar);
+      res.w = ar_finish(res.w, G[3], M[3], p.ar);
     } else {
       res.x = clampf(res.x, 0.f, 1.f); res.y = clampf(res.y, 0.f, 1.f);
       res.z = clampf(res.z, 0.f, 1.f); res.w = clampf(res.w, 0.f, 1.f);
@@ -726,71 +690,110 @@ __device__ __forceinline__ ZoomPos zoom_pos(int X, int W, int OW) {
   return {(int)q, (float)(num - q * den) / (float)den};
 }
 
-// Bilinear (FILTER LINEAR) fetch of one LUT texel at block column `blk` and
-// sub-position (sx, sy) of key block `key`: x = blk*9 + 8 sx, y = key*9 + 8 sy
-// (LUTPOS(x, 9) / (blocks, 288), ravu-zoom-r2.hook:23-31); clamp-to-edge.
-// With q > 0 the fractions are rounded to multiples of 1/q, as a texture
-// unit's fixed-point filter weights are (q = 256: 8 fractional bits).
-template <bool H16>
-__device__ __forceinline__ float4 lut_bilinear(const float4* lut, const uint2* luth, int hpitch, int rows, int cols,
-                                               int key, int blk, float sx, float sy, float q) {
-  const int pitch = H16 ? hpitch : cols;  // texels per stored row
-  const float fx8 = 8.0f * sx, fy8 = 8.0f * sy;
-  const float x0f = floorf(fx8), y0f = floorf(fy8);
-  float fx = fx8 - x0f, fy = fy8 - y0f;
-  if (q > 0.0f) {
-    fx = rintf(fx * q) / q;
-    fy = rintf(fy * q) / q;
-  }
-  const int xa = min(blk * 9 + (int)x0f, cols - 1), xb = min(xa + 1, cols - 1);
-  const int ya = clampi(key * 9 + (int)y0f, 0, rows - 1), yb = min(ya + 1, rows - 1);
-  const float4 v00 = lut_texel<H16>(lut, luth, (size_t)ya * pitch + xa);
-  const float4 v01 = lut_texel<H16>(lut, luth, (size_t)ya * pitch + xb);
-  const float4 v10 = lut_texel<H16>(lut, luth, (size_t)yb * pitch + xa);
-  const float4 v11 = lut_texel<H16>(lut, luth, (size_t)yb * pitch + xb);
-  const float gx = 1.0f - fx, gy = 1.0f - fy;
-  float4 r;
-  r.x = (v00.x * gx + v01.x * fx) * gy + (v10.x * gx + v11.x * fx) * fy;
-  r.y = (v00.y * gx + v01.y * fx) * gy + (v10.y * gx + v11.y * fx) * fy;
-  r.z = (v00.z * gx + v01.z * fx) * gy + (v10.z * gx + v11.z * fx) * fy;
-  r.w = (v00.w * gx + v01.w * fx) * gy + (v10.w * gx + v11.w * fx) * fy;
-  return r;
+// Texels (4 weights) of a key's half window at each of ravu-zoom's 9 x 9 LUT
+// points, and where texel t of point (row key * 9 + jy, jx) lies:
+//   FP32  as in the file, 9 neighbouring points' texels t side by side (144
+//         bytes): lanes with one key and different phases share a line
+//   FP16  by points, the point's texels side by side and padded to an even count,
+//         so that they come as 16-byte pairs
+// ravu-zoom-r2 / -r3, 1080p to 1.5x: FP16 by points 85 / 171 us against 132 / 217 us
+// as in the file; FP32 by points 121 / 330 us against FP32_FILE us as in the file.
+template <int R>
+__host__ __device__ constexpr int zoom_texels() {
+  return (2 * R * R + 3) / 4;
+}
+template <int R, bool H16>
+__host__ __device__ constexpr uint32_t zoom_texel_at(uint32_t row, uint32_t jx, uint32_t t) {
+  return H16 ? (row * 9 + jx) * ((zoom_texels<R>() + 1) & ~1) + t : (row * zoom_texels<R>() + t) * 9 + jx;
 }
 
-__device__ __forceinline__ float comp4(const float4& v, int i) {
-  return i == 0 ? v.x : (i == 1 ? v.y : (i == 2 ? v.z : v.w));
-}
+// The bilinear (FILTER LINEAR) position of one sub-position in a key's 9 x 9
+// points: x = 8 sx, y = key * 9 + 8 sy (LUTPOS(x, 9) / (blocks, 288),
+// ravu-zoom-r2.hook:23-31); rows clamp to the table's edge.  With q > 0 the
+// fractions are rounded to multiples of 1/q, as a texture unit's fixed-point
+// filter weights are (q = 256: 8 fractional bits).
+struct ZoomLut {
+  uint32_t row[2], col[2];  // rows floor(y), floor(y) + 1; columns floor(x), and the next (at most the
+                            // last one, whose weight is then 0)
+  float w[4];               // weights of (0, 0), (1, 0), (0, 1), (1, 1) (column, row)
+  __device__ __forceinline__ ZoomLut(int rows, int key, float sx, float sy, float q) {
+    const float fx8 = 8.0f * sx, fy8 = 8.0f * sy;
+    const float x0f = floorf(fx8), y0f = floorf(fy8);
+    float fx = fx8 - x0f, fy = fy8 - y0f;
+    if (q > 0.0f) {
+      fx = rintf(fx * q) / q;
+      fy = rintf(fy * q) / q;
+    }
+    col[0] = min((int)x0f, 8);
+    col[1] = min(col[0] + 1, 8u);
+    row[0] = clampi(key * 9 + (int)y0f, 0, rows - 1);
+    row[1] = min((int)row[0] + 1, rows - 1);
+    const float gx = 1.0f - fx, gy = 1.0f - fy;
+    w[0] = gx * gy;
+    w[1] = fx * gy;
+    w[2] = gx * fy;
+    w[3] = fx * fy;
+  }
+  // Texels 2t, 2t+1 of the interpolated point as FP32x2 pairs.
+  template <int R, bool H16>
+  __device__ __forceinline__ void texels(const float4* f, const uint2* h, int t, float2 (&out)[4]) const {
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const uint32_t y = row[k / 2], x = col[k % 2];
+      float4 a, b = make_float4(0.f, 0.f, 0.f, 0.f);
+      if constexpr (H16) {
+        lut_pair_h16(h, zoom_texel_at<R, true>(y, x, 2 * t), a, b);
+      } else {
+        a = __ldg(f + zoom_texel_at<R, false>(y, x, 2 * t));
+        if (2 * t + 1 < zoom_texels<R>()) b = __ldg(f + zoom_texel_at<R, false>(y, x, 2 * t + 1));
+      }
+      const float2 w2 = make_float2(w[k], w[k]);
+      const float2 v[4] = {make_float2(a.x, a.y), make_float2(a.z, a.w), make_float2(b.x, b.y), make_float2(b.z, b.w)};
+#pragma unroll
+      for (int j = 0; j < 4; j++) out[j] = k == 0 ? __fmul2_rn(v[j], w2) : __ffma2_rn(v[j], w2, out[j]);
+    }
+  }
+};
 
 // One thread per OUTPUT pixel; the tile is 32 x TR output pixels and stages the
 // input rectangle they touch (at most (32+N+1) x (TR+N+1) when upscaling;
 // its origin follows from the tile's source positions, as the compute
-// shader's rect, compute/ravu-zoom-ar-r2.hook:28-37): by clamped loads, or
-// (TMA staging, interior rectangles) from one TMA box per plane whose size
-// the host fits to the launch's scale factor (tma_box_of), converting just
-// the rectangle.
+// shader's rect, compute/ravu-zoom-ar-r2.hook:28-37): by quads of columns from
+// the multiple of 4 at or left of the rectangle, or (TMA staging, interior
+// rectangles) from one TMA box per plane whose size the host fits to the
+// launch's scale factor (tma_box_of), converting just the rectangle.
+// ZOOM_NUMS
 template <int R, int CM, bool AR, typename T, bool H16 = false, int TR = 8>
 struct ZoomTile {
   static constexpr int N = 2 * R, S = N * N, LO = R - 1;
   static constexpr int kRows = TR, kThreads = kTileW * TR;
   static constexpr bool kOutputTiles = true;
   static constexpr int RW = kTileW + N + 1, RH = TR + N + 1;
+  static constexpr int RP = (RW + 3 + 3) & ~3;  // row pitch: up to 3 lead columns
   static constexpr int C = CM == kLuma ? 1 : 3;
-  static constexpr int NB = (S / 2 + 3) / 4;  // LUT texels per half window
-  // input rectangle planes, then the source positions of the tile's 32
-  // columns and TR rows
-  static constexpr size_t smem_bytes =
-      (size_t)(C + (CM == kRgb ? 1 : 0)) * RW * RH * 4 + (kTileW + TR) * sizeof(ZoomPos);
+  static constexpr int PL = C + (CM == kRgb ? 1 : 0);
+  static constexpr int NT2 = (zoom_texels<R>() + 1) / 2;  // texel pairs of a LUT point
+  // input rectangle planes, then the source positions of the tile's 32 columns
+  // and TR rows
+  static constexpr size_t kPosAt = (size_t)PL * RP * RH * 4;
+  static constexpr size_t smem_bytes = kPosAt + (kTileW + TR) * sizeof(ZoomPos);
 
   static constexpr int kPlanes = C;
-  static constexpr int kMaxRegs = 0;  // the compiler's own allocation
+  static constexpr int kMaxRegs = PZ_ZOOM_REGS;
   // the largest TMA box: the largest rectangle plus up to 7 lead columns
   static constexpr int kBoxMaxW = (RW + 7 + 7) & ~7, kBoxMaxH = RH;
   using Elem = T;
 
+  // one staged texel: its values, its luma (RGB)
+  __device__ static __forceinline__ void put(float* tile, int at, const float (&v)[C]) {
+#pragma unroll
+    for (int c = 0; c < C; c++) tile[c * RP * RH + at] = v[c];
+    if constexpr (CM == kRgb) tile[C * RP * RH + at] = rgb_luma(v[0], v[1], v[2]);
+  }
+
   __device__ static void run(const RavuArgs& p, int X0, int Y0, float* smem, TmaCtx* tma = nullptr) {
     float* tile = smem;
-    float* ltile = smem + C * RW * RH;
-    ZoomPos* pos = reinterpret_cast<ZoomPos*>(smem + (C + (CM == kRgb ? 1 : 0)) * RW * RH);
+    ZoomPos* pos = reinterpret_cast<ZoomPos*>(reinterpret_cast<unsigned char*>(smem) + kPosAt);
     const int X1 = min(X0 + kTileW - 1, p.OW - 1), Y1 = min(Y0 + TR - 1, p.OH - 1);
     static_assert(kThreads >= kTileW + TR, "one thread per tile column and row");
     if (threadIdx.x < kTileW + TR) {  // one exact position per tile column / row
@@ -804,87 +807,109 @@ struct ZoomTile {
       if (threadIdx.x == 0 && p.err) atomicCAS(p.err, 0, kErrTileOverflow);
       return;
     }
+    const int off = rx & 3;  // the rectangle's first column in the tile
     // every operand of these tests is uniform across the CTA
-    int staged = 0;
     if (tma && tma->map && !tma->dead && rx >= 0 && ry >= 0 && rx + rw <= p.W && ry + rh <= p.H &&
         (rx & 7) + rw <= p.box_w && rh <= p.box_h) {
       const uint32_t pb = ((uint32_t)p.box_w * p.box_h * sizeof(T) + 127u) & ~127u;
-      staged = tma_stage_box<CM, kThreads, T>(p, tma, rx & ~7, ry, p.box_w, p.box_h, pb, rx & 7, rw, rh, RW,
-                                              RW * RH, tile, ltile);
-      if (staged < 0) return;
-    }
-    for (int i = threadIdx.x; !staged && i < rw * rh; i += kThreads) {
-      const int ty = i / rw, tx = i % rw;
-      const int gx = clampi(rx + tx, 0, p.W - 1), gy = clampi(ry + ty, 0, p.H - 1);
-      float v[3] = {0.f, 0.f, 0.f};
+      tma_issue_box<CM, T>(tma, rx & ~7, ry, p.box_w, p.box_h, pb);
+      if (!tma_wait_box(p, tma)) return;
+      for (int i = threadIdx.x; i < rw * rh; i += kThreads) {
+        const int ty = i / rw, tx = i % rw;
+        float v[C];
+#pragma unroll
+        for (int c = 0; c < C; c++)
+          v[c] = lds_f(reinterpret_cast<const T*>(tma->raw + c * pb) + ty * p.box_w + tx + (rx & 7));
+        put(tile, ty * RP + tx + off, v);
+      }
+    } else {
+      // loads of all planes first, then values, powers and luma
+      constexpr int QW = RP / 4, IT = (QW * RH + kThreads - 1) / kThreads;
+      Quad<T> q[C][IT];
+      auto each = [&](auto f) {
+#pragma unroll
+        for (int k = 0; k < IT; k++) {
+          const int i = threadIdx.x + k * kThreads, ty = i / QW, tx = i % QW * 4;
+          if (ty < rh && tx < off + rw) f(k, ty, tx);
+        }
+      };
 #pragma unroll
       for (int c = 0; c < C; c++) {
-        v[c] = ldp(static_cast<const T*>(p.in[c]) + (size_t)gy * p.in_pitch[c] + gx);
-        tile[c * RW * RH + ty * RW + tx] = v[c];
+        const T* in = static_cast<const T*>(p.in[c]);
+        const int pitch = p.in_pitch[c];
+        const bool aligned = quads_aligned(in, pitch);
+        each([&](int k, int ty, int tx) {
+          load_quad(q[c][k], in + (size_t)clampi(ry + ty, 0, p.H - 1) * pitch, rx - off + tx, p.W, aligned);
+        });
       }
-      if (CM == kRgb) ltile[ty * RW + tx] = rgb_luma(v[0], v[1], v[2]);
+      each([&](int k, int ty, int tx) {
+        float4 v[C];
+#pragma unroll
+        for (int c = 0; c < C; c++) v[c] = q[c][k].get();
+        float4* t4 = reinterpret_cast<float4*>(tile + ty * RP + tx);
+#pragma unroll
+        for (int c = 0; c < C; c++) t4[c * (RP * RH / 4)] = v[c];
+        if constexpr (CM == kRgb)
+          t4[C * (RP * RH / 4)] = make_float4(rgb_luma(v[0].x, v[1].x, v[2].x), rgb_luma(v[0].y, v[1].y, v[2].y),
+                                              rgb_luma(v[0].z, v[1].z, v[2].z), rgb_luma(v[0].w, v[1].w, v[2].w));
+      });
     }
     __syncthreads();
     const int X = X0 + threadIdx.x % kTileW, Y = Y0 + threadIdx.x / kTileW;
     if (X >= p.OW || Y >= p.OH) return;
     const ZoomPos px = pos[threadIdx.x % kTileW], py = pos[kTileW + threadIdx.x / kTileW];
-    const int bx = px.i - LO - rx, by = py.i - LO - ry;  // window origin in the tile
-    auto val = [&](int c, int k) { return tile[c * RW * RH + (by + k % N) * RW + bx + k / N]; };
-    auto lum = [&](int kx, int ky) {
-      return CM == kRgb ? ltile[(by + ky) * RW + bx + kx] : tile[(by + ky) * RW + bx + kx];
-    };
+    const int at = (py.i - LO - ry) * RP + px.i - LO - rx + off;  // window origin in the tile
+    const float* base = tile + at;
+    auto val = [&](int c, int k) { return base[c * RP * RH + k % N * RP + k / N]; };
+    auto lum = [&](int kx, int ky) { return base[(CM == kRgb ? C * RP * RH : 0) + ky * RP + kx]; };
     float a, b, d;
     structure_tensor<N, true>(lum, p.kp, a, b, d);
     const int key = ravu_key(a, b, d, p.kp);  // no +0.5 row centring (ravu-zoom-r2.hook:124)
     if (p.keys) p.keys[(size_t)Y * p.OW + X] = key;
-    const float sx = px.s, sy = py.s, ix = 1.0f - sx, iy = 1.0f - sy;
-    // anti-ringing sums per channel as FP32x2 pairs (hi, lo) and (hi2, lo2)
-    float res[C];
-    float2 HL[C], HL3[C];
+    const ZoomLut ls(p.lut_rows, key, px.s, py.s, p.lut_frac);
+    const ZoomLut li(p.lut_rows, key, 1.0f - px.s, 1.0f - py.s, p.lut_frac);
+    // taps i, i+1 in the lanes of res; anti-ringing sums per channel (ar_finish)
+    float2 res[C], G[C], M[C];
 #pragma unroll
-    for (int c = 0; c < C; c++) {
-      res[c] = 0.0f;
-      HL[c] = HL3[c] = make_float2(0.0f, 0.0f);
-    }
+    for (int c = 0; c < C; c++) res[c] = G[c] = M[c] = make_float2(0.0f, 0.0f);
 #pragma unroll
-    for (int blk = 0; blk < NB; blk++) {
-      const float4 ws = lut_bilinear<H16>(p.lut, p.lut_h, p.lut_h_pitch, p.lut_rows, p.lut_cols, key, blk, sx, sy, p.lut_frac);
-      const float4 wi = lut_bilinear<H16>(p.lut, p.lut_h, p.lut_h_pitch, p.lut_rows, p.lut_cols, key, blk, ix, iy, p.lut_frac);
-      float4 as = make_float4(0.f, 0.f, 0.f, 0.f), ai = as;
+    for (int t = 0; t < NT2; t++) {
+      float2 ws[4], wi[4], gs[4], gi[4];
+      ls.texels<R, H16>(p.lut, p.lut_h, t, ws);
+      li.texels<R, H16>(p.lut, p.lut_h, t, wi);
       if (AR) {  // the anti-ringing LUT stays FP32 in every form but mpv's (most of
                  // its values lie below FP16's normal range)
-        as = lut_bilinear<false>(p.lut_ar, nullptr, 0, p.lut_rows, p.lut_cols, key, blk, sx, sy, p.lut_frac);
-        ai = lut_bilinear<false>(p.lut_ar, nullptr, 0, p.lut_rows, p.lut_cols, key, blk, ix, iy, p.lut_frac);
+        ls.texels<R, false>(p.lut_ar, nullptr, t, gs);
+        li.texels<R, false>(p.lut_ar, nullptr, t, gi);
       }
 #pragma unroll
       for (int j = 0; j < 4; j++) {
-        const int i = blk * 4 + j;
-        if (i < S / 2) {
-          const int k2 = S - 1 - i;
+        const int i = t * 8 + 2 * j;
+        if (i >= S / 2) break;  // S / 2 is even
 #pragma unroll
-          for (int c = 0; c < C; c++) {
-            const float va = val(c, i), vb = val(c, k2);
-            res[c] += va * comp4(ws, j);
-            res[c] += vb * comp4(wi, j);
-            if (AR) {
-              float2 pa, pa3, pb, pb3;
-              ar_pow2(va, pa, pa3);
-              ar_pow2(vb, pb, pb3);
-              const float2 wa = make_float2(comp4(as, j), comp4(as, j));
-              const float2 wb = make_float2(comp4(ai, j), comp4(ai, j));
-              HL[c] = __ffma2_rn(pa, wa, HL[c]);
-              HL[c] = __ffma2_rn(pb, wb, HL[c]);
-              HL3[c] = __ffma2_rn(pa3, wa, HL3[c]);
-              HL3[c] = __ffma2_rn(pb3, wb, HL3[c]);
-            }
+        for (int c = 0; c < C; c++) {
+          const float va[2] = {val(c, i), val(c, i + 1)}, vb[2] = {val(c, S - 1 - i), val(c, S - 2 - i)};
+          res[c] = __ffma2_rn(make_float2(va[0], va[1]), ws[j], res[c]);
+          res[c] = __ffma2_rn(make_float2(vb[0], vb[1]), wi[j], res[c]);
+          if constexpr (AR) {
+            auto tap = [&](float v, float g) {
+              const float2 h = ar_pow32(v);
+              G[c] = __ffma2_rn(h, make_float2(g, g), G[c]);
+              M[c] = __ffma2_rn(__fmul2_rn(h, make_float2(v, v)), make_float2(g, g), M[c]);
+            };
+            tap(va[0], gs[j].x);
+            tap(va[1], gs[j].y);
+            tap(vb[0], gi[j].x);
+            tap(vb[1], gi[j].y);
           }
         }
       }
     }
 #pragma unroll
     for (int c = 0; c < C; c++) {
-      const float v = AR ? ar_finish(res[c], HL[c].y, HL[c].x, HL3[c].y, HL3[c].x, p.ar) : clampf(res[c], 0.f, 1.f);
-      stp(static_cast<T*>(p.out[c]) + (size_t)Y * p.out_pitch[c] + X, v);
+      const float r = res[c].x + res[c].y;
+      stp(static_cast<T*>(p.out[c]) + (size_t)Y * p.out_pitch[c] + X,
+          AR ? ar_finish(r, G[c], M[c], p.ar) : clampf(r, 0.f, 1.f));
     }
   }
 };
@@ -921,12 +946,26 @@ __global__ void __maxnreg__(Prog::kMaxRegs) tile_kernel_mr(const __grid_constant
   tile_body<Prog, TMA>(p, maps);
 }
 
-template <class Prog, bool TMA>
-void launch_tile_kernel(dim3 grid, size_t smem, cudaStream_t s, const RavuArgs& a, const TmaMaps& maps) {
-  if constexpr (Prog::kMaxRegs > 0)
-    tile_kernel_mr<Prog, TMA><<<grid, Prog::kThreads, smem, s>>>(a, maps);
-  else
-    tile_kernel<Prog, TMA><<<grid, Prog::kThreads, smem, s>>>(a, maps);
+// SMEM: bytes of dynamic shared memory.  Above 48 KB (ravu-zoom-ar of three
+// channels at 16 rows) the kernel is opted in once per device; two threads that
+// do so at once set the same value.
+template <class Prog, bool TMA, size_t SMEM>
+int launch_tile_kernel(dim3 grid, cudaStream_t s, const RavuArgs& a, const TmaMaps& maps) {
+  auto kern = [] {
+    if constexpr (Prog::kMaxRegs > 0) return tile_kernel_mr<Prog, TMA>;
+    else return tile_kernel<Prog, TMA>;
+  }();
+  if constexpr (SMEM > 48 * 1024) {
+    static std::atomic<bool> opted[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -95;
+    if (!opted[dev].load(std::memory_order_relaxed)) {
+      if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM) != cudaSuccess) return -5;
+      opted[dev].store(true, std::memory_order_relaxed);
+    }
+  }
+  kern<<<grid, Prog::kThreads, SMEM, s>>>(a, maps);
+  return 0;
 }
 
 bool encode_plane_map(CUtensorMap* map, const void* base, int W, int H, int pitch, int dtype, int box_w,
@@ -984,7 +1023,6 @@ bool encode_tma(RavuArgs* a, TmaMaps* maps) {
 // programs), staged by TMA when the frame asks for it and its planes map.
 template <class Prog>
 int launch_tiles(const RavuArgs& a, cudaStream_t s) {
-  static_assert(Prog::smem_bytes <= 48 * 1024, "tile program needs more than the default shared memory");
   const int fw = Prog::kOutputTiles ? a.OW : a.W, fh = Prog::kOutputTiles ? a.OH : a.H;
   const int tiles_w = (fw + kTileW - 1) / kTileW, tiles_h = (fh + Prog::kRows - 1) / Prog::kRows;
   TmaMaps maps;
@@ -993,13 +1031,10 @@ int launch_tiles(const RavuArgs& a, cudaStream_t s) {
     RavuArgs b = a;
     if (a.staging == 1 && encode_tma<Prog>(&b, &maps)) {
       constexpr size_t smem = ((Prog::smem_bytes + 127) & ~(size_t)127) + tma_landing_bytes<Prog>();
-      static_assert(smem <= 48 * 1024, "TMA staging needs more than the default shared memory");
-      launch_tile_kernel<Prog, true>(dim3(tiles_w, tiles_h), smem, s, b, maps);
-      return 0;
+      return launch_tile_kernel<Prog, true, smem>(dim3(tiles_w, tiles_h), s, b, maps);
     }
   }
-  launch_tile_kernel<Prog, false>(dim3(tiles_w, tiles_h), Prog::smem_bytes, s, a, maps);
-  return 0;
+  return launch_tile_kernel<Prog, false, Prog::smem_bytes>(dim3(tiles_w, tiles_h), s, a, maps);
 }
 
 // ------------------------------------------------------ persistent batches ---
