@@ -177,6 +177,13 @@ int pz_query(const pz_model* model, int in_width, int in_height, int dtype, cons
 /* Device scratch bytes pz_run needs for this model/input (0 if none). */
 size_t pz_scratch_bytes(const pz_model* model, const pz_plane* in, const pz_opts* opts);
 
+/* The scratch with which pz_run runs fastest and allocates nothing: what
+ * pz_scratch_bytes says, and for a ravu-zoom whose scale has few phases (1.5x,
+ * 1.75x, 2.25x; clamped-load staging) room for every key's interpolated weights
+ * at every phase, 16-byte aligned.  Without it such a zoom interpolates per
+ * pixel; the pixels are the same.  Host-only: no device call. */
+size_t pz_scratch_wanted(const pz_model* model, int in_width, int in_height, int dtype, const pz_opts* opts);
+
 /* Run the full hook chain of `model` on one frame.  n_in/n_out planes are
  * 1 (luma) or 3 (yuv/rgb, planar).  Output sizes: 2x (lite, ravu, nnedi3),
  * 3x (3x), or opts->out_width x out_height (zoom).  ravu-lite, ravu and the

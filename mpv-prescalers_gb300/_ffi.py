@@ -82,6 +82,8 @@ EXPORTS = {
     "pz_model_create": (ctypes.c_int, [ctypes.POINTER(ModelDesc), ctypes.POINTER(ctypes.c_void_p)]),
     "pz_model_destroy": (None, [ctypes.c_void_p]),
     "pz_scratch_bytes": (ctypes.c_size_t, [ctypes.c_void_p, ctypes.POINTER(Plane), ctypes.POINTER(Opts)]),
+    "pz_scratch_wanted": (ctypes.c_size_t, [ctypes.c_void_p, ctypes.c_int, ctypes.c_int, ctypes.c_int,
+                                            ctypes.POINTER(Opts)]),
     "pz_query": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.POINTER(Opts),
                                 ctypes.POINTER(QueryResult)]),
     "pz_run": (ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(Plane), ctypes.c_int, ctypes.POINTER(Plane),

@@ -69,6 +69,10 @@ __global__ void wait_selftest_kernel(int* err, unsigned long long limit_ns) {
     atomicCAS(err, 0, pz::kErrWaitTimeout);
 }
 
+size_t zoom_table_size(const pz_model* m, int W, int H, int OW, int OH, int* px, int* py) {
+  return pz::zoom_table_bytes(m->radius, m->ar != 0.0f, m->lut_rows / 9, W, H, OW, OH, px, py);
+}
+
 // `pairs`: the plane is written with 2-wide vector stores, so its base and
 // pitch must keep every even column 2-element aligned.
 int check_plane(const pz_plane& p, const char* what, int idx, bool pairs) {
@@ -469,6 +473,14 @@ size_t pz_scratch_bytes(const pz_model* m, const pz_plane* in, const pz_opts* o)
   return (size_t)2 * in->height * in->width * dtype_size(in->dtype);
 }
 
+size_t pz_scratch_wanted(const pz_model* m, int in_w, int in_h, int dtype, const pz_opts* o) {
+  pz_query_result q;
+  if (pz_query(m, in_w, in_h, dtype, o, &q)) return 0;
+  if (m->family != PZ_RAVU_ZOOM || o->staging) return q.scratch_bytes;
+  int px, py;
+  return zoom_table_size(m, in_w, in_h, q.out_width, q.out_height, &px, &py);
+}
+
 int pz_run(const pz_model* m, const pz_plane* in, int n_in, pz_plane* out, int n_out, const pz_opts* o,
            void* stream) {
   if (!m || !in || !out) return fail(PZ_EINVAL, "null argument");
@@ -583,7 +595,17 @@ int pz_run(const pz_model* m, const pz_plane* in, int n_in, pz_plane* out, int n
       case PZ_RAVU_LITE: rc = pz::launch_lite(a, m->radius, m->ar != 0.0f, dt, s); break;
       case PZ_RAVU_3X: rc = pz::launch_3x(a, m->radius, m->channels, dt, s); break;
       case PZ_RAVU: rc = pz::launch_lattice(a, m->radius, m->channels, dt, s); break;
-      case PZ_RAVU_ZOOM: rc = pz::launch_zoom(a, m->radius, m->channels, m->ar != 0.0f, dt, s); break;
+      case PZ_RAVU_ZOOM:
+        // with scratch for it, the weights of a scale of few phases are formed once
+        if (o->scratch && !a.staging && reinterpret_cast<uintptr_t>(o->scratch) % 16 == 0) {
+          const size_t need = zoom_table_size(m, W, H, OW, OH, &a.zpx, &a.zpy);
+          if (need && o->scratch_bytes >= need) {
+            if (!o->tile_rows) a.tile_rows = 4;
+            a.ztab = static_cast<const float4*>(o->scratch);
+            pz::launch_zoom_table(a, m->radius, m->ar != 0.0f, s);
+          }
+        }
+        rc = pz::launch_zoom(a, m->radius, m->channels, m->ar != 0.0f, dt, s); break;
       default: rc = PZ_EINVAL;
     }
     if (own_i11) cudaFreeAsync(a.i11, s);

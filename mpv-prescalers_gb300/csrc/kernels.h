@@ -30,6 +30,8 @@ struct RavuArgs {
   const uint2* lut_h;  // fast form: the LUT as FP16 texels (4 halves each), or null
   int lut_h_pitch;     // texels per FP16 LUT row (lut_cols rounded up to even)
   int box_w, box_h;    // ravu-zoom TMA staging: the box of this launch's tensor maps (texels x rows)
+  const float4* ztab;  // ravu-zoom: every key's weights at every phase of the scale (zoom_table_kernel), or null
+  int zpx, zpy;        // phases per axis: out / gcd(in, out)
   float* i11;          // ravu lattice: int11 plane, FP32 [C][H][W] (scratch)
   int i11_half;        // round int11 to FP16 before storing it (the mpv form)
   KeyParams kp;
@@ -57,6 +59,10 @@ int launch_lite(const RavuArgs& a, int radius, bool ar, int dtype, cudaStream_t 
 int launch_3x(const RavuArgs& a, int radius, int chmode, int dtype, cudaStream_t s);
 int launch_lattice(const RavuArgs& a, int radius, int chmode, int dtype, cudaStream_t s);
 int launch_zoom(const RavuArgs& a, int radius, int chmode, bool ar, int dtype, cudaStream_t s);
+// ravu-zoom's weight table for a scale of few phases: its bytes (0: too many
+// phases for the frame), and the launch that fills a.ztab.
+size_t zoom_table_bytes(int radius, bool ar, int keys, int W, int H, int OW, int OH, int* px, int* py);
+int launch_zoom_table(const RavuArgs& a, int radius, bool ar, cudaStream_t s);
 int launch_nnedi3_simt(const NnArgs& a, bool xpass, int dtype, cudaStream_t s);
 int launch_nnedi3_tc(const NnArgs& a, bool xpass, int dtype, cudaStream_t s);
 int launch_nnedi3_split(const NnArgs& a, bool xpass, int dtype, cudaStream_t s);

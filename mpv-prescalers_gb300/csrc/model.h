@@ -72,10 +72,11 @@ inline void select_lut(const pz_model* m, int precision, RavuArgs* a) {
 // the fastest on GB300 at 480p-1080p (1080p, fast form, 4 / 8 rows: ravu-r2 60.5
 // / 58.4 us, ravu-r3 78.8 / 79.7, ravu-r4 208.7 / 215.0, ravu-r4-yuv 279.7 /
 // 279.6, ravu-lite-r3 31.8 / 33.5, ravu-lite-ar-r4 76.9 / 76.9, ravu-3x-r3 45.2 /
-// 47.0; 16 rows is slower for every program).
+// 47.0, ravu-zoom-r3 at 1.5x 334 / 283 FP32; 16 rows is slower for every program).
 inline int default_tile_rows(const pz_model* m) {
   if (m->family == PZ_RAVU_LITE && (m->radius == 2 || (m->radius == 4 && m->ar != 0.0f))) return 8;
   if (m->family == PZ_RAVU && m->radius == 2 && m->channels == PZ_LUMA) return 8;
+  if (m->family == PZ_RAVU_ZOOM && m->radius == 3) return 8;
   return 4;
 }
 

@@ -26,9 +26,6 @@
 #include "async.cuh"
 #include "kernels.h"
 
-#ifndef PZ_ZOOM_REGS
-#define PZ_ZOOM_REGS 0
-#endif
 namespace pz {
 
 // Tile width in pixels (one warp per tile row); persistent batches run tiles
@@ -290,11 +287,15 @@ struct LiteTile {
   static constexpr bool kOutputTiles = false;
   static constexpr int TW = kTilePitch, TH = TR + N - 1;
   // the value tile and (AR) each texel's two 32nd powers, formed while staging
-  // and read as 8 bytes a tap: TABLE_NUMS
+  // and read as 8 bytes a tap (1080p, 4-row tiles: r3 fast 54.1 us, formed per tap
+  // 57.0; r4 fast 74.9 and 76.0; r2 39.8 and 41.8).  With FP32 texels, whose
+  // gathers already fill L1, r3 and r4 lose by it (57.0 us without, 61.0 with; 93
+  // and 102) and form them per tap
   static constexpr bool kTable = AR && (H16 || R == 2);
   static constexpr size_t smem_bytes = (size_t)TW * TH * (kTable ? 12 : 4);
 
   static constexpr int kPlanes = 1;
+  static constexpr bool kTma = true;
   // ravu-lite-ar-r4 at <= 48 registers (5 CTAs of 8 rows per SM) measured
   // 2 % faster; the other radii lose more to spills than they gain
   static constexpr int kMaxRegs = (R == 4 && AR) ? 48 : 0;
@@ -390,6 +391,7 @@ struct ThreeXTile {
   static constexpr int C = CM == kLuma ? 1 : 3;
   static constexpr size_t smem_bytes = (size_t)(C + (CM == kRgb ? 1 : 0)) * TW * TH * 4;
   static constexpr int kPlanes = C;
+  static constexpr bool kTma = true;
   static constexpr int kMaxRegs = 0;  // the compiler's own allocation
   using Elem = T;
 
@@ -501,6 +503,7 @@ struct Int11Tile {
   static constexpr int TW = kTilePitch, TH = TR + N - 1;
   static constexpr size_t smem_bytes = (size_t)(C + (CM == kRgb ? 1 : 0)) * TW * TH * 4;
   static constexpr int kPlanes = C;
+  static constexpr bool kTma = true;
   // r3 luma at 56 registers (of 66) is 1 % faster; the others lose by any cap
   static constexpr int kMaxRegs = R == 3 && CM == kLuma ? 56 : 0;
   using Elem = T;
@@ -604,6 +607,7 @@ struct LatticeTile {
   static constexpr int PL = C + (CM == kRgb ? 1 : 0);  // planes per tile set
   static constexpr size_t smem_bytes = (size_t)2 * PL * TW * TH * 4;
   static constexpr int kPlanes = C;
+  static constexpr bool kTma = true;
   // luma at r2 / r3 is 2-4 % faster under these caps (of 44 / 60 registers);
   // r4 and three channels lose by any (r3-yuv at 40: 162 against 126 us)
   static constexpr int kMaxRegs = CM == kLuma && R <= 3 ? (R == 2 ? 40 : 48) : 0;
@@ -697,7 +701,7 @@ __device__ __forceinline__ ZoomPos zoom_pos(int X, int W, int OW) {
 //   FP16  by points, the point's texels side by side and padded to an even count,
 //         so that they come as 16-byte pairs
 // ravu-zoom-r2 / -r3, 1080p to 1.5x: FP16 by points 85 / 171 us against 132 / 217 us
-// as in the file; FP32 by points 121 / 330 us against FP32_FILE us as in the file.
+// as in the file; FP32 by points 121 / 330 us against 135 / 283 us as in the file.
 template <int R>
 __host__ __device__ constexpr int zoom_texels() {
   return (2 * R * R + 3) / 4;
@@ -716,6 +720,7 @@ struct ZoomLut {
   uint32_t row[2], col[2];  // rows floor(y), floor(y) + 1; columns floor(x), and the next (at most the
                             // last one, whose weight is then 0)
   float w[4];               // weights of (0, 0), (1, 0), (0, 1), (1, 1) (column, row)
+  __device__ __forceinline__ ZoomLut() {}
   __device__ __forceinline__ ZoomLut(int rows, int key, float sx, float sy, float q) {
     const float fx8 = 8.0f * sx, fy8 = 8.0f * sy;
     const float x0f = floorf(fx8), y0f = floorf(fy8);
@@ -755,6 +760,39 @@ struct ZoomLut {
   }
 };
 
+// float4 of one half window's weights in the phase table; an entry holds the
+// two halves, then (AR) the anti-ringing weights' two.
+template <int R, bool AR>
+__host__ __device__ constexpr uint32_t zoom_entry() {
+  return zoom_texels<R>() * (AR ? 4 : 2);
+}
+
+// The weights of every key at every phase of a scale whose output positions
+// repeat after few pixels (1.5x: 3 x 3 phases; 2.25x: 9 x 9), [key][phase y]
+// [phase x][entry]: the same bilinear fetches as a pixel's own, once per launch
+// instead of once per pixel.  One thread per entry and texel pair.
+template <int R, bool AR, bool H16>
+__global__ void zoom_table_kernel(const __grid_constant__ RavuArgs p, float4* out) {
+  constexpr int NB = zoom_texels<R>(), NT2 = (NB + 1) / 2, PER = NT2 * (AR ? 4 : 2);
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int n = p.lut_rows / 9 * p.zpx * p.zpy;
+  if (i >= n * PER) return;
+  const int entry = i / PER, t = i % PER % NT2, part = i % PER / NT2;  // part: halves, then the AR halves
+  const int key = entry / (p.zpx * p.zpy), phase = entry % (p.zpx * p.zpy);
+  float sx = zoom_pos(phase % p.zpx, p.W, p.OW).s, sy = zoom_pos(phase / p.zpx, p.H, p.OH).s;
+  if (part & 1) {
+    sx = 1.0f - sx;
+    sy = 1.0f - sy;
+  }
+  const ZoomLut l(p.lut_rows, key, sx, sy, p.lut_frac);
+  float2 w[4];
+  if (part < 2) l.texels<R, H16>(p.lut, p.lut_h, t, w);
+  else l.texels<R, false>(p.lut_ar, nullptr, t, w);
+  float4* o = out + (size_t)entry * zoom_entry<R, AR>() + part * NB + 2 * t;
+  o[0] = make_float4(w[0].x, w[0].y, w[1].x, w[1].y);
+  if (2 * t + 1 < NB) o[1] = make_float4(w[2].x, w[2].y, w[3].x, w[3].y);
+}
+
 // One thread per OUTPUT pixel; the tile is 32 x TR output pixels and stages the
 // input rectangle they touch (at most (32+N+1) x (TR+N+1) when upscaling;
 // its origin follows from the tile's source positions, as the compute
@@ -762,8 +800,12 @@ struct ZoomLut {
 // the multiple of 4 at or left of the rectangle, or (TMA staging, interior
 // rectangles) from one TMA box per plane whose size the host fits to the
 // launch's scale factor (tma_box_of), converting just the rectangle.
-// ZOOM_NUMS
-template <int R, int CM, bool AR, typename T, bool H16 = false, int TR = 8>
+// Bound by L1, where the gathers of LUT texels go (86 %; 16-40 loads a pixel).
+// 1080p to 1.5x, without / with the phase table: ravu-zoom-r2 86 / 76 us fast (132
+// with a load per texel, scalar blends and texel staging), r3 FP32 283 / 121 us
+// (290), ravu-zoom-ar-r2-rgb fast 274 / 203 us (302).
+// TAB: the weights come from the launch's phase table, at the same bits.
+template <int R, int CM, bool AR, typename T, bool H16 = false, int TR = 8, bool TAB = false>
 struct ZoomTile {
   static constexpr int N = 2 * R, S = N * N, LO = R - 1;
   static constexpr int kRows = TR, kThreads = kTileW * TR;
@@ -779,7 +821,10 @@ struct ZoomTile {
   static constexpr size_t smem_bytes = kPosAt + (kTileW + TR) * sizeof(ZoomPos);
 
   static constexpr int kPlanes = C;
-  static constexpr int kMaxRegs = PZ_ZOOM_REGS;
+  static constexpr bool kTma = !TAB;  // the table goes with plain loads
+  // anti-ringing on FP32 texels: 4-8 % faster at 80 registers (of 96-126); any
+  // cap costs the other programs
+  static constexpr int kMaxRegs = AR && !H16 && !TAB ? 80 : 0;
   // the largest TMA box: the largest rectangle plus up to 7 lead columns
   static constexpr int kBoxMaxW = (RW + 7 + 7) & ~7, kBoxMaxH = RH;
   using Elem = T;
@@ -798,7 +843,9 @@ struct ZoomTile {
     static_assert(kThreads >= kTileW + TR, "one thread per tile column and row");
     if (threadIdx.x < kTileW + TR) {  // one exact position per tile column / row
       const int t = threadIdx.x;
-      pos[t] = t < kTileW ? zoom_pos(min(X0 + t, X1), p.W, p.OW) : zoom_pos(min(Y0 + t - kTileW, Y1), p.H, p.OH);
+      const int o = t < kTileW ? min(X0 + t, X1) : min(Y0 + t - kTileW, Y1);
+      pos[t] = t < kTileW ? zoom_pos(o, p.W, p.OW) : zoom_pos(o, p.H, p.OH);
+      if (TAB) pos[t].s = __int_as_float(t < kTileW ? o % p.zpx : o % p.zpy);  // its phase instead
     }
     __syncthreads();
     const int rx = pos[0].i - LO, ry = pos[kTileW].i - LO;
@@ -866,8 +913,32 @@ struct ZoomTile {
     structure_tensor<N, true>(lum, p.kp, a, b, d);
     const int key = ravu_key(a, b, d, p.kp);  // no +0.5 row centring (ravu-zoom-r2.hook:124)
     if (p.keys) p.keys[(size_t)Y * p.OW + X] = key;
-    const ZoomLut ls(p.lut_rows, key, px.s, py.s, p.lut_frac);
-    const ZoomLut li(p.lut_rows, key, 1.0f - px.s, 1.0f - py.s, p.lut_frac);
+    // the weights of taps 8t .. 8t+7 of a half window (0: from the front, 1: the
+    // mirrored taps from the back; +2: anti-ringing) as pairs
+    constexpr int NB = zoom_texels<R>();
+    const float4* entry = nullptr;
+    ZoomLut ls, li;
+    if constexpr (TAB) {
+      const int k = clampi(key, 0, p.lut_rows / 9 - 1) * p.zpy + __float_as_int(py.s);
+      entry = p.ztab + ((size_t)k * p.zpx + __float_as_int(px.s)) * zoom_entry<R, AR>();
+    } else {
+      ls = ZoomLut(p.lut_rows, key, px.s, py.s, p.lut_frac);
+      li = ZoomLut(p.lut_rows, key, 1.0f - px.s, 1.0f - py.s, p.lut_frac);
+    }
+    auto weights = [&](int part, int t, float2 (&w)[4]) {
+      if constexpr (TAB) {
+        const float4 a = __ldg(entry + part * NB + 2 * t);
+        const float4 b = 2 * t + 1 < NB ? __ldg(entry + part * NB + 2 * t + 1) : a;
+        w[0] = make_float2(a.x, a.y);
+        w[1] = make_float2(a.z, a.w);
+        w[2] = make_float2(b.x, b.y);
+        w[3] = make_float2(b.z, b.w);
+      } else {
+        const ZoomLut& l = part & 1 ? li : ls;
+        if (part < 2) l.texels<R, H16>(p.lut, p.lut_h, t, w);
+        else l.texels<R, false>(p.lut_ar, nullptr, t, w);
+      }
+    };
     // taps i, i+1 in the lanes of res; anti-ringing sums per channel (ar_finish)
     float2 res[C], G[C], M[C];
 #pragma unroll
@@ -875,12 +946,12 @@ struct ZoomTile {
 #pragma unroll
     for (int t = 0; t < NT2; t++) {
       float2 ws[4], wi[4], gs[4], gi[4];
-      ls.texels<R, H16>(p.lut, p.lut_h, t, ws);
-      li.texels<R, H16>(p.lut, p.lut_h, t, wi);
+      weights(0, t, ws);
+      weights(1, t, wi);
       if (AR) {  // the anti-ringing LUT stays FP32 in every form but mpv's (most of
                  // its values lie below FP16's normal range)
-        ls.texels<R, false>(p.lut_ar, nullptr, t, gs);
-        li.texels<R, false>(p.lut_ar, nullptr, t, gi);
+        weights(2, t, gs);
+        weights(3, t, gi);
       }
 #pragma unroll
       for (int j = 0; j < 4; j++) {
@@ -1027,7 +1098,7 @@ int launch_tiles(const RavuArgs& a, cudaStream_t s) {
   const int tiles_w = (fw + kTileW - 1) / kTileW, tiles_h = (fh + Prog::kRows - 1) / Prog::kRows;
   TmaMaps maps;
   std::memset(&maps, 0, sizeof maps);
-  if constexpr (Prog::kPlanes > 0) {
+  if constexpr (Prog::kTma) {
     RavuArgs b = a;
     if (a.staging == 1 && encode_tma<Prog>(&b, &maps)) {
       constexpr size_t smem = ((Prog::smem_bytes + 127) & ~(size_t)127) + tma_landing_bytes<Prog>();

@@ -7,11 +7,18 @@
 
 namespace pz {
 
+template <int R, int CM, bool AR, typename T, bool H16, int TR>
+int launch_zoom_one(const RavuArgs& a, cudaStream_t s) {
+  // the table's weights serve either form: they are FP32 once interpolated
+  if (a.ztab) return launch_tiles<ZoomTile<R, CM, AR, T, false, TR, true>>(a, s);
+  return launch_tiles<ZoomTile<R, CM, AR, T, H16, TR>>(a, s);
+}
+
 template <typename T, bool H16, int TR>
 int launch_zoom_t(const RavuArgs& a, int radius, int cm, bool ar, cudaStream_t s) {
-#define PZ_Z(R, CM)                                                     \
-  return ar ? launch_tiles<ZoomTile<R, CM, true, T, H16, TR>>(a, s)     \
-            : launch_tiles<ZoomTile<R, CM, false, T, H16, TR>>(a, s)
+#define PZ_Z(R, CM)                                              \
+  return ar ? launch_zoom_one<R, CM, true, T, H16, TR>(a, s)     \
+            : launch_zoom_one<R, CM, false, T, H16, TR>(a, s)
 #define PZ_Z_CM(R)                  \
   if (cm == kLuma) PZ_Z(R, kLuma);  \
   else if (cm == kYuv) PZ_Z(R, kYuv); \

@@ -340,8 +340,12 @@ class HookModel:
             keys = None
             if return_keys:
                 keys = torch.empty(self.key_shape(W, H, OW, OH), dtype=torch.int32, device=dev)
+            scratch = None
+            if self.family == "zoom":   # room for the weights of every phase, where the scale has few
+                n = self._scratch_wanted(W, H, pl[0], OW, OH, precision, staging)
+                scratch = torch.empty(n, dtype=torch.uint8, device=dev) if n else None
             self.run_raw(pl, res, out_size=(OW, OH), precision=precision, keys=keys, stream=stream,
-                         staging=staging, tile_rows=tile_rows)
+                         scratch=scratch, staging=staging, tile_rows=tile_rows)
             return self._pack(res, planes, as_list, keys, return_keys, full)
 
     def upscale_host(self, frames, out=None, out_size: Optional[Tuple[int, int]] = None, precision: str = "fp32",
@@ -451,6 +455,16 @@ class HookModel:
                 if k is None:
                     break
                 del pool[k]
+
+    def _scratch_wanted(self, W, H, plane, OW, OH, precision, staging) -> int:
+        """``pz_scratch_wanted`` of one frame."""
+        o = _ffi.Opts()
+        o.precision = PRECISIONS[precision]
+        o.out_width, o.out_height = OW, OH
+        o.staging = STAGINGS[staging or self.default_staging]
+        dt = _ffi.PZ_F32 if plane.element_size() == 4 else _ffi.PZ_F16
+        return int(_ffi.lib().pz_scratch_wanted(self.device_handle(plane.device.index), W, H, dt,
+                                                _ffi.ctypes.byref(o)))
 
     def key_shape(self, W, H, OW, OH):
         fam = self.family

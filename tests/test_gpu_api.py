@@ -225,6 +225,42 @@ def test_zoom_tma_rectangles_give_identical_pixels(name, osz, prec, dtype):
         assert torch.equal(hm.upscale(x, out_size=osz, precision=prec, staging="tma", tile_rows=rows), want), rows
 
 
+@pytest.mark.parametrize("name", ["ravu-zoom-r2", "ravu-zoom-r3-yuv", "ravu-zoom-ar-r2-rgb", "ravu-zoom-ar-r3"])
+@pytest.mark.parametrize("size,osz,table", [((721, 487), (1442, 974), True), ((720, 486), (1080, 729), True),
+                                            ((640, 484), (1120, 847), True), ((960, 400), (1200, 800), True),
+                                            ((640, 360), (960, 540), False), ((853, 479), (1501, 843), False)],
+                         ids=["2x", "1.5x", "1.75x", "1.25x2x", "small", "no-ratio"])
+@pytest.mark.parametrize("prec,dtype", [("fast", torch.float16), ("fp32", torch.float32), ("mpv", torch.float16)])
+def test_zoom_phase_table_gives_identical_pixels(name, size, osz, table, prec, dtype):
+    """With the scratch pz_scratch_wanted names, ravu-zoom takes its weights
+    from a table of the scale's phases: the pixels and keys of the general
+    path, at every tile height.  Small frames and scales of no simple ratio
+    want none."""
+    import ctypes
+    from mpv_prescalers_gb300 import _ffi
+    from mpv_prescalers_gb300.prescaler import PRECISIONS
+    hm, _ = synth.model_for(name)
+    W, H = size
+    x = torch.rand((hm.n_planes, H, W), device="cuda").to(dtype)
+    o = _ffi.Opts()
+    o.precision = PRECISIONS[prec]
+    o.out_width, o.out_height = osz
+    n = _ffi.lib().pz_scratch_wanted(hm.device_handle(0), W, H, 0 if dtype == torch.float32 else 1, ctypes.byref(o))
+    assert (n > 0) == table
+    scratch = torch.empty(max(n, 16), dtype=torch.uint8, device="cuda")
+
+    def run(**kw):
+        y = torch.empty((hm.n_planes, osz[1], osz[0]), device="cuda", dtype=dtype)
+        k = torch.empty(osz[::-1], device="cuda", dtype=torch.int32)
+        hm.run_raw(list(x.unbind(0)), list(y.unbind(0)), osz, precision=prec, keys=k, **kw)
+        return y, k
+
+    want, wkeys = run()
+    for rows in (None, 8, 16):
+        got, keys = run(scratch=scratch, tile_rows=rows)
+        assert torch.equal(got, want) and torch.equal(keys, wkeys), rows
+
+
 def test_zoom_tma_box_larger_than_the_plane_falls_back():
     hm, _ = synth.model_for("ravu-zoom-ar-r2")
     x = torch.rand((6, 20), device="cuda", dtype=torch.float16)   # smaller than any box
