@@ -196,6 +196,15 @@ size_t pz_scratch_wanted(const pz_model* model, int in_width, int in_height, int
 int pz_run(const pz_model* model, const pz_plane* in, int n_in, pz_plane* out, int n_out,
            const pz_opts* opts, void* cuda_stream);
 
+/* pz_run on n_frames frames of one tensor: plane c of frame f starts at element
+ * f * in_frame + c * in_plane of `in`, rows in_pitch elements apart; `out`
+ * likewise, at the output size pz_query reports.  `scratch` (pz_scratch_wanted
+ * bytes, or as for pz_run) replaces opts->scratch and serves the frames in turn;
+ * opts->keys must be NULL for more than one frame. */
+int pz_run_frames(const pz_model* model, const void* in, long long in_frame, long long in_plane, int in_pitch,
+                  void* out, long long out_frame, long long out_plane, int out_pitch, int n_frames, int width,
+                  int height, int dtype, const pz_opts* opts, void* scratch, size_t scratch_bytes, void* cuda_stream);
+
 /* ---- frames in host memory --------------------------------------------
  * For hosts that decode in software and hold frames in host memory: runs
  * the chain over n_frames frames, copying frame i in, running it and copying

@@ -88,6 +88,9 @@ EXPORTS = {
                                 ctypes.POINTER(QueryResult)]),
     "pz_run": (ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(Plane), ctypes.c_int, ctypes.POINTER(Plane),
                               ctypes.c_int, ctypes.POINTER(Opts), ctypes.c_void_p]),
+    "pz_run_frames": (ctypes.c_int, [ctypes.c_void_p] * 2 + [ctypes.c_longlong] * 2 + [ctypes.c_int, ctypes.c_void_p]
+                      + [ctypes.c_longlong] * 2 + [ctypes.c_int] * 5 + [ctypes.POINTER(Opts), ctypes.c_void_p,
+                                                                        ctypes.c_size_t, ctypes.c_void_p]),
     "pz_batch_work_bytes": (ctypes.c_size_t, [ctypes.POINTER(Job), ctypes.c_int]),
     "pz_batch_create": (ctypes.c_int, [ctypes.POINTER(Job), ctypes.c_int, ctypes.c_void_p, ctypes.c_size_t,
                                        ctypes.c_int, ctypes.c_void_p, ctypes.POINTER(ctypes.c_void_p)]),

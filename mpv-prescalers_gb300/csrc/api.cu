@@ -481,8 +481,10 @@ size_t pz_scratch_wanted(const pz_model* m, int in_w, int in_h, int dtype, const
   return zoom_table_size(m, in_w, in_h, q.out_width, q.out_height, &px, &py);
 }
 
-int pz_run(const pz_model* m, const pz_plane* in, int n_in, pz_plane* out, int n_out, const pz_opts* o,
-           void* stream) {
+// pz_run; table_filled: a call before it on this stream, with the same sizes and
+// options, has left ravu-zoom's phase table in the scratch.
+static int run_frame(const pz_model* m, const pz_plane* in, int n_in, pz_plane* out, int n_out, const pz_opts* o,
+                     void* stream, bool table_filled) {
   if (!m || !in || !out) return fail(PZ_EINVAL, "null argument");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int C = m->channels == PZ_LUMA ? 1 : 3;
@@ -602,7 +604,7 @@ int pz_run(const pz_model* m, const pz_plane* in, int n_in, pz_plane* out, int n
           if (need && o->scratch_bytes >= need) {
             if (!o->tile_rows) a.tile_rows = 4;
             a.ztab = static_cast<const float4*>(o->scratch);
-            pz::launch_zoom_table(a, m->radius, m->ar != 0.0f, s);
+            if (!table_filled) pz::launch_zoom_table(a, m->radius, m->ar != 0.0f, s);
           }
         }
         rc = pz::launch_zoom(a, m->radius, m->channels, m->ar != 0.0f, dt, s); break;
@@ -613,6 +615,34 @@ int pz_run(const pz_model* m, const pz_plane* in, int n_in, pz_plane* out, int n
   }
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "kernel launch");
+  return PZ_OK;
+}
+
+int pz_run(const pz_model* m, const pz_plane* in, int n_in, pz_plane* out, int n_out, const pz_opts* o, void* stream) {
+  return run_frame(m, in, n_in, out, n_out, o, stream, false);
+}
+
+int pz_run_frames(const pz_model* m, const void* in, long long in_frame, long long in_plane, int in_pitch, void* out,
+                  long long out_frame, long long out_plane, int out_pitch, int n_frames, int width, int height,
+                  int dtype, const pz_opts* opts, void* scratch, size_t scratch_bytes, void* stream) {
+  pz_query_result q;
+  if (const int rc = pz_query(m, width, height, dtype, opts, &q)) return rc;
+  if (!in || !out) return fail(PZ_EINVAL, "null planes");
+  pz_opts o{};
+  if (opts) o = *opts;
+  o.scratch = scratch;
+  o.scratch_bytes = scratch_bytes;
+  const long long es = (long long)dtype_size(dtype);
+  for (int f = 0; f < n_frames; f++) {
+    pz_plane pin[3], pout[3];
+    for (int c = 0; c < q.n_planes; c++) {
+      char* i = static_cast<char*>(const_cast<void*>(in)) + (f * in_frame + c * in_plane) * es;
+      char* d = static_cast<char*>(out) + (f * out_frame + c * out_plane) * es;
+      pin[c] = {i, width, height, in_pitch, dtype};
+      pout[c] = {d, q.out_width, q.out_height, out_pitch, dtype};
+    }
+    if (const int rc = run_frame(m, pin, q.n_planes, pout, q.n_planes, &o, stream, f > 0)) return rc;
+  }
   return PZ_OK;
 }
 

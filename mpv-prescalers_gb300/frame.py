@@ -32,6 +32,7 @@ import dataclasses
 from typing import List, Optional, Sequence, Tuple
 
 from . import _ffi
+from .prescaler import on_stream, raw_stream
 
 FILTERS = {"bilinear": _ffi.PZ_FILTER_BILINEAR, "catmull_rom": _ffi.PZ_FILTER_CATMULL_ROM}
 KINDS = ("yuv", "rgb", "gray")
@@ -148,14 +149,12 @@ def resample_plane(x, out_w: int, out_h: int, sx: float, ox: float, sy: float, o
     if filt not in FILTERS:
         raise ValueError(f"filter {filt!r} not in {sorted(FILTERS)}")
     if out is None:   # allocated on the stream that writes it
-        with torch.cuda.device(x.device), torch.cuda.stream(stream):
+        with on_stream(x.device, stream):
             out = torch.empty((out_h, out_w), dtype=x.dtype, device=x.device)
     dt = _ffi.PZ_F32 if x.dtype == torch.float32 else _ffi.PZ_F16
     pin = _ffi.Plane(x.data_ptr(), x.shape[1], x.shape[0], x.stride(0), dt)
     pout = _ffi.Plane(out.data_ptr(), out.shape[1], out.shape[0], out.stride(0), dt)
-    s = stream if stream is not None else torch.cuda.current_stream(x.device)
-    _ffi.check(_ffi.lib().pz_resample(_ffi.ctypes.byref(pin), _ffi.ctypes.byref(pout), sx, ox, sy, oy,
-                                      FILTERS[filt], s.cuda_stream))
+    _ffi.check(_ffi.lib().pz_resample(pin, pout, sx, ox, sy, oy, FILTERS[filt], raw_stream(x.device, stream)))
     return out
 
 
@@ -167,13 +166,16 @@ def prescale_frame(model, frame: Frame, out_size: Optional[Tuple[int, int]] = No
     torch = _torch()
     if frame.offset != (0.0, 0.0) and frame.offset != (0, 0):
         raise ValueError("the frame carries an uncorrected offset; correct it before the next prescaler")
-    plan = plan_frame(model, frame.kind, frame.sizes, out_size, frame.chroma_loc)
+    sizes, loc = tuple(frame.sizes), frame.chroma_loc
+    loc = loc if isinstance(loc, str) else tuple(loc)
+    plan = model._kept(("frame", frame.kind, sizes, None if out_size is None else tuple(out_size), loc),
+                       lambda: plan_frame(model, frame.kind, sizes, out_size, loc))
     if not plan.runs:
         return Frame(list(frame.planes), frame.kind, frame.chroma_loc, frame.offset)
     W, H = frame.sizes[0]
     planes = list(frame.planes)
     dev = planes[0].device
-    with torch.cuda.device(dev):
+    with on_stream(dev, None):
         if plan.upsample_chroma:
             (rx, ry), (lx, ly) = plan.chroma_scale, plan.chroma_origin
             planes[1:] = [resample_plane(p, W, H, rx, -lx * rx, ry, -ly * ry, cscale, stream=stream)

@@ -20,6 +20,7 @@ for the requested output size leaves the planes untouched, as mpv would.
 """
 from __future__ import annotations
 
+import contextlib
 import json
 import os
 import threading
@@ -58,6 +59,29 @@ def _torch():
     return torch
 
 
+def on_stream(dev, stream):
+    """The context in which work for ``stream`` on ``dev`` is queued and its
+    tensors allocated; none is needed on the current device's current stream
+    (entering torch's two costs more than a small frame's launch)."""
+    torch = _torch()
+    if stream is None and dev.index == torch.cuda.current_device():
+        return contextlib.nullcontext()
+    stack = contextlib.ExitStack()
+    stack.enter_context(torch.cuda.device(dev))
+    stack.enter_context(torch.cuda.stream(stream))
+    return stack
+
+
+def raw_stream(dev, stream) -> int:
+    """The ``cudaStream_t`` of ``stream``, or of the current stream on ``dev``."""
+    return _torch()._C._cuda_getCurrentRawStream(dev.index) if stream is None else stream.cuda_stream
+
+
+class _Plan:
+    """What one frame geometry and form needs of a call, worked out once."""
+    __slots__ = ("enabled", "out_size", "opts", "scratch")
+
+
 class HookModel:
     """A parsed prescaler with lazily created device copies of its data."""
 
@@ -74,6 +98,7 @@ class HookModel:
         self._host_work: Dict[Tuple[int, int], List[Tuple["torch.cuda.Event", "torch.Tensor"]]] = {}
         self._side: Dict[int, "torch.cuda.Stream"] = {}   # per device: the host pipeline's default stream
         self._host_opts: Dict[Tuple, "_ffi.Opts"] = {}    # pz_opts of host pipelines, per frame geometry
+        self._plans: Dict[Tuple, object] = {}             # per frame geometry and form, at most _PLANS_KEEP
 
     # ---- metadata -----------------------------------------------------
     @property
@@ -98,10 +123,10 @@ class HookModel:
 
     @property
     def default_staging(self) -> str:
-        """Halo staging used when none is asked for: TMA boxes for ravu-lite
-        (within 2 % of plain loads on GB300 at r2 and the anti-ringing r3 / r4:
-        ravu-lite-ar-r3 56 us per 1080p frame either way), plain loads for the
-        other programs (ravu-r3 79 against 83 us; 3x and zoom within 3 %)."""
+        """Halo staging of batch jobs that ask for none: TMA boxes for
+        ravu-lite, plain loads for the other programs.  Per-frame calls use plain
+        loads for all (1080p: ravu-lite-ar-r3 54 us either way, ravu-lite-r3 32
+        against 34 us, ravu-r3 79 against 83 us)."""
         return "tma" if self.family == "lite" else "ldg"
 
     @property
@@ -287,9 +312,8 @@ class HookModel:
         planes only, LUTs rounded to FP16, ravu-zoom LUT bilinear weights
         in 1/256 steps; NNEDI3 as "fp32").
         ``staging``: how RAVU tiles stage their input window: "ldg"
-        (clamped loads) or "tma" (TMA boxes for interior tiles), default
-        ``default_staging``; the pixels are identical, only the speed
-        differs (see ``batch.autotune_staging``).
+        (clamped loads, the default) or "tma" (TMA boxes for interior
+        tiles); the pixels are identical, only the speed differs (see ``batch.autotune_staging``).
         ``tile_rows``: RAVU tile height, 4, 8 or 16 rows of 32 pixels
         (default: the library's measured choice for the model's program, 4
         rows but for ravu-lite r2, ravu-lite-ar r4 and ravu-r2);
@@ -298,6 +322,10 @@ class HookModel:
         keys as int32 when ``return_keys``).
         """
         torch = _torch()
+        if stream is None and out is None and not return_keys and not isinstance(planes, (list, tuple)):
+            res = self._upscale_tensor(planes, out_size, precision, staging, tile_rows)
+            if res is not None:
+                return res
         if not isinstance(planes, (list, tuple)) and planes.dim() == 4:
             # a batch of frames [N][C][H][W]: one chain per frame, same stream
             # (the results are gathered on that stream, after the kernels)
@@ -323,14 +351,16 @@ class HookModel:
                 raise ValueError("planes must be float32 or float16")
             if p.shape != (H, W) or p.dtype != pl[0].dtype or p.stride(1) != 1:
                 raise ValueError("planes must share size/dtype and be row-contiguous")
-        if not self.enabled(W, H, out_size):
+        plan = self._plan(pl[0].device, W, H, pl[0].dtype, out_size, precision, staging, tile_rows)
+        if not plan.enabled:
             res = [p.clone() for p in pl]
             return self._pack(res, planes, as_list, None, return_keys)
-        OW, OH = self.output_size(W, H, out_size)
+        OW, OH = plan.out_size
         dev = pl[0].device
-        # results are allocated (and packed) on the stream that writes them,
-        # so the caching allocator orders their reuse after the kernels
-        with torch.cuda.device(dev), torch.cuda.stream(stream):
+        # results and scratch are allocated (and results packed) on the stream
+        # that writes them, so the caching allocator orders their reuse after the
+        # kernels
+        with on_stream(dev, stream):
             full = None
             if out is None:
                 full = torch.empty((len(pl), OH, OW), dtype=pl[0].dtype, device=dev)
@@ -340,13 +370,96 @@ class HookModel:
             keys = None
             if return_keys:
                 keys = torch.empty(self.key_shape(W, H, OW, OH), dtype=torch.int32, device=dev)
-            scratch = None
-            if self.family == "zoom":   # room for the weights of every phase, where the scale has few
-                n = self._scratch_wanted(W, H, pl[0], OW, OH, precision, staging)
-                scratch = torch.empty(n, dtype=torch.uint8, device=dev) if n else None
-            self.run_raw(pl, res, out_size=(OW, OH), precision=precision, keys=keys, stream=stream,
-                         scratch=scratch, staging=staging, tile_rows=tile_rows)
+            scratch = torch.empty(plan.scratch, dtype=torch.uint8, device=dev) if plan.scratch else None
+            self._run(pl, res, _ffi.Opts.from_buffer_copy(plan.opts), keys, stream, scratch)
             return self._pack(res, planes, as_list, keys, return_keys, full)
+
+    def _upscale_tensor(self, x, out_size, precision, staging, tile_rows):
+        """:meth:`upscale` of one tensor on the current stream in one native
+        call (all frames of a batch into one result); None where the general
+        path has more to do or to say (other devices, views whose rows are not
+        contiguous, a ``//!WHEN`` that is false, errors)."""
+        torch = _torch()
+        dev, dtype = x.device, x.dtype
+        if dev.type != "cuda" or dev.index != torch.cuda.current_device():
+            return None
+        if out_size is not None:
+            out_size = tuple(out_size)
+        key = (x.shape, x.stride(), dtype, dev, out_size, precision, staging, tile_rows)
+        call = self._plans.get(key) or self._kept(key, lambda: self._tensor_call(*key))
+        if call == "general":
+            return None
+        out_shape, from_in, from_out, scratch_bytes, opts = call
+        out = torch.empty(out_shape, dtype=dtype, device=dev)
+        scratch = torch.empty(scratch_bytes, dtype=torch.uint8, device=dev) if scratch_bytes else None
+        rc = _ffi.lib().pz_run_frames(self.device_handle(dev.index), x.data_ptr(), *from_in, out.data_ptr(), *from_out,
+                                      opts, scratch.data_ptr() if scratch_bytes else None, scratch_bytes,
+                                      raw_stream(dev, None))
+        if rc:
+            _ffi.check(rc)
+        return out
+
+    def _tensor_call(self, shape, st, dtype, dev, out_size, precision, staging, tile_rows):
+        """What :meth:`_upscale_tensor` hands ``pz_run_frames`` for tensors of
+        this geometry: (result's shape, the arguments after either pointer,
+        scratch bytes, options), or "general"."""
+        torch = _torch()
+        d = len(shape)
+        if not 2 <= d <= 4 or (dtype is not torch.float16 and dtype is not torch.float32) or 0 in shape:
+            return "general"
+        if st[-1] != 1 or (shape[-3] if d > 2 else 1) != self.n_planes:
+            return "general"
+        W, H = shape[-1], shape[-2]
+        plan = self._plan(dev, W, H, dtype, out_size, precision, staging, tile_rows)
+        if not plan.enabled:
+            return "general"
+        OW, OH = plan.out_size
+        n, c = shape[0] if d == 4 else 1, self.n_planes
+        return (shape[:-2] + (OH, OW), (st[0] if d == 4 else 0, st[-3] if d > 2 else 0, st[-2]),
+                (c * OH * OW, OH * OW, OW, n, W, H, _ffi.PZ_F32 if dtype is torch.float32 else _ffi.PZ_F16),
+                plan.scratch, plan.opts)
+
+    _PLANS_KEEP = 256   # frame geometries whose plans are kept
+
+    def _plan(self, dev, W, H, dtype, out_size, precision, staging, tile_rows) -> _Plan:
+        """The plan of one frame geometry and form (options, output size,
+        scratch; no device data), kept for the next call."""
+        def make():
+            p = _Plan()
+            p.enabled = self.enabled(W, H, out_size)
+            p.out_size, p.opts, p.scratch = (W, H), None, 0
+            if p.enabled:
+                p.out_size = self.output_size(W, H, out_size)
+                p.opts = self._opts(W, H, p.out_size, precision, staging, tile_rows)
+                dt = _ffi.PZ_F32 if dtype == _torch().float32 else _ffi.PZ_F16
+                p.scratch = int(_ffi.lib().pz_scratch_wanted(self.device_handle(dev.index), W, H, dt, p.opts))
+            return p
+        return self._kept((W, H, dtype, None if out_size is None else tuple(out_size), precision, staging, tile_rows),
+                          make)
+
+    def _kept(self, key, make):
+        """``make()``, a function of ``key`` and the model alone, kept for the next call."""
+        p = self._plans.get(key)
+        if p is None:
+            p = make()
+            with self._lock:
+                if len(self._plans) >= self._PLANS_KEEP:
+                    self._plans.clear()
+                self._plans[key] = p
+        return p
+
+    def _opts(self, W, H, out_size, precision, staging, tile_rows) -> "_ffi.Opts":
+        """The ``pz_opts`` of a call, without keys and scratch.  Staging that is
+        not asked for is by plain loads: since window tiles are staged in quads
+        they are as fast as TMA boxes or faster for every program."""
+        o = _ffi.Opts()
+        o.precision = PRECISIONS[precision]
+        o.out_width, o.out_height = out_size
+        if self.family == "nnedi3":
+            o.nnedi3_axes = self.nnedi3_axes(W, H, out_size)
+        o.staging = STAGINGS[staging or "ldg"]
+        o.tile_rows = check_tile_rows(tile_rows)
+        return o
 
     def upscale_host(self, frames, out=None, out_size: Optional[Tuple[int, int]] = None, precision: str = "fp32",
                      device=None, wait: bool = True, stream=None):
@@ -422,7 +535,6 @@ class HookModel:
             o.out_width, o.out_height = OW, OH
             if self.family == "nnedi3":
                 o.nnedi3_axes = self.nnedi3_axes(W, H, out_size)
-            o.staging = STAGINGS[self.default_staging]
             with self._lock:
                 o = self._host_opts.setdefault(key, o)
         return o
@@ -456,16 +568,6 @@ class HookModel:
                     break
                 del pool[k]
 
-    def _scratch_wanted(self, W, H, plane, OW, OH, precision, staging) -> int:
-        """``pz_scratch_wanted`` of one frame."""
-        o = _ffi.Opts()
-        o.precision = PRECISIONS[precision]
-        o.out_width, o.out_height = OW, OH
-        o.staging = STAGINGS[staging or self.default_staging]
-        dt = _ffi.PZ_F32 if plane.element_size() == 4 else _ffi.PZ_F16
-        return int(_ffi.lib().pz_scratch_wanted(self.device_handle(plane.device.index), W, H, dt,
-                                                _ffi.ctypes.byref(o)))
-
     def key_shape(self, W, H, OW, OH):
         fam = self.family
         if fam == "ravu":
@@ -480,29 +582,22 @@ class HookModel:
                 tile_rows=None):
         """Low-level call of ``pz_run`` on prepared tensors (no allocation
         besides the optional NNEDI3 scratch inside the library)."""
+        o = self._opts(pl[0].shape[1], pl[0].shape[0], out_size, precision, staging, tile_rows)
+        self._run(pl, res, o, keys, stream, scratch)
+
+    def _run(self, pl, res, o, keys, stream, scratch):
         torch = _torch()
         dt = _ffi.PZ_F32 if pl[0].dtype == torch.float32 else _ffi.PZ_F16
         n = len(pl)
-        pin = (_ffi.Plane * n)()
-        pout = (_ffi.Plane * n)()
-        for i, (p, r) in enumerate(zip(pl, res)):
-            pin[i] = _ffi.Plane(p.data_ptr(), p.shape[1], p.shape[0], p.stride(0), dt)
-            pout[i] = _ffi.Plane(r.data_ptr(), r.shape[1], r.shape[0], r.stride(0), dt)
-        o = _ffi.Opts()
-        o.precision = PRECISIONS[precision]
-        o.out_width, o.out_height = out_size
-        if self.family == "nnedi3":
-            o.nnedi3_axes = self.nnedi3_axes(pl[0].shape[1], pl[0].shape[0], out_size)
+        pin = (_ffi.Plane * n)(*[(p.data_ptr(), p.shape[1], p.shape[0], p.stride(0), dt) for p in pl])
+        pout = (_ffi.Plane * n)(*[(r.data_ptr(), r.shape[1], r.shape[0], r.stride(0), dt) for r in res])
         if keys is not None:
             o.keys = keys.data_ptr()
         if scratch is not None:
             o.scratch = scratch.data_ptr()
             o.scratch_bytes = scratch.numel() * scratch.element_size()
-        o.staging = STAGINGS[staging or self.default_staging]
-        o.tile_rows = check_tile_rows(tile_rows)
-        s = stream if stream is not None else torch.cuda.current_stream(pl[0].device)
-        h = self.device_handle(pl[0].device.index)
-        _ffi.check(_ffi.lib().pz_run(h, pin, n, pout, n, _ffi.ctypes.byref(o), s.cuda_stream))
+        dev = pl[0].device
+        _ffi.check(_ffi.lib().pz_run(self.device_handle(dev.index), pin, n, pout, n, o, raw_stream(dev, stream)))
 
     @staticmethod
     def _pack(res, planes, as_list, keys, return_keys, full=None):

@@ -140,6 +140,36 @@ def test_when_false_leaves_planes_untouched():
     assert y.shape == (80, 60)
 
 
+@pytest.mark.parametrize("name,osz", [("ravu-lite-ar-r3", None), ("ravu-r3-yuv", None), ("ravu-3x-r2-rgb", None),
+                                      ("ravu-zoom-ar-r2", (1440, 810)), ("nnedi3-nns32-win8x4", None)])
+def test_one_call_for_a_tensor_gives_the_planes_pixels(name, osz):
+    """A tensor on the current stream goes down in one native call; the same
+    planes as a list, with ``out`` or on a stream of their own take the
+    general path: the same pixels for whole tensors and for views (rows,
+    planes and frames further apart than they are long), frame by frame."""
+    hm, _ = synth.model_for(name)
+    C, (W, H) = hm.n_planes, (960, 540) if osz else (203, 57)
+    big = torch.rand((4, C + 1, H + 2, W + 5), device="cuda").to(torch.float16)
+    for x in (big[:3, :C, :H, :W], big[1:4:2, 1:, 2:, 5:], big[:2, :C, :H, :W].contiguous()):
+        y = hm.upscale(x, out_size=osz, precision="fast")
+        assert y.is_contiguous() and y.shape[:2] == x.shape[:2]
+        s = torch.cuda.Stream()
+        s.wait_stream(torch.cuda.current_stream())
+        z = hm.upscale(x, out_size=osz, precision="fast", stream=s)
+        torch.cuda.synchronize()
+        assert torch.equal(y, z)
+        for f in range(x.shape[0]):
+            want = hm.upscale(list(x[f].unbind(0)), out_size=osz, precision="fast")
+            assert all(torch.equal(a, b) for a, b in zip(y[f], want))
+            assert torch.equal(hm.upscale(x[f], out_size=osz, precision="fast"), y[f])
+    if C == 1:
+        assert torch.equal(hm.upscale(x[0, 0], out_size=osz, precision="fast"), y[0, 0])
+    with pytest.raises(ValueError):
+        hm.upscale(torch.rand((1, C + 1, H, W), device="cuda"), out_size=osz)
+    with pytest.raises(ValueError):
+        hm.upscale(big[:, :C].transpose(2, 3), out_size=osz)
+
+
 @pytest.mark.parametrize("name", ["ravu-lite-ar-r4", "ravu-lite-r2", "ravu-r3", "ravu-r4-rgb", "ravu-3x-r3-yuv",
                                   "ravu-zoom-ar-r2"])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
