@@ -43,6 +43,22 @@ def test_resample_matches_oracle(case, filt, dtype):
         assert np.array_equal(got, x)
 
 
+@pytest.mark.parametrize("w,h,ow,oh", [(260, 70, 260, 70), (131, 5, 131, 5), (4, 4, 4, 4), (1, 1, 3, 2), (96, 40, 103, 37)])
+@pytest.mark.parametrize("off", [(-0.5, -0.5), (0.25, -2.75), (1.0, 3.5), (-1e-9, -0.5), (-200.0, 90.25)])
+@pytest.mark.parametrize("filt", ["bilinear", "catmull_rom"])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+def test_shifts_match_oracle(w, h, ow, oh, off, filt, dtype):
+    """Unit-scale shifts run by 4 x 4 blocks: whole and ragged blocks, planes
+    read in quads and not, every column phase, positions whose floor is not
+    floor(offset) (-1e-9), starts far outside."""
+    x = synth.luma_plane(h, w, 73)
+    if dtype == torch.float16:
+        x = x.astype(np.float16).astype(np.float64)
+    got = F.resample_plane(torch.from_numpy(x).to("cuda", dtype), ow, oh, 1.0, off[0], 1.0, off[1], filt)
+    want = ores.resample(x, ow, oh, 1.0, off[0], 1.0, off[1], filt)
+    assert np.abs(got.double().cpu().numpy() - want).max() <= (2e-6 if dtype == torch.float32 else 1e-3)
+
+
 def test_resample_rejects_bad_arguments():
     x = torch.zeros((8, 8), device="cuda")
     with pytest.raises(Exception, match="out of range"):
