@@ -365,14 +365,18 @@ int pz_model_create(const pz_model_desc* d, pz_model** out) {
     return fail(PZ_EINVAL, "ravu-zoom anti-ringing needs the _ar LUT and a strength");
   }
   m->lut_rows = d->lut_rows;
-  m->lut_cols = d->lut_cols;
   // ravu-zoom's tables are held by LUT point (zoom_texel_at, ravu_tiles.cuh),
-  // the others as in the file; FP16 texels in rows padded to an even count, so
-  // that texel pairs are 16-byte loads
+  // the others by rows.  ravu's FP32 rows are padded to an odd texel count: a warp
+  // gathers texel q of 32 rows at once, and the file's 8 texels a row at r4 (128
+  // bytes) put all of them in one of L1's 8 16-byte banks, its 2 at r2 in 4 (the
+  // others' counts are odd): 1080p ravu-r4 131 us, 209 unpadded; ravu-r4-yuv 204,
+  // 279; ravu-r2 58.1, 58.4.  FP16 rows are padded to an even count,
+  // so that texel pairs are 16-byte loads.
   const bool zoom = d->family == PZ_RAVU_ZOOM;
   const int nb = need_cols / 9;
   m->lut_h_pitch = zoom ? 9 * ((nb + 1) & ~1) : (d->lut_cols + 1) & ~1;
-  const size_t nval = (size_t)d->lut_rows * d->lut_cols * 4, bytes = nval * 4;
+  m->lut_pitch = d->family == PZ_RAVU ? d->lut_cols | 1 : d->lut_cols;
+  const size_t nval = (size_t)d->lut_rows * m->lut_pitch * 4, bytes = nval * 4;
   auto laid_out = [&](const float* src, bool half, std::vector<float>* r) {
     for (int y = 0; y < d->lut_rows; y++)
       for (int c = 0; c < d->lut_cols; c++) {
@@ -382,7 +386,7 @@ int pz_model_create(const pz_model_desc* d, pz_model** out) {
           at = d->radius == 2 ? (half ? pz::zoom_texel_at<2, true>(y, x, t) : pz::zoom_texel_at<2, false>(y, x, t))
                               : (half ? pz::zoom_texel_at<3, true>(y, x, t) : pz::zoom_texel_at<3, false>(y, x, t));
         } else {
-          at = (size_t)y * (half ? m->lut_h_pitch : d->lut_cols) + c;
+          at = (size_t)y * (half ? m->lut_h_pitch : m->lut_pitch) + c;
         }
         std::memcpy(&(*r)[at * 4], &src[((size_t)y * d->lut_cols + c) * 4], 16);
       }

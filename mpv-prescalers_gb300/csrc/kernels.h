@@ -18,9 +18,9 @@ struct RavuArgs {
   int out_pitch[3];
   int W, H;          // input size
   int OW, OH;        // output size
-  const float4* lut;     // [lut_rows][lut_cols] texels
+  const float4* lut;     // [lut_rows][lut_pitch] texels
   const float4* lut_ar;  // zoom-ar only
-  int lut_rows, lut_cols;
+  int lut_rows, lut_pitch;
   float ar;
   int32_t* keys;     // optional raw-key output
   int* err;          // device error word (kErr*)
@@ -28,7 +28,7 @@ struct RavuArgs {
   int tile_rows;     // tile height of the per-frame launches: 4, 8 or 16 rows
   float lut_frac;    // zoom LUT bilinear fraction steps (0: exact FP32)
   const uint2* lut_h;  // fast form: the LUT as FP16 texels (4 halves each), or null
-  int lut_h_pitch;     // texels per FP16 LUT row (lut_cols rounded up to even)
+  int lut_h_pitch;     // texels per FP16 LUT row (even)
   int box_w, box_h;    // ravu-zoom TMA staging: the box of this launch's tensor maps (texels x rows)
   const float4* ztab;  // ravu-zoom: every key's weights at every phase of the scale (zoom_table_kernel), or null
   int zpx, zpy;        // phases per axis: out / gcd(in, out)

@@ -15,7 +15,7 @@ struct pz_model {
   float4* d_lut_ar16 = nullptr;
   __half* d_lut_h = nullptr;     // the LUT as FP16 texels (fast form), rows padded
   int lut_h_pitch = 0;           // to an even texel count (16-byte texel pairs)
-  int lut_rows = 0, lut_cols = 0;
+  int lut_rows = 0, lut_pitch = 0;  // keys (ravu-zoom: key * 9 rows); FP32 texels per stored row
   pz::KeyParams kp{};
   int nns = 0, win_w = 0, win_h = 0;
   float* d_wts = nullptr;   // [nns][2][T]
@@ -58,7 +58,7 @@ inline void select_lut(const pz_model* m, int precision, RavuArgs* a) {
   a->lut = mpv ? m->d_lut16 : m->d_lut;
   a->lut_ar = mpv ? m->d_lut_ar16 : m->d_lut_ar;
   a->lut_rows = m->lut_rows;
-  a->lut_cols = m->lut_cols;
+  a->lut_pitch = m->lut_pitch;
   a->lut_frac = mpv ? 256.0f : 0.0f;
   const bool h = fast_half_lut(m, precision);
   a->lut_h = h ? reinterpret_cast<const uint2*>(m->d_lut_h) : nullptr;
@@ -69,9 +69,9 @@ inline void select_lut(const pz_model* m, int precision, RavuArgs* a) {
 }
 
 // Tile height of a model's per-frame launches when the caller asks for none,
-// the fastest on GB300 at 480p-1080p (1080p, fast form, 4 / 8 rows: ravu-r2 60.5
-// / 58.4 us, ravu-r3 78.8 / 79.7, ravu-r4 208.7 / 215.0, ravu-r4-yuv 279.7 /
-// 279.6, ravu-lite-r3 31.8 / 33.5, ravu-lite-ar-r4 76.9 / 76.9, ravu-3x-r3 45.2 /
+// the fastest on GB300 at 480p-1080p (1080p, fast form, 4 / 8 rows: ravu-r2 60.2
+// / 58.1 us, ravu-r3 78.7 / 79.7, ravu-r4 131.3 / 131.0, ravu-r4-yuv 203.7 /
+// 203.7, ravu-lite-r3 31.8 / 33.5, ravu-lite-ar-r4 76.9 / 76.9, ravu-3x-r3 45.2 /
 // 47.0, ravu-zoom-r3 at 1.5x 334 / 283 FP32; 16 rows is slower for every program).
 inline int default_tile_rows(const pz_model* m) {
   if (m->family == PZ_RAVU_LITE && (m->radius == 2 || (m->radius == 4 && m->ar != 0.0f))) return 8;

@@ -320,7 +320,7 @@ struct LiteTile {
     structure_tensor<N, false, kPackedTensor>(get, p.kp, a, b, d);
     const int key = ravu_key(a, b, d, p.kp);
     if (p.keys) p.keys[(size_t)gy * p.W + gx] = key;
-    const size_t row = (size_t)min(max(key, 0), p.lut_rows - 1) * (H16 ? p.lut_h_pitch : p.lut_cols);
+    const size_t row = (size_t)min(max(key, 0), p.lut_rows - 1) * (H16 ? p.lut_h_pitch : p.lut_pitch);
     float4 w_next;  // H16: the odd texel of the pair loaded at the even one
     static_assert(S / 2 % 2 == 0, "texel pairs start at even columns");
     // FP32x2 sums: P = sum va*w, Q = sum vb*w, res = P + Q.wzyx; the
@@ -411,7 +411,7 @@ struct ThreeXTile {
     if (p.keys) p.keys[(size_t)gy * p.W + gx] = key;
     // 3x rows hold 2 * ceil(S / 2) texels: even, so the FP32 texel pairs are
     // 32-byte aligned without padding (1.2x over two 16-byte loads)
-    const size_t row = (size_t)min(max(key, 0), p.lut_rows - 1) * (H16 ? p.lut_h_pitch : p.lut_cols);
+    const size_t row = (size_t)min(max(key, 0), p.lut_rows - 1) * (H16 ? p.lut_h_pitch : p.lut_pitch);
     // res0 += a*w0 + b*w1.wzyx; res1 += a*w1 + b*w0.wzyx, as FP32x2 sums
     // P0 = sum a*w0, P1 = sum a*w1, Q0 = sum b*w0, Q1 = sum b*w1 (pairs .xy, .zw)
     float2 P0[C][2], P1[C][2], Q0[C][2], Q1[C][2];
@@ -524,7 +524,7 @@ struct Int11Tile {
     for (int e = 0; e < P; e++) {
       const int key = ravu_key(a[e], b[e], d[e], p.kp);
       if (p.keys && gy + e < p.H) p.keys[(size_t)(gy + e) * p.W + gx] = key;
-      L[e] = p.lut + (size_t)min(max(key, 0), p.lut_rows - 1) * p.lut_cols;
+      L[e] = p.lut + (size_t)min(max(key, 0), p.lut_rows - 1) * p.lut_pitch;
     }
     if (C > 1 || R == 4) asm volatile("" ::: "memory");  // no window value stays in a register from here
     float2 acc[P][C];
@@ -592,9 +592,9 @@ __host__ __device__ constexpr int lat_dy(int X, int Y) {
 // the lattice: every lattice value is loaded once per use (key, filter) and
 // channel for the two, and a tap is one lane of an FP32x2 product with its
 // weight (no sums of mirrored taps first: the two windows mirror differently).
-// Bound by issue (69 %) and by L1 (76 %).  1080p, both passes together: ravu-r3
-// 79.0 us (100.9 us with each window by itself and texel staging), ravu-r4 209
-// (266), ravu-r4-yuv 279 (330).  It then holds all four samples of its output 2x2 block
+// Bound by issue (69 %) and by L1 (76-80 %).  1080p, both passes together: ravu-r3
+// 78.7 us (100.9 us with each window by itself and texel staging), ravu-r4 131
+// (266), ravu-r4-yuv 204 (330).  It then holds all four samples of its output 2x2 block
 // -- input (0,0), int10 (1,0), int01 (0,1), int11 (1,1) -- and writes them as two
 // pixel-pair rows.
 template <int R, int CM, typename T, int TR = 8>
@@ -645,7 +645,7 @@ struct LatticeTile {
     for (int e = 0; e < 2; e++) {
       const int key = ravu_key(a[e], b[e], d[e], p.kp);
       if (p.keys) p.keys[(size_t)(1 + e) * plane + (size_t)gy * p.W + gx] = key;
-      const float4* L = p.lut + (size_t)min(max(key, 0), p.lut_rows - 1) * p.lut_cols;
+      const float4* L = p.lut + (size_t)min(max(key, 0), p.lut_rows - 1) * p.lut_pitch;
 #pragma unroll
       for (int q = 0; q < (S / 2 + 3) / 4; q++) w[e][q] = __ldg(L + q);
     }
@@ -760,11 +760,14 @@ struct ZoomLut {
   }
 };
 
-// float4 of one half window's weights in the phase table; an entry holds the
-// two halves, then (AR) the anti-ringing weights' two.
+// float4 of an entry of the phase table: the weights of the two half windows,
+// then (AR) the anti-ringing weights' two, padded to an odd count: a warp's loads
+// gather from 32 entries at once, and at an even stride they meet in few of L1's
+// 8 16-byte banks (1080p to 1.5x: ravu-zoom-ar-r2 97 us, 158 at 8 float4;
+// ravu-zoom-r2 62 us, 76 at 4).
 template <int R, bool AR>
 __host__ __device__ constexpr uint32_t zoom_entry() {
-  return zoom_texels<R>() * (AR ? 4 : 2);
+  return zoom_texels<R>() * (AR ? 4 : 2) + 1;
 }
 
 // The weights of every key at every phase of a scale whose output positions
@@ -801,9 +804,9 @@ __global__ void zoom_table_kernel(const __grid_constant__ RavuArgs p, float4* ou
 // rectangles) from one TMA box per plane whose size the host fits to the
 // launch's scale factor (tma_box_of), converting just the rectangle.
 // Bound by L1, where the gathers of LUT texels go (86 %; 16-40 loads a pixel).
-// 1080p to 1.5x, without / with the phase table: ravu-zoom-r2 86 / 76 us fast (132
-// with a load per texel, scalar blends and texel staging), r3 FP32 283 / 121 us
-// (290), ravu-zoom-ar-r2-rgb fast 274 / 203 us (302).
+// 1080p to 1.5x, without / with the phase table: ravu-zoom-r2 86 / 62 us fast (132
+// with a load per texel, scalar blends and texel staging), r3 FP32 283 / 111 us
+// (290), ravu-zoom-ar-r2-rgb fast 274 / 187 us (302).
 // TAB: the weights come from the launch's phase table, at the same bits.
 template <int R, int CM, bool AR, typename T, bool H16 = false, int TR = 8, bool TAB = false>
 struct ZoomTile {

@@ -48,8 +48,8 @@ void launch_table(const RavuArgs& a, cudaStream_t s) {
 
 // The table pays where it holds far fewer entries than the frame has pixels (an
 // entry costs about what a pixel saves) and the frame is large enough for one
-// more launch (some 4 us): 1080p to 1.5x, 9 phases, 203 against 274 us
-// (ravu-zoom-ar-r2-rgb); 1080p to 2.25x, 81 phases, 153 against 281 us
+// more launch (some 4 us): 1080p to 1.5x, 9 phases, 187 against 274 us
+// (ravu-zoom-ar-r2-rgb); 1080p to 2.25x, 81 phases, 145 against 281 us
 // (ravu-zoom-r2); 720x576 to 1080p, 120 phases and 60 pixels an entry, 38 against
 // 60 us; 854x480 to 1.75x, 49 phases and 89 pixels an entry, 63 against 68 us.
 // Scales of no simple ratio have as many phases as pixels and take none.
@@ -58,8 +58,9 @@ size_t zoom_table_bytes(int radius, bool ar, int keys, int W, int H, int OW, int
   *py = OH / gcd(H, OH);
   const long long entries = (long long)keys * *px * *py, pixels = (long long)OW * OH;
   if (pixels < 1 << 19 || entries * 8 > pixels) return 0;
-  const int nb = radius == 2 ? zoom_texels<2>() : zoom_texels<3>();
-  return (size_t)entries * nb * (ar ? 4 : 2) * sizeof(float4);
+  const uint32_t e = radius == 2 ? (ar ? zoom_entry<2, true>() : zoom_entry<2, false>())
+                                 : (ar ? zoom_entry<3, true>() : zoom_entry<3, false>());
+  return (size_t)entries * e * sizeof(float4);
 }
 
 int launch_zoom_table(const RavuArgs& a, int radius, bool ar, cudaStream_t s) {
