@@ -69,15 +69,17 @@ inline void select_lut(const pz_model* m, int precision, RavuArgs* a) {
 }
 
 // Tile height of a model's per-frame launches when the caller asks for none,
-// the fastest on GB300 at 480p-1080p (1080p, fast form, 4 / 8 rows: ravu-r2 60.2
-// / 58.1 us, ravu-r3 78.7 / 79.7, ravu-r4 131.3 / 131.0, ravu-r4-yuv 203.7 /
-// 203.7, ravu-lite-r3 31.8 / 33.5, ravu-lite-ar-r4 76.9 / 76.9, ravu-3x-r3 45.2 /
-// 47.0, ravu-zoom-r3 at 1.5x 334 / 283 FP32; 16 rows is slower for every program).
+// the fastest on GB300 at 480p-1080p (1080p, fast form, 4 / 8 rows: ravu-lite-r3
+// 31.3 / 30.0 us, ravu-lite-ar-r4 72.4 / 71.3, ravu-3x-r3 44.1 / 43.2, ravu-r2 60.2 /
+// 58.1, ravu-r3 78.7 / 79.7, ravu-r4 131.3 / 131.0, ravu-r4-yuv 203.7 / 203.7,
+// ravu-zoom-r2 at 1.5x 85.8 / 85.7, ravu-zoom-r3 FP32 334 / 283; 16 rows is slower
+// for nearly every program).
 inline int default_tile_rows(const pz_model* m) {
-  if (m->family == PZ_RAVU_LITE && (m->radius == 2 || (m->radius == 4 && m->ar != 0.0f))) return 8;
-  if (m->family == PZ_RAVU && m->radius == 2 && m->channels == PZ_LUMA) return 8;
-  if (m->family == PZ_RAVU_ZOOM && m->radius == 3) return 8;
-  return 4;
+  switch (m->family) {
+    case PZ_RAVU: return m->radius == 2 && m->channels == PZ_LUMA ? 8 : 4;
+    case PZ_RAVU_ZOOM: return m->radius == 3 ? 8 : 4;
+    default: return 8;
+  }
 }
 
 // The neurons of an NNEDI3 model, as the doubling passes take them.

@@ -16,7 +16,7 @@
 // Input tiles are 32 x TR input pixels (zoom: output pixels), TR = 4, 8 or 16
 // rows (a template argument of every program; 8 is the reference's own
 // workgroup height, compute/ravu-lite-r3.hook:22); thread t handles column
-// t % 32 of row t / 32 (int11: of the P rows from P * (t / 32)).  Out-of-range reads replicate the edge texel (the mpv
+// t % 32 of row t / 32 (lite, 3x, int11: of the P rows from P * (t / 32)).  Out-of-range reads replicate the edge texel (the mpv
 // texture border mode).
 #pragma once
 #include <atomic>
@@ -272,6 +272,12 @@ __device__ __forceinline__ void lut_pair_h16(const uint2* h, size_t i, float4& a
   b = make_float4(b01.x, b01.y, b23.x, b23.y);
 }
 
+// Windows of a thread's P pixels, one below the other.
+struct OffDown {
+  __host__ __device__ static constexpr int x(int) { return 0; }
+  __host__ __device__ static constexpr int y(int e) { return e; }
+};
+
 // ------------------------------------------------------------ ravu-lite ---
 // Does lite LUT column c take part in the anti-ringing sums?  r2: every
 // tap; r3/r4: the 13-tap diamond |dx|+|dy| <= 2 (ravu-lite-ar-r3.hook:93-170).
@@ -283,7 +289,13 @@ __host__ __device__ constexpr bool lite_ar_col(int c) {
 template <int R, bool AR, typename T, bool H16 = false, int TR = 8>
 struct LiteTile {
   static constexpr int N = 2 * R - 1, S = N * N, HALO = R - 1;
-  static constexpr int kRows = TR, kThreads = kTileW * TR;
+  // two pixels of a column per thread, keys first: shared loads and derivatives
+  // of the two windows (1080p at 8 rows, one / two / four pixels a thread:
+  // ravu-lite-r4 fast 61.0 / 53.3 / 53.1 us, -ar-r3 54.1 / 49.6 / 50.0, -ar-r4 76.7 /
+  // 71.3 / 78.6, r3 FP32 48.7 / 46.6 / 46.6).  Bound by L1 (80-93 %): a 16-byte
+  // gather from 32 LUT rows takes 12-13 wavefronts.
+  static constexpr int P = 2;
+  static constexpr int kRows = TR, kThreads = kTileW * TR / P;
   static constexpr bool kOutputTiles = false;
   static constexpr int TW = kTilePitch, TH = TR + N - 1;
   // the value tile and (AR) each texel's two 32nd powers, formed while staging
@@ -296,9 +308,7 @@ struct LiteTile {
 
   static constexpr int kPlanes = 1;
   static constexpr bool kTma = true;
-  // ravu-lite-ar-r4 at <= 48 registers (5 CTAs of 8 rows per SM) measured
-  // 2 % faster; the other radii lose more to spills than they gain
-  static constexpr int kMaxRegs = (R == 4 && AR) ? 48 : 0;
+  static constexpr int kMaxRegs = 0;  // any cap costs 1-5 % (64 and 80 measured)
   // ravu-lite-ar-r2 / -r3 measured 2-5 % slower with the packed structure
   // tensor (register allocation of the anti-ringing sums)
   static constexpr bool kPackedTensor = !(R <= 3 && AR);
@@ -310,17 +320,29 @@ struct LiteTile {
     if (!stage_frame<kLuma, TH, kThreads, T, kTable>(p, tma, x0, y0 - HALO, tile, NoStage(), reinterpret_cast<float4*>(pow)))
       return;
     __syncthreads();
-    const int tx = threadIdx.x % kTileW, ty = threadIdx.x / kTileW;
+    const int tx = threadIdx.x % kTileW, ty = threadIdx.x / kTileW * P;
     const int gx = x0 + tx, gy = y0 + ty;
     if (gx >= p.W || gy >= p.H) return;
-    const float* base = tile + ty * TW + tx + kLead - HALO;
-    const float2* pbase = reinterpret_cast<const float2*>(pow) + ty * TW + tx + kLead - HALO;
+    const int at = ty * TW + tx + kLead - HALO;
+    float a[P], b[P], d[P];
+    structure_tensors<N, false, kPackedTensor, P, OffDown>([&](int X, int Y) { return tile[at + Y * TW + X]; }, p.kp, a,
+                                                           b, d);
+    size_t rows[P];
+#pragma unroll
+    for (int e = 0; e < P; e++) {
+      const int key = ravu_key(a[e], b[e], d[e], p.kp);
+      if (p.keys && gy + e < p.H) p.keys[(size_t)(gy + e) * p.W + gx] = key;
+      rows[e] = (size_t)min(max(key, 0), p.lut_rows - 1) * (H16 ? p.lut_h_pitch : p.lut_pitch);
+    }
+#pragma unroll
+    for (int e = 0; e < P; e++)
+      if (gy + e < p.H) filter(p, rows[e], tile + at + e * TW, reinterpret_cast<const float2*>(pow) + at + e * TW, gx, gy + e);
+  }
+
+  // one pixel's four outputs: its LUT row, its window and (kTable) powers
+  __device__ static __forceinline__ void filter(const RavuArgs& p, size_t row, const float* base, const float2* pbase,
+                                                int gx, int gy) {
     auto get = [&](int kx, int ky) { return base[ky * TW + kx]; };
-    float a, b, d;
-    structure_tensor<N, false, kPackedTensor>(get, p.kp, a, b, d);
-    const int key = ravu_key(a, b, d, p.kp);
-    if (p.keys) p.keys[(size_t)gy * p.W + gx] = key;
-    const size_t row = (size_t)min(max(key, 0), p.lut_rows - 1) * (H16 ? p.lut_h_pitch : p.lut_pitch);
     float4 w_next;  // H16: the odd texel of the pair loaded at the even one
     static_assert(S / 2 % 2 == 0, "texel pairs start at even columns");
     // FP32x2 sums: P = sum va*w, Q = sum vb*w, res = P + Q.wzyx; the
@@ -385,7 +407,11 @@ struct LiteTile {
 template <int R, int CM, typename T, bool H16 = false, int TR = 8>
 struct ThreeXTile {
   static constexpr int N = 2 * R - 1, S = N * N, HALO = R - 1;
-  static constexpr int kRows = TR, kThreads = kTileW * TR;
+  // two pixels of a column per thread, as in LiteTile (1080p at 8 rows, one / two /
+  // four pixels a thread: r3 fast 47.3 / 43.2 / 44.0 us, r4 FP32 128.0 / 108.5 /
+  // 110.7, r3-rgb fast 93.0 / 84.5 / 91.5)
+  static constexpr int P = 2;
+  static constexpr int kRows = TR, kThreads = kTileW * TR / P;
   static constexpr bool kOutputTiles = false;
   static constexpr int TW = kTilePitch, TH = TR + N - 1;
   static constexpr int C = CM == kLuma ? 1 : 3;
@@ -399,19 +425,30 @@ struct ThreeXTile {
     float* tile = smem;
     if (!stage_frame<CM, TH, kThreads, T>(p, tma, x0, y0 - HALO, tile)) return;
     __syncthreads();
-    const int tx = threadIdx.x % kTileW, ty = threadIdx.x / kTileW;
+    const int tx = threadIdx.x % kTileW, ty = threadIdx.x / kTileW * P;
     const int gx = x0 + tx, gy = y0 + ty;
     if (gx >= p.W || gy >= p.H) return;
     const float* base = tile + ty * TW + tx + kLead - HALO;
-    auto val = [&](int c, int t) { return base[c * TW * TH + t % N * TW + t / N]; };
-    auto lum = [&](int kx, int ky) { return base[(CM == kRgb ? C * TW * TH : 0) + ky * TW + kx]; };
-    float a, b, d;
-    structure_tensor<N, false>(lum, p.kp, a, b, d);
-    const int key = ravu_key(a, b, d, p.kp);
-    if (p.keys) p.keys[(size_t)gy * p.W + gx] = key;
+    const float* lbase = base + (CM == kRgb ? C * TW * TH : 0);
+    float a[P], b[P], d[P];
+    structure_tensors<N, false, true, P, OffDown>([&](int X, int Y) { return lbase[Y * TW + X]; }, p.kp, a, b, d);
     // 3x rows hold 2 * ceil(S / 2) texels: even, so the FP32 texel pairs are
     // 32-byte aligned without padding (1.2x over two 16-byte loads)
-    const size_t row = (size_t)min(max(key, 0), p.lut_rows - 1) * (H16 ? p.lut_h_pitch : p.lut_pitch);
+    size_t rows[P];
+#pragma unroll
+    for (int e = 0; e < P; e++) {
+      const int key = ravu_key(a[e], b[e], d[e], p.kp);
+      if (p.keys && gy + e < p.H) p.keys[(size_t)(gy + e) * p.W + gx] = key;
+      rows[e] = (size_t)min(max(key, 0), p.lut_rows - 1) * (H16 ? p.lut_h_pitch : p.lut_pitch);
+    }
+#pragma unroll
+    for (int e = 0; e < P; e++)
+      if (gy + e < p.H) filter(p, rows[e], base + e * TW, gx, gy + e);
+  }
+
+  // one pixel's 3 x 3 outputs: its LUT row and its windows
+  __device__ static __forceinline__ void filter(const RavuArgs& p, size_t row, const float* base, int gx, int gy) {
+    auto val = [&](int c, int t) { return base[c * TW * TH + t % N * TW + t / N]; };
     // res0 += a*w0 + b*w1.wzyx; res1 += a*w1 + b*w0.wzyx, as FP32x2 sums
     // P0 = sum a*w0, P1 = sum a*w1, Q0 = sum b*w0, Q1 = sum b*w1 (pairs .xy, .zw)
     float2 P0[C][2], P1[C][2], Q0[C][2], Q1[C][2];
@@ -477,11 +514,6 @@ struct ThreeXTile {
 };
 
 // ------------------------------------------------------ ravu lattice -----
-// Windows of a thread's P pixels, one below the other.
-struct OffDown {
-  __host__ __device__ static constexpr int x(int) { return 0; }
-  __host__ __device__ static constexpr int y(int e) { return e; }
-};
 
 // int11: the keyed filter over the input window (ravu-r3.hook:15-146):
 // res[c] = sum over the S/2 mirrored tap pairs of (x_i + x_{S-1-i}) * w_i, the

@@ -40,7 +40,7 @@ _CHANNEL_CODE = {"luma": _ffi.PZ_LUMA, "yuv": _ffi.PZ_YUV, "rgb": _ffi.PZ_RGB}
 PRECISIONS = {"fp32": _ffi.PZ_PREC_FP32, "fast": _ffi.PZ_PREC_FAST, "mpv": _ffi.PZ_PREC_MPV}
 # RAVU halo staging: clamped loads, or TMA boxes for interior tiles
 STAGINGS = {"ldg": 0, "tma": 1}
-# RAVU tile heights (rows of 32 pixels, one thread per pixel); None: the
+# RAVU tile heights (rows of 32 pixels); None: the
 # library's measured default for the model's program
 TILE_ROWS = (4, 8, 16)
 
@@ -315,8 +315,7 @@ class HookModel:
         (clamped loads, the default) or "tma" (TMA boxes for interior
         tiles); the pixels are identical, only the speed differs (see ``batch.autotune_staging``).
         ``tile_rows``: RAVU tile height, 4, 8 or 16 rows of 32 pixels
-        (default: the library's measured choice for the model's program, 4
-        rows but for ravu-lite r2, ravu-lite-ar r4 and ravu-r2);
+        (default: the library's measured choice for the model's program);
         again only the speed differs (see ``batch.autotune_tiles``).
         Returns the upscaled planes in the input's form (and the raw LUT
         keys as int32 when ``return_keys``).
