@@ -130,8 +130,8 @@ typedef struct {
                               clamped loads: TMA fills zeros, not the edge)  */
   int tile_rows;           /* RAVU tile height: 4, 8 or 16 rows of 32 pixels
                               (input pixels; ravu-zoom: output pixels); 0: the
-                              program's measured default (ravu-lite, ravu-3x,
-                              ravu-r2, ravu-zoom r3: 8, the others 4).  The pixels do not depend on it.  The
+                              program's measured default (8; ravu-zoom r2: 4,
+                              ravu-r4 of three channels: 16).  The pixels do not depend on it.  The
                               persistent batch kernels run 8-row tiles
                               whatever this says.                           */
 } pz_opts;

@@ -69,17 +69,14 @@ inline void select_lut(const pz_model* m, int precision, RavuArgs* a) {
 }
 
 // Tile height of a model's per-frame launches when the caller asks for none,
-// the fastest on GB300 at 480p-1080p (1080p, fast form, 4 / 8 rows: ravu-lite-r3
-// 31.3 / 30.0 us, ravu-lite-ar-r4 72.4 / 71.3, ravu-3x-r3 44.1 / 43.2, ravu-r2 60.2 /
-// 58.1, ravu-r3 78.7 / 79.7, ravu-r4 131.3 / 131.0, ravu-r4-yuv 203.7 / 203.7,
-// ravu-zoom-r2 at 1.5x 85.8 / 85.7, ravu-zoom-r3 FP32 334 / 283; 16 rows is slower
-// for nearly every program).
+// the fastest on GB300 at 480p-1080p (1080p, fast form, 4 / 8 / 16 rows:
+// ravu-lite-r3 31.3 / 30.0 / 31.3 us, ravu-lite-ar-r4 72.4 / 71.3 / 79.5, ravu-3x-r3
+// 44.1 / 43.2 / 45.6, ravu-r2 58.1 / 54.2 / 54.2, ravu-r3 74.9 / 74.6 / 78.6, ravu-r4
+// 116.4 / 114.3 / 118.4, ravu-r3-yuv 121.9 / 117.8 / 128.1, ravu-r4-yuv 210.6 /
+// 198.0 / 188.7; ravu-zoom at 1.5x, 4 / 8: r2 85.8 / 85.7, r3 FP32 334 / 283).
 inline int default_tile_rows(const pz_model* m) {
-  switch (m->family) {
-    case PZ_RAVU: return m->radius == 2 && m->channels == PZ_LUMA ? 8 : 4;
-    case PZ_RAVU_ZOOM: return m->radius == 3 ? 8 : 4;
-    default: return 8;
-  }
+  if (m->family == PZ_RAVU && m->radius == 4 && m->channels != PZ_LUMA) return 16;
+  return m->family == PZ_RAVU_ZOOM && m->radius == 2 ? 4 : 8;
 }
 
 // The neurons of an NNEDI3 model, as the doubling passes take them.

@@ -16,7 +16,7 @@
 // Input tiles are 32 x TR input pixels (zoom: output pixels), TR = 4, 8 or 16
 // rows (a template argument of every program; 8 is the reference's own
 // workgroup height, compute/ravu-lite-r3.hook:22); thread t handles column
-// t % 32 of row t / 32 (lite, 3x, int11: of the P rows from P * (t / 32)).  Out-of-range reads replicate the edge texel (the mpv
+// t % 32 of row t / 32 (zoom; the others: of the P rows from P * (t / 32)).  Out-of-range reads replicate the edge texel (the mpv
 // texture border mode).
 #pragma once
 #include <atomic>
@@ -599,9 +599,10 @@ struct Int11Tile {
 // interleaves input and int11 pixels.  int01's window is int10's one step back
 // along kx, so both are windows of one lattice (X, Y): int10 at X = kx, int01
 // at X = kx - 1.
+// The windows of the pixel below lie one step back along X and one on along Y.
 struct OffLattice {
-  __host__ __device__ static constexpr int x(int e) { return -e; }
-  __host__ __device__ static constexpr int y(int) { return 0; }
+  __host__ __device__ static constexpr int x(int e) { return -(e % 2) - e / 2; }
+  __host__ __device__ static constexpr int y(int e) { return e / 2; }
 };
 // Where lattice point (X, Y) lies: 0 = input, 1 = int11, at offset (dx, dy).
 template <int N>
@@ -620,19 +621,22 @@ __host__ __device__ constexpr int lat_dy(int X, int Y) {
 // int10 + int01: both lattice filters per input pixel (ravu-r3.hook:148-437).
 // The input tile and the int11 tile (from the FP32 int11 plane, clamped to
 // its edge: the clamp-to-edge of the int11 texture) are staged; each thread
-// evaluates both windows of a pixel, which share all but one column each of
-// the lattice: every lattice value is loaded once per use (key, filter) and
-// channel for the two, and a tap is one lane of an FP32x2 product with its
-// weight (no sums of mirrored taps first: the two windows mirror differently).
-// Bound by issue (69 %) and by L1 (76-80 %).  1080p, both passes together: ravu-r3
-// 78.7 us (100.9 us with each window by itself and texel staging), ravu-r4 131
-// (266), ravu-r4-yuv 204 (330).  It then holds all four samples of its output 2x2 block
-// -- input (0,0), int10 (1,0), int01 (0,1), int11 (1,1) -- and writes them as two
-// pixel-pair rows.
+// evaluates both windows of P = 2 pixels, one below the other.  The keys of all
+// four windows come first: they share most loads and derivatives.  A pixel's
+// filters then load every lattice value once for its two windows, and a tap is
+// one lane of an FP32x2 product with its weight (no sums of mirrored taps first:
+// the two windows mirror differently).  The thread holds all four samples of an
+// output 2x2 block -- input (0,0), int10 (1,0), int01 (0,1), int11 (1,1) -- and
+// writes them as two pixel-pair rows.
+// Bound by issue (69 %) and by L1 (76-80 %).  1080p, both passes together at 8
+// rows, one / two pixels a thread: ravu-r2 56.2 / 54.2 us, ravu-r3 78.7 (4 rows) /
+// 74.6 (100.9 with each window by itself and texel staging), ravu-r4 131 / 114
+// (266), ravu-r3-yuv 125 / 118 (153), ravu-r4-yuv 204 / 198, 189 at 16 rows (330).
 template <int R, int CM, typename T, int TR = 8>
 struct LatticeTile {
   static constexpr int N = 2 * R, S = N * N;
-  static constexpr int kRows = TR, kThreads = kTileW * TR;
+  static constexpr int P = 2;
+  static constexpr int kRows = TR, kThreads = kTileW * TR / P;
   static constexpr bool kOutputTiles = false;
   static constexpr int TW = kTilePitch, TH = TR + N - 1;
   static constexpr int C = CM == kLuma ? 1 : 3;
@@ -640,9 +644,9 @@ struct LatticeTile {
   static constexpr size_t smem_bytes = (size_t)2 * PL * TW * TH * 4;
   static constexpr int kPlanes = C;
   static constexpr bool kTma = true;
-  // luma at r2 / r3 is 2-4 % faster under these caps (of 44 / 60 registers);
-  // r4 and three channels lose by any (r3-yuv at 40: 162 against 126 us)
-  static constexpr int kMaxRegs = CM == kLuma && R <= 3 ? (R == 2 ? 40 : 48) : 0;
+  // r4 luma at 80 registers (of 100) is 2 % faster; the others lose by any cap
+  // (r4-yuv at 80: 207 against 198 us, at 64: 259)
+  static constexpr int kMaxRegs = R == 4 && CM == kLuma ? 80 : 0;
   using Elem = T;
 
   __device__ static void run(const RavuArgs& p, int x0, int y0, float* smem, TmaCtx* tma = nullptr) {
@@ -661,53 +665,61 @@ struct LatticeTile {
     } i11{{}, p, t11, x0, y0 - R};
     if (!stage_frame<CM, TH, kThreads, T>(p, tma, x0, y0 - (R - 1), tin, i11)) return;
     __syncthreads();
-    const int tx = threadIdx.x % kTileW, ty = threadIdx.x / kTileW;
+    const int tx = threadIdx.x % kTileW, ty = threadIdx.x / kTileW * P;
     const int gx = x0 + tx, gy = y0 + ty;
     if (gx >= p.W || gy >= p.H) return;
     const float* bin = tin + (ty + R - 1) * TW + tx + kLead;
     const float* b11 = t11 + (ty + R) * TW + tx + kLead;
-    auto val = [&](int c, int X, int Y) {
-      return (lat_src<N>(X, Y) == 0 ? bin : b11)[c * TW * TH + lat_dy<N>(X, Y) * TW + lat_dx<N>(X, Y)];
+    auto point = [&](int c, int X, int Y, int down) {
+      return (lat_src<N>(X, Y) == 0 ? bin : b11)[c * TW * TH + (lat_dy<N>(X, Y) + down) * TW + lat_dx<N>(X, Y)];
     };
-    float a[2], b[2], d[2];
-    structure_tensors<N, true, true, 2, OffLattice>(
-        [&](int X, int Y) { return val(CM == kRgb ? C : 0, X, Y); }, p.kp, a, b, d);  // rgb: the luma tile is plane C
-    float4 w[2][(S / 2 + 3) / 4];
+    float a[2 * P], b[2 * P], d[2 * P];
+    structure_tensors<N, true, true, 2 * P, OffLattice>(
+        [&](int X, int Y) { return point(CM == kRgb ? C : 0, X, Y, 0); }, p.kp, a, b, d);  // rgb: the luma tile is plane C
+    const float4* rows[2 * P];
 #pragma unroll
-    for (int e = 0; e < 2; e++) {
+    for (int e = 0; e < 2 * P; e++) {
       const int key = ravu_key(a[e], b[e], d[e], p.kp);
-      if (p.keys) p.keys[(size_t)(1 + e) * plane + (size_t)gy * p.W + gx] = key;
-      const float4* L = p.lut + (size_t)min(max(key, 0), p.lut_rows - 1) * p.lut_pitch;
-#pragma unroll
-      for (int q = 0; q < (S / 2 + 3) / 4; q++) w[e][q] = __ldg(L + q);
+      if (p.keys && gy + e / 2 < p.H) p.keys[(size_t)(1 + e % 2) * plane + (size_t)(gy + e / 2) * p.W + gx] = key;
+      rows[e] = p.lut + (size_t)min(max(key, 0), p.lut_rows - 1) * p.lut_pitch;
     }
     if (C > 1 || R == 4) asm volatile("" ::: "memory");  // no window value stays in a register from here
-    // weights i, i+1 (i even) of window e as a pair
-    auto wpair = [&](int e, int i) {
-      const float4& q = w[e][i / 4];
-      return i % 4 == 0 ? make_float2(q.x, q.y) : make_float2(q.z, q.w);
-    };
 #pragma unroll
-    for (int c = 0; c < C; c++) {
-      float2 acc[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+    for (int down = 0; down < P; down++) {
+      if (gy + down >= p.H) break;
+      auto val = [&](int c, int X, int Y) { return point(c, X, Y, down); };
+      float4 w[2][(S / 2 + 3) / 4];
 #pragma unroll
-      for (int X = -1; X < N; X++) {
+      for (int e = 0; e < 2; e++)
 #pragma unroll
-        for (int Y = 0; Y < N; Y += 2) {
-          const float v0 = val(c, X, Y), v1 = val(c, X, Y + 1);
+        for (int q = 0; q < (S / 2 + 3) / 4; q++) w[e][q] = __ldg(rows[2 * down + e] + q);
+      // weights i, i+1 (i even) of window e as a pair
+      auto wpair = [&](int e, int i) {
+        const float4& q = w[e][i / 4];
+        return i % 4 == 0 ? make_float2(q.x, q.y) : make_float2(q.z, q.w);
+      };
 #pragma unroll
-          for (int e = 0; e < 2; e++) {
-            const int i = (X + e) * N + Y;  // taps i, i+1 of window e; the upper half mirrors the lower
-            if (i < 0 || i >= S) continue;
-            if (i < S / 2) acc[e] = __ffma2_rn(make_float2(v0, v1), wpair(e, i), acc[e]);
-            else acc[e] = __ffma2_rn(make_float2(v1, v0), wpair(e, S - 2 - i), acc[e]);
+      for (int c = 0; c < C; c++) {
+        float2 acc[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+#pragma unroll
+        for (int X = -1; X < N; X++) {
+#pragma unroll
+          for (int Y = 0; Y < N; Y += 2) {
+            const float v0 = val(c, X, Y), v1 = val(c, X, Y + 1);
+#pragma unroll
+            for (int e = 0; e < 2; e++) {
+              const int i = (X + e) * N + Y;  // taps i, i+1 of window e; the upper half mirrors the lower
+              if (i < 0 || i >= S) continue;
+              if (i < S / 2) acc[e] = __ffma2_rn(make_float2(v0, v1), wpair(e, i), acc[e]);
+              else acc[e] = __ffma2_rn(make_float2(v1, v0), wpair(e, S - 2 - i), acc[e]);
+            }
           }
         }
+        T* o = static_cast<T*>(p.out[c]) + (size_t)(2 * (gy + down)) * p.out_pitch[c] + 2 * gx;
+        // row 2i: input, int10; row 2i+1: int01, int11 (ravu-r3.hook:424-437)
+        stp2(o, bin[c * TW * TH + down * TW], clampf(acc[0].x + acc[0].y, 0.f, 1.f));
+        stp2(o + p.out_pitch[c], clampf(acc[1].x + acc[1].y, 0.f, 1.f), b11[c * TW * TH + down * TW]);
       }
-      T* o = static_cast<T*>(p.out[c]) + (size_t)(2 * gy) * p.out_pitch[c] + 2 * gx;
-      // row 2i: input, int10; row 2i+1: int01, int11 (ravu-r3.hook:424-437)
-      stp2(o, bin[c * TW * TH], clampf(acc[0].x + acc[0].y, 0.f, 1.f));
-      stp2(o + p.out_pitch[c], clampf(acc[1].x + acc[1].y, 0.f, 1.f), b11[c * TW * TH]);
     }
   }
 };
