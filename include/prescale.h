@@ -198,9 +198,10 @@ int pz_run(const pz_model* model, const pz_plane* in, int n_in, pz_plane* out, i
 
 /* pz_run on n_frames frames of one tensor: plane c of frame f starts at element
  * f * in_frame + c * in_plane of `in`, rows in_pitch elements apart; `out`
- * likewise, at the output size pz_query reports.  `scratch` (pz_scratch_wanted
- * bytes, or as for pz_run) replaces opts->scratch and serves the frames in turn;
- * opts->keys must be NULL for more than one frame. */
+ * likewise, at the output size pz_query reports.  `scratch` replaces
+ * opts->scratch: with n_frames times pz_scratch_bytes of it (and clamped-load
+ * staging) each pass of the chain is one launch for all frames, else it serves
+ * the frames in turn; opts->keys must be NULL for more than one frame. */
 int pz_run_frames(const pz_model* model, const void* in, long long in_frame, long long in_plane, int in_pitch,
                   void* out, long long out_frame, long long out_plane, int out_pitch, int n_frames, int width,
                   int height, int dtype, const pz_opts* opts, void* scratch, size_t scratch_bytes, void* cuda_stream);

@@ -485,10 +485,12 @@ size_t pz_scratch_wanted(const pz_model* m, int in_w, int in_h, int dtype, const
   return zoom_table_size(m, in_w, in_h, q.out_width, q.out_height, &px, &py);
 }
 
-// pz_run; table_filled: a call before it on this stream, with the same sizes and
-// options, has left ravu-zoom's phase table in the scratch.
+// pz_run on `frames` frames whose planes lie in_frame / out_frame elements apart
+// (more than one: scratch for each given, plain loads, no keys).  table_filled: a
+// call before it on this stream, with the same sizes and options, has left
+// ravu-zoom's phase table in the scratch.
 static int run_frame(const pz_model* m, const pz_plane* in, int n_in, pz_plane* out, int n_out, const pz_opts* o,
-                     void* stream, bool table_filled) {
+                     void* stream, bool table_filled, int frames = 1, long long in_frame = 0, long long out_frame = 0) {
   if (!m || !in || !out) return fail(PZ_EINVAL, "null argument");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int C = m->channels == PZ_LUMA ? 1 : 3;
@@ -543,23 +545,26 @@ static int run_frame(const pz_model* m, const pz_plane* in, int n_in, pz_plane* 
         own_tmp = true;
       }
     }
-    auto pass = [&](bool xpass, const void* src, int sw, int sh, int spitch, void* dst, int dpitch) {
+    auto pass = [&](bool xpass, const void* src, int sw, int sh, int spitch, long long sframe, void* dst, int dpitch,
+                    long long dframe) {
       a.in = src;
       a.in_pitch = spitch;
       a.out = dst;
       a.out_pitch = dpitch;
       a.W = sw;
       a.H = sh;
+      a.frames = frames;
+      a.in_frame = sframe;
+      a.out_frame = dframe;
       return pz::launch_nnedi3(a, precision, xpass, dt, s);
     };
     rc = 0;
     if (ax == 3) {
-      rc = pass(false, in[0].data, W, H, in[0].pitch, tmp, W);
-      if (!rc) rc = pass(true, tmp, W, 2 * H, W, out[0].data, out[0].pitch);
-    } else if (ax == 1) {
-      rc = pass(false, in[0].data, W, H, in[0].pitch, out[0].data, out[0].pitch);
+      const long long doubled = 2LL * H * W;
+      rc = pass(false, in[0].data, W, H, in[0].pitch, in_frame, tmp, W, doubled);
+      if (!rc) rc = pass(true, tmp, W, 2 * H, W, doubled, out[0].data, out[0].pitch, out_frame);
     } else {
-      rc = pass(true, in[0].data, W, H, in[0].pitch, out[0].data, out[0].pitch);
+      rc = pass(ax != 1, in[0].data, W, H, in[0].pitch, in_frame, out[0].data, out[0].pitch, out_frame);
     }
     if (own_tmp) cudaFreeAsync(tmp, s);
     if (rc) return fail(rc, "NNEDI3 launch configuration not supported");
@@ -575,6 +580,9 @@ static int run_frame(const pz_model* m, const pz_plane* in, int n_in, pz_plane* 
     a.H = H;
     a.OW = OW;
     a.OH = OH;
+    a.frames = frames;
+    a.in_frame = in_frame;
+    a.out_frame = out_frame;
     pz::select_lut(m, o ? o->precision : PZ_PREC_FP32, &a);
     a.ar = m->ar;
     a.keys = o ? o->keys : nullptr;
@@ -637,7 +645,11 @@ int pz_run_frames(const pz_model* m, const void* in, long long in_frame, long lo
   o.scratch = scratch;
   o.scratch_bytes = scratch_bytes;
   const long long es = (long long)dtype_size(dtype);
-  for (int f = 0; f < n_frames; f++) {
+  // all frames in one launch per pass (at most 1024: the tile numbers of one
+  // launch stay far below 2^31, its grid within bounds) where each has scratch of its own
+  const bool together = !o.staging && !o.keys && out_frame % 2 == 0 && q.scratch_bytes * (size_t)n_frames <= scratch_bytes;
+  const int step = together ? 1024 : 1;
+  for (int f = 0; f < n_frames; f += step) {
     pz_plane pin[3], pout[3];
     for (int c = 0; c < q.n_planes; c++) {
       char* i = static_cast<char*>(const_cast<void*>(in)) + (f * in_frame + c * in_plane) * es;
@@ -645,7 +657,8 @@ int pz_run_frames(const pz_model* m, const void* in, long long in_frame, long lo
       pin[c] = {i, width, height, in_pitch, dtype};
       pout[c] = {d, q.out_width, q.out_height, out_pitch, dtype};
     }
-    if (const int rc = run_frame(m, pin, q.n_planes, pout, q.n_planes, &o, stream, f > 0)) return rc;
+    const int n = n_frames - f < step ? n_frames - f : step;
+    if (const int rc = run_frame(m, pin, q.n_planes, pout, q.n_planes, &o, stream, f > 0, n, in_frame, out_frame)) return rc;
   }
   return PZ_OK;
 }

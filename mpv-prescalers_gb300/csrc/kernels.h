@@ -18,6 +18,8 @@ struct RavuArgs {
   int out_pitch[3];
   int W, H;          // input size
   int OW, OH;        // output size
+  int frames;        // frames of one launch (0 counts as 1; plain loads only), elements apart:
+  long long in_frame, out_frame;
   const float4* lut;     // [lut_rows][lut_pitch] texels
   const float4* lut_ar;  // zoom-ar only
   int lut_rows, lut_pitch;
@@ -44,6 +46,8 @@ struct NnArgs {
   void* out;
   int out_pitch;
   int W, H;                 // size of the pass input
+  int frames;               // frames of one launch (tensor cores; 0 counts as 1), elements apart:
+  long long in_frame, out_frame;
   int nns, win_h;           // window is 8 x win_h (double_y orientation)
   const float* wts;         // [nns][2][T]: A row then B row per neuron (FP32)
   const float* cs;          // [nns][2]: column sums of A and B

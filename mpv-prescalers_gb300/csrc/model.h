@@ -108,7 +108,16 @@ inline int launch_nnedi3(const NnArgs& a, int precision, bool xpass, int dtype, 
     if (precision == PZ_PREC_FAST) return launch_nnedi3_tc(a, xpass, dtype, s);
     if (a.wts_s) return launch_nnedi3_split(a, xpass, dtype, s);
   }
-  return launch_nnedi3_simt(a, xpass, dtype, s);
+  // one frame a launch
+  NnArgs b = a;
+  b.frames = 1;
+  const size_t es = dtype == PZ_F32 ? 4 : 2;
+  for (int f = 0; f < (a.frames > 0 ? a.frames : 1); f++) {
+    b.in = static_cast<const char*>(a.in) + f * a.in_frame * (long long)es;
+    b.out = static_cast<char*>(a.out) + f * a.out_frame * (long long)es;
+    if (const int rc = launch_nnedi3_simt(b, xpass, dtype, s)) return rc;
+  }
+  return 0;
 }
 
 // Scratch of a ravu lattice chain: the int11 plane, FP32 [channels][H][W].

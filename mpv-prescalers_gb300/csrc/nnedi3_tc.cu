@@ -158,13 +158,30 @@ struct TcShape {
   static_assert(NG >= 1 && NG * 2 * CCOL <= 512, "operands must fit shared and tensor memory");
 };
 
+// t / d for 0 <= t < 2^31 by a multiplication (t advances by hundreds of tiles,
+// and a division costs as much as a neuron pair).
+struct FastDiv {
+  uint32_t m, s, d;
+  __host__ explicit FastDiv(uint32_t div) : d(div) {
+    s = 0;
+    while ((1ull << s) < div) s++;
+    m = (uint32_t)(((1ull << 32) * ((1ull << s) - div)) / div + 1);
+  }
+  __device__ __forceinline__ uint32_t operator()(uint32_t t) const { return (__umulhi(t, m) + t) >> s; }
+};
+// The tiles of a launch: 32 x 4 pixels, row by row, frame after frame.
+struct Tiles {
+  FastDiv x, y;  // tiles per row, rows of tiles per frame
+  int n;
+};
+
 // Neurons are processed in chunks of NC (32, or 16 for nns16): chunk k's
 // accumulator holds NC softmax-branch and NC Elliott-branch columns; the MMA
 // of chunk k+2 is issued as soon as every warp of the group has read chunk k.
 // Operand B is stored chunk-major: rows [2*NC*k, 2*NC*k + NC) are the
 // softmax weights of neurons k*NC.., the next NC rows their Elliott weights.
 template <int WH, int NNS, bool XP, typename T, bool SPLIT>
-__global__ void __launch_bounds__(TcShape<WH, NNS, XP, SPLIT>::THREADS, 1) nn_tc_kernel(const __grid_constant__ NnArgs p) {
+__global__ void __launch_bounds__(TcShape<WH, NNS, XP, SPLIT>::THREADS, 1) nn_tc_kernel(const __grid_constant__ NnArgs p, const __grid_constant__ Tiles tiles) {
   using S = TcShape<WH, NNS, XP, SPLIT>;
   constexpr int NT = S::NT, KP = S::KP, NC = S::NC, NCH = S::NCH, CCOL = S::CCOL, NG = S::NG;
   constexpr int TW = S::TW, TH = S::TH;
@@ -212,8 +229,7 @@ __global__ void __launch_bounds__(TcShape<WH, NNS, XP, SPLIT>::THREADS, 1) nn_tc
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = tmem_base;
-  const int tiles_x = (p.W + 31) / 32, tiles_y = (p.H + 3) / 4;
-  const int ntiles = tiles_x * tiles_y;
+  const int ntiles = tiles.n;
   const int stride = NG * gridDim.x;  // tiles go over the SMs first, then over each SM's groups
 
   // true once the phase has completed; false when the CTA has given up
@@ -278,16 +294,25 @@ __global__ void __launch_bounds__(TcShape<WH, NNS, XP, SPLIT>::THREADS, 1) nn_tc
     // the window tile of a later tile, loaded into registers ahead of use
     constexpr int PF = (TW * TH + kGroup - 1) / kGroup;
     float pre[PF];
+    // frame, row and column of tile t
+    auto locate = [&](int t, int& f, int& y0) {
+      const int row = tiles.x(t);
+      f = tiles.y(row);
+      y0 = (row - f * (int)tiles.y.d) * 4;
+      return (t - row * (int)tiles.x.d) * 32;
+    };
     auto prefetch = [&](int t) {
       if (t >= ntiles) return;
-      const int px0 = (t % tiles_x) * 32, py0 = (t / tiles_x) * 4;
+      int f, py0;
+      const int px0 = locate(t, f, py0);
+      const T* src = in + f * p.in_frame;
 #pragma unroll
       for (int r = 0; r < PF; r++) {
         const int i = m + r * kGroup;
         if (i < TW * TH) {
           const int ty = i / TW, tx = i % TW;
           const int gx = clampi(px0 + S::OX0 + tx, 0, p.W - 1), gy = clampi(py0 + S::OY0 + ty, 0, p.H - 1);
-          pre[r] = ldp(in + (size_t)gy * p.in_pitch + gx);
+          pre[r] = ldp(src + (size_t)gy * p.in_pitch + gx);
         }
       }
     };
@@ -428,14 +453,17 @@ __global__ void __launch_bounds__(TcShape<WH, NNS, XP, SPLIT>::THREADS, 1) nn_tc
           }
         }
       }
-      const int gx = (t % tiles_x) * 32 + lane, gy = (t / tiles_x) * 4 + py;
+      int f, gy;
+      const int gx = locate(t, f, gy) + lane;
+      gy += py;
+      T* dst = out + f * p.out_frame;
       if (gx < p.W && gy < p.H && !*aborted) {
         const float v = clampf(cur.mean + 5.0f * (vsum.x + vsum.y) / (wsum.x + wsum.y) * cur.stdv, 0.0f, 1.0f);
         if (XP) {
-          stp2(out + (size_t)gy * p.out_pitch + 2 * gx, cur.orig, v);
+          stp2(dst + (size_t)gy * p.out_pitch + 2 * gx, cur.orig, v);
         } else {
-          stp(out + (size_t)(2 * gy) * p.out_pitch + gx, cur.orig);
-          stp(out + (size_t)(2 * gy + 1) * p.out_pitch + gx, v);
+          stp(dst + (size_t)(2 * gy) * p.out_pitch + gx, cur.orig);
+          stp(dst + (size_t)(2 * gy + 1) * p.out_pitch + gx, v);
         }
       }
       cur = nxt;
@@ -464,8 +492,9 @@ int launch_one(const NnArgs& a, cudaStream_t s) {
     configured[dev] = true;
   }
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int ntiles = ((a.W + 31) / 32) * ((a.H + 3) / 4);
-  kern<<<ntiles < sms ? ntiles : sms, S::THREADS, S::SMEM, s>>>(a);
+  Tiles tiles{FastDiv((a.W + 31) / 32), FastDiv((a.H + 3) / 4), 0};
+  tiles.n = (int)(tiles.x.d * tiles.y.d) * (a.frames > 0 ? a.frames : 1);
+  kern<<<tiles.n < sms ? tiles.n : sms, S::THREADS, S::SMEM, s>>>(a, tiles);
   return 0;
 }
 

@@ -32,6 +32,16 @@ namespace pz {
 // of kBatchTileRows rows.
 constexpr int kTileW = 32, kBatchTileRows = 8;
 
+// Plane c of frame f.
+template <typename T>
+__device__ __forceinline__ const T* plane_in(const RavuArgs& p, int c, int f) {
+  return static_cast<const T*>(p.in[c]) + f * p.in_frame;
+}
+template <typename T>
+__device__ __forceinline__ T* plane_out(const RavuArgs& p, int c, int f) {
+  return static_cast<T*>(p.out[c]) + f * p.out_frame;
+}
+
 __host__ __device__ constexpr int cabs(int v) { return v < 0 ? -v : v; }
 
 // The window tiles of the frame-tile programs: 40 columns starting 4 left of
@@ -229,7 +239,7 @@ struct NoStage {
   __device__ __forceinline__ void store() {}
 };
 template <int CM, int TH, int NT, typename T, bool POW = false, class Also = NoStage>
-__device__ __forceinline__ bool stage_frame(const RavuArgs& p, TmaCtx* t, int x0, int y0, float* tile,
+__device__ __forceinline__ bool stage_frame(const RavuArgs& p, TmaCtx* t, int f, int x0, int y0, float* tile,
                                             Also&& also = NoStage(), float4* pow = nullptr) {
   TileStage<CM, TH, NT, T> st;
   constexpr int C = CM == kLuma ? 1 : 3, BW = tma_box_w<kTilePitch>();
@@ -246,7 +256,7 @@ __device__ __forceinline__ bool stage_frame(const RavuArgs& p, TmaCtx* t, int x0
     for (int c = 0; c < C; c++)
       st.s[c].load_box(reinterpret_cast<const T*>(t->raw + c * pb) + (wx - bx), BW);
   } else {
-    st.load([&](int c, int& pitch) { pitch = p.in_pitch[c]; return static_cast<const T*>(p.in[c]); }, p.W, p.H, x0, y0);
+    st.load([&](int c, int& pitch) { pitch = p.in_pitch[c]; return plane_in<T>(p, c, f); }, p.W, p.H, x0, y0);
     also.load();
   }
   st.template store<POW>(tile, pow);
@@ -314,10 +324,10 @@ struct LiteTile {
   static constexpr bool kPackedTensor = !(R <= 3 && AR);
   using Elem = T;
 
-  __device__ static void run(const RavuArgs& p, int x0, int y0, float* smem, TmaCtx* tma = nullptr) {
+  __device__ static void run(const RavuArgs& p, int f, int x0, int y0, float* smem, TmaCtx* tma = nullptr) {
     float* tile = smem;
     float* pow = tile + TW * TH;
-    if (!stage_frame<kLuma, TH, kThreads, T, kTable>(p, tma, x0, y0 - HALO, tile, NoStage(), reinterpret_cast<float4*>(pow)))
+    if (!stage_frame<kLuma, TH, kThreads, T, kTable>(p, tma, f, x0, y0 - HALO, tile, NoStage(), reinterpret_cast<float4*>(pow)))
       return;
     __syncthreads();
     const int tx = threadIdx.x % kTileW, ty = threadIdx.x / kTileW * P;
@@ -336,12 +346,13 @@ struct LiteTile {
     }
 #pragma unroll
     for (int e = 0; e < P; e++)
-      if (gy + e < p.H) filter(p, rows[e], tile + at + e * TW, reinterpret_cast<const float2*>(pow) + at + e * TW, gx, gy + e);
+      if (gy + e < p.H) 
+        filter(p, f, rows[e], tile + at + e * TW, reinterpret_cast<const float2*>(pow) + at + e * TW, gx, gy + e);
   }
 
   // one pixel's four outputs: its LUT row, its window and (kTable) powers
-  __device__ static __forceinline__ void filter(const RavuArgs& p, size_t row, const float* base, const float2* pbase,
-                                                int gx, int gy) {
+  __device__ static __forceinline__ void filter(const RavuArgs& p, int f, size_t row, const float* base,
+                                                const float2* pbase, int gx, int gy) {
     auto get = [&](int kx, int ky) { return base[ky * TW + kx]; };
     float4 w_next;  // H16: the odd texel of the pair loaded at the even one
     static_assert(S / 2 % 2 == 0, "texel pairs start at even columns");
@@ -396,7 +407,7 @@ struct LiteTile {
       res.z = clampf(res.z, 0.f, 1.f); res.w = clampf(res.w, 0.f, 1.f);
     }
     // res[0..3] -> offsets (0,0), (0,1), (1,0), (1,1)  (compute/ravu-lite-r3.hook:101-104)
-    T* out = static_cast<T*>(p.out[0]);
+    T* out = plane_out<T>(p, 0, f);
     const int op = p.out_pitch[0];
     stp2(out + (size_t)(2 * gy) * op + 2 * gx, res.x, res.z);
     stp2(out + (size_t)(2 * gy + 1) * op + 2 * gx, res.y, res.w);
@@ -421,9 +432,9 @@ struct ThreeXTile {
   static constexpr int kMaxRegs = 0;  // the compiler's own allocation
   using Elem = T;
 
-  __device__ static void run(const RavuArgs& p, int x0, int y0, float* smem, TmaCtx* tma = nullptr) {
+  __device__ static void run(const RavuArgs& p, int f, int x0, int y0, float* smem, TmaCtx* tma = nullptr) {
     float* tile = smem;
-    if (!stage_frame<CM, TH, kThreads, T>(p, tma, x0, y0 - HALO, tile)) return;
+    if (!stage_frame<CM, TH, kThreads, T>(p, tma, f, x0, y0 - HALO, tile)) return;
     __syncthreads();
     const int tx = threadIdx.x % kTileW, ty = threadIdx.x / kTileW * P;
     const int gx = x0 + tx, gy = y0 + ty;
@@ -443,11 +454,12 @@ struct ThreeXTile {
     }
 #pragma unroll
     for (int e = 0; e < P; e++)
-      if (gy + e < p.H) filter(p, rows[e], base + e * TW, gx, gy + e);
+      if (gy + e < p.H) filter(p, f, rows[e], base + e * TW, gx, gy + e);
   }
 
   // one pixel's 3 x 3 outputs: its LUT row and its windows
-  __device__ static __forceinline__ void filter(const RavuArgs& p, size_t row, const float* base, int gx, int gy) {
+  __device__ static __forceinline__ void filter(const RavuArgs& p, int f, size_t row, const float* base, int gx,
+                                                int gy) {
     auto val = [&](int c, int t) { return base[c * TW * TH + t % N * TW + t / N]; };
     // res0 += a*w0 + b*w1.wzyx; res1 += a*w1 + b*w0.wzyx, as FP32x2 sums
     // P0 = sum a*w0, P1 = sum a*w1, Q0 = sum b*w0, Q1 = sum b*w1 (pairs .xy, .zw)
@@ -501,7 +513,7 @@ struct ThreeXTile {
                                     clampf(r1[c].z, 0.f, 1.f), clampf(r1[c].w, 0.f, 1.f));
       // imageStore(gid*3 + (dx,dy)): res0 -> (0,0),(0,1),(0,2),(1,0); centre (1,1);
       // res1 -> (1,2),(2,0),(2,1),(2,2)   (compute/ravu-3x-r2.hook:106-114)
-      T* o = static_cast<T*>(p.out[c]);
+      T* o = plane_out<T>(p, c, f);
       const size_t op = p.out_pitch[c];
       T* r = o + (size_t)(3 * gy) * op + 3 * gx;
       stp(r, a0.x); stp(r + 1, a0.w); stp(r + 2, a1.y);
@@ -540,9 +552,9 @@ struct Int11Tile {
   static constexpr int kMaxRegs = R == 3 && CM == kLuma ? 56 : 0;
   using Elem = T;
 
-  __device__ static void run(const RavuArgs& p, int x0, int y0, float* smem, TmaCtx* tma = nullptr) {
+  __device__ static void run(const RavuArgs& p, int f, int x0, int y0, float* smem, TmaCtx* tma = nullptr) {
     float* tile = smem;
-    if (!stage_frame<CM, TH, kThreads, T>(p, tma, x0, y0 - HALO, tile)) return;
+    if (!stage_frame<CM, TH, kThreads, T>(p, tma, f, x0, y0 - HALO, tile)) return;
     __syncthreads();
     const int tx = threadIdx.x % kTileW, ty = threadIdx.x / kTileW * P;
     const int gx = x0 + tx, gy = y0 + ty;
@@ -588,7 +600,7 @@ struct Int11Tile {
       for (int c = 0; c < C; c++) {
         float v = clampf(acc[e][c].x + acc[e][c].y, 0.f, 1.f);
         if (p.i11_half) v = __half2float(__float2half_rn(v));
-        p.i11[c * plane + (size_t)(gy + e) * p.W + gx] = v;
+        p.i11[(f * C + c) * plane + (size_t)(gy + e) * p.W + gx] = v;
       }
     }
   }
@@ -649,7 +661,7 @@ struct LatticeTile {
   static constexpr int kMaxRegs = R == 4 && CM == kLuma ? 80 : 0;
   using Elem = T;
 
-  __device__ static void run(const RavuArgs& p, int x0, int y0, float* smem, TmaCtx* tma = nullptr) {
+  __device__ static void run(const RavuArgs& p, int f, int x0, int y0, float* smem, TmaCtx* tma = nullptr) {
     float* tin = smem;                      // input, rows y0-(R-1) ..
     float* t11 = smem + PL * TW * TH;       // int11, rows y0-R ..
     const size_t plane = (size_t)p.W * p.H;
@@ -657,13 +669,13 @@ struct LatticeTile {
       TileStage<CM, TH, kThreads, float> st;
       const RavuArgs& p;
       float* t11;
-      int x0, y0;
+      int f, x0, y0;
       __device__ __forceinline__ void load() {
-        st.load([&](int c, int& pitch) { pitch = p.W; return p.i11 + (size_t)c * p.W * p.H; }, p.W, p.H, x0, y0);
+        st.load([&](int c, int& pitch) { pitch = p.W; return p.i11 + (size_t)(f * C + c) * p.W * p.H; }, p.W, p.H, x0, y0);
       }
       __device__ __forceinline__ void store() { st.store(t11); }
-    } i11{{}, p, t11, x0, y0 - R};
-    if (!stage_frame<CM, TH, kThreads, T>(p, tma, x0, y0 - (R - 1), tin, i11)) return;
+    } i11{{}, p, t11, f, x0, y0 - R};
+    if (!stage_frame<CM, TH, kThreads, T>(p, tma, f, x0, y0 - (R - 1), tin, i11)) return;
     __syncthreads();
     const int tx = threadIdx.x % kTileW, ty = threadIdx.x / kTileW * P;
     const int gx = x0 + tx, gy = y0 + ty;
@@ -715,7 +727,7 @@ struct LatticeTile {
             }
           }
         }
-        T* o = static_cast<T*>(p.out[c]) + (size_t)(2 * (gy + down)) * p.out_pitch[c] + 2 * gx;
+        T* o = plane_out<T>(p, c, f) + (size_t)(2 * (gy + down)) * p.out_pitch[c] + 2 * gx;
         // row 2i: input, int10; row 2i+1: int01, int11 (ravu-r3.hook:424-437)
         stp2(o, bin[c * TW * TH + down * TW], clampf(acc[0].x + acc[0].y, 0.f, 1.f));
         stp2(o + p.out_pitch[c], clampf(acc[1].x + acc[1].y, 0.f, 1.f), b11[c * TW * TH + down * TW]);
@@ -883,7 +895,7 @@ struct ZoomTile {
     if constexpr (CM == kRgb) tile[C * RP * RH + at] = rgb_luma(v[0], v[1], v[2]);
   }
 
-  __device__ static void run(const RavuArgs& p, int X0, int Y0, float* smem, TmaCtx* tma = nullptr) {
+  __device__ static void run(const RavuArgs& p, int f, int X0, int Y0, float* smem, TmaCtx* tma = nullptr) {
     float* tile = smem;
     ZoomPos* pos = reinterpret_cast<ZoomPos*>(reinterpret_cast<unsigned char*>(smem) + kPosAt);
     const int X1 = min(X0 + kTileW - 1, p.OW - 1), Y1 = min(Y0 + TR - 1, p.OH - 1);
@@ -929,7 +941,7 @@ struct ZoomTile {
       };
 #pragma unroll
       for (int c = 0; c < C; c++) {
-        const T* in = static_cast<const T*>(p.in[c]);
+        const T* in = plane_in<T>(p, c, f);
         const int pitch = p.in_pitch[c];
         const bool aligned = quads_aligned(in, pitch);
         each([&](int k, int ty, int tx) {
@@ -1026,13 +1038,14 @@ struct ZoomTile {
 #pragma unroll
     for (int c = 0; c < C; c++) {
       const float r = res[c].x + res[c].y;
-      stp(static_cast<T*>(p.out[c]) + (size_t)Y * p.out_pitch[c] + X,
+      stp(plane_out<T>(p, c, f) + (size_t)Y * p.out_pitch[c] + X,
           AR ? ar_finish(r, G[c], M[c], p.ar) : clampf(r, 0.f, 1.f));
     }
   }
 };
 
-// One CTA per tile of a single frame; with TMA the frame tile of interior
+// One CTA per tile of a frame (grid z: the frame); with TMA (one frame a
+// launch) the frame tile of interior
 // tiles comes in by cp.async.bulk.tensor.
 template <class Prog, bool TMA>
 __device__ __forceinline__ void tile_body(const RavuArgs& p, const TmaMaps& maps) {
@@ -1044,10 +1057,10 @@ __device__ __forceinline__ void tile_body(const RavuArgs& p, const TmaMaps& maps
     __syncthreads();
     TmaCtx ctx{maps.map, smem_u32(&mbar),
                reinterpret_cast<unsigned char*>(tile_smem) + ((Prog::smem_bytes + 127) & ~(size_t)127), 0u, 0};
-    Prog::run(p, blockIdx.x * kTileW, blockIdx.y * Prog::kRows, smem, &ctx);
+    Prog::run(p, 0, blockIdx.x * kTileW, blockIdx.y * Prog::kRows, smem, &ctx);
     tma_drain(&ctx);
   } else {
-    Prog::run(p, blockIdx.x * kTileW, blockIdx.y * Prog::kRows, smem, nullptr);
+    Prog::run(p, blockIdx.z, blockIdx.x * kTileW, blockIdx.y * Prog::kRows, smem, nullptr);
   }
 }
 
@@ -1152,7 +1165,8 @@ int launch_tiles(const RavuArgs& a, cudaStream_t s) {
       return launch_tile_kernel<Prog, true, smem>(dim3(tiles_w, tiles_h), s, b, maps);
     }
   }
-  return launch_tile_kernel<Prog, false, Prog::smem_bytes>(dim3(tiles_w, tiles_h), s, a, maps);
+  return launch_tile_kernel<Prog, false, Prog::smem_bytes>(dim3(tiles_w, tiles_h, a.frames > 0 ? a.frames : 1), s, a,
+                                                            maps);
 }
 
 // ------------------------------------------------------ persistent batches ---
@@ -1242,7 +1256,7 @@ __device__ __forceinline__ void persistent_body(const DevJob* __restrict__ jobs,
     // No barrier after the tile: the next tile's staging and argument copy
     // come after the next claim barrier, which every thread reaches only
     // when done with this tile.
-    Prog::run(s_args, (t % tw) * kTileW, (t / tw) * Prog::kRows, smem, Prog::kPlanes > 0 ? &ctx : nullptr);
+    Prog::run(s_args, 0, (t % tw) * kTileW, (t / tw) * Prog::kRows, smem, Prog::kPlanes > 0 ? &ctx : nullptr);
   }
   tma_drain(&ctx);
 }

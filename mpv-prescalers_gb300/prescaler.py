@@ -414,9 +414,11 @@ class HookModel:
             return "general"
         OW, OH = plan.out_size
         n, c = shape[0] if d == 4 else 1, self.n_planes
+        # scratch for every frame (one launch per pass), unless that is much memory
+        scratch = plan.scratch * n if self.family in ("ravu", "nnedi3") and plan.scratch * n <= 1 << 30 else plan.scratch
         return (shape[:-2] + (OH, OW), (st[0] if d == 4 else 0, st[-3] if d > 2 else 0, st[-2]),
                 (c * OH * OW, OH * OW, OW, n, W, H, _ffi.PZ_F32 if dtype is torch.float32 else _ffi.PZ_F16),
-                plan.scratch, plan.opts)
+                scratch, plan.opts)
 
     _PLANS_KEEP = 256   # frame geometries whose plans are kept
 
