@@ -35,10 +35,10 @@
 // Bound by issue and latency in the blend (12 packed or scalar instructions
 // and 6 MUFU for four neurons) at four warps a scheduler (60 % issue, 37 % MUFU,
 // 23 % tensor pipe; 96 registers and 512 TMEM columns allow no fifth group).
-// 1080p to 2160p, nns128 8x6: 365 us fast (384 us with scalar sums over neuron
-// pairs; 438 us as four CTAs an SM, each with its own copy of B and a CTA barrier
-// per chunk), 485 us split (523 us; 4919 us on the CUDA cores); nns256 8x6 at
-// 720p 279 us fast (443 us: two CTAs an SM had room).
+// 1080p to 2160p, nns128 8x6: 330 us fast (384 us with scalar sums over neuron
+// pairs and rolled chunks; 438 us as four CTAs an SM, each with its own copy of B
+// and a CTA barrier per chunk), 488 us split (523 us; 4919 us on the CUDA cores);
+// nns256 8x6 at 720p 243 us fast (443 us: two CTAs an SM had room).
 //
 // Every mbarrier wait is bounded (kWaitNs of %globaltimer).  A wait that runs
 // out sets the CTA's abort flag: from then on nobody waits, nothing is stored,
@@ -404,24 +404,33 @@ __global__ void __launch_bounds__(TcShape<WH, NNS, XP, SPLIT>::THREADS, 1) nn_tc
     int c = 0;
     for (; t < ntiles; t += stride) {
       float2 wsum = make_float2(0.0f, 0.0f), vsum = wsum;
-      // the accumulators in steps of 16 neurons, both branches' columns; a
-      // step's loads are in flight during the arithmetic of the step before
+      // the accumulators in steps of 16 neurons, both branches' columns
       float s1[2][16], s2[2][16];
       constexpr int STEPS = NC / 16;
+      // a step's loads are in flight during the arithmetic of the step before,
+      // across chunks too but for the tile's last (the next tile is normalised
+      // before it); the chunks are unrolled, so that no load in flight crosses a
+      // loop's edge.  nns128 8x6 fast, 1080p: rolled 353 us, unrolled 334, and ahead
+      // 330.  Split, the MMAs bound it: ahead loses 2 %, and so does unrolling
+      // from four chunks on (nns128 488 / 498 us, nns64 8x4 at 480p 67 / 63).
+      constexpr bool AHEAD = STEPS == 2 && !SPLIT;
+      constexpr int UNROLL = SPLIT && NCH > 2 ? 1 : NCH;
       auto load = [&](int b, int q) {
         tmem_ld16(lane_addr + b * CCOL + 16 * q, s1[q]);
         tmem_ld16(lane_addr + b * CCOL + NC + 16 * q, s2[q]);
       };
-#pragma unroll 1
+#pragma unroll UNROLL
       for (int k = 0; k < NCH; k++, c++) {
-        const int b = c & 1;
-        (void)wait(&B.full[b], (c >> 1) & 1);
-        tc_fence_after();
-        if (k == NCH - 1 && t + stride < ntiles) {
-          nxt = normalise();
-          prefetch(t + 2 * stride);
+        const int b = NCH % 2 == 0 ? k & 1 : c & 1;
+        if (!AHEAD || k == 0 || k == NCH - 1) {  // not in flight yet
+          (void)wait(&B.full[b], (c >> 1) & 1);
+          tc_fence_after();
+          if (k == NCH - 1 && t + stride < ntiles) {
+            nxt = normalise();
+            prefetch(t + 2 * stride);
+          }
+          load(b, 0);
         }
-        load(b, 0);
 #pragma unroll
         for (int q = 0; q < STEPS; q++) {
           tmem_wait16(s1[q], s2[q]);
@@ -431,6 +440,11 @@ __global__ void __launch_bounds__(TcShape<WH, NNS, XP, SPLIT>::THREADS, 1) nn_tc
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(&B.empty[b]));
+            if (AHEAD && k + 1 < NCH - 1) {
+              (void)wait(&B.full[b ^ 1], ((c + 1) >> 1) & 1);
+              tc_fence_after();
+              load(b ^ 1, 0);
+            }
           }
           // sum of e s / (1 + |s|): neurons j and j+2 (and j+1, j+3) share one
           // reciprocal, of the product of their denominators
