@@ -69,7 +69,7 @@ __global__ void wait_selftest_kernel(int* err, unsigned long long limit_ns) {
     atomicCAS(err, 0, pz::kErrWaitTimeout);
 }
 
-size_t zoom_table_size(const pz_model* m, int W, int H, int OW, int OH, int* px, int* py) {
+size_t zoom_table_size(const pz_model* m, int W, int H, int OW, int OH, pz::FastDiv* px, pz::FastDiv* py) {
   return pz::zoom_table_bytes(m->radius, m->ar != 0.0f, m->lut_rows / 9, W, H, OW, OH, px, py);
 }
 
@@ -481,7 +481,7 @@ size_t pz_scratch_wanted(const pz_model* m, int in_w, int in_h, int dtype, const
   pz_query_result q;
   if (pz_query(m, in_w, in_h, dtype, o, &q)) return 0;
   if (m->family != PZ_RAVU_ZOOM || o->staging) return q.scratch_bytes;
-  int px, py;
+  pz::FastDiv px, py;
   return zoom_table_size(m, in_w, in_h, q.out_width, q.out_height, &px, &py);
 }
 
@@ -610,6 +610,7 @@ static int run_frame(const pz_model* m, const pz_plane* in, int n_in, pz_plane* 
       case PZ_RAVU_3X: rc = pz::launch_3x(a, m->radius, m->channels, dt, s); break;
       case PZ_RAVU: rc = pz::launch_lattice(a, m->radius, m->channels, dt, s); break;
       case PZ_RAVU_ZOOM:
+        pz::zoom_divisors(&a);
         // with scratch for it, the weights of a scale of few phases are formed once
         if (o->scratch && !a.staging && reinterpret_cast<uintptr_t>(o->scratch) % 16 == 0) {
           const size_t need = zoom_table_size(m, W, H, OW, OH, &a.zpx, &a.zpy);

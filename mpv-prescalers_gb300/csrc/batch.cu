@@ -129,6 +129,7 @@ int build_tables(const pz_job* jobs, int n, std::vector<pz::DevJob>* table, pz_b
     a.kp = m->kp;
     d.prog = en.prog;
     const bool zoom = m->family == PZ_RAVU_ZOOM;
+    if (zoom) pz::zoom_divisors(&a);
     const int tw = ((zoom ? a.OW : a.W) + pz::kTileW - 1) / pz::kTileW;
     const int th = ((zoom ? a.OH : a.H) + pz::kBatchTileRows - 1) / pz::kBatchTileRows;
     a.tile_rows = pz::kBatchTileRows;

@@ -33,6 +33,18 @@ struct KeyParams {
 // Device-side error word shared by all kernels: first failure wins.
 enum : int { kErrNone = 0, kErrTileOverflow = 1, kErrWaitTimeout = 2, kErrQueue = 3 };
 
+// t / d for 0 <= t < 2^31 by a multiplication, with the divisor fixed on the host.
+struct FastDiv {
+  uint32_t m, s, d;
+  __device__ __forceinline__ uint32_t operator()(uint32_t t) const { return (__umulhi(t, m) + t) >> s; }
+};
+inline FastDiv fast_div(uint32_t d) {
+  FastDiv f{0, 0, d};
+  while ((1ull << f.s) < d) f.s++;
+  f.m = (uint32_t)(((1ull << 32) * ((1ull << f.s) - d)) / d + 1);
+  return f;
+}
+
 // ------------------------------------------------------------- plane I/O --
 __device__ __forceinline__ float ldp(const float* p) { return __ldg(p); }
 __device__ __forceinline__ float ldp(const __half* p) {

@@ -33,7 +33,8 @@ struct RavuArgs {
   int lut_h_pitch;     // texels per FP16 LUT row (even)
   int box_w, box_h;    // ravu-zoom TMA staging: the box of this launch's tensor maps (texels x rows)
   const float4* ztab;  // ravu-zoom: every key's weights at every phase of the scale (zoom_table_kernel), or null
-  int zpx, zpy;        // phases per axis: out / gcd(in, out)
+  FastDiv zpx, zpy;    // phases per axis: out / gcd(in, out)
+  FastDiv zx, zy;      // ravu-zoom: 2 * out per axis (d = 0: positions need 64 bits)
   float* i11;          // ravu lattice: int11 plane, FP32 [C][H][W] (scratch)
   int i11_half;        // round int11 to FP16 before storing it (the mpv form)
   KeyParams kp;
@@ -63,9 +64,15 @@ int launch_lite(const RavuArgs& a, int radius, bool ar, int dtype, cudaStream_t 
 int launch_3x(const RavuArgs& a, int radius, int chmode, int dtype, cudaStream_t s);
 int launch_lattice(const RavuArgs& a, int radius, int chmode, int dtype, cudaStream_t s);
 int launch_zoom(const RavuArgs& a, int radius, int chmode, bool ar, int dtype, cudaStream_t s);
+// The divisors of ravu-zoom's source positions ((2X + 1) W - OW) / (2 OW).
+inline void zoom_divisors(RavuArgs* a) {
+  const bool fits = (2ll * a->OW + 1) * a->W < 1ll << 31 && (2ll * a->OH + 1) * a->H < 1ll << 31;
+  a->zx = fits ? fast_div(2 * a->OW) : FastDiv{0, 0, 0};
+  a->zy = fits ? fast_div(2 * a->OH) : FastDiv{0, 0, 0};
+}
 // ravu-zoom's weight table for a scale of few phases: its bytes (0: too many
 // phases for the frame), and the launch that fills a.ztab.
-size_t zoom_table_bytes(int radius, bool ar, int keys, int W, int H, int OW, int OH, int* px, int* py);
+size_t zoom_table_bytes(int radius, bool ar, int keys, int W, int H, int OW, int OH, FastDiv* px, FastDiv* py);
 int launch_zoom_table(const RavuArgs& a, int radius, bool ar, cudaStream_t s);
 int launch_nnedi3_simt(const NnArgs& a, bool xpass, int dtype, cudaStream_t s);
 int launch_nnedi3_tc(const NnArgs& a, bool xpass, int dtype, cudaStream_t s);

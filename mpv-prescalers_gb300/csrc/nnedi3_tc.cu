@@ -158,20 +158,9 @@ struct TcShape {
   static_assert(NG >= 1 && NG * 2 * CCOL <= 512, "operands must fit shared and tensor memory");
 };
 
-// t / d for 0 <= t < 2^31 by a multiplication (t advances by hundreds of tiles,
-// and a division costs as much as a neuron pair).
-struct FastDiv {
-  uint32_t m, s, d;
-  __host__ explicit FastDiv(uint32_t div) : d(div) {
-    s = 0;
-    while ((1ull << s) < div) s++;
-    m = (uint32_t)(((1ull << 32) * ((1ull << s) - div)) / div + 1);
-  }
-  __device__ __forceinline__ uint32_t operator()(uint32_t t) const { return (__umulhi(t, m) + t) >> s; }
-};
 // The tiles of a launch: 32 x 4 pixels, row by row, frame after frame.
 struct Tiles {
-  FastDiv x, y;  // tiles per row, rows of tiles per frame
+  FastDiv x, y;  // tiles per row, rows of tiles per frame (a division costs as much as a neuron pair)
   int n;
 };
 
@@ -506,7 +495,7 @@ int launch_one(const NnArgs& a, cudaStream_t s) {
     configured[dev] = true;
   }
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  Tiles tiles{FastDiv((a.W + 31) / 32), FastDiv((a.H + 3) / 4), 0};
+  Tiles tiles{fast_div((a.W + 31) / 32), fast_div((a.H + 3) / 4), 0};
   tiles.n = (int)(tiles.x.d * tiles.y.d) * (a.frames > 0 ? a.frames : 1);
   kern<<<tiles.n < sms ? tiles.n : sms, S::THREADS, S::SMEM, s>>>(a, tiles);
   return 0;

@@ -742,8 +742,14 @@ struct ZoomPos {
   float s;  // fract(pos - 0.5)
 };
 
-// pos - 0.5 = ((2X+1) W - OW) / (2 OW), taken exactly (centre-aligned map).
-__device__ __forceinline__ ZoomPos zoom_pos(int X, int W, int OW) {
+// pos - 0.5 = ((2X+1) W - OW) / (2 OW), taken exactly (centre-aligned map);
+// `d`: 2 OW, or d.d = 0 where the numerator needs 64 bits.
+__device__ __forceinline__ ZoomPos zoom_pos(int X, int W, int OW, const FastDiv& d) {
+  if (d.d) {
+    const int num = (2 * X + 1) * W - OW;  // > -2 OW: W < OW
+    const int q = num < 0 ? -1 : (int)d(num);
+    return {q, (float)(num - q * (int)d.d) / (float)(int)d.d};
+  }
   const long long num = (2LL * X + 1) * W - OW;
   const long long den = 2LL * OW;
   const long long q = num >= 0 ? num / den : -((-num + den - 1) / den);
@@ -834,11 +840,11 @@ template <int R, bool AR, bool H16>
 __global__ void zoom_table_kernel(const __grid_constant__ RavuArgs p, float4* out) {
   constexpr int NB = zoom_texels<R>(), NT2 = (NB + 1) / 2, PER = NT2 * (AR ? 4 : 2);
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int n = p.lut_rows / 9 * p.zpx * p.zpy;
+  const int phases = (int)(p.zpx.d * p.zpy.d), n = p.lut_rows / 9 * phases;
   if (i >= n * PER) return;
   const int entry = i / PER, t = i % PER % NT2, part = i % PER / NT2;  // part: halves, then the AR halves
-  const int key = entry / (p.zpx * p.zpy), phase = entry % (p.zpx * p.zpy);
-  float sx = zoom_pos(phase % p.zpx, p.W, p.OW).s, sy = zoom_pos(phase / p.zpx, p.H, p.OH).s;
+  const int key = entry / phases, phase = entry % phases, py = p.zpx(phase), px = phase - py * (int)p.zpx.d;
+  float sx = zoom_pos(px, p.W, p.OW, p.zx).s, sy = zoom_pos(py, p.H, p.OH, p.zy).s;
   if (part & 1) {
     sx = 1.0f - sx;
     sy = 1.0f - sy;
@@ -862,7 +868,7 @@ __global__ void zoom_table_kernel(const __grid_constant__ RavuArgs p, float4* ou
 // Bound by L1, where the gathers of LUT texels go (86 %; 16-40 loads a pixel).
 // 1080p to 1.5x, without / with the phase table: ravu-zoom-r2 86 / 62 us fast (132
 // with a load per texel, scalar blends and texel staging), r3 FP32 283 / 111 us
-// (290), ravu-zoom-ar-r2-rgb fast 274 / 187 us (302).
+// (290), ravu-zoom-ar-r2-rgb fast 274 / 165 us (302).
 // TAB: the weights come from the launch's phase table, at the same bits.
 template <int R, int CM, bool AR, typename T, bool H16 = false, int TR = 8, bool TAB = false>
 struct ZoomTile {
@@ -874,10 +880,13 @@ struct ZoomTile {
   static constexpr int C = CM == kLuma ? 1 : 3;
   static constexpr int PL = C + (CM == kRgb ? 1 : 0);
   static constexpr int NT2 = (zoom_texels<R>() + 1) / 2;  // texel pairs of a LUT point
-  // input rectangle planes, then the source positions of the tile's 32 columns
-  // and TR rows
-  static constexpr size_t kPosAt = (size_t)PL * RP * RH * 4;
-  static constexpr size_t smem_bytes = kPosAt + (kTileW + TR) * sizeof(ZoomPos);
+  // input rectangle planes, then the powers of the first CT channels: with the
+  // phase table's weights and three channels, forming all powers per tap keeps
+  // the FMA pipe 75 % busy, L1 58 %; two channels' powers from shared memory, once
+  // per texel, balance them (1080p to 1.5x: 0 / 1 / 2 / 3 channels 187 / 177 / 171 /
+  // 179 us; to 2.25x 412 / 397 / 397 / 428; luma at 1.75x 73 / 78)
+  static constexpr int CT = AR && TAB && C == 3 ? 2 : 0;
+  static constexpr size_t smem_bytes = (size_t)(PL + 2 * CT) * RP * RH * 4;
 
   static constexpr int kPlanes = C;
   static constexpr bool kTma = !TAB;  // the table goes with plain loads
@@ -897,18 +906,17 @@ struct ZoomTile {
 
   __device__ static void run(const RavuArgs& p, int f, int X0, int Y0, float* smem, TmaCtx* tma = nullptr) {
     float* tile = smem;
-    ZoomPos* pos = reinterpret_cast<ZoomPos*>(reinterpret_cast<unsigned char*>(smem) + kPosAt);
-    const int X1 = min(X0 + kTileW - 1, p.OW - 1), Y1 = min(Y0 + TR - 1, p.OH - 1);
-    static_assert(kThreads >= kTileW + TR, "one thread per tile column and row");
-    if (threadIdx.x < kTileW + TR) {  // one exact position per tile column / row
-      const int t = threadIdx.x;
-      const int o = t < kTileW ? min(X0 + t, X1) : min(Y0 + t - kTileW, Y1);
-      pos[t] = t < kTileW ? zoom_pos(o, p.W, p.OW) : zoom_pos(o, p.H, p.OH);
-      if (TAB) pos[t].s = __int_as_float(t < kTileW ? o % p.zpx : o % p.zpy);  // its phase instead
-    }
-    __syncthreads();
-    const int rx = pos[0].i - LO, ry = pos[kTileW].i - LO;
-    const int rw = pos[X1 - X0].i + R - rx + 1, rh = pos[kTileW + Y1 - Y0].i + R - ry + 1;
+    float2* pow = reinterpret_cast<float2*>(smem + PL * RP * RH);
+    // exact source positions: lane l of every warp takes column X0 + l and row
+    // Y0 + min(l, TR - 1); the tile's corners and the warp's own row come by shuffles
+    // (no barrier; as 64-bit divisions shared through memory they held every tile
+    // up: ravu-zoom-ar-r2-rgb at 1.5x 171 us, now 165; -ar-r2 at 2.25x 252, now 223)
+    const int lane = threadIdx.x % kTileW, warp = threadIdx.x / kTileW;
+    const int X = X0 + lane, Y = Y0 + warp, oy = min(Y0 + min(lane, TR - 1), p.OH - 1);
+    ZoomPos px = zoom_pos(min(X, p.OW - 1), p.W, p.OW, p.zx), rows = zoom_pos(oy, p.H, p.OH, p.zy);
+    const ZoomPos py = {__shfl_sync(~0u, rows.i, warp), __shfl_sync(~0u, rows.s, warp)};
+    const int rx = __shfl_sync(~0u, px.i, 0) - LO, ry = __shfl_sync(~0u, rows.i, 0) - LO;
+    const int rw = __shfl_sync(~0u, px.i, 31) + R - rx + 1, rh = __shfl_sync(~0u, rows.i, 31) + R - ry + 1;
     if (rw > RW || rh > RH) {  // only reachable when downscaling, which the host rejects
       if (threadIdx.x == 0 && p.err) atomicCAS(p.err, 0, kErrTileOverflow);
       return;
@@ -954,16 +962,22 @@ struct ZoomTile {
         for (int c = 0; c < C; c++) v[c] = q[c][k].get();
         float4* t4 = reinterpret_cast<float4*>(tile + ty * RP + tx);
 #pragma unroll
-        for (int c = 0; c < C; c++) t4[c * (RP * RH / 4)] = v[c];
+        for (int c = 0; c < C; c++) {
+          t4[c * (RP * RH / 4)] = v[c];
+          if (c < CT) {
+            const float2 a = ar_pow32(v[c].x), b = ar_pow32(v[c].y), e = ar_pow32(v[c].z), d = ar_pow32(v[c].w);
+            float4* p4 = reinterpret_cast<float4*>(pow + c * RP * RH + ty * RP + tx);
+            p4[0] = make_float4(a.x, a.y, b.x, b.y);
+            p4[1] = make_float4(e.x, e.y, d.x, d.y);
+          }
+        }
         if constexpr (CM == kRgb)
           t4[C * (RP * RH / 4)] = make_float4(rgb_luma(v[0].x, v[1].x, v[2].x), rgb_luma(v[0].y, v[1].y, v[2].y),
                                               rgb_luma(v[0].z, v[1].z, v[2].z), rgb_luma(v[0].w, v[1].w, v[2].w));
       });
     }
     __syncthreads();
-    const int X = X0 + threadIdx.x % kTileW, Y = Y0 + threadIdx.x / kTileW;
     if (X >= p.OW || Y >= p.OH) return;
-    const ZoomPos px = pos[threadIdx.x % kTileW], py = pos[kTileW + threadIdx.x / kTileW];
     const int at = (py.i - LO - ry) * RP + px.i - LO - rx + off;  // window origin in the tile
     const float* base = tile + at;
     auto val = [&](int c, int k) { return base[c * RP * RH + k % N * RP + k / N]; };
@@ -978,8 +992,9 @@ struct ZoomTile {
     const float4* entry = nullptr;
     ZoomLut ls, li;
     if constexpr (TAB) {
-      const int k = clampi(key, 0, p.lut_rows / 9 - 1) * p.zpy + __float_as_int(py.s);
-      entry = p.ztab + ((size_t)k * p.zpx + __float_as_int(px.s)) * zoom_entry<R, AR>();
+      const int phx = X - (int)(p.zpx(X) * p.zpx.d), phy = Y - (int)(p.zpy(Y) * p.zpy.d);
+      const int k = clampi(key, 0, p.lut_rows / 9 - 1) * (int)p.zpy.d + phy;
+      entry = p.ztab + ((size_t)k * p.zpx.d + phx) * zoom_entry<R, AR>();
     } else {
       ls = ZoomLut(p.lut_rows, key, px.s, py.s, p.lut_frac);
       li = ZoomLut(p.lut_rows, key, 1.0f - px.s, 1.0f - py.s, p.lut_frac);
@@ -1022,15 +1037,15 @@ struct ZoomTile {
           res[c] = __ffma2_rn(make_float2(va[0], va[1]), ws[j], res[c]);
           res[c] = __ffma2_rn(make_float2(vb[0], vb[1]), wi[j], res[c]);
           if constexpr (AR) {
-            auto tap = [&](float v, float g) {
-              const float2 h = ar_pow32(v);
+            auto tap = [&](float v, int k, float g) {
+              const float2 h = c < CT ? pow[c * RP * RH + at + k % N * RP + k / N] : ar_pow32(v);
               G[c] = __ffma2_rn(h, make_float2(g, g), G[c]);
               M[c] = __ffma2_rn(__fmul2_rn(h, make_float2(v, v)), make_float2(g, g), M[c]);
             };
-            tap(va[0], gs[j].x);
-            tap(va[1], gs[j].y);
-            tap(vb[0], gi[j].x);
-            tap(vb[1], gi[j].y);
+            tap(va[0], i, gs[j].x);
+            tap(va[1], i + 1, gs[j].y);
+            tap(vb[0], S - 1 - i, gi[j].x);
+            tap(vb[1], S - 2 - i, gi[j].y);
           }
         }
       }

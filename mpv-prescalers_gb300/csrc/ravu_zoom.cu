@@ -38,7 +38,7 @@ int gcd(int a, int b) {
 
 template <int R, bool AR>
 void launch_table(const RavuArgs& a, cudaStream_t s) {
-  const int n = a.lut_rows / 9 * a.zpx * a.zpy * ((zoom_texels<R>() + 1) / 2) * (AR ? 4 : 2);
+  const int n = a.lut_rows / 9 * (int)(a.zpx.d * a.zpy.d) * ((zoom_texels<R>() + 1) / 2) * (AR ? 4 : 2);
   float4* out = const_cast<float4*>(a.ztab);
   if (a.lut_h) zoom_table_kernel<R, AR, true><<<(n + 127) / 128, 128, 0, s>>>(a, out);
   else zoom_table_kernel<R, AR, false><<<(n + 127) / 128, 128, 0, s>>>(a, out);
@@ -53,10 +53,11 @@ void launch_table(const RavuArgs& a, cudaStream_t s) {
 // (ravu-zoom-r2); 720x576 to 1080p, 120 phases and 60 pixels an entry, 38 against
 // 60 us; 854x480 to 1.75x, 49 phases and 89 pixels an entry, 63 against 68 us.
 // Scales of no simple ratio have as many phases as pixels and take none.
-size_t zoom_table_bytes(int radius, bool ar, int keys, int W, int H, int OW, int OH, int* px, int* py) {
-  *px = OW / gcd(W, OW);
-  *py = OH / gcd(H, OH);
-  const long long entries = (long long)keys * *px * *py, pixels = (long long)OW * OH;
+size_t zoom_table_bytes(int radius, bool ar, int keys, int W, int H, int OW, int OH, FastDiv* px,
+                        FastDiv* py) {
+  *px = fast_div(OW / gcd(W, OW));
+  *py = fast_div(OH / gcd(H, OH));
+  const long long entries = (long long)keys * px->d * py->d, pixels = (long long)OW * OH;
   if (pixels < 1 << 19 || entries * 8 > pixels) return 0;
   const uint32_t e = radius == 2 ? (ar ? zoom_entry<2, true>() : zoom_entry<2, false>())
                                  : (ar ? zoom_entry<3, true>() : zoom_entry<3, false>());
