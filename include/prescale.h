@@ -306,6 +306,9 @@ int pz_nnedi3_run_static(const pz_model* model, const pz_plane* in, pz_plane* ou
 typedef enum { PZ_FILTER_BILINEAR = 0, PZ_FILTER_CATMULL_ROM = 1 } pz_filter;
 int pz_resample(const pz_plane* in, pz_plane* out, float sx, float ox, float sy, float oy, int filter,
                 void* cuda_stream);
+/* The same for 1 to 4 planes that share sizes and dtype, in one launch. */
+int pz_resample_planes(const pz_plane* in, pz_plane* out, int n_planes, float sx, float ox, float sy, float oy,
+                       int filter, void* cuda_stream);
 
 #ifdef __cplusplus
 }

@@ -107,6 +107,9 @@ EXPORTS = {
                                    ctypes.c_size_t, ctypes.c_int, ctypes.c_void_p]),
     "pz_resample": (ctypes.c_int, [ctypes.POINTER(Plane), ctypes.POINTER(Plane), ctypes.c_float, ctypes.c_float,
                                    ctypes.c_float, ctypes.c_float, ctypes.c_int, ctypes.c_void_p]),
+    "pz_resample_planes": (ctypes.c_int, [ctypes.POINTER(Plane), ctypes.POINTER(Plane), ctypes.c_int, ctypes.c_float,
+                                          ctypes.c_float, ctypes.c_float, ctypes.c_float, ctypes.c_int,
+                                          ctypes.c_void_p]),
     "pz_check_device_error": (ctypes.c_int, [ctypes.c_void_p]),
     "pz_selftest_wait": (ctypes.c_int, [ctypes.c_longlong, ctypes.c_void_p]),
 }

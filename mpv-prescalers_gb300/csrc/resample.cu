@@ -23,11 +23,14 @@
 namespace pz {
 namespace {
 
+// Planes of one size (grid z) through one resampling.
+constexpr int kMaxPlanes = 4;
 struct ResampleArgs {
-  const void* in;
-  void* out;
-  int in_w, in_h, in_pitch;
-  int out_w, out_h, out_pitch;
+  const void* in[kMaxPlanes];
+  void* out[kMaxPlanes];
+  int in_pitch[kMaxPlanes], out_pitch[kMaxPlanes];
+  int in_w, in_h;
+  int out_w, out_h;
   float sx, ox, sy, oy;
 };
 
@@ -63,7 +66,8 @@ __device__ __forceinline__ int tap_weights(float s, int x, float o, float (&w)[T
 
 template <int TAPS, typename T>
 __device__ __forceinline__ float resample_one(const ResampleArgs& a, int x, int y) {
-  const T* in = static_cast<const T*>(a.in);
+  const T* in = static_cast<const T*>(a.in[blockIdx.z]);
+  const int pitch = a.in_pitch[blockIdx.z];
   float wx[TAPS], wy[TAPS];
   const int iu = tap_weights<TAPS>(a.sx, x, a.ox, wx), iv = tap_weights<TAPS>(a.sy, y, a.oy, wy);
   constexpr int K0 = TAPS == 2 ? 0 : -1;
@@ -73,7 +77,7 @@ __device__ __forceinline__ float resample_one(const ResampleArgs& a, int x, int 
   float acc = 0.0f;
 #pragma unroll
   for (int j = 0; j < TAPS; j++) {
-    const T* row = in + (size_t)clampi(iv + K0 + j, 0, a.in_h - 1) * a.in_pitch;
+    const T* row = in + (size_t)clampi(iv + K0 + j, 0, a.in_h - 1) * pitch;
     float r = 0.0f;
 #pragma unroll
     for (int i = 0; i < TAPS; i++) r += wx[i] * ldp(row + cx[i]);
@@ -83,11 +87,11 @@ __device__ __forceinline__ float resample_one(const ResampleArgs& a, int x, int 
 }
 
 template <int TAPS, typename T>
-__global__ void __launch_bounds__(256) resample_kernel(const ResampleArgs a) {
+__global__ void __launch_bounds__(256) resample_kernel(const __grid_constant__ ResampleArgs a) {
   const int x = blockIdx.x * 32 + (threadIdx.x & 31);
   const int y = blockIdx.y * 8 + (threadIdx.x >> 5);
   if (x >= a.out_w || y >= a.out_h) return;
-  stp(static_cast<T*>(a.out) + (size_t)y * a.out_pitch + x, resample_one<TAPS, T>(a, x, y));
+  stp(static_cast<T*>(a.out[blockIdx.z]) + (size_t)y * a.out_pitch[blockIdx.z] + x, resample_one<TAPS, T>(a, x, y));
 }
 
 // Shifts: one thread per 4 x 4 block of outputs.  Neighbouring outputs share
@@ -101,11 +105,12 @@ __global__ void __launch_bounds__(256) resample_kernel(const ResampleArgs a) {
 // texel by texel.  Catmull-Rom, 3840x2160 FP16: 20.5 us (61.6 us), 2560x1440 10.4
 // (28.9); bilinear 10.7 (26.7).
 template <int TAPS, int OFF, typename T>
-__global__ void __launch_bounds__(256) shift_kernel(const ResampleArgs a) {
+__global__ void __launch_bounds__(256) shift_kernel(const __grid_constant__ ResampleArgs a) {
   constexpr int K0 = TAPS == 2 ? 0 : -1, QUADS = (OFF + TAPS + 3 + 3) / 4;
   const int X = (blockIdx.x * 32 + (threadIdx.x & 31)) * 4, Y = (blockIdx.y * 8 + (threadIdx.x >> 5)) * 4;
   if (X >= a.out_w || Y >= a.out_h) return;
-  T* out = static_cast<T*>(a.out) + (size_t)Y * a.out_pitch + X;
+  const int in_pitch = a.in_pitch[blockIdx.z], out_pitch = a.out_pitch[blockIdx.z];
+  T* out = static_cast<T*>(a.out[blockIdx.z]) + (size_t)Y * out_pitch + X;
   const int nx = min(4, a.out_w - X), ny = min(4, a.out_h - Y);
   float wx[4][TAPS], wy[4][TAPS];
   int iu[4], iv[4];
@@ -120,11 +125,11 @@ __global__ void __launch_bounds__(256) shift_kernel(const ResampleArgs a) {
   for (int k = 1; k < 4; k++) whole = whole && iu[k] == iu[0] + k && iv[k] == iv[0] + k;
   if (!whole) {
     for (int j = 0; j < ny; j++)
-      for (int i = 0; i < nx; i++) stp(out + (size_t)j * a.out_pitch + i, resample_one<TAPS, T>(a, X + i, Y + j));
+      for (int i = 0; i < nx; i++) stp(out + (size_t)j * out_pitch + i, resample_one<TAPS, T>(a, X + i, Y + j));
     return;
   }
-  const T* in = static_cast<const T*>(a.in);
-  const bool aligned = quads_aligned(in, a.in_pitch);
+  const T* in = static_cast<const T*>(a.in[blockIdx.z]);
+  const bool aligned = quads_aligned(in, in_pitch);
   float acc[4][4];
 #pragma unroll
   for (int j = 0; j < 4; j++)
@@ -132,7 +137,7 @@ __global__ void __launch_bounds__(256) shift_kernel(const ResampleArgs a) {
     for (int i = 0; i < 4; i++) acc[j][i] = 0.0f;
 #pragma unroll
   for (int row = 0; row < TAPS + 3; row++) {
-    const T* src = in + (size_t)clampi(iv[0] + K0 + row, 0, a.in_h - 1) * a.in_pitch;
+    const T* src = in + (size_t)clampi(iv[0] + K0 + row, 0, a.in_h - 1) * in_pitch;
     float v[QUADS * 4];
 #pragma unroll
     for (int q = 0; q < QUADS; q++) {
@@ -154,11 +159,11 @@ __global__ void __launch_bounds__(256) shift_kernel(const ResampleArgs a) {
         if (row - j >= 0 && row - j < TAPS) acc[j][i] += wy[j][row - j] * r;
     }
   }
-  const bool quads = nx == 4 && quads_aligned(static_cast<const T*>(a.out), a.out_pitch);
+  const bool quads = nx == 4 && quads_aligned(static_cast<const T*>(a.out[blockIdx.z]), out_pitch);
 #pragma unroll
   for (int j = 0; j < 4; j++) {
     if (j >= ny) break;
-    T* o = out + (size_t)j * a.out_pitch;
+    T* o = out + (size_t)j * out_pitch;
     if (quads) {
       st_quad(o, acc[j]);
     } else {
@@ -168,12 +173,12 @@ __global__ void __launch_bounds__(256) shift_kernel(const ResampleArgs a) {
 }
 
 template <int TAPS, typename T>
-void launch_resample(const ResampleArgs& a, cudaStream_t s) {
+void launch_resample(const ResampleArgs& a, int planes, cudaStream_t s) {
   if (a.sx != 1.0f || a.sy != 1.0f) {
-    resample_kernel<TAPS, T><<<dim3((a.out_w + 31) / 32, (a.out_h + 7) / 8), 256, 0, s>>>(a);
+    resample_kernel<TAPS, T><<<dim3((a.out_w + 31) / 32, (a.out_h + 7) / 8, planes), 256, 0, s>>>(a);
     return;
   }
-  const dim3 grid((a.out_w + 127) / 128, (a.out_h + 31) / 32);
+  const dim3 grid((a.out_w + 127) / 128, (a.out_h + 31) / 32, planes);
   switch (((int)floorf(a.ox) + (TAPS == 2 ? 0 : -1)) & 3) {
     case 0: shift_kernel<TAPS, 0, T><<<grid, 256, 0, s>>>(a); break;
     case 1: shift_kernel<TAPS, 1, T><<<grid, 256, 0, s>>>(a); break;
@@ -197,9 +202,27 @@ int check_rs_plane(const pz_plane* p, const char* what) {
 
 extern "C" int pz_resample(const pz_plane* in, pz_plane* out, float sx, float ox, float sy, float oy, int filter,
                            void* stream) {
-  int rc;
-  if ((rc = pz::check_rs_plane(in, "in")) || (rc = pz::check_rs_plane(out, "out"))) return rc;
-  if (in->dtype != out->dtype) return pz::set_error(PZ_EINVAL, "input and output dtypes differ");
+  return pz_resample_planes(in, out, 1, sx, ox, sy, oy, filter, stream);
+}
+
+extern "C" int pz_resample_planes(const pz_plane* in, pz_plane* out, int n_planes, float sx, float ox, float sy,
+                                  float oy, int filter, void* stream) {
+  if (n_planes < 1 || n_planes > pz::kMaxPlanes)
+    return pz::set_error(PZ_EINVAL, "%d planes: 1 to %d", n_planes, pz::kMaxPlanes);
+  pz::ResampleArgs a{};
+  for (int c = 0; c < n_planes; c++) {
+    int rc;
+    if ((rc = pz::check_rs_plane(in ? in + c : nullptr, "in")) || (rc = pz::check_rs_plane(out ? out + c : nullptr, "out")))
+      return rc;
+    if (in[c].dtype != out[c].dtype) return pz::set_error(PZ_EINVAL, "input and output dtypes differ");
+    if (in[c].width != in->width || in[c].height != in->height || out[c].width != out->width ||
+        out[c].height != out->height || in[c].dtype != in->dtype)
+      return pz::set_error(PZ_EINVAL, "the planes of one call share sizes and dtype");
+    a.in[c] = in[c].data;
+    a.out[c] = out[c].data;
+    a.in_pitch[c] = in[c].pitch;
+    a.out_pitch[c] = out[c].pitch;
+  }
   if (filter != PZ_FILTER_BILINEAR && filter != PZ_FILTER_CATMULL_ROM)
     return pz::set_error(PZ_EINVAL, "unknown filter %d", filter);
   // every sample position must stay a finite float well inside int range
@@ -208,12 +231,20 @@ extern "C" int pz_resample(const pz_plane* in, pz_plane* out, float sx, float ox
   const float vy0 = oy, vy1 = sy * (float)(out->height - 1) + oy;
   if (!(fabsf(ux0) < lim && fabsf(ux1) < lim && fabsf(vy0) < lim && fabsf(vy1) < lim))
     return pz::set_error(PZ_EINVAL, "sample positions out of range");
-  pz::ResampleArgs a{in->data, out->data, in->width, in->height, in->pitch,
-                     out->width, out->height, out->pitch, sx, ox, sy, oy};
+  a.in_w = in->width;
+  a.in_h = in->height;
+  a.out_w = out->width;
+  a.out_h = out->height;
+  a.sx = sx;
+  a.ox = ox;
+  a.sy = sy;
+  a.oy = oy;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const bool f16 = in->dtype == PZ_F16;
-  if (filter == PZ_FILTER_BILINEAR) f16 ? pz::launch_resample<2, __half>(a, s) : pz::launch_resample<2, float>(a, s);
-  else f16 ? pz::launch_resample<4, __half>(a, s) : pz::launch_resample<4, float>(a, s);
+  if (filter == PZ_FILTER_BILINEAR)
+    f16 ? pz::launch_resample<2, __half>(a, n_planes, s) : pz::launch_resample<2, float>(a, n_planes, s);
+  else
+    f16 ? pz::launch_resample<4, __half>(a, n_planes, s) : pz::launch_resample<4, float>(a, n_planes, s);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return pz::set_error(PZ_EIO, "resample launch: %s", cudaGetErrorString(e));
   return PZ_OK;

@@ -141,21 +141,36 @@ def resample_plane(x, out_w: int, out_h: int, sx: float, ox: float, sy: float, o
                    filt: str = "catmull_rom", out=None, stream=None):
     """``out(x, y) = interp(in, sx*x + ox, sy*y + oy)`` on the device
     (``pz_resample``; texel centres at integers, edges replicated)."""
+    return _resample([x], out_w, out_h, sx, ox, sy, oy, filt, [out], stream)[0]
+
+
+def _resample(xs, out_w, out_h, sx, ox, sy, oy, filt, outs, stream):
+    """:func:`resample_plane` of planes of one size and dtype, in one launch."""
     torch = _torch()
-    if not x.is_cuda or x.dim() != 2 or x.stride(1) != 1:
-        raise ValueError("resample_plane takes a row-contiguous CUDA [H][W] tensor")
-    if x.dtype not in (torch.float32, torch.float16):
-        raise ValueError("planes must be float32 or float16")
+    for x in xs:
+        if not x.is_cuda or x.dim() != 2 or x.stride(1) != 1:
+            raise ValueError("resample_plane takes a row-contiguous CUDA [H][W] tensor")
+        if x.dtype not in (torch.float32, torch.float16):
+            raise ValueError("planes must be float32 or float16")
     if filt not in FILTERS:
         raise ValueError(f"filter {filt!r} not in {sorted(FILTERS)}")
-    if out is None:   # allocated on the stream that writes it
-        with on_stream(x.device, stream):
-            out = torch.empty((out_h, out_w), dtype=x.dtype, device=x.device)
-    dt = _ffi.PZ_F32 if x.dtype == torch.float32 else _ffi.PZ_F16
-    pin = _ffi.Plane(x.data_ptr(), x.shape[1], x.shape[0], x.stride(0), dt)
-    pout = _ffi.Plane(out.data_ptr(), out.shape[1], out.shape[0], out.stride(0), dt)
-    _ffi.check(_ffi.lib().pz_resample(pin, pout, sx, ox, sy, oy, FILTERS[filt], raw_stream(x.device, stream)))
-    return out
+    dev, dtype, n = xs[0].device, xs[0].dtype, len(xs)
+    if outs[0] is None:   # allocated on the stream that writes them
+        with on_stream(dev, stream):
+            outs = list(torch.empty((n, out_h, out_w), dtype=dtype, device=dev).unbind(0))
+    dt = _ffi.PZ_F32 if dtype == torch.float32 else _ffi.PZ_F16
+    pin = (_ffi.Plane * n)(*[(x.data_ptr(), x.shape[1], x.shape[0], x.stride(0), dt) for x in xs])
+    pout = (_ffi.Plane * n)(*[(o.data_ptr(), o.shape[1], o.shape[0], o.stride(0), dt) for o in outs])
+    _ffi.check(_ffi.lib().pz_resample_planes(pin, pout, n, sx, ox, sy, oy, FILTERS[filt], raw_stream(dev, stream)))
+    return outs
+
+
+def _together(xs, *args):
+    """:func:`_resample` in one launch where the planes agree in size, type and
+    device, else one by one."""
+    if all((x.shape, x.dtype, x.device) == (xs[0].shape, xs[0].dtype, xs[0].device) for x in xs):
+        return _resample(xs, *args[:-1], [None] * len(xs), args[-1])
+    return [_resample([x], *args[:-1], [None], args[-1])[0] for x in xs]
 
 
 def prescale_frame(model, frame: Frame, out_size: Optional[Tuple[int, int]] = None, precision: str = "fp32",
@@ -178,8 +193,7 @@ def prescale_frame(model, frame: Frame, out_size: Optional[Tuple[int, int]] = No
     with on_stream(dev, None):
         if plan.upsample_chroma:
             (rx, ry), (lx, ly) = plan.chroma_scale, plan.chroma_origin
-            planes[1:] = [resample_plane(p, W, H, rx, -lx * rx, ry, -ly * ry, cscale, stream=stream)
-                          for p in planes[1:]]
+            planes[1:] = _together(planes[1:], W, H, rx, -lx * rx, ry, -ly * ry, cscale, stream)
         src = [planes[i] for i in plan.prescaled]
         dt = src[0].dtype
         if any(p.dtype != dt for p in src):
@@ -188,7 +202,7 @@ def prescale_frame(model, frame: Frame, out_size: Optional[Tuple[int, int]] = No
         off = plan.offset
         if isinstance(off, tuple) and off != (0.0, 0.0) and offset_filter is not None:
             OW, OH = plan.out_size
-            up = [resample_plane(p, OW, OH, 1.0, off[0], 1.0, off[1], offset_filter, stream=stream) for p in up]
+            up = _together(up, OW, OH, 1.0, off[0], 1.0, off[1], offset_filter, stream)
             off = (0.0, 0.0)
         out = list(frame.planes)
         for i, p in zip(plan.prescaled, up):
