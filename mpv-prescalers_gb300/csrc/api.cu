@@ -90,8 +90,8 @@ int check_plane(const pz_plane& p, const char* what, int idx, bool pairs) {
 }
 
 // The tensor-core operands B [2*nns][KP] of an NNEDI3 model, chunk-major:
-// chunk c of NC neurons (NC = 32, or nns when below) is NC softmax-branch rows
-// followed by NC Elliott-branch rows.  Row = [weights (T taps), sum of the
+// chunk c of NC neurons (nnedi3_tc_chunk) is NC softmax-branch rows followed by
+// NC Elliott-branch rows.  Row = [weights (T taps), sum of the
 // weights, the bias in pieces, 0...]; against A rows [x_hat, mean*invstd, 1, 1,
 // 1, 0...] the MMA yields the whole pre-activation <x,w>*invstd + b.  Softmax
 // rows are scaled by log2(e) so the epilogue takes exp2 directly.  Stored as
@@ -106,14 +106,15 @@ int check_plane(const pz_plane& p, const char* what, int idx, bool pairs) {
 //          when a value is not finite or the power lies outside 2^-8..2^30,
 //          where the blend's products could leave FP32's range.
 int upload_operands(pz_model* m, const std::vector<float>& w, const std::vector<float>& bias) {
-  const int n = m->nns, T = m->win_w * m->win_h, NC = pz::nnedi3_tc_chunk(n);
+  const int n = m->nns, T = m->win_w * m->win_h;
+  const int NCH = pz::nnedi3_tc_chunk(n, m->win_h, false), NCS = pz::nnedi3_tc_chunk(n, m->win_h, true);
   const int KP = (T + 4 + 15) / 16 * 16;  // taps, mean term, three bias pieces, padded to a K step
   const double kLog2e = 1.4426950408889634;
-  std::vector<double> v((size_t)2 * n * (T + 2));  // [row][weights, sum, bias], row as stored
+  std::vector<double> v((size_t)2 * n * (T + 2));  // [2 * neuron + branch][weights, sum, bias]
   double top = 0.0;
   bool finite = true;
   for (int r = 0; r < 2 * n; r++) {
-    const int k = r / (2 * NC) * NC + r % NC, br = r % (2 * NC) / NC;
+    const int k = r / 2, br = r % 2;
     const double scale = br == 0 ? kLog2e : 1.0;
     double* row = &v[(size_t)r * (T + 2)];
     double sum = 0.0;
@@ -134,28 +135,31 @@ int upload_operands(pz_model* m, const std::vector<float>& w, const std::vector<
   const bool split = finite && exp2 >= -8 && exp2 <= 30;
   const __half zero = __float2half_rn(0.0f);
   std::vector<__half> h(piece, zero), s(2 * piece, zero);
-  auto at = [&](int r, int t) { return (size_t)(r >> 3) * 8 * KP + (t >> 3) * 64 + (r & 7) * 8 + (t & 7); };
+  auto at = [&](int row, int t, int NC) {  // element t of the neuron and branch `row`
+    const int k = row / 2, r = k / NC * 2 * NC + row % 2 * NC + k % NC;
+    return (size_t)(r >> 3) * 8 * KP + (t >> 3) * 64 + (r & 7) * 8 + (t & 7);
+  };
   auto half_of = [](double x) { return __float2half_rn((float)x); };
   auto val = [](__half x) { return (double)__half2float(x); };
   for (int r = 0; r < 2 * n; r++) {
     const double* row = &v[(size_t)r * (T + 2)];
     for (int t = 0; t <= T; t++) {
-      h[at(r, t)] = half_of(row[t]);
+      h[at(r, t, NCH)] = half_of(row[t]);
       if (split) {
         const double x = std::ldexp(row[t], exp2);
         const __half hi = half_of(x);
-        s[at(r, t)] = hi;
-        s[piece + at(r, t)] = half_of(x - val(hi));
+        s[at(r, t, NCS)] = hi;
+        s[piece + at(r, t, NCS)] = half_of(x - val(hi));
       }
     }
     double b = row[T + 1], x = split ? std::ldexp(b, exp2) : 0.0;
     for (int t = T + 1; t <= T + 3; t++) {  // two pieces (fast form), three (split)
       if (t < T + 3) {
-        h[at(r, t)] = half_of(b);
-        b -= val(h[at(r, t)]);
+        h[at(r, t, NCH)] = half_of(b);
+        b -= val(h[at(r, t, NCH)]);
       }
-      s[at(r, t)] = half_of(x);
-      x -= val(s[at(r, t)]);
+      s[at(r, t, NCS)] = half_of(x);
+      x -= val(s[at(r, t, NCS)]);
     }
   }
   int rc = upload(&m->d_wts_h, h.data(), piece * 2);

@@ -98,7 +98,7 @@ inline NnArgs nn_args(const pz_model* m, int* err) {
 // One doubling pass in the form `precision` asks for.  The fast form runs
 // its neurons on the tensor cores in FP16; every other form keeps FP32 values
 // and runs them there as two FP16 pieces each.  1080p to 2160p, FP32 planes,
-// split against CUDA cores: nns128 8x6 488 against 4919 us, nns16 8x4 189
+// split against CUDA cores: nns128 8x6 455 against 4919 us, nns16 8x4 189
 // against 491 us; 160x90 nns32 8x4 the same (both are the two launches).  The
 // error against 64 bits is 0.5-0.65x the CUDA cores' for every nns and window
 // (nns128 8x6 at 640x360: 8.6e-8 against 1.46e-7 relative).  Models of other

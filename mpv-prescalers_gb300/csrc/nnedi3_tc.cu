@@ -16,8 +16,9 @@
 //      followed by mean*invstd and ones, which multiply B's columns of weight
 //      sums and biases;
 //   2. the group's issuing thread runs tcgen05.mma.kind::f16 (M = 128, N = 64,
-//      K = 16) for 32-neuron chunks into two alternating TMEM accumulators and
-//      commits each to an mbarrier;
+//      K = 16) for 32-neuron chunks into two alternating TMEM accumulators (or
+//      N = 128 for 64-neuron chunks into one: tc_chunk) and commits each to an
+//      mbarrier;
 //   3. each warp reads its 32 TMEM lanes with tcgen05.ld.32x32b and runs the
 //      blend in FP32: e = exp2(s1) (softmax rows of B are in log2 units),
 //      wsum += e, vsum += e * s2 / (1 + |s2|).
@@ -37,7 +38,7 @@
 // 23 % tensor pipe; 96 registers and 512 TMEM columns allow no fifth group).
 // 1080p to 2160p, nns128 8x6: 330 us fast (384 us with scalar sums over neuron
 // pairs and rolled chunks; 438 us as four CTAs an SM, each with its own copy of B
-// and a CTA barrier per chunk), 488 us split (523 us; 4919 us on the CUDA cores);
+// and a CTA barrier per chunk), 455 us split (523 us; 4919 us on the CUDA cores);
 // nns256 8x6 at 720p 243 us fast (443 us: two CTAs an SM had room).
 //
 // Every mbarrier wait is bounded (kWaitNs of %globaltimer).  A wait that runs
@@ -130,12 +131,26 @@ __device__ __forceinline__ void group_sync(int g) {
   asm volatile("bar.sync %0, %1;" ::"r"(g + 1), "n"(kGroup) : "memory");
 }
 
+// Neurons per chunk.  Split operands are bound by the MMAs, whose A is read from
+// shared memory once per instruction whatever its N: 64 neurons (N = 128) take
+// two thirds of the shared-memory time of 32 (N = 64), and then one accumulator
+// per group (its MMAs wait for the blend's last read) is all that fits four
+// groups.  FP32, chunks of 32 / 64: nns128 8x6 at 1080p 491 / 455 us, nns128 8x4 at
+// 720p 186 / 179, nns256 8x4 at 1080p 674 / 607, nns64 8x6 316 / 300; but nns64
+// 8x4, with little to multiply, 256 / 267, and nns256 8x6, two groups, at 720p 468 /
+// 487.  The fast form, bound by the blend, keeps 32 and two accumulators.
+constexpr int tc_chunk(int nns, int wh, bool split) {
+  const bool wide = split && (nns == 128 || (nns == 256 && wh == 4) || (nns == 64 && wh == 6));
+  return nns < 32 ? nns : (wide ? 64 : 32);
+}
+
 // Shape of one instantiation.
 template <int WH, int NNS, bool XP, bool SPLIT>
 struct TcShape {
   static constexpr int NT = 8 * WH;                   // window taps
   static constexpr int KP = (NT + 4 + 15) / 16 * 16;  // K: taps, mean term, bias pieces, zero pad
-  static constexpr int NC = NNS < 32 ? NNS : 32;      // neurons per chunk
+  static constexpr int NC = tc_chunk(NNS, WH, SPLIT);     // neurons per chunk
+  static constexpr int NBUF = NC == 64 ? 1 : 2;       // chunk buffers per group
   static constexpr int NCH = NNS / NC;                // chunks per tile
   static constexpr int CCOL = 2 * NC;                 // TMEM columns per chunk buffer
   static constexpr int NP = SPLIT ? 2 : 1;            // FP16 pieces per operand value
@@ -152,10 +167,10 @@ struct TcShape {
   static constexpr int fit = (int)((kSmemMax - NP * BPIECE) / GROUP_BYTES);
   static constexpr int NG = fit < 4 ? fit : 4;
   static constexpr int THREADS = NG * (kGroup + 32);
-  static constexpr uint32_t TCOLS = NG * 2 * CCOL <= 64 ? 64 : (NG * 2 * CCOL <= 128 ? 128 : (NG * 2 * CCOL <= 256 ? 256 : 512));
+  static constexpr uint32_t TCOLS = NG * NBUF * CCOL <= 64 ? 64 : (NG * NBUF * CCOL <= 128 ? 128 : (NG * NBUF * CCOL <= 256 ? 256 : 512));
   static constexpr uint32_t SMEM = NP * BPIECE + NG * GROUP_BYTES;
   static_assert(NNS % NC == 0 && NC % 16 == 0, "neuron count must be a multiple of 16");
-  static_assert(NG >= 1 && NG * 2 * CCOL <= 512, "operands must fit shared and tensor memory");
+  static_assert(NG >= 1 && NG * NBUF * CCOL <= 512, "operands must fit shared and tensor memory");
 };
 
 // The tiles of a launch: 32 x 4 pixels, row by row, frame after frame.
@@ -164,15 +179,15 @@ struct Tiles {
   int n;
 };
 
-// Neurons are processed in chunks of NC (32, or 16 for nns16): chunk k's
-// accumulator holds NC softmax-branch and NC Elliott-branch columns; the MMA
-// of chunk k+2 is issued as soon as every warp of the group has read chunk k.
+// Neurons are processed in chunks of NC: chunk k's accumulator holds NC
+// softmax-branch and NC Elliott-branch columns; the MMA of the next chunk for
+// an accumulator is issued as soon as every warp of the group has read it.
 // Operand B is stored chunk-major: rows [2*NC*k, 2*NC*k + NC) are the
 // softmax weights of neurons k*NC.., the next NC rows their Elliott weights.
 template <int WH, int NNS, bool XP, typename T, bool SPLIT>
 __global__ void __launch_bounds__(TcShape<WH, NNS, XP, SPLIT>::THREADS, 1) nn_tc_kernel(const __grid_constant__ NnArgs p, const __grid_constant__ Tiles tiles) {
   using S = TcShape<WH, NNS, XP, SPLIT>;
-  constexpr int NT = S::NT, KP = S::KP, NC = S::NC, NCH = S::NCH, CCOL = S::CCOL, NG = S::NG;
+  constexpr int NT = S::NT, KP = S::KP, NC = S::NC, NCH = S::NCH, CCOL = S::CCOL, NG = S::NG, NBUF = S::NBUF;
   constexpr int TW = S::TW, TH = S::TH;
   constexpr uint32_t SBO = KP * 16;  // bytes between 8-row groups (A and B)
   constexpr uint32_t LBO = 128;      // bytes between K-adjacent core matrices
@@ -240,13 +255,13 @@ __global__ void __launch_bounds__(TcShape<WH, NNS, XP, SPLIT>::THREADS, 1) nn_tc
       GroupBars& B = bars[g];
       constexpr uint32_t IDESC = instr_desc(128, CCOL);
       const uint32_t a_addr = smem_u32(sB + S::NP * S::BPIECE + g * S::GROUP_BYTES), b_addr = smem_u32(sB);
-      const uint32_t dcol = tmem + g * 2 * CCOL;
+      const uint32_t dcol = tmem + g * NBUF * CCOL;
       bool ok = wait(&bbar, 0u);
       int c = 0, it = 0;  // chunks and tiles issued so far
       for (int t = g * gridDim.x + blockIdx.x; ok && t < ntiles; t += stride, it++) {
         if (!(ok = wait(&B.afull, it & 1))) break;
         for (int k = 0; k < NCH; k++, c++) {
-          const int b = c & 1, u = c >> 1;
+          const int b = c % NBUF, u = c / NBUF;
           if (u > 0 && !(ok = wait(&B.empty[b], (u - 1) & 1))) break;
           tc_fence_after();
           // D[b] = A x B[chunk]^T over the whole K; completion on full[b]
@@ -388,7 +403,7 @@ __global__ void __launch_bounds__(TcShape<WH, NNS, XP, SPLIT>::THREADS, 1) nn_tc
       cur = normalise();
       prefetch(t + stride);
     }
-    const uint32_t lane_addr = tmem + g * 2 * CCOL + ((uint32_t)(py * 32) << 16);
+    const uint32_t lane_addr = tmem + g * NBUF * CCOL + ((uint32_t)(py * 32) << 16);
     const float one = SPLIT ? p.split_one : 1.0f, unit = SPLIT ? p.split_unit : 1.0f;
     int c = 0;
     for (; t < ntiles; t += stride) {
@@ -401,18 +416,18 @@ __global__ void __launch_bounds__(TcShape<WH, NNS, XP, SPLIT>::THREADS, 1) nn_tc
       // before it); the chunks are unrolled, so that no load in flight crosses a
       // loop's edge.  nns128 8x6 fast, 1080p: rolled 353 us, unrolled 334, and ahead
       // 330.  Split, the MMAs bound it: ahead loses 2 %, and so does unrolling
-      // from four chunks on (nns128 488 / 498 us, nns64 8x4 at 480p 67 / 63).
+      // from four chunks on (nns64 8x4 at 480p, two chunks: 67 rolled, 63 unrolled).
       constexpr bool AHEAD = STEPS == 2 && !SPLIT;
       constexpr int UNROLL = SPLIT && NCH > 2 ? 1 : NCH;
       auto load = [&](int b, int q) {
-        tmem_ld16(lane_addr + b * CCOL + 16 * q, s1[q]);
-        tmem_ld16(lane_addr + b * CCOL + NC + 16 * q, s2[q]);
+        tmem_ld16(lane_addr + b * CCOL + 16 * q, s1[q & 1]);
+        tmem_ld16(lane_addr + b * CCOL + NC + 16 * q, s2[q & 1]);
       };
 #pragma unroll UNROLL
       for (int k = 0; k < NCH; k++, c++) {
-        const int b = NCH % 2 == 0 ? k & 1 : c & 1;
+        const int b = NBUF == 1 ? 0 : (NCH % 2 == 0 ? k & 1 : c & 1);
         if (!AHEAD || k == 0 || k == NCH - 1) {  // not in flight yet
-          (void)wait(&B.full[b], (c >> 1) & 1);
+          (void)wait(&B.full[b], (c / NBUF) & 1);
           tc_fence_after();
           if (k == NCH - 1 && t + stride < ntiles) {
             nxt = normalise();
@@ -422,7 +437,7 @@ __global__ void __launch_bounds__(TcShape<WH, NNS, XP, SPLIT>::THREADS, 1) nn_tc
         }
 #pragma unroll
         for (int q = 0; q < STEPS; q++) {
-          tmem_wait16(s1[q], s2[q]);
+          tmem_wait16(s1[q & 1], s2[q & 1]);
           if (q + 1 < STEPS) {
             load(b, q + 1);
           } else {  // this warp has read buffer b
@@ -443,11 +458,11 @@ __global__ void __launch_bounds__(TcShape<WH, NNS, XP, SPLIT>::THREADS, 1) nn_tc
 #pragma unroll
             for (int h = 0; h < 2; h++) {
               const int i = j + 2 * h;
-              float2 l = make_float2(s1[q][i], s1[q][i + 1]);
+              float2 l = make_float2(s1[q & 1][i], s1[q & 1][i + 1]);
               if (SPLIT) l = __fmul2_rn(l, make_float2(unit, unit));
               const float2 e = make_float2(exp2f_approx(l.x), exp2f_approx(l.y));
-              d[h] = make_float2(one + fabsf(s2[q][i]), one + fabsf(s2[q][i + 1]));
-              n[h] = __fmul2_rn(e, make_float2(s2[q][i], s2[q][i + 1]));
+              d[h] = make_float2(one + fabsf(s2[q & 1][i]), one + fabsf(s2[q & 1][i + 1]));
+              n[h] = __fmul2_rn(e, make_float2(s2[q & 1][i], s2[q & 1][i + 1]));
               wsum = __fadd2_rn(wsum, e);
             }
             const float2 dd = __fmul2_rn(d[0], d[1]);
@@ -526,7 +541,7 @@ bool nnedi3_tc_supported(int nns, int win_h) {
   return (nns == 16 || nns == 32 || nns == 64 || nns == 128 || nns == 256) && (win_h == 4 || win_h == 6);
 }
 
-int nnedi3_tc_chunk(int nns) { return nns < 32 ? nns : 32; }
+int nnedi3_tc_chunk(int nns, int win_h, bool split) { return tc_chunk(nns, win_h, split); }
 
 int launch_nnedi3_tc(const NnArgs& a, bool xpass, int dtype, cudaStream_t s) {
   if (!a.wts_h || !a.err) return -22;
