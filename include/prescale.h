@@ -192,7 +192,8 @@ size_t pz_scratch_wanted(const pz_model* model, int in_width, int in_height, int
  * axes, the row-doubled plane (2 * W * H * element size); ravu, the FP32
  * int11 plane between its two launches (planes * W * H * 4 bytes, 4-byte
  * aligned).  When opts->scratch is NULL and scratch is needed, it is
- * allocated stream-ordered and freed. */
+ * allocated stream-ordered and freed.  A ravu-zoom that is given enough of it
+ * (pz_scratch_wanted) keeps its weights there; it needs none. */
 int pz_run(const pz_model* model, const pz_plane* in, int n_in, pz_plane* out, int n_out,
            const pz_opts* opts, void* cuda_stream);
 

@@ -182,9 +182,12 @@ def prescale_frame(model, frame: Frame, out_size: Optional[Tuple[int, int]] = No
     if frame.offset != (0.0, 0.0) and frame.offset != (0, 0):
         raise ValueError("the frame carries an uncorrected offset; correct it before the next prescaler")
     sizes, loc = tuple(frame.sizes), frame.chroma_loc
-    loc = loc if isinstance(loc, str) else tuple(loc)
-    plan = model._kept(("frame", frame.kind, sizes, None if out_size is None else tuple(out_size), loc),
-                       lambda: plan_frame(model, frame.kind, sizes, out_size, loc))
+
+    def make():
+        return plan_frame(model, frame.kind, sizes, out_size, loc)
+
+    plan = (model._kept(("frame", frame.kind, sizes, None if out_size is None else tuple(out_size), loc), make)
+            if isinstance(loc, str) else make())   # other sitings: anything with two numbers, or unused
     if not plan.runs:
         return Frame(list(frame.planes), frame.kind, frame.chroma_loc, frame.offset)
     W, H = frame.sizes[0]

@@ -108,3 +108,11 @@ def test_chain_offset_of_every_reference_file(reference_dir):
         assert hm.hook_point == hooks[hm.channels], f
     nn = HookModel(models.load_model(os.path.join(reference_dir, "compute", "nnedi3-nns32-win8x4.hook")))
     assert nn.chain_offset(64, 36, out_size=(64, 72)) == (0.0, -0.5)
+
+
+@pytest.mark.parametrize("loc", [None, [0.0, 0.5], "left"])
+def test_a_frame_that_passes_through_takes_any_siting(loc):
+    class Plane:   # an RGB frame under a LUMA hook reaches no device
+        shape = (36, 64)
+    f = F.prescale_frame(m("ravu-lite-r3"), F.Frame([Plane()] * 3, "rgb", loc))
+    assert f.chroma_loc is loc and len(f.planes) == 3
