@@ -140,7 +140,8 @@ def test_when_false_leaves_planes_untouched():
     assert y.shape == (80, 60)
 
 
-@pytest.mark.parametrize("name,osz", [("ravu-lite-ar-r3", None), ("ravu-r3-yuv", None), ("ravu-3x-r2-rgb", None),
+@pytest.mark.parametrize("name,osz", [("ravu-lite-ar-r3", None), ("ravu-r3-yuv", None), ("ravu-r4-yuv", None),
+                                      ("ravu-r4", None), ("ravu-3x-r2-rgb", None),
                                       ("ravu-zoom-ar-r2", (1440, 810)), ("nnedi3-nns32-win8x4", None)])
 def test_one_call_for_a_tensor_gives_the_planes_pixels(name, osz):
     """A tensor on the current stream goes down in one native call; the same
@@ -313,7 +314,8 @@ def test_staging_autotuner(tmp_path):
     assert best in ("ldg", "tma") and set(times) == {"ldg", "tma"}
 
 
-@pytest.mark.parametrize("name,osz", [("ravu-lite-ar-r3", None), ("ravu-r3-yuv", None), ("ravu-3x-r2-rgb", None),
+@pytest.mark.parametrize("name,osz", [("ravu-lite-ar-r3", None), ("ravu-r3-yuv", None), ("ravu-r4-yuv", None),
+                                      ("ravu-r4", None), ("ravu-3x-r2-rgb", None),
                                       ("ravu-zoom-ar-r2", (101, 77)), ("nnedi3-nns16-win8x4", None),
                                       ("nnedi3-nns16-win8x4", (40, 60)), ("nnedi3-nns16-win8x4", (80, 30))])
 def test_query_matches_the_python_geometry(name, osz):
