@@ -560,6 +560,7 @@ static int run_frame(const pz_model* m, const pz_plane* in, int n_in, pz_plane* 
       a.frames = frames;
       a.in_frame = sframe;
       a.out_frame = dframe;
+      a.after = src == tmp && tmp;
       return pz::launch_nnedi3(a, precision, xpass, dt, s);
     };
     rc = 0;
@@ -622,6 +623,7 @@ static int run_frame(const pz_model* m, const pz_plane* in, int n_in, pz_plane* 
             if (!o->tile_rows) a.tile_rows = 4;
             a.ztab = static_cast<const float4*>(o->scratch);
             if (!table_filled) pz::launch_zoom_table(a, m->radius, m->ar != 0.0f, s);
+            a.after = !table_filled;
           }
         }
         rc = pz::launch_zoom(a, m->radius, m->channels, m->ar != 0.0f, dt, s); break;

@@ -12,6 +12,13 @@
 
 namespace pz {
 
+// Programmatic dependent launch: a kernel that a later one depends on lets that
+// one's CTAs begin once all of its own have (pdl_trigger); the later one waits
+// before it reads what the first wrote, until the first is complete and its
+// stores are visible (pdl_wait; nothing to wait for in any other launch).
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 constexpr float kFltEps = 1.192092896e-7f;   // the shaders' epsilon literal
 constexpr float kPi = 3.141592653589793f;    // the shaders' pi literal
 

@@ -8,6 +8,27 @@
 
 namespace pz {
 
+// Launches `kern`; `after`: its prerequisite is the launch just before it on the
+// stream, whose CTAs have all begun when this one's may (pdl_trigger, pdl_wait): its
+// CTAs fill the SMs that the other's last wave leaves idle and run up to their wait.
+// One after the other / overlapped: ravu-r3 854x480 26.9 / 24.2 us, 1080p 74.6 / 73.9,
+// ravu-r3-yuv 720p 60.1 / 57.2, ravu-zoom-r2 720p to 1080p (its phase table first)
+// 33.1 / 31.6, nnedi3-nns64-win8x4 FP32 854x480 63.9 / 62.1.
+template <class... P, class... A>
+void launch_kernel(void (*kern)(P...), dim3 grid, int threads, size_t smem, cudaStream_t s, bool after, const A&... a) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c{};
+  c.gridDim = grid;
+  c.blockDim = dim3(threads);
+  c.dynamicSmemBytes = smem;
+  c.stream = s;
+  c.attrs = &at;
+  c.numAttrs = after ? 1 : 0;
+  cudaLaunchKernelEx(&c, kern, a...);  // errors: cudaGetLastError, as for the other launches
+}
+
 enum ChMode : int { kLuma = 0, kYuv = 1, kRgb = 2 };
 
 // One RAVU-family dispatch.  Planes are [H][W] with per-plane pitches.
@@ -18,6 +39,7 @@ struct RavuArgs {
   int out_pitch[3];
   int W, H;          // input size
   int OW, OH;        // output size
+  int after;         // launched right after its prerequisite (launch_kernel)
   int frames;        // frames of one launch (0 counts as 1; plain loads only), elements apart:
   long long in_frame, out_frame;
   const float4* lut;     // [lut_rows][lut_pitch] texels
@@ -47,6 +69,7 @@ struct NnArgs {
   void* out;
   int out_pitch;
   int W, H;                 // size of the pass input
+  int after;                // launched right after its prerequisite (launch_kernel; tensor cores)
   int frames;               // frames of one launch (tensor cores; 0 counts as 1), elements apart:
   long long in_frame, out_frame;
   int nns, win_h;           // window is 8 x win_h (double_y orientation)

@@ -127,6 +127,9 @@ __device__ __forceinline__ void mbar_arrive(uint32_t mbar) {
 }
 
 // Barrier among the 128 threads of group g (named barriers 1..4; 0 is the CTA's).
+__device__ __forceinline__ float to_float(float v) { return v; }
+__device__ __forceinline__ float to_float(__half v) { return __half2float(v); }
+
 __device__ __forceinline__ void group_sync(int g) {
   asm volatile("bar.sync %0, %1;" ::"r"(g + 1), "n"(kGroup) : "memory");
 }
@@ -223,6 +226,9 @@ __global__ void __launch_bounds__(TcShape<WH, NNS, XP, SPLIT>::THREADS, 1) nn_tc
         "l"(reinterpret_cast<uint64_t>(SPLIT ? p.wts_s : p.wts_h)), "r"(S::NP * S::BPIECE), "r"(smem_u32(&bbar))
         : "memory");
   }
+  // the row pass's CTAs may still run (they hold the tensor memory) until here
+  pdl_wait();
+  pdl_trigger();
   if (warp == 0) {
     __syncwarp();
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base)),
@@ -316,7 +322,7 @@ __global__ void __launch_bounds__(TcShape<WH, NNS, XP, SPLIT>::THREADS, 1) nn_tc
         if (i < TW * TH) {
           const int ty = i / TW, tx = i % TW;
           const int gx = clampi(px0 + S::OX0 + tx, 0, p.W - 1), gy = clampi(py0 + S::OY0 + ty, 0, p.H - 1);
-          pre[r] = ldp(src + (size_t)gy * p.in_pitch + gx);
+          pre[r] = to_float(src[(size_t)gy * p.in_pitch + gx]);  // plain loads: pdl_wait
         }
       }
     };
@@ -512,7 +518,7 @@ int launch_one(const NnArgs& a, cudaStream_t s) {
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   Tiles tiles{fast_div((a.W + 31) / 32), fast_div((a.H + 3) / 4), 0};
   tiles.n = (int)(tiles.x.d * tiles.y.d) * (a.frames > 0 ? a.frames : 1);
-  kern<<<tiles.n < sms ? tiles.n : sms, S::THREADS, S::SMEM, s>>>(a, tiles);
+  launch_kernel(kern, dim3(tiles.n < sms ? tiles.n : sms), S::THREADS, S::SMEM, s, a.after, a, tiles);
   return 0;
 }
 

@@ -84,6 +84,19 @@ struct Quad<__half> {
   }
 };
 
+// FP32 texels that the launch before may still be writing when this one begins
+// (pdl_wait): read with plain loads, not as data constant for the kernel.
+struct FreshFloat {
+  float v;
+};
+template <>
+struct Quad<FreshFloat> : Quad<float> {
+  __device__ __forceinline__ void load(const FreshFloat* p) { v = *reinterpret_cast<const float4*>(p); }
+  __device__ __forceinline__ void load1(const FreshFloat* p, int a, int b, int c, int d) {
+    v = make_float4(p[a].v, p[b].v, p[c].v, p[d].v);
+  }
+};
+
 // May a plane be read in quads (at columns that are multiples of 4)?
 template <typename T>
 __device__ __forceinline__ bool quads_aligned(const T* in, int pitch) {
@@ -553,6 +566,7 @@ struct Int11Tile {
   using Elem = T;
 
   __device__ static void run(const RavuArgs& p, int f, int x0, int y0, float* smem, TmaCtx* tma = nullptr) {
+    pdl_trigger();  // the lattice launch
     float* tile = smem;
     if (!stage_frame<CM, TH, kThreads, T>(p, tma, f, x0, y0 - HALO, tile)) return;
     __syncthreads();
@@ -666,12 +680,16 @@ struct LatticeTile {
     float* t11 = smem + PL * TW * TH;       // int11, rows y0-R ..
     const size_t plane = (size_t)p.W * p.H;
     struct {
-      TileStage<CM, TH, kThreads, float> st;
+      TileStage<CM, TH, kThreads, FreshFloat> st;
       const RavuArgs& p;
       float* t11;
       int f, x0, y0;
       __device__ __forceinline__ void load() {
-        st.load([&](int c, int& pitch) { pitch = p.W; return p.i11 + (size_t)(f * C + c) * p.W * p.H; }, p.W, p.H, x0, y0);
+        pdl_wait();  // the input tile's loads are in flight
+        st.load([&](int c, int& pitch) {
+          pitch = p.W;
+          return reinterpret_cast<const FreshFloat*>(p.i11) + (size_t)(f * C + c) * p.W * p.H;
+        }, p.W, p.H, x0, y0);
       }
       __device__ __forceinline__ void store() { st.store(t11); }
     } i11{{}, p, t11, f, x0, y0 - R};
@@ -839,6 +857,7 @@ __host__ __device__ constexpr uint32_t zoom_entry() {
 template <int R, bool AR, bool H16>
 __global__ void zoom_table_kernel(const __grid_constant__ RavuArgs p, float4* out) {
   constexpr int NB = zoom_texels<R>(), NT2 = (NB + 1) / 2, PER = NT2 * (AR ? 4 : 2);
+  pdl_trigger();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int phases = (int)(p.zpx.d * p.zpy.d), n = p.lut_rows / 9 * phases;
   if (i >= n * PER) return;
@@ -994,6 +1013,7 @@ struct ZoomTile {
     if constexpr (TAB) {
       const int phx = X - (int)(p.zpx(X) * p.zpx.d), phy = Y - (int)(p.zpy(Y) * p.zpy.d);
       const int k = clampi(key, 0, p.lut_rows / 9 - 1) * (int)p.zpy.d + phy;
+      pdl_wait();
       entry = p.ztab + ((size_t)k * p.zpx.d + phx) * zoom_entry<R, AR>();
     } else {
       ls = ZoomLut(p.lut_rows, key, px.s, py.s, p.lut_frac);
@@ -1001,8 +1021,8 @@ struct ZoomTile {
     }
     auto weights = [&](int part, int t, float2 (&w)[4]) {
       if constexpr (TAB) {
-        const float4 a = __ldg(entry + part * NB + 2 * t);
-        const float4 b = 2 * t + 1 < NB ? __ldg(entry + part * NB + 2 * t + 1) : a;
+        const float4 a = entry[part * NB + 2 * t];  // written by a launch this one may overlap
+        const float4 b = 2 * t + 1 < NB ? entry[part * NB + 2 * t + 1] : a;
         w[0] = make_float2(a.x, a.y);
         w[1] = make_float2(a.z, a.w);
         w[2] = make_float2(b.x, b.y);
@@ -1125,7 +1145,7 @@ int launch_tile_kernel(dim3 grid, cudaStream_t s, const RavuArgs& a, const TmaMa
       opted[dev].store(true, std::memory_order_relaxed);
     }
   }
-  kern<<<grid, Prog::kThreads, SMEM, s>>>(a, maps);
+  launch_kernel(kern, grid, Prog::kThreads, SMEM, s, a.after, a, maps);
   return 0;
 }
 

@@ -336,3 +336,37 @@ def test_query_matches_the_python_geometry(name, osz):
     if hm.family == "ravu":   # the FP32 int11 plane between the two lattice launches
         want_scratch = hm.n_planes * W * H * 4
     assert r.scratch_bytes == want_scratch
+
+
+@pytest.mark.parametrize("name,size,osz,precision", [
+    ("ravu-r3", (203, 57), None, "fp32"), ("ravu-r4-yuv", (640, 360), None, "fast"),
+    ("ravu-zoom-ar-r2", (960, 540), (1440, 810), "fast"), ("nnedi3-nns16-win8x4", (96, 40), None, "fp32"),
+    ("nnedi3-nns64-win8x6", (320, 180), None, "fast")])
+def test_chains_queued_back_to_back_and_captured(name, size, osz, precision):
+    """A chain's second launch begins while its first still runs, waits for it,
+    and a chain queued behind another one reuses its scratch: frames queued
+    without a wait, and replayed from a graph, are the frames made one by one."""
+    hm, _ = synth.model_for(name)
+    (W, H), C = size, hm.n_planes
+    xs = [torch.rand((C, H, W), device="cuda").to(torch.float16) for _ in range(6)]
+    OW, OH = osz or (2 * W, 2 * H)
+    scratch = torch.empty(16 << 20, dtype=torch.uint8, device="cuda")
+
+    def run(x, out):
+        hm.run_raw(list(x.unbind(0)), list(out.unbind(0)), (OW, OH), precision=precision, scratch=scratch)
+
+    outs = [[torch.zeros((C, OH, OW), dtype=torch.float16, device="cuda") for _ in xs] for _ in range(3)]
+    for x, o in zip(xs, outs[0]):
+        run(x, o)
+        torch.cuda.synchronize()
+    for x, o in zip(xs, outs[1]):
+        run(x, o)
+    g = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(g):
+        for x, o in zip(xs, outs[2]):
+            run(x, o)
+    g.replay()
+    torch.cuda.synchronize()
+    for a, b, c in zip(*outs):
+        assert torch.equal(a, b) and torch.equal(a, c)
