@@ -314,8 +314,7 @@ def test_staging_autotuner(tmp_path):
     assert best in ("ldg", "tma") and set(times) == {"ldg", "tma"}
 
 
-@pytest.mark.parametrize("name,osz", [("ravu-lite-ar-r3", None), ("ravu-r3-yuv", None), ("ravu-r4-yuv", None),
-                                      ("ravu-r4", None), ("ravu-3x-r2-rgb", None),
+@pytest.mark.parametrize("name,osz", [("ravu-lite-ar-r3", None), ("ravu-r3-yuv", None), ("ravu-3x-r2-rgb", None),
                                       ("ravu-zoom-ar-r2", (101, 77)), ("nnedi3-nns16-win8x4", None),
                                       ("nnedi3-nns16-win8x4", (40, 60)), ("nnedi3-nns16-win8x4", (80, 30))])
 def test_query_matches_the_python_geometry(name, osz):
