@@ -104,7 +104,8 @@ int check_plane(const pz_plane& p, const char* what, int idx, bool pairs) {
 //          then keeps 22 bits or more, and a smaller one an absolute error of
 //          2^-39 of the largest.  Not made (the CUDA cores run the model)
 //          when a value is not finite or the power lies outside 2^-8..2^30,
-//          where the blend's products could leave FP32's range.
+//          so that the blend's product of two denominators, of at most 2^37
+//          each, and its reciprocal stay within FP32's normal range.
 int upload_operands(pz_model* m, const std::vector<float>& w, const std::vector<float>& bias) {
   const int n = m->nns, T = m->win_w * m->win_h;
   const int NCH = pz::nnedi3_tc_chunk(n, m->win_h, false), NCS = pz::nnedi3_tc_chunk(n, m->win_h, true);

@@ -410,7 +410,7 @@ __global__ void __launch_bounds__(TcShape<WH, NNS, XP, SPLIT>::THREADS, 1) nn_tc
       prefetch(t + stride);
     }
     const uint32_t lane_addr = tmem + g * NBUF * CCOL + ((uint32_t)(py * 32) << 16);
-    const float one = SPLIT ? p.split_one : 1.0f, unit = SPLIT ? p.split_unit : 1.0f;
+    const float one = SPLIT ? p.split_one : 1.0f, half_unit = SPLIT ? 0.5f * p.split_unit : 1.0f;
     int c = 0;
     for (; t < ntiles; t += stride) {
       float2 wsum = make_float2(0.0f, 0.0f), vsum = wsum;
@@ -457,23 +457,36 @@ __global__ void __launch_bounds__(TcShape<WH, NNS, XP, SPLIT>::THREADS, 1) nn_tc
             }
           }
           // sum of e s / (1 + |s|): neurons j and j+2 (and j+1, j+3) share one
-          // reciprocal, of the product of their denominators
+          // reciprocal, of the product of their denominators.  Split: s / (1 + |s|)
+          // (the scale cancels in it) is formed before e comes in, and e = 2^l is the
+          // square of 2^(l/2), so that no product leaves FP32's range before e does
+          // and e reaches down into the subnormals: logits of -95 to 88 as by expf
+          // (e s (1 + |s|) at the model's scale was infinite from logits of 70 on, e
+          // zero below -87; nns128 8x6 at 1080p 440 us so, now 476)
 #pragma unroll
           for (int j = 0; j < 16; j += 4) {
-            float2 n[2], d[2];
+            float2 e[2], n[2], d[2];  // n: s (split), e s
 #pragma unroll
             for (int h = 0; h < 2; h++) {
               const int i = j + 2 * h;
               float2 l = make_float2(s1[q & 1][i], s1[q & 1][i + 1]);
-              if (SPLIT) l = __fmul2_rn(l, make_float2(unit, unit));
-              const float2 e = make_float2(exp2f_approx(l.x), exp2f_approx(l.y));
+              if (SPLIT) l = __fmul2_rn(l, make_float2(half_unit, half_unit));
+              e[h] = make_float2(exp2f_approx(l.x), exp2f_approx(l.y));
+              if (SPLIT) e[h] = __fmul2_rn(e[h], e[h]);
               d[h] = make_float2(one + fabsf(s2[q & 1][i]), one + fabsf(s2[q & 1][i + 1]));
-              n[h] = __fmul2_rn(e, make_float2(s2[q & 1][i], s2[q & 1][i + 1]));
-              wsum = __fadd2_rn(wsum, e);
+              n[h] = make_float2(s2[q & 1][i], s2[q & 1][i + 1]);
+              if (!SPLIT) n[h] = __fmul2_rn(e[h], n[h]);
+              wsum = __fadd2_rn(wsum, e[h]);
             }
             const float2 dd = __fmul2_rn(d[0], d[1]);
-            const float2 nn = __ffma2_rn(n[0], d[1], __fmul2_rn(n[1], d[0]));
-            vsum = __ffma2_rn(nn, make_float2(rcp_approx(dd.x), rcp_approx(dd.y)), vsum);
+            if (SPLIT) {
+              const float2 r = make_float2(rcp_approx(dd.x), rcp_approx(dd.y));
+              vsum = __ffma2_rn(e[0], __fmul2_rn(__fmul2_rn(n[0], d[1]), r), vsum);
+              vsum = __ffma2_rn(e[1], __fmul2_rn(__fmul2_rn(n[1], d[0]), r), vsum);
+            } else {
+              const float2 nn = __ffma2_rn(n[0], d[1], __fmul2_rn(n[1], d[0]));
+              vsum = __ffma2_rn(nn, make_float2(rcp_approx(dd.x), rcp_approx(dd.y)), vsum);
+            }
           }
         }
       }

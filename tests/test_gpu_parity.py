@@ -263,6 +263,32 @@ def test_nnedi3_tensor_core_tiles(name, H, W):
     assert np.abs(y - ref[0]).max() <= 2e-3
 
 
+@pytest.mark.parametrize("name", ["nnedi3-nns32-win8x4", "nnedi3-nns128-win8x6"])
+@pytest.mark.parametrize("elliott", [1.0, 13.0, 133.0], ids=["w", "13w", "133w"])
+@pytest.mark.parametrize("logit", [-95.0, -86.0, 60.0, 70.0, 80.0])
+def test_nnedi3_fp32_large_logits(name, elliott, logit):
+    """Softmax logits over the range of FP32's exp (down to its subnormals),
+    beside Elliott arguments of some 1, 10 and 100, in the plain FP32 form's
+    row pass.  A logit below 128 in units of log2 carries at most 5 roundings
+    of 2^-17: e is off by 5 * 2^-17 * ln 2 = 2.6e-5, the mean of values in
+    [-1, 1] by twice that, the pixel by 5 std (std <= 1/2) times it: 1.3e-4,
+    and the usual 1e-5.  At -95 an e of at least 2^-138.5 is a multiple of
+    2^-149: 1.7e-4 more, 8.6e-4 in the pixel."""
+    import dataclasses
+    from mpv_prescalers_gb300.prescaler import HookModel
+    m = synth.synthetic_model(name)
+    bias = logit + np.random.default_rng(3).normal(0.0, 0.3, m.nns)
+    m = dataclasses.replace(m, bias_a=bias.astype(np.float32), weights_a=m.weights_a * np.float32(0.2),
+                            weights_b=m.weights_b * np.float32(elliott))
+    H, W = 48, 96
+    x = synth.luma_plane(H, W, 51)
+    y = HookModel(m).upscale(torch.from_numpy(x).cuda(), out_size=(W, 2 * H)).cpu().numpy().astype(np.float64)
+    ref, info = oracle.nnedi3_upscale(m, x, axes="y")
+    err = np.abs(y - ref[0])
+    err[1::2][info["boundary_y"]] = 0.0
+    assert err.max() <= (1.3e-4 if logit > -90 else 1.3e-4 + 8.6e-4) + TOL_FP32
+
+
 def test_nnedi3_fp32_on_the_variance_gate():
     """Windows with variance near FLT_EPS: a plane of 0.5 with +-d
     perturbations on a few pixels so that var ~ eps; the bound per gate
