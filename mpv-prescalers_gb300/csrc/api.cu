@@ -650,6 +650,7 @@ int pz_run_frames(const pz_model* m, const void* in, long long in_frame, long lo
   if (!in || !out) return fail(PZ_EINVAL, "null planes");
   pz_opts o{};
   if (opts) o = *opts;
+  if (!scratch) scratch_bytes = 0;  // no room, whatever the caller counted
   o.scratch = scratch;
   o.scratch_bytes = scratch_bytes;
   const long long es = (long long)dtype_size(dtype);

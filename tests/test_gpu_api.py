@@ -369,3 +369,22 @@ def test_chains_queued_back_to_back_and_captured(name, size, osz, precision):
     torch.cuda.synchronize()
     for a, b, c in zip(*outs):
         assert torch.equal(a, b) and torch.equal(a, c)
+
+
+@pytest.mark.parametrize("name", ["ravu-r3", "ravu-r2-yuv", "nnedi3-nns32-win8x4"])
+def test_frames_without_scratch_ignore_its_byte_count(name):
+    """pz_run_frames without a scratch buffer has room for no frame, whatever
+    byte count comes with the null pointer: it allocates for one frame at a
+    time, and the frames are the same."""
+    import ctypes
+    from mpv_prescalers_gb300 import _ffi
+    hm, _ = synth.model_for(name)
+    n, C, H, W = 3, hm.n_planes, 40, 56
+    x = torch.rand((n, C, H, W), device="cuda")
+    y = torch.empty((n, C, 2 * H, 2 * W), device="cuda")
+    o = _ffi.Opts()
+    o.out_width, o.out_height = 2 * W, 2 * H
+    _ffi.check(_ffi.lib().pz_run_frames(
+        hm.device_handle(0), x.data_ptr(), C * H * W, H * W, W, y.data_ptr(), 4 * C * H * W, 4 * H * W, 2 * W, n, W, H,
+        _ffi.PZ_F32, ctypes.byref(o), None, 1 << 30, torch.cuda.current_stream().cuda_stream))
+    assert torch.equal(y, hm.upscale(x))
