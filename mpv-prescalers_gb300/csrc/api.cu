@@ -645,6 +645,8 @@ int pz_run(const pz_model* m, const pz_plane* in, int n_in, pz_plane* out, int n
 int pz_run_frames(const pz_model* m, const void* in, long long in_frame, long long in_plane, int in_pitch, void* out,
                   long long out_frame, long long out_plane, int out_pitch, int n_frames, int width, int height,
                   int dtype, const pz_opts* opts, void* scratch, size_t scratch_bytes, void* stream) {
+  if (n_frames <= 0) return fail(PZ_EINVAL, "n_frames %d", n_frames);
+  if (n_frames > 1 && opts && opts->keys) return fail(PZ_EINVAL, "opts->keys holds the keys of one frame, not of %d", n_frames);
   pz_query_result q;
   if (const int rc = pz_query(m, width, height, dtype, opts, &q)) return rc;
   if (!in || !out) return fail(PZ_EINVAL, "null planes");
@@ -656,7 +658,7 @@ int pz_run_frames(const pz_model* m, const void* in, long long in_frame, long lo
   const long long es = (long long)dtype_size(dtype);
   // all frames in one launch per pass (at most 1024: the tile numbers of one
   // launch stay far below 2^31, its grid within bounds) where each has scratch of its own
-  const bool together = !o.staging && !o.keys && out_frame % 2 == 0 && q.scratch_bytes * (size_t)n_frames <= scratch_bytes;
+  const bool together = !o.staging && out_frame % 2 == 0 && q.scratch_bytes * (size_t)n_frames <= scratch_bytes;
   const int step = together ? 1024 : 1;
   for (int f = 0; f < n_frames; f += step) {
     pz_plane pin[3], pout[3];

@@ -105,3 +105,17 @@ def test_host_pipeline_arguments_are_checked_on_the_host(lib):
     assert lib.pz_run_host(None, None, None, 1, 8, 8, _ffi.PZ_F16, None, None, 0, 0, None) == _ffi.PZ_EINVAL
     assert b"null" in lib.pz_last_error()
     assert lib.pz_run_host_work_bytes(None, 8, 8, _ffi.PZ_F16, None) == 0
+
+
+def test_frame_arguments_are_checked_on_the_host(lib):
+    import ctypes
+    o = _ffi.Opts()
+
+    def run(n):
+        return lib.pz_run_frames(None, None, 0, 0, 0, None, 0, 0, 0, n, 8, 8, _ffi.PZ_F16, ctypes.byref(o), None, 0, None)
+
+    for n in (0, -1):
+        assert run(n) == _ffi.PZ_EINVAL and b"n_frames" in lib.pz_last_error()
+    o.keys = 4096   # never dereferenced
+    assert run(2) == _ffi.PZ_EINVAL and b"keys" in lib.pz_last_error()
+    assert run(1) == _ffi.PZ_EINVAL and b"null" in lib.pz_last_error()
