@@ -177,8 +177,8 @@ int pz_query(const pz_model* model, int in_width, int in_height, int dtype, cons
 /* Device scratch bytes pz_run needs for this model/input (0 if none). */
 size_t pz_scratch_bytes(const pz_model* model, const pz_plane* in, const pz_opts* opts);
 
-/* The scratch with which pz_run runs fastest and allocates nothing: what
- * pz_scratch_bytes says, and for a ravu-zoom whose scale has few phases (1.5x,
+/* The scratch with which pz_run_with_scratch and pz_run_frames run fastest and
+ * allocate nothing: what pz_scratch_bytes says, and for a ravu-zoom whose scale has few phases (1.5x,
  * 1.75x, 2.25x; clamped-load staging) room for every key's interpolated weights
  * at every phase, 16-byte aligned.  Without it such a zoom interpolates per
  * pixel; the pixels are the same.  Host-only: no device call. */
@@ -192,17 +192,25 @@ size_t pz_scratch_wanted(const pz_model* model, int in_width, int in_height, int
  * axes, the row-doubled plane (2 * W * H * element size); ravu, the FP32
  * int11 plane between its two launches (planes * W * H * 4 bytes, 4-byte
  * aligned).  When opts->scratch is NULL and scratch is needed, it is
- * allocated stream-ordered and freed.  A ravu-zoom that is given enough of it
- * (pz_scratch_wanted) keeps its weights there; it needs none. */
+ * allocated stream-ordered and freed.  A chain that needs none (pz_scratch_bytes
+ * says 0: lite, 3x, zoom, nnedi3 along one axis) leaves opts->scratch alone, so
+ * that a host may hand one buffer to such calls on several streams. */
 int pz_run(const pz_model* model, const pz_plane* in, int n_in, pz_plane* out, int n_out,
            const pz_opts* opts, void* cuda_stream);
+
+/* pz_run with `scratch` in place of opts->scratch, this call's own until the
+ * stream has passed it: a ravu-zoom that is given enough (pz_scratch_wanted) and
+ * 16-byte aligned scratch keeps its weights there. */
+int pz_run_with_scratch(const pz_model* model, const pz_plane* in, int n_in, pz_plane* out, int n_out,
+                        const pz_opts* opts, void* scratch, size_t scratch_bytes, void* cuda_stream);
 
 /* pz_run on n_frames frames of one tensor: plane c of frame f starts at element
  * f * in_frame + c * in_plane of `in`, rows in_pitch elements apart; `out`
  * likewise, at the output size pz_query reports.  `scratch` replaces
- * opts->scratch: with n_frames times pz_scratch_bytes of it (and clamped-load
- * staging) each pass of the chain is one launch for all frames, else it serves
- * the frames in turn; opts->keys must be NULL for more than one frame. */
+ * opts->scratch, as in pz_run_with_scratch: with n_frames times pz_scratch_bytes
+ * of it (and clamped-load staging) each pass of the chain is one launch for all
+ * frames, else it serves the frames in turn; opts->keys must be NULL for more
+ * than one frame. */
 int pz_run_frames(const pz_model* model, const void* in, long long in_frame, long long in_plane, int in_pitch,
                   void* out, long long out_frame, long long out_plane, int out_pitch, int n_frames, int width,
                   int height, int dtype, const pz_opts* opts, void* scratch, size_t scratch_bytes, void* cuda_stream);

@@ -88,6 +88,9 @@ EXPORTS = {
                                 ctypes.POINTER(QueryResult)]),
     "pz_run": (ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(Plane), ctypes.c_int, ctypes.POINTER(Plane),
                               ctypes.c_int, ctypes.POINTER(Opts), ctypes.c_void_p]),
+    "pz_run_with_scratch": (ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(Plane), ctypes.c_int, ctypes.POINTER(Plane),
+                                           ctypes.c_int, ctypes.POINTER(Opts), ctypes.c_void_p, ctypes.c_size_t,
+                                           ctypes.c_void_p]),
     "pz_run_frames": (ctypes.c_int, [ctypes.c_void_p] * 2 + [ctypes.c_longlong] * 2 + [ctypes.c_int, ctypes.c_void_p]
                       + [ctypes.c_longlong] * 2 + [ctypes.c_int] * 5 + [ctypes.POINTER(Opts), ctypes.c_void_p,
                                                                         ctypes.c_size_t, ctypes.c_void_p]),

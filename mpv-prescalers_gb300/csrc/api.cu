@@ -490,12 +490,17 @@ size_t pz_scratch_wanted(const pz_model* m, int in_w, int in_h, int dtype, const
   return zoom_table_size(m, in_w, in_h, q.out_width, q.out_height, &px, &py);
 }
 
+// ravu-zoom's phase table (ravu_zoom.cu) and a call's scratch.
+enum ZoomTable {
+  kNoTable,      // the scratch is not to be written by a ravu-zoom
+  kMakeTable,    // it takes the table, if there is room
+  kTableFilled,  // a call before on this stream, with the same sizes and options, has left the table there
+};
+
 // pz_run on `frames` frames whose planes lie in_frame / out_frame elements apart
-// (more than one: scratch for each given, plain loads, no keys).  table_filled: a
-// call before it on this stream, with the same sizes and options, has left
-// ravu-zoom's phase table in the scratch.
+// (more than one: scratch for each given, plain loads, no keys).
 static int run_frame(const pz_model* m, const pz_plane* in, int n_in, pz_plane* out, int n_out, const pz_opts* o,
-                     void* stream, bool table_filled, int frames = 1, long long in_frame = 0, long long out_frame = 0) {
+                     void* stream, ZoomTable table, int frames = 1, long long in_frame = 0, long long out_frame = 0) {
   if (!m || !in || !out) return fail(PZ_EINVAL, "null argument");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int C = m->channels == PZ_LUMA ? 1 : 3;
@@ -618,13 +623,13 @@ static int run_frame(const pz_model* m, const pz_plane* in, int n_in, pz_plane* 
       case PZ_RAVU_ZOOM:
         pz::zoom_divisors(&a);
         // with scratch for it, the weights of a scale of few phases are formed once
-        if (o->scratch && !a.staging && reinterpret_cast<uintptr_t>(o->scratch) % 16 == 0) {
+        if (table != kNoTable && o->scratch && !a.staging && reinterpret_cast<uintptr_t>(o->scratch) % 16 == 0) {
           const size_t need = zoom_table_size(m, W, H, OW, OH, &a.zpx, &a.zpy);
           if (need && o->scratch_bytes >= need) {
             if (!o->tile_rows) a.tile_rows = 4;
             a.ztab = static_cast<const float4*>(o->scratch);
-            if (!table_filled) pz::launch_zoom_table(a, m->radius, m->ar != 0.0f, s);
-            a.after = !table_filled;
+            if (table == kMakeTable) pz::launch_zoom_table(a, m->radius, m->ar != 0.0f, s);
+            a.after = table == kMakeTable;
           }
         }
         rc = pz::launch_zoom(a, m->radius, m->channels, m->ar != 0.0f, dt, s); break;
@@ -639,7 +644,16 @@ static int run_frame(const pz_model* m, const pz_plane* in, int n_in, pz_plane* 
 }
 
 int pz_run(const pz_model* m, const pz_plane* in, int n_in, pz_plane* out, int n_out, const pz_opts* o, void* stream) {
-  return run_frame(m, in, n_in, out, n_out, o, stream, false);
+  return run_frame(m, in, n_in, out, n_out, o, stream, kNoTable);
+}
+
+int pz_run_with_scratch(const pz_model* m, const pz_plane* in, int n_in, pz_plane* out, int n_out, const pz_opts* opts,
+                        void* scratch, size_t scratch_bytes, void* stream) {
+  pz_opts o{};
+  if (opts) o = *opts;
+  o.scratch = scratch;
+  o.scratch_bytes = scratch ? scratch_bytes : 0;
+  return run_frame(m, in, n_in, out, n_out, &o, stream, kMakeTable);
 }
 
 int pz_run_frames(const pz_model* m, const void* in, long long in_frame, long long in_plane, int in_pitch, void* out,
@@ -669,7 +683,9 @@ int pz_run_frames(const pz_model* m, const void* in, long long in_frame, long lo
       pout[c] = {d, q.out_width, q.out_height, out_pitch, dtype};
     }
     const int n = n_frames - f < step ? n_frames - f : step;
-    if (const int rc = run_frame(m, pin, q.n_planes, pout, q.n_planes, &o, stream, f > 0, n, in_frame, out_frame)) return rc;
+    if (const int rc = run_frame(m, pin, q.n_planes, pout, q.n_planes, &o, stream, f > 0 ? kTableFilled : kMakeTable, n,
+                                 in_frame, out_frame))
+      return rc;
   }
   return PZ_OK;
 }

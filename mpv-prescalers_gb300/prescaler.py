@@ -370,7 +370,14 @@ class HookModel:
             if return_keys:
                 keys = torch.empty(self.key_shape(W, H, OW, OH), dtype=torch.int32, device=dev)
             scratch = torch.empty(plan.scratch, dtype=torch.uint8, device=dev) if plan.scratch else None
-            self._run(pl, res, _ffi.Opts.from_buffer_copy(plan.opts), keys, stream, scratch)
+            pin, pout, n = self._planes(pl, res)
+            o = plan.opts
+            if keys is not None:
+                o = _ffi.Opts.from_buffer_copy(o)
+                o.keys = keys.data_ptr()
+            _ffi.check(_ffi.lib().pz_run_with_scratch(
+                self.device_handle(dev.index), pin, n, pout, n, o, scratch.data_ptr() if plan.scratch else None,
+                plan.scratch, raw_stream(dev, stream)))
             return self._pack(res, planes, as_list, keys, return_keys, full)
 
     def _upscale_tensor(self, x, out_size, precision, staging, tile_rows):
@@ -582,23 +589,24 @@ class HookModel:
     def run_raw(self, pl, res, out_size, precision="fp32", keys=None, stream=None, scratch=None, staging=None,
                 tile_rows=None):
         """Low-level call of ``pz_run`` on prepared tensors (no allocation
-        besides the optional NNEDI3 scratch inside the library)."""
+        besides the optional scratch inside the library)."""
         o = self._opts(pl[0].shape[1], pl[0].shape[0], out_size, precision, staging, tile_rows)
-        self._run(pl, res, o, keys, stream, scratch)
-
-    def _run(self, pl, res, o, keys, stream, scratch):
-        torch = _torch()
-        dt = _ffi.PZ_F32 if pl[0].dtype == torch.float32 else _ffi.PZ_F16
-        n = len(pl)
-        pin = (_ffi.Plane * n)(*[(p.data_ptr(), p.shape[1], p.shape[0], p.stride(0), dt) for p in pl])
-        pout = (_ffi.Plane * n)(*[(r.data_ptr(), r.shape[1], r.shape[0], r.stride(0), dt) for r in res])
         if keys is not None:
             o.keys = keys.data_ptr()
         if scratch is not None:
             o.scratch = scratch.data_ptr()
             o.scratch_bytes = scratch.numel() * scratch.element_size()
+        pin, pout, n = self._planes(pl, res)
         dev = pl[0].device
         _ffi.check(_ffi.lib().pz_run(self.device_handle(dev.index), pin, n, pout, n, o, raw_stream(dev, stream)))
+
+    @staticmethod
+    def _planes(pl, res):
+        """The ``pz_plane`` arrays of input and output planes, and their number."""
+        dt = _ffi.PZ_F32 if pl[0].dtype == _torch().float32 else _ffi.PZ_F16
+        n = len(pl)
+        return ((_ffi.Plane * n)(*[(p.data_ptr(), p.shape[1], p.shape[0], p.stride(0), dt) for p in pl]),
+                (_ffi.Plane * n)(*[(r.data_ptr(), r.shape[1], r.shape[0], r.stride(0), dt) for r in res]), n)
 
     @staticmethod
     def _pack(res, planes, as_list, keys, return_keys, full=None):

@@ -388,3 +388,68 @@ def test_frames_without_scratch_ignore_its_byte_count(name):
         hm.device_handle(0), x.data_ptr(), C * H * W, H * W, W, y.data_ptr(), 4 * C * H * W, 4 * H * W, 2 * W, n, W, H,
         _ffi.PZ_F32, ctypes.byref(o), None, 1 << 30, torch.cuda.current_stream().cuda_stream))
     assert torch.equal(y, hm.upscale(x))
+
+
+@pytest.mark.parametrize("name,size,osz", [("ravu-zoom-r2", (960, 540), (1440, 810)),
+                                           ("ravu-zoom-ar-r3", (960, 540), (1920, 1080)),
+                                           ("ravu-lite-r3", (96, 54), None), ("ravu-3x-r2", (96, 54), None)])
+def test_scratch_that_a_chain_does_not_need_is_left_alone(name, size, osz):
+    """pz_run does not write to the scratch of a chain for which
+    pz_scratch_bytes says 0: a host may hand one buffer to all its calls."""
+    hm, _ = synth.model_for(name)
+    W, H = size
+    x = torch.rand((H, W), device="cuda", dtype=torch.float16)
+    OW, OH = hm.output_size(W, H, osz)
+    y = torch.empty((OH, OW), device="cuda", dtype=torch.float16)
+    scratch = torch.full((64 << 20,), 0x5A, dtype=torch.uint8, device="cuda")
+    hm.run_raw([x], [y], (OW, OH), precision="fast", scratch=scratch)
+    assert torch.equal(y, hm.upscale(x, out_size=osz, precision="fast"))
+    assert bool((scratch == 0x5A).all())
+
+
+@pytest.mark.parametrize("name", ["ravu-zoom-r2", "ravu-zoom-r3-yuv", "ravu-zoom-ar-r2-rgb", "ravu-zoom-ar-r3"])
+@pytest.mark.parametrize("size,osz", [((721, 487), (1442, 974)), ((720, 486), (1080, 729)), ((960, 400), (1200, 800))],
+                         ids=["2x", "1.5x", "1.25x2x"])
+@pytest.mark.parametrize("prec,dtype", [("fast", torch.float16), ("fp32", torch.float32), ("mpv", torch.float16)])
+def test_zoom_phase_table_in_a_calls_own_scratch(name, size, osz, prec, dtype):
+    """Calls with scratch of their own (a list of planes, a tensor, with keys,
+    into given outputs) take the weights from the phase table: the pixels and
+    keys of the general path, at every tile height; queued behind one another
+    in one scratch, and replayed from a graph."""
+    import ctypes
+    from mpv_prescalers_gb300 import _ffi
+    from mpv_prescalers_gb300.prescaler import PRECISIONS
+    hm, _ = synth.model_for(name)
+    C, (W, H), (OW, OH) = hm.n_planes, size, osz
+    xs = [torch.rand((C, H, W), device="cuda").to(dtype) for _ in range(3)]
+    want = [torch.empty((C, OH, OW), device="cuda", dtype=dtype) for _ in xs]
+    wkeys = torch.empty((OH, OW), device="cuda", dtype=torch.int32)
+    for x, y in reversed(list(zip(xs, want))):
+        hm.run_raw(list(x.unbind(0)), list(y.unbind(0)), osz, precision=prec, keys=wkeys)
+    for rows in (None, 4, 8, 16):
+        got, keys = hm.upscale(list(xs[0].unbind(0)), out_size=osz, precision=prec, tile_rows=rows, return_keys=True)
+        assert all(torch.equal(a, b) for a, b in zip(got, want[0])) and torch.equal(keys, wkeys), rows
+        assert torch.equal(hm.upscale(xs[0], out_size=osz, precision=prec, tile_rows=rows), want[0]), rows
+    o = _ffi.Opts()
+    o.precision = PRECISIONS[prec]
+    o.out_width, o.out_height = osz
+    n = _ffi.lib().pz_scratch_wanted(hm.device_handle(0), W, H, 0 if dtype == torch.float32 else 1, ctypes.byref(o))
+    scratch = torch.zeros(n, dtype=torch.uint8, device="cuda")
+    outs = [torch.zeros_like(y) for y in want]
+
+    def queue():
+        for x, y in zip(xs, outs):
+            pin, pout, c = hm._planes(list(x.unbind(0)), list(y.unbind(0)))
+            _ffi.check(_ffi.lib().pz_run_with_scratch(hm.device_handle(0), pin, c, pout, c, ctypes.byref(o),
+                                                      scratch.data_ptr(), n, torch.cuda.current_stream().cuda_stream))
+
+    queue()
+    assert all(torch.equal(a, b) for a, b in zip(outs, want)) and bool((scratch != 0).any())
+    for y in outs:
+        y.zero_()
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        queue()
+    g.replay()
+    assert all(torch.equal(a, b) for a, b in zip(outs, want))
