@@ -46,13 +46,19 @@ void launch_table(const RavuArgs& a, cudaStream_t s) {
 
 }  // namespace
 
-// The table pays where it holds far fewer entries than the frame has pixels (an
+// The table pays where it holds fewer entries than the frame has pixels (an
 // entry costs about what a pixel saves) and the frame is large enough for one
-// more launch (some 4 us): 1080p to 1.5x, 9 phases, 187 against 274 us
-// (ravu-zoom-ar-r2-rgb); 1080p to 2.25x, 81 phases, 145 against 281 us
-// (ravu-zoom-r2); 720x576 to 1080p, 120 phases and 60 pixels an entry, 38 against
-// 60 us; 854x480 to 1.75x, 49 phases and 89 pixels an entry, 63 against 68 us.
-// Scales of no simple ratio have as many phases as pixels and take none.
+// more launch (some 4 us).  Gain over weights per pixel, least (ravu-zoom-r2-rgb
+// fast) to most (ravu-zoom-ar-r2 FP32), at 720p, 1080p and 2160p outputs, by
+// pixels an entry: 8 1.05-1.97x, 18 1.10-2.46x, 32 1.09-2.40x, 72 1.13-2.73x, 3200
+// (1.5x) 1.28-2.85x; 1080p to 1.5x ravu-zoom-ar-r2-rgb 187 against 274 us.  Tables
+// beyond L2 still pay: ravu-zoom-ar-r3 to 2160p at 8 pixels an entry, 348 MB, 706
+// against 1087 us.  But they are scratch of every call: kTableMax leaves every
+// output up to 2160p its table and bounds the larger ones', up to 42 bytes a pixel
+// (1.4 GB at 7680x4320).  Scales of no simple ratio have as many phases as pixels
+// and take none.
+constexpr size_t kTableMax = (size_t)512 << 20;
+
 size_t zoom_table_bytes(int radius, bool ar, int keys, int W, int H, int OW, int OH, FastDiv* px,
                         FastDiv* py) {
   *px = fast_div(OW / gcd(W, OW));
@@ -61,7 +67,8 @@ size_t zoom_table_bytes(int radius, bool ar, int keys, int W, int H, int OW, int
   if (pixels < 1 << 19 || entries * 8 > pixels) return 0;
   const uint32_t e = radius == 2 ? (ar ? zoom_entry<2, true>() : zoom_entry<2, false>())
                                  : (ar ? zoom_entry<3, true>() : zoom_entry<3, false>());
-  return (size_t)entries * e * sizeof(float4);
+  const size_t bytes = (size_t)entries * e * sizeof(float4);
+  return bytes <= kTableMax ? bytes : 0;
 }
 
 int launch_zoom_table(const RavuArgs& a, int radius, bool ar, cudaStream_t s) {

@@ -453,3 +453,17 @@ def test_zoom_phase_table_in_a_calls_own_scratch(name, size, osz, prec, dtype):
         queue()
     g.replay()
     assert all(torch.equal(a, b) for a, b in zip(outs, want))
+
+
+@pytest.mark.parametrize("size,osz,table", [((2624, 1476), (3840, 2160), 288 * 3600 * 21 * 16), ((2592, 1458), (3840, 2160), 1),
+                                            ((4928, 2772), (7680, 4320), 0), ((5120, 2880), (7680, 4320), 1)])
+def test_zoom_phase_table_is_bounded(size, osz, table):
+    """Every 2160p output whose scale has few phases has room for its table;
+    14400 phases of an 8K output do not (1.4 GB), 9 do."""
+    import ctypes
+    from mpv_prescalers_gb300 import _ffi
+    hm, _ = synth.model_for("ravu-zoom-ar-r3")
+    o = _ffi.Opts()
+    o.out_width, o.out_height = osz
+    n = _ffi.lib().pz_scratch_wanted(hm.device_handle(0), *size, _ffi.PZ_F16, ctypes.byref(o))
+    assert n <= 512 << 20 and (n >= table if table else n == 0)
