@@ -77,6 +77,19 @@ def raw_stream(dev, stream) -> int:
     return _torch()._C._cuda_getCurrentRawStream(dev.index) if stream is None else stream.cuda_stream
 
 
+def scratch_for(nbytes: int, dev):
+    """A call's scratch on ``dev``, allocated on the current stream; None where
+    none is needed, or the device has no room (a ravu-zoom then interpolates
+    per pixel, and the library allocates what a chain cannot do without)."""
+    torch = _torch()
+    if not nbytes:
+        return None
+    try:
+        return torch.empty(nbytes, dtype=torch.uint8, device=dev)
+    except torch.cuda.OutOfMemoryError:
+        return None
+
+
 class _Plan:
     """What one frame geometry and form needs of a call, worked out once."""
     __slots__ = ("enabled", "out_size", "opts", "scratch")
@@ -369,14 +382,14 @@ class HookModel:
             keys = None
             if return_keys:
                 keys = torch.empty(self.key_shape(W, H, OW, OH), dtype=torch.int32, device=dev)
-            scratch = torch.empty(plan.scratch, dtype=torch.uint8, device=dev) if plan.scratch else None
+            scratch = scratch_for(plan.scratch, dev)
             pin, pout, n = self._planes(pl, res)
             o = plan.opts
             if keys is not None:
                 o = _ffi.Opts.from_buffer_copy(o)
                 o.keys = keys.data_ptr()
             _ffi.check(_ffi.lib().pz_run_with_scratch(
-                self.device_handle(dev.index), pin, n, pout, n, o, scratch.data_ptr() if plan.scratch else None,
+                self.device_handle(dev.index), pin, n, pout, n, o, scratch.data_ptr() if scratch is not None else None,
                 plan.scratch, raw_stream(dev, stream)))
             return self._pack(res, planes, as_list, keys, return_keys, full)
 
@@ -397,9 +410,9 @@ class HookModel:
             return None
         out_shape, from_in, from_out, scratch_bytes, opts = call
         out = torch.empty(out_shape, dtype=dtype, device=dev)
-        scratch = torch.empty(scratch_bytes, dtype=torch.uint8, device=dev) if scratch_bytes else None
+        scratch = scratch_for(scratch_bytes, dev)
         rc = _ffi.lib().pz_run_frames(self.device_handle(dev.index), x.data_ptr(), *from_in, out.data_ptr(), *from_out,
-                                      opts, scratch.data_ptr() if scratch_bytes else None, scratch_bytes,
+                                      opts, scratch.data_ptr() if scratch is not None else None, scratch_bytes,
                                       raw_stream(dev, None))
         if rc:
             _ffi.check(rc)

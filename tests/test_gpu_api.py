@@ -467,3 +467,24 @@ def test_zoom_phase_table_is_bounded(size, osz, table):
     o.out_width, o.out_height = osz
     n = _ffi.lib().pz_scratch_wanted(hm.device_handle(0), *size, _ffi.PZ_F16, ctypes.byref(o))
     assert n <= 512 << 20 and (n >= table if table else n == 0)
+
+
+@pytest.mark.parametrize("name,osz", [("ravu-zoom-ar-r2", (1440, 810)), ("ravu-r3", None), ("nnedi3-nns16-win8x4", None)])
+def test_upscale_without_room_for_scratch(name, osz, monkeypatch):
+    """Scratch that the device has no room for is done without: a ravu-zoom
+    interpolates per pixel, a batch runs frame by frame in scratch that the
+    library allocates; as a tensor, a batch and a list."""
+    hm, _ = synth.model_for(name)
+    x = torch.rand((2, 1, 540, 960), device="cuda", dtype=torch.float16)
+    want = hm.upscale(x, out_size=osz)
+    empty = torch.empty
+
+    def no_room(*args, **kw):
+        if kw.get("dtype") is torch.uint8:
+            raise torch.cuda.OutOfMemoryError("no room")
+        return empty(*args, **kw)
+
+    monkeypatch.setattr(torch, "empty", no_room)
+    assert torch.equal(hm.upscale(x, out_size=osz), want)
+    assert torch.equal(hm.upscale(x[0], out_size=osz), want[0])
+    assert torch.equal(hm.upscale([x[1, 0]], out_size=osz)[0], want[1, 0])
