@@ -104,15 +104,19 @@ int check_plane(const pz_plane& p, const char* what, int idx, bool pairs) {
 //          then keeps 22 bits or more, and a smaller one an absolute error of
 //          2^-39 of the largest.  Not made (the CUDA cores run the model)
 //          when a value is not finite or the power lies outside 2^-8..2^30,
-//          so that the blend's product of two denominators, of at most 2^37
-//          each, and its reciprocal stay within FP32's normal range.
+//          so that the blend's product of two denominators, of at most 2^31
+//          each, and its reciprocal stay within FP32's normal range.  Whether its
+//          numerators may leave FP32's range (nn_tc_kernel marks such pixels) is
+//          bounded here: a window's x_hat has norm sqrt(T) and no mean, and its
+//          mean term is at most 60000, so that a pre-activation is at most
+//          sqrt(T) |w - mean(w)| + 60000 |sum w| + |bias|.
 int upload_operands(pz_model* m, const std::vector<float>& w, const std::vector<float>& bias) {
   const int n = m->nns, T = m->win_w * m->win_h;
   const int NCH = pz::nnedi3_tc_chunk(n, m->win_h, false), NCS = pz::nnedi3_tc_chunk(n, m->win_h, true);
   const int KP = (T + 4 + 15) / 16 * 16;  // taps, mean term, three bias pieces, padded to a K step
   const double kLog2e = 1.4426950408889634;
   std::vector<double> v((size_t)2 * n * (T + 2));  // [2 * neuron + branch][weights, sum, bias]
-  double top = 0.0;
+  double top = 0.0, most[2] = {0.0, 0.0};  // largest pre-activation per branch (softmax: log2 units)
   bool finite = true;
   for (int r = 0; r < 2 * n; r++) {
     const int k = r / 2, br = r % 2;
@@ -126,6 +130,9 @@ int upload_operands(pz_model* m, const std::vector<float>& w, const std::vector<
     }
     row[T] = sum * scale;
     row[T + 1] = bias[2 * k + br] * scale;
+    double norm2 = 0.0;
+    for (int t = 0; t < T; t++) norm2 += (row[t] - row[T] / T) * (row[t] - row[T] / T);
+    most[br] = std::max(most[br], std::sqrt(T * norm2) + 60000.0 * std::fabs(row[T]) + std::fabs(row[T + 1]));
     for (int t = 0; t < T + 2; t++) {
       finite = finite && std::isfinite(row[t]);
       top = std::max(top, std::fabs(row[t]));
@@ -166,6 +173,10 @@ int upload_operands(pz_model* m, const std::vector<float>& w, const std::vector<
   int rc = upload(&m->d_wts_h, h.data(), piece * 2);
   if (!rc && split) {
     m->split_one = (float)std::ldexp(1.0, exp2);
+    // e s (1 + |s|) at the square of the scale, over all neurons, with room for
+    // the roundings; and one e of at least 2^-89
+    const double top2 = most[0] + 2.0 * (exp2 + std::log2(1.0 + most[1])) + std::log2((double)n);
+    m->may_mark = !(top2 < 126.0 && most[0] < 89.0);
     rc = upload(&m->d_wts_s, s.data(), 2 * piece * 2);
   }
   return rc;
@@ -567,7 +578,7 @@ static int run_frame(const pz_model* m, const pz_plane* in, int n_in, pz_plane* 
       a.in_frame = sframe;
       a.out_frame = dframe;
       a.after = src == tmp && tmp;
-      return pz::launch_nnedi3(a, precision, xpass, dt, s);
+      return pz::launch_nnedi3(m, a, precision, xpass, dt, s);
     };
     rc = 0;
     if (ax == 3) {

@@ -70,7 +70,7 @@ struct NnArgs {
   int out_pitch;
   int W, H;                 // size of the pass input
   int after;                // launched right after its prerequisite (launch_kernel; tensor cores)
-  int frames;               // frames of one launch (tensor cores; 0 counts as 1), elements apart:
+  int frames;               // frames (of one launch: tensor cores; 0 counts as 1), elements apart:
   long long in_frame, out_frame;
   int nns, win_h;           // window is 8 x win_h (double_y orientation)
   const float* wts;         // [nns][2][T]: A row then B row per neuron (FP32)
@@ -98,6 +98,8 @@ inline void zoom_divisors(RavuArgs* a) {
 size_t zoom_table_bytes(int radius, bool ar, int keys, int W, int H, int OW, int OH, FastDiv* px, FastDiv* py);
 int launch_zoom_table(const RavuArgs& a, int radius, bool ar, cudaStream_t s);
 int launch_nnedi3_simt(const NnArgs& a, bool xpass, int dtype, cudaStream_t s);
+// The pixels that launch_nnedi3_split, on the same arguments, has marked.
+int launch_nnedi3_marked(const NnArgs& a, bool xpass, int dtype, cudaStream_t s);
 int launch_nnedi3_tc(const NnArgs& a, bool xpass, int dtype, cudaStream_t s);
 int launch_nnedi3_split(const NnArgs& a, bool xpass, int dtype, cudaStream_t s);
 bool nnedi3_tc_supported(int nns, int win_h);

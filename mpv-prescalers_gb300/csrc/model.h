@@ -24,6 +24,7 @@ struct pz_model {
   __half* d_wts_h = nullptr;
   __half* d_wts_s = nullptr;  // split operand of the plain FP32 form (null: CUDA cores)
   float split_one = 1.0f;     // the power of two it is scaled by
+  bool may_mark = true;       // may its pixels leave the split blend's range?
   int device = 0;
 };
 
@@ -102,22 +103,18 @@ inline NnArgs nn_args(const pz_model* m, int* err) {
 // against 491 us; 160x90 nns32 8x4 the same (both are the two launches).  The
 // error against 64 bits is 0.5-0.65x the CUDA cores' for every nns and window
 // (nns128 8x6 at 640x360: 8.6e-8 against 1.46e-7 relative).  Models of other
-// shapes, or with weights that the pieces cannot hold, stay on the CUDA cores.
-inline int launch_nnedi3(const NnArgs& a, int precision, bool xpass, int dtype, cudaStream_t s) {
+// shapes, or with weights that the pieces cannot hold, stay on the CUDA cores;
+// and so do single pixels of models whose pre-activations may leave the split
+// blend's range (may_mark), by a second launch that looks for them.
+inline int launch_nnedi3(const pz_model* m, const NnArgs& a, int precision, bool xpass, int dtype, cudaStream_t s) {
   if (nnedi3_tc_supported(a.nns, a.win_h)) {
     if (precision == PZ_PREC_FAST) return launch_nnedi3_tc(a, xpass, dtype, s);
-    if (a.wts_s) return launch_nnedi3_split(a, xpass, dtype, s);
+    if (a.wts_s) {
+      const int rc = launch_nnedi3_split(a, xpass, dtype, s);
+      return rc || !m->may_mark ? rc : launch_nnedi3_marked(a, xpass, dtype, s);
+    }
   }
-  // one frame a launch
-  NnArgs b = a;
-  b.frames = 1;
-  const size_t es = dtype == PZ_F32 ? 4 : 2;
-  for (int f = 0; f < (a.frames > 0 ? a.frames : 1); f++) {
-    b.in = static_cast<const char*>(a.in) + f * a.in_frame * (long long)es;
-    b.out = static_cast<char*>(a.out) + f * a.out_frame * (long long)es;
-    if (const int rc = launch_nnedi3_simt(b, xpass, dtype, s)) return rc;
-  }
-  return 0;
+  return launch_nnedi3_simt(a, xpass, dtype, s);
 }
 
 // Scratch of a ravu lattice chain: the int11 plane, FP32 [channels][H][W].

@@ -110,7 +110,7 @@ extern "C" int pz_nnedi3_run_static(const pz_model* m, const pz_plane* in, pz_pl
     a.out_pitch = dpitch;
     a.W = sw;
     a.H = sh;
-    return pz::launch_nnedi3(a, precision, xpass, dt, s);
+    return pz::launch_nnedi3(m, a, precision, xpass, dt, s);
   };
   if (ax == 3) {
     rc = pass(false, in->data, W, H, in->pitch, addr.scratch, W);

@@ -410,7 +410,7 @@ __global__ void __launch_bounds__(TcShape<WH, NNS, XP, SPLIT>::THREADS, 1) nn_tc
       prefetch(t + stride);
     }
     const uint32_t lane_addr = tmem + g * NBUF * CCOL + ((uint32_t)(py * 32) << 16);
-    const float one = SPLIT ? p.split_one : 1.0f, half_unit = SPLIT ? 0.5f * p.split_unit : 1.0f;
+    const float one = SPLIT ? p.split_one : 1.0f, unit = SPLIT ? p.split_unit : 1.0f;
     int c = 0;
     for (; t < ntiles; t += stride) {
       float2 wsum = make_float2(0.0f, 0.0f), vsum = wsum;
@@ -457,36 +457,23 @@ __global__ void __launch_bounds__(TcShape<WH, NNS, XP, SPLIT>::THREADS, 1) nn_tc
             }
           }
           // sum of e s / (1 + |s|): neurons j and j+2 (and j+1, j+3) share one
-          // reciprocal, of the product of their denominators.  Split: s / (1 + |s|)
-          // (the scale cancels in it) is formed before e comes in, and e = 2^l is the
-          // square of 2^(l/2), so that no product leaves FP32's range before e does
-          // and e reaches down into the subnormals: logits of -95 to 88 as by expf
-          // (e s (1 + |s|) at the model's scale was infinite from logits of 70 on, e
-          // zero below -87; nns128 8x6 at 1080p 440 us so, now 476)
+          // reciprocal, of the product of their denominators
 #pragma unroll
           for (int j = 0; j < 16; j += 4) {
-            float2 e[2], n[2], d[2];  // n: s (split), e s
+            float2 n[2], d[2];
 #pragma unroll
             for (int h = 0; h < 2; h++) {
               const int i = j + 2 * h;
               float2 l = make_float2(s1[q & 1][i], s1[q & 1][i + 1]);
-              if (SPLIT) l = __fmul2_rn(l, make_float2(half_unit, half_unit));
-              e[h] = make_float2(exp2f_approx(l.x), exp2f_approx(l.y));
-              if (SPLIT) e[h] = __fmul2_rn(e[h], e[h]);
+              if (SPLIT) l = __fmul2_rn(l, make_float2(unit, unit));
+              const float2 e = make_float2(exp2f_approx(l.x), exp2f_approx(l.y));
               d[h] = make_float2(one + fabsf(s2[q & 1][i]), one + fabsf(s2[q & 1][i + 1]));
-              n[h] = make_float2(s2[q & 1][i], s2[q & 1][i + 1]);
-              if (!SPLIT) n[h] = __fmul2_rn(e[h], n[h]);
-              wsum = __fadd2_rn(wsum, e[h]);
+              n[h] = __fmul2_rn(e, make_float2(s2[q & 1][i], s2[q & 1][i + 1]));
+              wsum = __fadd2_rn(wsum, e);
             }
             const float2 dd = __fmul2_rn(d[0], d[1]);
-            if (SPLIT) {
-              const float2 r = make_float2(rcp_approx(dd.x), rcp_approx(dd.y));
-              vsum = __ffma2_rn(e[0], __fmul2_rn(__fmul2_rn(n[0], d[1]), r), vsum);
-              vsum = __ffma2_rn(e[1], __fmul2_rn(__fmul2_rn(n[1], d[0]), r), vsum);
-            } else {
-              const float2 nn = __ffma2_rn(n[0], d[1], __fmul2_rn(n[1], d[0]));
-              vsum = __ffma2_rn(nn, make_float2(rcp_approx(dd.x), rcp_approx(dd.y)), vsum);
-            }
+            const float2 nn = __ffma2_rn(n[0], d[1], __fmul2_rn(n[1], d[0]));
+            vsum = __ffma2_rn(nn, make_float2(rcp_approx(dd.x), rcp_approx(dd.y)), vsum);
           }
         }
       }
@@ -495,7 +482,20 @@ __global__ void __launch_bounds__(TcShape<WH, NNS, XP, SPLIT>::THREADS, 1) nn_tc
       gy += py;
       T* dst = out + f * p.out_frame;
       if (gx < p.W && gy < p.H && !*aborted) {
-        const float v = clampf(cur.mean + 5.0f * (vsum.x + vsum.y) / (wsum.x + wsum.y) * cur.stdv, 0.0f, 1.0f);
+        const float ws = wsum.x + wsum.y, vs = vsum.x + vsum.y;
+        float v = clampf(cur.mean + 5.0f * vs / ws * cur.stdv, 0.0f, 1.0f);
+        // The split blend multiplies e by s (1 + |s|) and the square of its scale
+        // before it divides: from logits of about 70 on that is infinite, and stays
+        // so or turns to NaN in the sums, where e itself is good to 88; and e is
+        // flushed below 2^-126, which 256 neurons may feel where their sum is below
+        // 2^-90 (logits below -62).  Such a window's pixel is marked by a NaN, which is
+        // stored for no other, and launch_nnedi3_marked takes it in plain FP32.
+        // Forming s / (1 + |s|) first and e as the square of 2^(l/2) instead keeps
+        // every pixel in range, but costs all of them (nns128 8x6 at 1080p 476 us,
+        // 438) and 1 % of accuracy; an FP32 pixel called from here 454 us; the mark 441.
+        if (SPLIT && (ws < 0x1p-90f || !(fabsf(vs) < INFINITY)) && fabsf(cur.mean) < INFINITY &&
+            fabsf(cur.stdv) < INFINITY)
+          v = NAN;
         if (XP) {
           stp2(dst + (size_t)gy * p.out_pitch + 2 * gx, cur.orig, v);
         } else {

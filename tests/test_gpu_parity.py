@@ -289,6 +289,37 @@ def test_nnedi3_fp32_large_logits(name, elliott, logit):
     assert err.max() <= (1.3e-4 if logit > -90 else 1.3e-4 + 8.6e-4) + TOL_FP32
 
 
+@pytest.mark.parametrize("name", ["nnedi3-nns16-win8x4", "nnedi3-nns256-win8x6"])
+@pytest.mark.parametrize("sign", [1.0, -1.0])
+def test_nnedi3_fp32_some_large_logits(name, sign):
+    """Softmax weights that sum to 1 (-1): a window's logits lie around its
+    mean over its deviation.  In one half of a frame, a checkerboard of 0.4 +-
+    0.0055, that is 73, beyond the split blend's range and, with the 5 that the
+    centred weights and the bias add, below the 88 of FP32's exp; in the other, 0.4
+    +- 0.2, it is 2.  A logit of 78 that is off by 2^-20 of itself moves a mean of
+    values in [-1, 1] by 1.5e-4 and the pixel by 5 deviations times that: 4e-6 on
+    the one half, 2^-20 * 7 * 2 * 1 = 1.3e-5 on the other (the two halves' windows
+    mix along the seam, at larger deviations).  Each axis by itself, and a batch of
+    frames as its frames."""
+    import dataclasses
+    from mpv_prescalers_gb300.prescaler import HookModel
+    m = synth.synthetic_model(name)
+    m = dataclasses.replace(m, weights_a=m.weights_a + np.float32(sign / (8 * m.win_h)))
+    hm = HookModel(m)
+    H, W = 37, 70
+    yy, xx = np.mgrid[:H, :W]
+    x = (0.4 + np.where(xx < W // 2, 0.0055, 0.2) * (1 - 2 * ((xx + yy) % 2))).astype(np.float32)
+    xt = torch.from_numpy(x).cuda()
+    for axis, size in (("y", (W, 2 * H)), ("x", (2 * W, H))):
+        y = hm.upscale(xt, out_size=size).cpu().numpy().astype(np.float64)
+        ref, _ = oracle.nnedi3_upscale(m, x, axes=axis)
+        assert np.abs(y - ref[0]).max() <= 2e-5
+    batch = torch.stack([xt, xt.flip(1), xt * 0.5])[:, None]
+    y = hm.upscale(batch)
+    for i in range(3):
+        assert torch.equal(y[i], hm.upscale(batch[i]))
+
+
 def test_nnedi3_fp32_on_the_variance_gate():
     """Windows with variance near FLT_EPS: a plane of 0.5 with +-d
     perturbations on a few pixels so that var ~ eps; the bound per gate
