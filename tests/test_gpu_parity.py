@@ -320,6 +320,34 @@ def test_nnedi3_fp32_some_large_logits(name, sign):
         assert torch.equal(y[i], hm.upscale(batch[i]))
 
 
+@pytest.mark.parametrize("name,scale", [("nnedi3-nns24-win8x4", 0), ("nnedi3-nns40-win8x6", 0),
+                                        ("nnedi3-nns32-win8x4", -40), ("nnedi3-nns16-win8x6", -40)])
+@pytest.mark.parametrize("axes", ["y", "x", "yx"])
+def test_nnedi3_on_the_cuda_cores(name, scale, axes):
+    """Neuron counts that the tensor-core kernel is not built for, and weights
+    too small for its FP16 pieces (the largest below 2^-17), run on the CUDA
+    cores, in the fast form too where the count is the reason: plain FP32
+    against the oracle, and a batch whose frames lie apart as its frames."""
+    import dataclasses
+    from mpv_prescalers_gb300.prescaler import HookModel
+    m = synth.synthetic_model(name)
+    if scale:
+        m = dataclasses.replace(m, **{k: getattr(m, k) * np.float32(2.0 ** scale)
+                                      for k in ("weights_a", "weights_b", "bias_a", "bias_b")})
+    hm = HookModel(m)
+    H, W = 27, 35
+    _check_nnedi3_fp32(hm, synth.luma_plane(H, W, 51), axes)
+    size = (2 * W if "x" in axes else W, 2 * H if "y" in axes else H)
+    big = torch.from_numpy(synth.luma_plane(3 * (H + 2), W + 3, 52)).cuda().reshape(3, 1, H + 2, W + 3)
+    for x in (big[:, :, 1:H + 1, 2:W + 2], big[::2, :, 1:H + 1, 2:W + 2].half()):
+        y = hm.upscale(x, out_size=size)
+        for i in range(x.shape[0]):
+            assert torch.equal(y[i], hm.upscale(x[i], out_size=size))
+            assert torch.equal(y[i, 0], hm.upscale([x[i, 0]], out_size=size)[0])
+        if not scale:
+            assert torch.equal(y, hm.upscale(x, out_size=size, precision="fast"))
+
+
 def test_nnedi3_fp32_on_the_variance_gate():
     """Windows with variance near FLT_EPS: a plane of 0.5 with +-d
     perturbations on a few pixels so that var ~ eps; the bound per gate
