@@ -19,7 +19,6 @@
 // t % 32 of row t / 32 (zoom; the others: of the P rows from P * (t / 32)).  Out-of-range reads replicate the edge texel (the mpv
 // texture border mode).
 #pragma once
-#include <atomic>
 #include <cstddef>
 #include <cstring>
 
@@ -1127,26 +1126,15 @@ __global__ void __maxnreg__(Prog::kMaxRegs) tile_kernel_mr(const __grid_constant
   tile_body<Prog, TMA>(p, maps);
 }
 
-// SMEM: bytes of dynamic shared memory.  Above 48 KB (ravu-zoom-ar of three
-// channels at 16 rows) the kernel is opted in once per device; two threads that
-// do so at once set the same value.
+// SMEM: bytes of dynamic shared memory.
 template <class Prog, bool TMA, size_t SMEM>
-int launch_tile_kernel(dim3 grid, cudaStream_t s, const RavuArgs& a, const TmaMaps& maps) {
+void launch_tile_kernel(dim3 grid, cudaStream_t s, const RavuArgs& a, const TmaMaps& maps) {
+  static_assert(SMEM <= 48 * 1024, "tile program needs more than the default shared memory");
   auto kern = [] {
     if constexpr (Prog::kMaxRegs > 0) return tile_kernel_mr<Prog, TMA>;
     else return tile_kernel<Prog, TMA>;
   }();
-  if constexpr (SMEM > 48 * 1024) {
-    static std::atomic<bool> opted[64];
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -95;
-    if (!opted[dev].load(std::memory_order_relaxed)) {
-      if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM) != cudaSuccess) return -5;
-      opted[dev].store(true, std::memory_order_relaxed);
-    }
-  }
   launch_kernel(kern, grid, Prog::kThreads, SMEM, s, a.after, a, maps);
-  return 0;
 }
 
 bool encode_plane_map(CUtensorMap* map, const void* base, int W, int H, int pitch, int dtype, int box_w,
@@ -1212,15 +1200,18 @@ int launch_tiles(const RavuArgs& a, cudaStream_t s) {
     RavuArgs b = a;
     if (a.staging == 1 && encode_tma<Prog>(&b, &maps)) {
       constexpr size_t smem = ((Prog::smem_bytes + 127) & ~(size_t)127) + tma_landing_bytes<Prog>();
-      return launch_tile_kernel<Prog, true, smem>(dim3(tiles_w, tiles_h), s, b, maps);
+      launch_tile_kernel<Prog, true, smem>(dim3(tiles_w, tiles_h), s, b, maps);
+      return 0;
     }
   }
   if constexpr (kHasOneFrame<Prog>) {
-    if (a.frames <= 1)
-      return launch_tile_kernel<OneFrame<Prog>, false, Prog::smem_bytes>(dim3(tiles_w, tiles_h), s, a, maps);
+    if (a.frames <= 1) {
+      launch_tile_kernel<OneFrame<Prog>, false, Prog::smem_bytes>(dim3(tiles_w, tiles_h), s, a, maps);
+      return 0;
+    }
   }
-  return launch_tile_kernel<Prog, false, Prog::smem_bytes>(dim3(tiles_w, tiles_h, a.frames > 0 ? a.frames : 1), s, a,
-                                                            maps);
+  launch_tile_kernel<Prog, false, Prog::smem_bytes>(dim3(tiles_w, tiles_h, a.frames > 0 ? a.frames : 1), s, a, maps);
+  return 0;
 }
 
 // ------------------------------------------------------ persistent batches ---
