@@ -40,7 +40,10 @@ struct KeyParams {
 // Device-side error word shared by all kernels: first failure wins.
 enum : int { kErrNone = 0, kErrTileOverflow = 1, kErrWaitTimeout = 2, kErrQueue = 3 };
 
-// t / d for 0 <= t < 2^31 by a multiplication, with the divisor fixed on the host.
+// t / d for 0 <= t < 2^31 by a multiplication, with the divisor fixed on the host
+// (Granlund and Montgomery, Division by Invariant Integers using Multiplication,
+// 1994, figure 4.1: m' = floor(2^32 (2^s - d) / d) + 1, s = ceil(log2 d); their two
+// shifts are one, as the sum fits 32 bits for these t).
 struct FastDiv {
   uint32_t m, s, d;
   __device__ __forceinline__ uint32_t operator()(uint32_t t) const { return (__umulhi(t, m) + t) >> s; }
@@ -102,50 +105,40 @@ __device__ __forceinline__ float deriv(const G& s, int p) {
 
 // Gaussian-weighted sum of (gx^2, gx gy, gy^2) over the gradient points:
 // the whole window when N <= 4, else the window minus a one-tap border.
-// `get(kx, ky)` returns the key input at window grid (kx, ky).  PACKED: a
-// and d accumulate as one FP32x2 pair, a += gx (gx w), d += gy (gy w),
-// b += (gx w) gy (three instructions per point instead of six), and where
+// `get(kx, ky)` returns the key input at window grid (kx, ky).  a and d
+// accumulate as one FP32x2 pair, a += gx (gx w), d += gy (gy w), b += (gx w) gy
+// (three instructions per point instead of six), and where
 // both stencils of a point share one scale c the scale moves into the weight
 // (gwf = gw c^2: the unscaled differences are used).  Each term then rounds
 // a few times differently from the shader's gx * gx * w, far inside the
 // key's FP32 boundary budget.
-template <int N, bool FOUR, bool PACKED = true, class Get>
+template <int N, bool FOUR, class Get>
 __device__ __forceinline__ void structure_tensor(const Get& get, const KeyParams& kp, float& a,
                                                  float& b, float& d) {
   constexpr int P0 = N <= 4 ? 0 : 1;
   constexpr int P1 = N <= 4 ? N : N - 1;
   float2 ad = make_float2(0.0f, 0.0f);
-  a = 0.0f;
   b = 0.0f;
-  d = 0.0f;
   int i = 0;
 #pragma unroll
   for (int px = P0; px < P1; px++) {
 #pragma unroll
     for (int py = P0; py < P1; py++) {
-      const bool fold = PACKED && stencil_kind(N, FOUR, px) == stencil_kind(N, FOUR, py);
+      const bool fold = stencil_kind(N, FOUR, px) == stencil_kind(N, FOUR, py);
       auto sx = [&](int q) { return get(q, py); };
       auto sy = [&](int q) { return get(px, q); };
       const float gx = fold ? deriv_unscaled<N, FOUR>(sx, px) : deriv<N, FOUR>(sx, px);
       const float gy = fold ? deriv_unscaled<N, FOUR>(sy, py) : deriv<N, FOUR>(sy, py);
       const float w = fold ? kp.gwf[i] : kp.gw[i];
       i++;
-      if constexpr (PACKED) {
-        const float2 g2 = make_float2(gx, gy);
-        const float2 gw2 = __fmul2_rn(g2, make_float2(w, w));
-        ad = __ffma2_rn(g2, gw2, ad);
-        b = fmaf(gw2.x, gy, b);
-      } else {
-        a += gx * gx * w;
-        b += gx * gy * w;
-        d += gy * gy * w;
-      }
+      const float2 g2 = make_float2(gx, gy);
+      const float2 gw2 = __fmul2_rn(g2, make_float2(w, w));
+      ad = __ffma2_rn(g2, gw2, ad);
+      b = fmaf(gw2.x, gy, b);
     }
   }
-  if constexpr (PACKED) {
-    a = ad.x;
-    d = ad.y;
-  }
+  a = ad.x;
+  d = ad.y;
 }
 
 // The structure tensors of E windows of one lattice that a thread evaluates
@@ -153,7 +146,8 @@ __device__ __forceinline__ void structure_tensor(const Get& get, const KeyParams
 // and `get(X, Y)` returns the key input at lattice point (X, Y).  The points run
 // in lattice order, so that a derivative that several windows share (the same
 // stencil at the same point) is formed once; each window's own sums see their
-// terms in the order and rounding of structure_tensor<PACKED>.
+// terms in the order and (PACKED) rounding of structure_tensor; else each lane
+// rounds as the shader's a += gx * gx * w.
 template <int N, bool FOUR, bool PACKED, int E, class Off, class Get>
 __device__ __forceinline__ void structure_tensors(const Get& get, const KeyParams& kp, float (&a)[E], float (&b)[E],
                                                   float (&d)[E]) {
