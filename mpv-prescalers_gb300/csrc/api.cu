@@ -89,6 +89,8 @@ int check_plane(const pz_plane& p, const char* what, int idx, bool pairs) {
   return PZ_OK;
 }
 
+constexpr double kLog2e = 1.4426950408889634;
+
 // The tensor-core operands B [2*nns][KP] of an NNEDI3 model, chunk-major:
 // chunk c of NC neurons (nnedi3_tc_chunk) is NC softmax-branch rows followed by
 // NC Elliott-branch rows.  Row = [weights (T taps), sum of the
@@ -110,76 +112,86 @@ int check_plane(const pz_plane& p, const char* what, int idx, bool pairs) {
 //          bounded here: a window's x_hat has norm sqrt(T) and no mean, and its
 //          mean term is at most 60000, so that a pre-activation is at most
 //          sqrt(T) |w - mean(w)| + 60000 |sum w| + |bias|.
+//
+// One block per row (the softmax or Elliott branch of a neuron), one thread per
+// element; `up`: the power of two, 0: no pieces.  On the device, where its three
+// conversions a value cost nothing: nns256 8x6 loads in LOADNEW ms, in 0.70 with
+// them on the host.
+__global__ void operand_kernel(const float* wts, const float* bias, int T, int KP, int nch, int ncs, double up,
+                               __half* h, __half* s) {
+  const int r = blockIdx.x, t = threadIdx.x;
+  const size_t piece = (size_t)gridDim.x * KP;
+  const float* w = wts + (size_t)r * T;
+  const double scale = r % 2 == 0 ? kLog2e : 1.0;
+  double x = 0.0;
+  if (t < T) x = w[t];
+  if (t == T)
+    for (int i = 0; i < T; i++) x += w[i];
+  if (t > T && t <= T + 3) x = bias[r];
+  x *= scale;
+  auto at = [&](int nc) {
+    const int k = r / 2, row = k / nc * 2 * nc + r % 2 * nc + k % nc;
+    return (size_t)(row >> 3) * 8 * KP + (t >> 3) * 64 + (row & 7) * 8 + (t & 7);
+  };
+  // piece j of v: the FP16 value of what the pieces before it leave
+  auto take = [](double v, int j) {
+    __half p = __float2half_rn((float)v);
+    for (; j > 0; j--) {
+      v -= (double)__half2float(p);
+      p = __float2half_rn((float)v);
+    }
+    return p;
+  };
+  const int j = t > T ? t - T - 1 : 0;  // a bias has an element for each of its pieces
+  h[at(nch)] = j < 2 ? take(x, j) : __float2half_rn(0.0f);
+  if (up > 0.0) {
+    s[at(ncs)] = j < 3 ? take(x * up, j) : __float2half_rn(0.0f);
+    s[piece + at(ncs)] = t <= T ? take(x * up, 1) : __float2half_rn(0.0f);
+  }
+}
+
+// The operands from the FP32 weights and biases that the model already holds on
+// the device (w, bias: on the host).
 int upload_operands(pz_model* m, const std::vector<float>& w, const std::vector<float>& bias) {
   const int n = m->nns, T = m->win_w * m->win_h;
-  const int NCH = pz::nnedi3_tc_chunk(n, m->win_h, false), NCS = pz::nnedi3_tc_chunk(n, m->win_h, true);
   const int KP = (T + 4 + 15) / 16 * 16;  // taps, mean term, three bias pieces, padded to a K step
-  const double kLog2e = 1.4426950408889634;
-  std::vector<double> v((size_t)2 * n * (T + 2));  // [2 * neuron + branch][weights, sum, bias]
   double top = 0.0, most[2] = {0.0, 0.0};  // largest pre-activation per branch (softmax: log2 units)
   bool finite = true;
   for (int r = 0; r < 2 * n; r++) {
-    const int k = r / 2, br = r % 2;
-    const double scale = br == 0 ? kLog2e : 1.0;
-    double* row = &v[(size_t)r * (T + 2)];
-    double sum = 0.0;
+    const float* row = &w[(size_t)r * T];
+    const double scale = r % 2 == 0 ? kLog2e : 1.0;
+    double sum = 0.0, squares = 0.0, largest = std::fabs(bias[r]);
     for (int t = 0; t < T; t++) {
-      const double x = w[((size_t)k * 2 + br) * T + t];
+      const double x = row[t];
       sum += x;
-      row[t] = x * scale;
+      squares += x * x;
+      largest = std::max(largest, std::fabs(x));
     }
-    row[T] = sum * scale;
-    row[T + 1] = bias[2 * k + br] * scale;
-    double norm2 = 0.0;
-    for (int t = 0; t < T; t++) norm2 += (row[t] - row[T] / T) * (row[t] - row[T] / T);
-    most[br] = std::max(most[br], std::sqrt(T * norm2) + 60000.0 * std::fabs(row[T]) + std::fabs(row[T + 1]));
-    for (int t = 0; t < T + 2; t++) {
-      finite = finite && std::isfinite(row[t]);
-      top = std::max(top, std::fabs(row[t]));
-    }
+    largest = std::max(largest, std::fabs(sum));
+    const double norm = std::sqrt(std::max(squares - sum * sum / T, 0.0));
+    most[r % 2] = std::max(most[r % 2], (std::sqrt((double)T) * norm + 60000.0 * std::fabs(sum) + std::fabs(bias[r])) * scale);
+    finite = finite && std::isfinite(squares + sum + bias[r]);
+    top = std::max(top, largest * scale);
   }
-  const size_t piece = (size_t)2 * n * KP;
   const int exp2 = top > 0.0 && finite ? 13 - std::ilogb(top) : 0;
   const bool split = finite && exp2 >= -8 && exp2 <= 30;
-  const __half zero = __float2half_rn(0.0f);
-  std::vector<__half> h(piece, zero), s(2 * piece, zero);
-  auto at = [&](int row, int t, int NC) {  // element t of the neuron and branch `row`
-    const int k = row / 2, r = k / NC * 2 * NC + row % 2 * NC + k % NC;
-    return (size_t)(r >> 3) * 8 * KP + (t >> 3) * 64 + (r & 7) * 8 + (t & 7);
-  };
-  auto half_of = [](double x) { return __float2half_rn((float)x); };
-  auto val = [](__half x) { return (double)__half2float(x); };
-  for (int r = 0; r < 2 * n; r++) {
-    const double* row = &v[(size_t)r * (T + 2)];
-    for (int t = 0; t <= T; t++) {
-      h[at(r, t, NCH)] = half_of(row[t]);
-      if (split) {
-        const double x = std::ldexp(row[t], exp2);
-        const __half hi = half_of(x);
-        s[at(r, t, NCS)] = hi;
-        s[piece + at(r, t, NCS)] = half_of(x - val(hi));
-      }
-    }
-    double b = row[T + 1], x = split ? std::ldexp(b, exp2) : 0.0;
-    for (int t = T + 1; t <= T + 3; t++) {  // two pieces (fast form), three (split)
-      if (t < T + 3) {
-        h[at(r, t, NCH)] = half_of(b);
-        b -= val(h[at(r, t, NCH)]);
-      }
-      s[at(r, t, NCS)] = half_of(x);
-      x -= val(s[at(r, t, NCS)]);
-    }
-  }
-  int rc = upload(&m->d_wts_h, h.data(), piece * 2);
-  if (!rc && split) {
+  const size_t piece = (size_t)2 * n * KP * sizeof(__half);
+  cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&m->d_wts_h), piece);
+  if (e == cudaSuccess && split) e = cudaMalloc(reinterpret_cast<void**>(&m->d_wts_s), 2 * piece);
+  if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc");
+  operand_kernel<<<2 * n, KP>>>(m->d_wts, m->d_bias, T, KP, pz::nnedi3_tc_chunk(n, m->win_h, false),
+                                pz::nnedi3_tc_chunk(n, m->win_h, true), split ? std::ldexp(1.0, exp2) : 0.0, m->d_wts_h,
+                                m->d_wts_s);
+  if ((e = cudaGetLastError()) != cudaSuccess || (e = cudaStreamSynchronize(nullptr)) != cudaSuccess)
+    return cuda_fail(e, "NNEDI3 operands");
+  if (split) {
     m->split_one = (float)std::ldexp(1.0, exp2);
     // e s (1 + |s|) at the square of the scale, over all neurons, with room for
     // the roundings; and one e of at least 2^-89
     const double top2 = most[0] + 2.0 * (exp2 + std::log2(1.0 + most[1])) + std::log2((double)n);
     m->may_mark = !(top2 < 126.0 && most[0] < 89.0);
-    rc = upload(&m->d_wts_s, s.data(), 2 * piece * 2);
   }
-  return rc;
+  return PZ_OK;
 }
 
 }  // namespace
@@ -392,42 +404,48 @@ int pz_model_create(const pz_model_desc* d, pz_model** out) {
   const int nb = need_cols / 9;
   m->lut_h_pitch = zoom ? 9 * ((nb + 1) & ~1) : (d->lut_cols + 1) & ~1;
   m->lut_pitch = d->family == PZ_RAVU ? d->lut_cols | 1 : d->lut_cols;
-  const size_t nval = (size_t)d->lut_rows * m->lut_pitch * 4, bytes = nval * 4;
-  auto laid_out = [&](const float* src, bool half, std::vector<float>* r) {
-    for (int y = 0; y < d->lut_rows; y++)
-      for (int c = 0; c < d->lut_cols; c++) {
-        size_t at;
-        if (zoom) {
-          const uint32_t x = c % 9, t = c / 9;
-          at = d->radius == 2 ? (half ? pz::zoom_texel_at<2, true>(y, x, t) : pz::zoom_texel_at<2, false>(y, x, t))
-                              : (half ? pz::zoom_texel_at<3, true>(y, x, t) : pz::zoom_texel_at<3, false>(y, x, t));
-        } else {
-          at = (size_t)y * (half ? m->lut_h_pitch : m->lut_pitch) + c;
-        }
-        std::memcpy(&(*r)[at * 4], &src[((size_t)y * d->lut_cols + c) * 4], 16);
-      }
+  const size_t rows = d->lut_rows, cols = d->lut_cols, bytes = rows * m->lut_pitch * 16;
+  // FP32 rows as they are stored: the file's own where the pitch is (ravu-zoom's
+  // FP32 order is the file's)
+  std::vector<float> room;
+  auto padded = [&](const float* src) {
+    if ((size_t)m->lut_pitch == cols) return src;
+    room.assign(bytes / 4, 0.0f);
+    for (size_t y = 0; y < rows; y++) std::memcpy(&room[y * m->lut_pitch * 4], src + y * cols * 4, cols * 16);
+    return (const float*)room.data();
   };
-  auto rounded = [](std::vector<float> r) {  // every value rounded to FP16 (round to nearest even)
-    for (float& v : r) v = __half2float(__float2half_rn(v));
-    return r;
+  // every value rounded to FP16 (round to nearest even), as FP32 and as halves
+  std::vector<float> rounded(rows * cols * 4);
+  std::vector<__half> halves(rows * cols * 4);
+  auto round16 = [&](const float* src) {
+    for (size_t i = 0; i < halves.size(); i++) {
+      halves[i] = __float2half_rn(src[i]);
+      rounded[i] = __half2float(halves[i]);
+    }
+    return (const float*)rounded.data();
   };
-  std::vector<float> lut(nval), luthf((size_t)d->lut_rows * m->lut_h_pitch * 4, 0.0f);
-  laid_out(d->lut, false, &lut);
-  laid_out(d->lut, true, &luthf);
-  std::vector<__half> luth(luthf.size());
-  for (size_t i = 0; i < luthf.size(); i++) luth[i] = __float2half_rn(luthf[i]);
-  if ((rc = upload(&m->d_lut, lut.data(), bytes)) || (rc = upload(&m->d_lut16, rounded(lut).data(), bytes)) ||
-      (rc = upload(&m->d_lut_h, luth.data(), luth.size() * 2))) {
+  if ((rc = upload(&m->d_lut, padded(d->lut), bytes)) || (rc = upload(&m->d_lut16, padded(round16(d->lut)), bytes))) {
     pz_model_destroy(m);
     return rc;
   }
-  if (d->lut_ar) {
-    std::vector<float> ar(nval);
-    laid_out(d->lut_ar, false, &ar);
-    if ((rc = upload(&m->d_lut_ar, ar.data(), bytes)) || (rc = upload(&m->d_lut_ar16, rounded(ar).data(), bytes))) {
-      pz_model_destroy(m);
-      return rc;
+  std::vector<__half> luth(rows * m->lut_h_pitch * 4, __float2half_rn(0.0f));
+  for (size_t y = 0; y < rows; y++) {
+    const __half* src = &halves[y * cols * 4];
+    if (!zoom) {
+      std::memcpy(&luth[y * m->lut_h_pitch * 4], src, cols * 8);
+      continue;
     }
+    for (uint32_t t = 0, c = 0; c < cols; t++)
+      for (uint32_t x = 0; x < 9; x++, c++) {
+        const size_t at = d->radius == 2 ? pz::zoom_texel_at<2, true>(y, x, t) : pz::zoom_texel_at<3, true>(y, x, t);
+        std::memcpy(&luth[at * 4], src + c * 4, 8);
+      }
+  }
+  if ((rc = upload(&m->d_lut_h, luth.data(), luth.size() * 2)) ||
+      (d->lut_ar && ((rc = upload(&m->d_lut_ar, padded(d->lut_ar), bytes)) ||
+                     (rc = upload(&m->d_lut_ar16, padded(round16(d->lut_ar)), bytes))))) {
+    pz_model_destroy(m);
+    return rc;
   }
   *out = m;
   return PZ_OK;
