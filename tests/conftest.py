@@ -60,6 +60,7 @@ def _no_silent_device_errors(request):
 
 @pytest.fixture(scope="session")
 def reference_dir():
-    if not os.path.isdir(REFERENCE):
+    # an empty folder is no checkout either (as for build())
+    if not os.path.isdir(REFERENCE) or not any(f.endswith(".hook") for f in os.listdir(REFERENCE)):
         pytest.skip("reference .hook files not present on this machine")
     return REFERENCE
