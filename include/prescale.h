@@ -65,7 +65,8 @@ typedef enum { PZ_F32 = 0, PZ_F16 = 1 } pz_dtype;
 typedef enum {
   PZ_PREC_FP32 = 0,  /* plain FP32 everywhere; NNEDI3's contraction of FP32
                         values on the tensor cores, each value as two FP16
-                        pieces (no further from 64 bits than FP32 FMAs)      */
+                        pieces (measured against 64 bits: 0.5-0.65x the
+                        error of FP32 FMAs, for weights that sum to zero)    */
   PZ_PREC_FAST = 1,  /* FP16 tensor-core NNEDI3 neurons; ravu-lite / 3x /
                         zoom read their LUTs as FP16 texels (half the L1
                         gather traffic; zoom-ar's anti-ringing LUT stays

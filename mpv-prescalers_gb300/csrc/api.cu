@@ -115,7 +115,7 @@ constexpr double kLog2e = 1.4426950408889634;
 //
 // One block per row (the softmax or Elliott branch of a neuron), one thread per
 // element; `up`: the power of two, 0: no pieces.  On the device, where its three
-// conversions a value cost nothing: nns256 8x6 loads in LOADNEW ms, in 0.70 with
+// conversions a value cost nothing: nns256 8x6 loads in 0.19 ms, in 0.70 with
 // them on the host.
 __global__ void operand_kernel(const float* wts, const float* bias, int T, int KP, int nch, int ncs, double up,
                                __half* h, __half* s) {

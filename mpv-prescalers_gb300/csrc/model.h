@@ -99,10 +99,12 @@ inline NnArgs nn_args(const pz_model* m, int* err) {
 // One doubling pass in the form `precision` asks for.  The fast form runs
 // its neurons on the tensor cores in FP16; every other form keeps FP32 values
 // and runs them there as two FP16 pieces each.  1080p to 2160p, FP32 planes,
-// split against CUDA cores: nns128 8x6 455 against 4919 us, nns16 8x4 189
+// split against CUDA cores: nns128 8x6 441 against 4919 us, nns16 8x4 176
 // against 491 us; 160x90 nns32 8x4 the same (both are the two launches).  The
 // error against 64 bits is 0.5-0.65x the CUDA cores' for every nns and window
-// (nns128 8x6 at 640x360: 8.6e-8 against 1.46e-7 relative).  Models of other
+// with weights that sum to zero, as the files' do (nns128 8x6 at 640x360: 8.5e-8
+// against 1.46e-7 relative); with Elliott weights 130 times as large it is 0.75-1.1x
+// (largest error 1.8e-6 against 4.3e-7, nns32 8x4), with logits of 60 0.9-1.5x.  Models of other
 // shapes, or with weights that the pieces cannot hold, stay on the CUDA cores;
 // and so do single pixels of models whose pre-activations may leave the split
 // blend's range (may_mark), by a second launch that looks for them.

@@ -29,17 +29,22 @@
 // first MMAs run under that blend.
 //
 // SPLIT (the plain FP32 form): every operand value is two FP16 pieces, hi +
-// lo, which together hold 22-24 bits, and a chunk is three products, A_lo B_hi
-// + A_hi B_lo + A_hi B_hi in FP32, the small ones first.  A power of two (the
-// model's) scales B so that its pieces stay clear of FP16's subnormals.
+// lo, and a chunk is three products, A_lo B_hi + A_hi B_lo + A_hi B_hi in FP32, the
+// small ones first.  The pieces hold 22 bits of a value at least, but a low piece
+// ends at FP16's 2^-24: x_hat, whose root mean square is 1, keeps an absolute error
+// of 2^-25 below 2^-3 (scaled by 16, which removes that, the error against 64 bits
+// is the same); in B, which a power of two of the model's scales, that is 2^-39 of
+// the largest value.  A_lo B_lo, at most 2^-22 of a product, is left out.  The
+// sums, rounded once a K step instead of once a term, more than make up for it:
+// the error against 64 bits is 0.5-0.65x the CUDA cores' (launch_nnedi3).
 //
 // Bound by issue and latency in the blend (12 packed or scalar instructions
 // and 6 MUFU for four neurons) at four warps a scheduler (60 % issue, 37 % MUFU,
 // 23 % tensor pipe; 96 registers and 512 TMEM columns allow no fifth group).
-// 1080p to 2160p, nns128 8x6: 330 us fast (384 us with scalar sums over neuron
+// 1080p to 2160p, nns128 8x6: 325 us fast (384 us with scalar sums over neuron
 // pairs and rolled chunks; 438 us as four CTAs an SM, each with its own copy of B
-// and a CTA barrier per chunk), 455 us split (523 us; 4919 us on the CUDA cores);
-// nns256 8x6 at 720p 243 us fast (443 us: two CTAs an SM had room).
+// and a CTA barrier per chunk), 441 us split (523 us; 4919 us on the CUDA cores);
+// nns256 8x6 at 720p 240 us fast (443 us: two CTAs an SM had room).
 //
 // Every mbarrier wait is bounded (kWaitNs of %globaltimer).  A wait that runs
 // out sets the CTA's abort flag: from then on nobody waits, nothing is stored,
@@ -126,10 +131,10 @@ __device__ __forceinline__ void mbar_arrive(uint32_t mbar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(mbar) : "memory");
 }
 
-// Barrier among the 128 threads of group g (named barriers 1..4; 0 is the CTA's).
 __device__ __forceinline__ float to_float(float v) { return v; }
 __device__ __forceinline__ float to_float(__half v) { return __half2float(v); }
 
+// Barrier among the 128 threads of group g (named barriers 1..4; 0 is the CTA's).
 __device__ __forceinline__ void group_sync(int g) {
   asm volatile("bar.sync %0, %1;" ::"r"(g + 1), "n"(kGroup) : "memory");
 }
@@ -138,10 +143,10 @@ __device__ __forceinline__ void group_sync(int g) {
 // shared memory once per instruction whatever its N: 64 neurons (N = 128) take
 // two thirds of the shared-memory time of 32 (N = 64), and then one accumulator
 // per group (its MMAs wait for the blend's last read) is all that fits four
-// groups.  FP32, chunks of 32 / 64: nns128 8x6 at 1080p 491 / 455 us, nns128 8x4 at
-// 720p 186 / 179, nns256 8x4 at 1080p 674 / 607, nns64 8x6 316 / 300; but nns64
-// 8x4, with little to multiply, 256 / 267, and nns256 8x6, two groups, at 720p 468 /
-// 487.  The fast form, bound by the blend, keeps 32 and two accumulators.
+// groups.  FP32, chunks of 32 / 64: nns128 8x6 at 1080p 486 / 444 us, nns128 8x4 at
+// 720p 183 / 177, nns256 8x4 at 1080p 670 / 603, nns64 8x6 321 / 298; but nns64
+// 8x4, with little to multiply, 255 / 266, and nns256 8x6, two groups, at 720p 464 /
+// 483.  The fast form, bound by the blend, keeps 32 and two accumulators.
 constexpr int tc_chunk(int nns, int wh, bool split) {
   const bool wide = split && (nns == 128 || (nns == 256 && wh == 4) || (nns == 64 && wh == 6));
   return nns < 32 ? nns : (wide ? 64 : 32);

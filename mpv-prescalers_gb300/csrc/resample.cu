@@ -102,8 +102,9 @@ __global__ void __launch_bounds__(256) resample_kernel(const __grid_constant__ R
 // 8 % of the copy bandwidth).  OFF: column of the first tap within its quad,
 // (floor(ox) + first tap) mod 4, the same for every thread.  A block whose
 // positions do not step by whole texels (the rounding of x + ox far from 0) goes
-// texel by texel.  Catmull-Rom, 3840x2160 FP16: 20.5 us (61.6 us), 2560x1440 10.4
-// (28.9); bilinear 10.7 (26.7).
+// texel by texel.  3840x2160 FP16, planes in L2 / from memory: Catmull-Rom 20.6 / 28.9
+// us (one texel a thread 61.6 / 61.7), bilinear 12.2 / 18.3 (26.8 / 30.9); 2560x1440
+// Catmull-Rom 10.6 (28.9).
 template <int TAPS, int OFF, typename T>
 __global__ void __launch_bounds__(256) shift_kernel(const __grid_constant__ ResampleArgs a) {
   constexpr int K0 = TAPS == 2 ? 0 : -1, QUADS = (OFF + TAPS + 3 + 3) / 4;
